@@ -793,7 +793,8 @@ def run_ours(args):
     # per step: assemble, the factorization (one persistent launch), then two solves (permute in,
     # forward, backward, permute out), the first one after the factorization also computing the
     # diagonal super-block inverses
-    launches_per_step = 1 + info.factor_launches + 4 + 4 + (1 if info.inverse_bytes else 0)
+    # assembly, factorization, two solves (permutations, tiny leaves and sweeps), block inverses
+    launches_per_step = 1 + info.factor_launches + 6 + 6 + (3 if info.inverse_bytes else 0)
     if rank == 0:
         line = {
             "metric": METRIC, "value": replicas.job_rate(flops * K, world, fac_ms) / 1e12, "unit": "TFLOP/s",

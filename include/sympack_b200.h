@@ -127,7 +127,7 @@ typedef struct spb_info {
   double backward_error;   /* componentwise-free backward error of the last solve, if computed */
   int32_t dense_root_width; /* always 0 (a former cluster solve of the root; kept for layout) */
   int32_t pad_;
-  int64_t inverse_bytes;    /* device bytes of the diagonal super-block inverses of one operand */
+  int64_t inverse_bytes;    /* device bytes of the diagonal block and super-block inverses of one operand */
   double factor_sched_us;   /* makespan the persistent factorization's ordering simulation predicts */
   int32_t factor_tasks;     /* tasks of the persistent factorization */
   int32_t pad2_;

@@ -75,15 +75,20 @@ struct spb_handle {
   bool trace_fresh = false;        // the last factorization was traced in the current task order
   int32_t* dinvp0 = nullptr;
   int32_t* dlevel_sn = nullptr;
-  spb::SolveTask* dfwd = nullptr;
-  spb::SolveTask* dbwd = nullptr;
+  spb::SolveRec* dfwd = nullptr;   // records of the solve tasks
+  spb::SolveRec* dbwd = nullptr;
+  spb::SolveRec* dfsubs = nullptr;
+  spb::SolveRec* dbsubs = nullptr;
   int32_t* dexpected = nullptr;
   int32_t* dtiny = nullptr;        // leaf supernodes of the forward sweep's T tasks
   int32_t* dsparent = nullptr;
   int32_t* dsync = nullptr;  // solve counters (spb::solve_sync_ints)
   void* dInv = nullptr;      // diagonal super-block inverses of the forward operand (L, or L D for LDL^T)
   void* dInvB = nullptr;     // LDL^T: inverses of the backward operand (unit L); else dInv
+  double* dInv1 = nullptr;   // inverses of the one-block supernodes' diagonal blocks (forward operand)
+  double* dInv1B = nullptr;  // LDL^T: those of the backward operand; else dInv1
   spb::InvItem* dinvitems = nullptr;
+  spb::Inv1Item* dinv1items = nullptr;
   bool inv_stale = true;     // inverses not yet computed for the current factor
   Status* dstatus = nullptr;
   // precision form: original matrix as full CSR (FP64) and refinement buffers
@@ -174,6 +179,7 @@ void release_device(spb_handle* h) {
   h->dW = nullptr;
   h->dX = h->dZ = h->dB = h->dR = h->dD = h->dXo = nullptr;
   h->dInv = h->dInvB = nullptr;
+  h->dInv1 = h->dInv1B = nullptr;
   h->dsplit = nullptr;
   h->dsplit_off = nullptr;
   h->dtmaps = nullptr;
@@ -416,7 +422,7 @@ int ensure_rhs_capacity(spb_handle* h, int nrhs) {
   return SPB_OK;
 }
 
-// Diagonal super-block inverses of the current factor, computed by the first solve
+// Diagonal block and super-block inverses of the current factor, computed by the first solve
 // after a factorization.
 void ensure_inverses(spb_handle* h) {
   if (!h->inv_stale) return;
@@ -424,23 +430,32 @@ void ensure_inverses(spb_handle* h) {
   const int count = (int)P.inv_items.size();
   spb::dev::launch_sb_inverse(h->stream, h->ldl ? (const void*)h->dW : h->dL, h->dInv, h->fp32, h->dmeta,
                               h->dinvitems, count, P.solve_sb);
-  if (h->ldl) spb::dev::launch_sb_inverse(h->stream, h->dL, h->dInvB, false, h->dmeta, h->dinvitems, count, P.solve_sb);
+  const int count1 = (int)P.inv1_items.size();
+  spb::dev::launch_diag_inverse(h->stream, h->ldl ? (const void*)h->dW : h->dL, h->dInv1, h->fp32, h->dinv1items,
+                                P.inv1_narrow, count1);
+  if (h->ldl) {
+    spb::dev::launch_sb_inverse(h->stream, h->dL, h->dInvB, false, h->dmeta, h->dinvitems, count, P.solve_sb);
+    spb::dev::launch_diag_inverse(h->stream, h->dL, h->dInv1B, false, h->dinv1items, P.inv1_narrow, count1);
+  }
   h->inv_stale = false;
 }
 
 // Forward and backward persistent sweeps on the permuted right-hand sides X (n x nrhs,
 // ld n; the solution replaces them), with Z (same shape) between the sweeps and the
-// counters in sync; 64 right-hand sides per pass.  prof: record the per-pass events.
-void enqueue_sweeps(spb_handle* h, double* X, double* Z, int32_t* sync, int nrhs, bool prof) {
+// counters of `groups` groups of kSolveGroup right-hand sides in sync; that many groups per
+// pass.  prof: record the per-pass events.
+void enqueue_sweeps(spb_handle* h, double* X, double* Z, int32_t* sync, int groups, int nrhs, bool prof) {
   const spb::Plan& P = h->plan;
-  const int ns = P.nsuper;
-  for (int c0 = 0; c0 < nrhs; c0 += 64) {
+  const size_t ints = spb::solve_sync_ints(P);
+  const int step = spb::kSolveGroup * groups;
+  for (int c0 = 0, pass = 0; c0 < nrhs; c0 += step, ++pass) {
     // counters must start at zero
-    cudaMemsetAsync(sync, 0, sizeof(int32_t) * spb::solve_sync_ints(P), h->stream);
+    cudaMemsetAsync(sync, 0, sizeof(int32_t) * ints * groups, h->stream);
     spb::dev::PSolveArgs a{};
     // LDL^T: the forward sweep solves with L D (diagonal D), the backward one with unit L
     a.L = h->ldl ? (void*)h->dW : h->dL;
     a.Inv = h->dInv;
+    a.Inv1 = h->dInv1;
     a.fp32 = h->fp32;
     a.meta = h->dmeta;
     a.rows = h->drows;
@@ -451,20 +466,19 @@ void enqueue_sweeps(spb_handle* h, double* X, double* Z, int32_t* sync, int nrhs
     a.X = X + (int64_t)c0 * h->sym.n;
     a.Z = Z + (int64_t)c0 * h->sym.n;
     a.ldx = h->sym.n;
-    a.nrhs = std::min(64, nrhs - c0);
+    a.nrhs = std::min(step, nrhs - c0);
     a.expected = h->dexpected;
     a.tiny = h->dtiny;
-    a.arrived = sync + 2;
+    a.ntiny = (int)P.tiny.size();
+    a.sync = sync;
+    a.sync_stride = (int64_t)ints;
     a.status = h->dstatus;
     a.spin_limit = h->wait_limit;
-    a.sb = P.solve_sb;
-    a.tpt = P.solve_tpt;
-    const size_t e0 = 4 * (size_t)(c0 / 64);
-    a.tasks = h->dfwd;
-    a.ntasks = (int)P.fwd_tasks.size();
+    const size_t e0 = 4 * (size_t)pass;
+    a.recs = h->dfwd;
+    a.subs = h->dfsubs;
+    a.ntasks = (int)P.fwd_recs.size();
     a.counter = sync;
-    a.blkdone = sync + 2 + ns;
-    a.upd = sync + 2 + 3 * (size_t)ns;
     a.trace = prof ? h->dtrace : nullptr;
     const size_t pass_bytes = sizeof(double) * (size_t)h->sym.n * a.nrhs;
     if (prof) cudaEventRecord(h->events[e0], h->stream);
@@ -473,12 +487,13 @@ void enqueue_sweeps(spb_handle* h, double* X, double* Z, int32_t* sync, int nrhs
     if (prof) cudaEventRecord(h->events[e0 + 1], h->stream);
     a.L = h->dL;
     a.Inv = h->ldl ? h->dInvB : h->dInv;
-    a.tasks = h->dbwd;
-    a.ntasks = (int)P.bwd_tasks.size();
+    a.Inv1 = h->ldl ? h->dInv1B : h->dInv1;
+    a.recs = h->dbwd;
+    a.subs = h->dbsubs;
+    a.ntasks = (int)P.bwd_recs.size();
     a.counter = sync + 1;
-    a.blkdone = sync + 2 + 2 * ns;
-    a.upd = sync + 2 + 3 * (size_t)ns + P.nsb_total;
     a.trace = prof && h->dtrace ? h->dtrace + 4 * P.fwd_tasks.size() : nullptr;
+    a.tiny_task0 = (int64_t)(P.bwd_tasks.size() - (P.tiny.size() + spb::kTinyBatch - 1) / spb::kTinyBatch);
     if (prof) cudaEventRecord(h->events[e0 + 2], h->stream);
     cudaMemsetAsync(a.X, 0, pass_bytes, h->stream);  // the backward DI tasks add into X
     spb::dev::launch_solve_persistent(h->stream, a, false);
@@ -496,7 +511,7 @@ void enqueue_solve(spb_handle* h, int nrhs) {
   ensure_inverses(h);
   if (prof) cudaEventRecord(h->events[ie + 1], h->stream);
   h->prof_inverse = prof && inv;
-  enqueue_sweeps(h, h->dX, h->dZ, h->dsync, nrhs, prof);
+  enqueue_sweeps(h, h->dX, h->dZ, h->dsync, spb::kSolveGroups, nrhs, prof);
 }
 
 // Per-sweep device times of the last profiled solve.
@@ -868,13 +883,15 @@ int64_t predict_bytes(const spb_handle* h, bool fp32, int nrhs) {
   t += b(P.panel_items.size(), sizeof(spb::PanelItem));
   t += b((int64_t)std::max(1, P.max_diag_slots) * (int64_t)spb::dev::kDiagSlotDoubles, 8);
   t += b(P.tile_items.size(), sizeof(spb::TileItem)) + b(n, 4) + b(ns, 4);
-  t += b(P.fwd_tasks.size(), sizeof(spb::SolveTask)) + b(P.bwd_tasks.size(), sizeof(spb::SolveTask));
-  t += b(P.fwd_pending.size(), 4) + b(P.tiny.size(), 4) + b(P.sparent.size(), 4) +
-       b((int64_t)spb::solve_sync_ints(P), 4);
+  t += b(P.fwd_recs.size(), sizeof(spb::SolveRec)) + b(P.bwd_recs.size(), sizeof(spb::SolveRec));
+  t += b(P.fwd_subs.size(), sizeof(spb::SolveRec)) + b(P.bwd_subs.size(), sizeof(spb::SolveRec));
+  t += b(P.fwd_wait.size(), 4) + b(P.tiny.size(), 4) + b(P.sparent.size(), 4) +
+       b((int64_t)spb::solve_sync_ints(P) * spb::kSolveGroups, 4);
   t += b(P.inv_elems, fp32 ? sizeof(float) : sizeof(double)) + b(P.inv_items.size(), sizeof(spb::InvItem));
+  t += b(P.inv1_elems, sizeof(double)) + b(P.inv1_items.size(), sizeof(spb::Inv1Item));
   t += b(P.ftasks.size(), sizeof(spb::FTask)) + b(P.fwaits.size(), sizeof(spb::FWait)) + b(P.fsigs.size(), 4) +
        b(P.nfctr + 1, 4);
-  if (o.decomposition == SPB_DECOMPOSITION_LDL) t += b(P.inv_elems, sizeof(double));
+  if (o.decomposition == SPB_DECOMPOSITION_LDL) t += b(P.inv_elems, sizeof(double)) + b(P.inv1_elems, sizeof(double));
   t += b(1, sizeof(Status));
   if (fp32) {
     int64_t offdiag = 0;
@@ -956,18 +973,22 @@ int install_device(spb_handle* h) {
   SPB_CK(h, dalloc(h, &h->dtiles, P.tile_items.size()));
   SPB_CK(h, dalloc(h, &h->dinvp0, invp0.size()));
   SPB_CK(h, dalloc(h, &h->dlevel_sn, lsn.size()));
-  SPB_CK(h, dalloc(h, &h->dfwd, P.fwd_tasks.size()));
-  SPB_CK(h, dalloc(h, &h->dbwd, P.bwd_tasks.size()));
-  SPB_CK(h, dalloc(h, &h->dexpected, P.fwd_pending.size()));
+  SPB_CK(h, dalloc(h, &h->dfwd, P.fwd_recs.size()));
+  SPB_CK(h, dalloc(h, &h->dbwd, P.bwd_recs.size()));
+  SPB_CK(h, dalloc(h, &h->dfsubs, P.fwd_subs.size()));
+  SPB_CK(h, dalloc(h, &h->dbsubs, P.bwd_subs.size()));
+  SPB_CK(h, dalloc(h, &h->dexpected, P.fwd_wait.size()));
   SPB_CK(h, dalloc(h, &h->dtiny, P.tiny.size()));
   SPB_CK(h, dalloc(h, &h->dsparent, P.sparent.size()));
-  SPB_CK(h, dalloc(h, &h->dsync, spb::solve_sync_ints(P)));
+  SPB_CK(h, dalloc(h, &h->dsync, spb::solve_sync_ints(P) * spb::kSolveGroups));
   {
     unsigned char* inv = nullptr;
     SPB_CK(h, dalloc(h, &inv, (size_t)P.inv_elems * h->elem));
     h->dInv = inv;
   }
   SPB_CK(h, dalloc(h, &h->dinvitems, P.inv_items.size()));
+  SPB_CK(h, dalloc(h, &h->dInv1, (size_t)P.inv1_elems));
+  SPB_CK(h, dalloc(h, &h->dinv1items, P.inv1_items.size()));
   SPB_CK(h, dalloc(h, &h->dftasks, P.ftasks.size()));
   SPB_CK(h, dalloc(h, &h->dfwaits, P.fwaits.size()));
   SPB_CK(h, dalloc(h, &h->dfsigs, P.fsigs.size()));
@@ -976,8 +997,10 @@ int install_device(spb_handle* h) {
     double* invb = nullptr;
     SPB_CK(h, dalloc(h, &invb, (size_t)P.inv_elems));
     h->dInvB = invb;
+    SPB_CK(h, dalloc(h, &h->dInv1B, (size_t)P.inv1_elems));
   } else {
     h->dInvB = h->dInv;
+    h->dInv1B = h->dInv1;
   }
   h->inv_stale = true;
   SPB_CK(h, dalloc(h, &h->dstatus, 1));
@@ -997,12 +1020,15 @@ int install_device(spb_handle* h) {
   SPB_CK(h, up(h->dtiles, P.tile_items.data(), P.tile_items.size() * sizeof(spb::TileItem)));
   SPB_CK(h, up(h->dinvp0, invp0.data(), invp0.size() * 4));
   SPB_CK(h, up(h->dlevel_sn, lsn.data(), lsn.size() * 4));
-  SPB_CK(h, up(h->dfwd, P.fwd_tasks.data(), P.fwd_tasks.size() * sizeof(spb::SolveTask)));
-  SPB_CK(h, up(h->dbwd, P.bwd_tasks.data(), P.bwd_tasks.size() * sizeof(spb::SolveTask)));
-  SPB_CK(h, up(h->dexpected, P.fwd_pending.data(), P.fwd_pending.size() * 4));
+  SPB_CK(h, up(h->dfwd, P.fwd_recs.data(), P.fwd_recs.size() * sizeof(spb::SolveRec)));
+  SPB_CK(h, up(h->dbwd, P.bwd_recs.data(), P.bwd_recs.size() * sizeof(spb::SolveRec)));
+  SPB_CK(h, up(h->dfsubs, P.fwd_subs.data(), P.fwd_subs.size() * sizeof(spb::SolveRec)));
+  SPB_CK(h, up(h->dbsubs, P.bwd_subs.data(), P.bwd_subs.size() * sizeof(spb::SolveRec)));
+  SPB_CK(h, up(h->dexpected, P.fwd_wait.data(), P.fwd_wait.size() * 4));
   SPB_CK(h, up(h->dtiny, P.tiny.data(), P.tiny.size() * 4));
   SPB_CK(h, up(h->dsparent, P.sparent.data(), P.sparent.size() * 4));
   SPB_CK(h, up(h->dinvitems, P.inv_items.data(), P.inv_items.size() * sizeof(spb::InvItem)));
+  SPB_CK(h, up(h->dinv1items, P.inv1_items.data(), P.inv1_items.size() * sizeof(spb::Inv1Item)));
   SPB_CK(h, up(h->dftasks, P.ftasks.data(), P.ftasks.size() * sizeof(spb::FTask)));
   SPB_CK(h, up(h->dfwaits, P.fwaits.data(), P.fwaits.size() * sizeof(spb::FWait)));
   SPB_CK(h, up(h->dfsigs, P.fsigs.data(), P.fsigs.size() * 4));
@@ -1406,7 +1432,8 @@ int spb_get_info(spb_handle* h, spb_info* info) {
   info->dense_root_width = 0;  // the cluster root solve gave way to the super-block solve
   info->factor_sched_us = P.fsim_us;
   info->factor_tasks = (int32_t)P.ftasks.size();
-  info->inverse_bytes = P.inv_elems * (int64_t)(h->opt.precision == SPB_PRECISION_FP32_IR ? 4 : 8);
+  info->inverse_bytes =
+      P.inv_elems * (int64_t)(h->opt.precision == SPB_PRECISION_FP32_IR ? 4 : 8) + P.inv1_elems * (int64_t)sizeof(double);
   info->ir_iterations = h->ir_iterations;
   info->backward_error = h->backward_error;
   return SPB_OK;
@@ -1521,7 +1548,7 @@ int spb_debug_stall(spb_handle* h, int32_t supernode) {
   if (!h->have_symbolic || h->device < 0) return fail(h, SPB_ERR_STATE, "debug_stall: needs a device handle");
   const int ns = h->plan.nsuper;
   if (supernode >= ns) return fail(h, SPB_ERR_INVALID, "debug_stall: supernode out of range");
-  std::vector<int32_t> e = h->plan.fwd_pending;
+  std::vector<int32_t> e = h->plan.fwd_wait;
   if (supernode >= 0) e[supernode] += 1;
   SPB_CK(h, cudaMemcpyAsync(h->dexpected, e.data(), e.size() * 4, cudaMemcpyHostToDevice, h->stream));
   SPB_CK(h, cudaStreamSynchronize(h->stream));
@@ -1735,7 +1762,9 @@ extern "C" int spb_solve_device_noalloc(spb_handle* h, const double* d_rhs, doub
   int32_t* sync = reinterpret_cast<int32_t*>(base + 2 * kNoAllocXBytes);
   spb::dev::launch_permute_in(h->stream, X, n, d_rhs, ld, h->dinvp0, n, nrhs);
   ensure_inverses(h);  // the first solve after a factorization computes them (arena of the analysis)
-  enqueue_sweeps(h, X, Z, sync, nrhs, false);
+  const size_t ints = spb::solve_sync_ints(h->plan) * sizeof(int32_t);  // as many groups as the counters have room for
+  const int groups = (int)std::min<size_t>(spb::kSolveGroups, kNoAllocSyncBytes / ints);
+  enqueue_sweeps(h, X, Z, sync, groups, nrhs, false);
   spb::dev::launch_permute_out(h->stream, d_x, ld, X, n, h->dinvp0, n, nrhs);
   SPB_CK(h, cudaGetLastError());
   return check_solve_status(h);

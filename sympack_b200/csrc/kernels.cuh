@@ -81,13 +81,14 @@ void launch_factor_persistent(cudaStream_t st, const FactorArgs& a, const Factor
 
 // Solves work on the permuted right-hand sides X (n x nrhs, column-major, leading dimension ldx).
 
-// Persistent sweeps (one launch each).  counter, arrived, blkdone and upd must
-// be zero at launch; expected[s] is the number of forward arrivals (off-diagonal
-// task, target) that write rows of supernode s.  Forward: Y = X (accumulated),
-// solution to Z; backward: Z (accumulated), solution to X.
+// Sweeps: one persistent launch each, beside one launch for the tiny leaves.  The
+// counters must be zero at launch; expected[s] is the number of forward arrivals
+// (off-diagonal task, target) that write rows of supernode s, the tiny leaves' aside.
+// Forward: Y = X (accumulated), solution to Z; backward: Z (accumulated), solution to X.
 struct PSolveArgs {
   const void* L;     // factor arena (double, or float when fp32): L, or L D for the LDL^T forward sweep
   const void* Inv;   // diagonal super-block inverses of that operand (same type)
+  const double* Inv1;  // inverses of its one-block supernodes' diagonal blocks
   bool fp32;
   const SnMeta* meta;
   const int32_t* rows;
@@ -98,17 +99,17 @@ struct PSolveArgs {
   double* X;
   double* Z;
   int64_t ldx;       // leading dimension of X and Z
-  int nrhs;  // <= 64
-  const SolveTask* tasks;
+  int nrhs;  // <= kSolveGroup * kSolveGroups
+  const SolveRec* recs;
+  const SolveRec* subs;
   int ntasks;
-  const int32_t* tiny;  // leaf supernodes of the forward T tasks (Plan::tiny)
+  const int32_t* tiny;  // tiny leaf supernodes (Plan::tiny)
+  int ntiny;
+  int64_t tiny_task0;   // place of their first batch in the task list (trace)
   int32_t* counter;
   const int32_t* expected;
-  int32_t* arrived;
-  int32_t* blkdone;  // per supernode: finished diagonal tasks of this sweep
-  int32_t* upd;      // per super-block (meta.sboff + p): updates landed
-  int sb;            // 64-column blocks per super-block (Plan::solve_sb)
-  int tpt;           // tiles per DI / U / V / O / W task (Plan::solve_tpt)
+  int32_t* sync;     // counters of the first group of right-hand sides (SolveRec's counter numbers index it)
+  int64_t sync_stride;  // from one group's counters to the next one's
   Status* status;
   long long spin_limit;  // polls (about 128 ns apart) before a wait gives up
   unsigned long long* trace;  // optional, 4 per task: grabbed, dependencies met, done (ns), s << 8 | kind
@@ -119,6 +120,10 @@ void launch_solve_persistent(cudaStream_t st, const PSolveArgs& a, bool forward)
 // written to Inv in 64 x 64 tiles at meta.ioff.
 void launch_sb_inverse(cudaStream_t st, const void* L, void* Inv, bool fp32, const SnMeta* meta,
                        const InvItem* items, int count, int sb);
+// Inverses of the diagonal blocks of L's one-block supernodes (Plan::inv1_items, the first
+// `narrow` of them of at most kInv1Narrow columns), in FP64.
+void launch_diag_inverse(cudaStream_t st, const void* L, double* Inv, bool fp32, const Inv1Item* items, int narrow,
+                         int count);
 
 // Precision form (FP64 refinement): gather CSR values, residual r = b - A x,
 // per-column max |v| (out zeroed by the caller), max row sum of |A|, x += d.

@@ -2,6 +2,8 @@
 
 #include <algorithm>
 #include <atomic>
+#include <climits>
+#include <cstdint>
 #include <queue>
 #include <stdexcept>
 #include <system_error>
@@ -13,6 +15,7 @@ namespace spb {
 static int64_t round_up(int64_t x, int64_t m) { return (x + m - 1) / m * m; }
 
 static void build_factor_dag(Plan& P, const PlanParams& prm, const std::vector<double>* measured_us = nullptr);
+static void build_solve_recs(Plan& P);
 
 Plan build_plan(const Symbolic& sym, const PlanParams& prm) {
   Plan P;
@@ -428,7 +431,184 @@ Plan build_plan(const Symbolic& sym, const PlanParams& prm) {
   for (size_t i = 0; i < P.tiny.size(); i += kTinyBatch)  // the tiny leaves last
     P.bwd_tasks.push_back(SolveTask{P.tiny[i], 6, (int32_t)i,
                                     (int32_t)std::min<size_t>(kTinyBatch, P.tiny.size() - i)});
+  build_solve_recs(P);
   return P;
+}
+
+// Device records of the solve tasks, and the places of the one-block supernodes' inverses.
+static void build_solve_recs(Plan& P) {
+  const int ns = P.nsuper, SB = P.solve_sb, TPT = P.solve_tpt;
+  if (std::max(P.fwd_tasks.size(), P.bwd_tasks.size()) >= ((size_t)1 << 28))
+    throw std::runtime_error("plan: more than 2^28 solve tasks");
+  if (P.rows.size() > (size_t)INT32_MAX) throw std::runtime_error("plan: row lists beyond 2^31 entries");
+  std::vector<uint8_t> tiny(ns, 0);
+  for (int32_t s : P.tiny) tiny[s] = 1;
+  std::vector<int64_t> inv(ns, -1);
+  for (int pass = 0; pass < 2; ++pass) {
+    for (int s = 0; s < ns; ++s) {
+      const SnMeta& m = P.meta[s];
+      if (m.w > 64 || tiny[s] || (m.w <= kInv1Narrow) != (pass == 0)) continue;
+      inv[s] = P.inv1_elems;
+      P.inv1_items.push_back(Inv1Item{m.off, P.inv1_elems, m.ld, m.w});
+      P.inv1_elems += (int64_t)m.w * m.w;
+    }
+    if (pass == 0) P.inv1_narrow = (int32_t)P.inv1_items.size();
+  }
+  // counters, as the sweeps lay them out (solve_sync_ints)
+  const int arrived = 2, done_f = 2 + ns, done_b = 2 + 2 * ns, upd_f = 2 + 3 * ns, upd_b = upd_f + P.nsb_total;
+  const int full_di = solve_di_tasks(SB, TPT);
+  auto make = [&](const SolveTask& t, bool fwd) {
+    SolveRec r{};
+    const int s = t.s, kind = t.kind;
+    const SnMeta& m = P.meta[s];
+    const int nblk = (m.w + 63) / 64, nsb = (nblk + SB - 1) / SB, nlast = nblk - (nsb - 1) * SB;
+    const int noff = (m.h - m.w + 63) / 64;
+    const int p = t.i & 0xffffff, q0 = t.i >> 24, b0 = p * SB, nb = std::min(SB, nblk - b0);
+    r.kind = kind;
+    r.s = s;
+    r.ld = m.ld;
+    r.inv = inv[s];
+    r.wait = r.sig = -1;
+    // DI tasks of super-blocks p0 .. p1 - 1
+    auto di_range = [&](int p0, int p1) {
+      return (p1 - p0) * full_di + (p1 == nsb ? solve_di_tasks(nlast, TPT) - full_di : 0);
+    };
+    const int col0 = (b0 + q0) * 64;  // first column (forward) or row (V) of the task's tiles
+    const int cols = std::min(m.w - col0, 64 * std::min(TPT, nb - q0));
+    if (kind == 4 || kind == 0) {  // F / D, G / B
+      r.a = m.off;
+      r.m = m.w;
+      r.k = kind == 4 ? m.h - m.w : 0;
+      r.x0 = m.fc;
+      r.y0 = (int32_t)(m.lidx + m.w);
+      if (fwd) {
+        r.wait = arrived + s;  // the target is read from the expected counts
+        if (kind == 0) r.sig = done_f + s;
+        if (r.k > 0) {
+          r.g0 = P.row_group[m.lidx + m.w];
+          r.ng = P.row_group[m.lidx + m.h - 1] - r.g0 + 1;
+        }
+      } else {
+        r.sig = done_b + s;
+        if (kind == 4) {
+          const int par = P.sparent[s];
+          if (par >= 0) r.wait = done_b + par, r.target = solve_done_count(P.meta[par].w, SB, TPT);
+        } else {
+          r.wait = upd_b + m.sboff;
+          r.target = noff;
+        }
+      }
+    } else if (kind == 5) {
+      const int rb = t.t, blk = b0 + rb;  // row block of the super-block
+      const int64_t base = m.ioff + (int64_t)p * inv_tiles(SB) * 4096;
+      r.ld = 64;
+      r.m = std::min(64, m.w - blk * 64);
+      r.y0 = m.fc + blk * 64;
+      r.sig = (fwd ? done_f : done_b) + s;
+      if (fwd) {
+        r.a = base + ((int64_t)rb * (rb + 1) / 2 + q0) * 4096;
+        const int q1 = std::min(rb + 1, q0 + TPT);
+        r.k = std::min(m.w, (b0 + q1) * 64) - col0;
+        r.x0 = m.fc + col0;
+        r.wait = upd_f + m.sboff + p;
+        r.target = p * nb * solve_ntask(SB, TPT);
+      } else {  // tiles (rb + j, rb), j = q0 ..
+        r.a = base;
+        const int j1 = std::min(nb - rb, q0 + TPT);
+        r.g0 = rb + q0;
+        r.ng = rb;
+        r.x0 = m.fc + (blk + q0) * 64;
+        r.k = std::min(m.w, (blk + j1) * 64) - (blk + q0) * 64;
+        r.wait = upd_b + m.sboff + p;
+        const int later = p < nsb - 1 ? (nsb - 2 - p) * solve_ntask(SB, TPT) + solve_ntask(nlast, TPT) : 0;
+        r.target = noff * solve_ntask(nb, TPT) + nb * later;
+      }
+    } else if (kind == 1) {  // U, V: the diagonal part's other blocks
+      r.m = std::min(64, m.w - t.t * 64);
+      r.k = cols;
+      r.x0 = m.fc + col0;
+      r.y0 = m.fc + t.t * 64;
+      r.a = fwd ? m.off + (int64_t)t.t * 64 + (int64_t)col0 * m.ld : m.off + col0 + (int64_t)t.t * 64 * m.ld;
+      r.wait = (fwd ? done_f : done_b) + s;
+      r.target = fwd ? di_range(0, p + 1) : di_range(p, nsb);
+      r.sig = (fwd ? upd_f : upd_b) + m.sboff + t.t / SB;
+    } else {  // O (2), W (3): an off-diagonal tile
+      const int r0 = m.w + t.t * 64, br = std::min(64, m.h - r0);
+      r.a = m.off + r0 + (int64_t)col0 * m.ld;
+      if (fwd) {
+        r.m = br;
+        r.k = cols;
+        r.x0 = m.fc + col0;
+        r.y0 = (int32_t)(m.lidx + r0);
+        r.wait = done_f + s;
+        r.target = nblk == 1 ? 1 : di_range(0, p + 1);
+        r.g0 = P.row_group[m.lidx + r0];
+        r.ng = P.row_group[m.lidx + r0 + br - 1] - r.g0 + 1;
+      } else {
+        r.m = cols;
+        r.k = br;
+        r.x0 = (int32_t)(m.lidx + r0);
+        r.y0 = m.fc + col0;
+        const int par = P.sparent[s];
+        if (par >= 0) r.wait = done_b + par, r.target = solve_done_count(P.meta[par].w, SB, TPT);
+        r.sig = upd_b + m.sboff + p;
+      }
+    }
+    return r;
+  };
+  // small F / G tasks of a level go to batches, enough of them to keep every CTA slot busy
+  // before a batch holds more than one
+  const int slots = 2 * 148;
+  std::vector<int32_t> nsmall(P.nlevels, 0);
+  auto small = [&](const SolveTask& t) {
+    const SnMeta& m = P.meta[t.s];
+    return t.kind == 4 && m.w <= kWarpMaxW && m.h - m.w <= kWarpMaxOff;
+  };
+  for (const SolveTask& t : P.fwd_tasks)
+    if (small(t)) ++nsmall[P.level[t.s]];
+  auto fill = [&](const std::vector<SolveTask>& tasks, bool fwd, std::vector<SolveRec>& recs,
+                  std::vector<SolveRec>& subs) {
+    int level = -1;
+    SolveRec batch{};
+    auto flush = [&]() {
+      if (batch.m > 0) recs.push_back(batch);
+      batch = SolveRec{};
+      batch.kind = 7;
+      batch.wait = batch.sig = -1;
+      batch.x0 = (int32_t)subs.size();
+    };
+    flush();
+    recs.reserve(tasks.size());
+    for (size_t i = 0; i < tasks.size(); ++i) {
+      const SolveTask& t = tasks[i];
+      if (t.kind == 6) continue;
+      if (P.level[t.s] != level) {
+        flush();
+        level = P.level[t.s];
+      }
+      SolveRec r = make(t, fwd);
+      r.kind |= (int32_t)(i << 3);
+      if (!small(t)) {
+        recs.push_back(r);
+        continue;
+      }
+      subs.push_back(r);
+      batch.s = t.s;
+      if (++batch.m >= std::min(8, std::max(1, (nsmall[level] + slots - 1) / slots))) flush();
+    }
+    flush();
+  };
+  fill(P.fwd_tasks, true, P.fwd_recs, P.fwd_subs);
+  fill(P.bwd_tasks, false, P.bwd_recs, P.bwd_subs);
+  P.fwd_wait = P.fwd_pending;
+  for (int32_t s : P.tiny) {
+    const SnMeta& m = P.meta[s];
+    for (int r = m.w, last = -1; r < m.h; ++r) {
+      const int t = P.supmember0[P.rows[m.lidx + r]];
+      if (t != last) --P.fwd_wait[t];
+      last = t;
+    }
+  }
 }
 
 std::vector<int64_t> build_assembly_map(const Symbolic& sym, const Plan& P, const int64_t* colptr,

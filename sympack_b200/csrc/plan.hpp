@@ -144,6 +144,28 @@ struct SolveTask {
 };
 inline int32_t pack_task_i(int p, int q0) { return p | (q0 << 24); }
 
+// A solve task as the kernels read it: where its operand, its right-hand-side rows and its
+// output rows lie, what it waits for and what it signals, worked out once per structure so
+// that a task starts after one load (counter numbers index the sweep counters, see
+// solve_sync_ints).  The T tasks have none (kernels of their own before the forward and
+// after the backward sweep); small F / G tasks of one level share a batch record (kind 7:
+// their records are the m of the sub-record list from x0 on, one per warp); every other
+// SolveTask has one record, in order.
+struct alignas(16) SolveRec {
+  int64_t a;       // element offset of the operand's first element (panel arena; DI: inverse arena)
+  int64_t inv;     // one-block supernodes: element offset of the diagonal block's inverse
+  int32_t kind;    // SolveTask::kind | place in the task list << 3
+  int32_t s;
+  int32_t ld;      // leading dimension of the operand
+  int32_t m, k;    // outputs and inner length (F, G, D, B: panel columns and off-diagonal rows)
+  int32_t x0, y0;  // first right-hand-side row and first output row; the gathered side of O, F, W and G
+                   // counts in the concatenated row lists
+  int32_t wait, target;  // counter and the value to reach (wait < 0: none)
+  int32_t sig;     // counter to bump (-1: none)
+  int32_t g0, ng;  // O, F: relative-index groups of its rows; backward DI: first tile row and its column
+};
+static_assert(sizeof(SolveRec) == 64, "one 64-byte record per solve task");
+
 // Task counts of the super-block solve (host and device): tasks of a run of `tiles`
 // tiles, and the DI tasks of a super-block of nb blocks (sum over its rows r of the
 // tasks of r + 1 tiles; the same sum counts the backward rows of nb - r tiles).
@@ -179,6 +201,15 @@ struct InvItem {
   int32_t j;
   int32_t pad;
 };
+
+// Diagonal block of a one-block supernode that the inverse kernel inverts.
+struct Inv1Item {
+  int64_t a;    // element offset of the block in the panel arena
+  int64_t inv;  // element offset of its inverse
+  int32_t ld;
+  int32_t w;
+};
+constexpr int kInv1Narrow = 32;
 
 // 64 x 64 tiles of the inverse of a super-block of nb blocks (lower triangle of tiles).
 inline int64_t inv_tiles(int nb) { return (int64_t)nb * (nb + 1) / 2; }
@@ -229,6 +260,9 @@ struct Plan {
   // and per supernode the number of forward off-diagonal tiles writing its rows
   std::vector<SolveTask> fwd_tasks, bwd_tasks;
   std::vector<int32_t> fwd_pending;
+  std::vector<SolveRec> fwd_recs, bwd_recs;  // the same tasks as device records
+  std::vector<SolveRec> fwd_subs, bwd_subs;  // the records of their batches
+  std::vector<int32_t> fwd_wait;             // arrivals the forward sweep waits for (without the tiny leaves')
   std::vector<int32_t> tiny;  // leaf supernodes of the forward T tasks
   int32_t nblk_total = 0;  // 64-column blocks over all supernodes
   int32_t nsb_total = 0;   // solve super-blocks over all supernodes (per-super-block counters)
@@ -237,6 +271,11 @@ struct Plan {
   // diagonal super-block inverses: arena size (elements) and one item per (super-block, column block)
   int64_t inv_elems = 0;
   std::vector<InvItem> inv_items;
+  // inverses of the diagonal blocks of one-block supernodes (FP64, w x w column-major each):
+  // items of at most kInv1Narrow columns first
+  int64_t inv1_elems = 0;
+  std::vector<Inv1Item> inv1_items;
+  int32_t inv1_narrow = 0;
   // algorithmic bytes of one sweep: every panel element read once
   double solve_sweep_bytes = 0.0;
 };
@@ -246,6 +285,11 @@ struct Plan {
 constexpr int kSolveFusedTiles = 16;
 // Tiny leaf supernodes (at most kTinyMaxW columns and kTinyMaxElems panel entries) are
 // solved forward one per thread, kTinyBatch to a task.
+// Small F / G tasks: supernodes of at most kWarpMaxW columns and kWarpMaxOff off-diagonal
+// rows, one per warp.  Right-hand sides are solved in groups of kSolveGroup columns, each
+// group with counters of its own, at most kSolveGroups groups at a time.
+constexpr int kWarpMaxW = 16, kWarpMaxOff = 128;
+constexpr int kSolveGroup = 16, kSolveGroups = 4;
 constexpr int kTinyMaxW = 4, kTinyMaxElems = 64, kTinyBatch = 128;
 
 // Tunables of the plan.
@@ -277,7 +321,7 @@ Plan build_plan(const Symbolic& s, const PlanParams& p = PlanParams());
 // counts of tasks, waits and signals do not change; the dependency counters neither.
 void reorder_factor_tasks(Plan& P, const PlanParams& prm, const std::vector<double>& us);
 
-// int32 counters one persistent solve pass uses: two task counters, then per
+// int32 counters one group of right-hand sides uses: two task counters, then per
 // supernode arrivals and forward / backward done blocks, then per super-block
 // forward / backward update counts.  Sized by 64-column blocks (at least as many
 // as super-blocks).

@@ -17,10 +17,24 @@
 // inverse (k_sb_inverse, once per factorization), so the sb dependent block
 // solves of a substitution become sb independent row-block products: the chain
 // of a wide supernode has two steps per super-block (its DI products, then the
-// updates of the next super-block) instead of one per 64 columns.  The forward
-// sweep reads the permuted right-hand sides Y (accumulating the descendants'
-// contributions there) and writes its solution to Z; the backward sweep
-// accumulates into Z and writes the final solution X.
+// updates of the next super-block) instead of one per 64 columns.  The diagonal
+// block of a one-block supernode is applied through its inverse too
+// (k_diag_inverse).  The forward sweep reads the permuted right-hand sides Y
+// (accumulating the descendants' contributions there) and writes its solution
+// to Z; the backward sweep accumulates into Z and writes the final solution X.
+//
+// Every task is a product of a stored operand with a few right-hand-side columns.
+// The sweeps are bound by the chain of dependent tasks, each a few global round
+// trips, so a task does everything that needs no right-hand side before it waits:
+// one 64-byte record (SolveRec) says where everything is, the operand is loaded
+// straight into registers in the layout of the FP64 tensor-core fragments
+// (mma.sync m16n8k4: 32 entries per thread cover a 64 x 128 tile pair), and after
+// the wait only the right-hand sides pass through shared memory.  The products run
+// on the FP64 tensor pipe for one right-hand side too: an 8-column group costs no
+// more issue slots than scalar FMAs with their shared-memory reads would.
+// FP32 factors are widened as they enter a product.
+#include <type_traits>
+
 #include "kernels.cuh"
 
 namespace spb {
@@ -28,15 +42,28 @@ namespace dev {
 
 namespace {
 
-constexpr int kT = 64;         // rows / columns per task unit
-constexpr int kPld = 65;       // padded leading dimension of a staged 64 x 64 tile
+constexpr int kT = 64;         // rows / columns per tile
+constexpr int kPld = 65;       // padded leading dimension of a staged 64 x 64 tile (inverse kernels)
 constexpr int kThreads = 256;
-// staged tile (64 x 65), right-hand-side staging (64 x 64), and the accumulator of kR
-// right-hand sides; kR = 16 keeps three CTAs per SM
-template <int kR>
-constexpr size_t solve_smem() { return (size_t)(kT * kPld + kT * kT + kT * kR) * sizeof(double); }
-template <int kR>
-constexpr int solve_min_blocks() { return kR <= 16 ? 3 : 2; }
+// Leading dimensions (doubles) of the operands staged in shared memory: 4 mod 16, so that
+// the fragment reads (8 rows or columns a leading dimension apart x 4 consecutive) of a
+// half warp fall on 16 different banks.
+constexpr int kInvLd = 68;     // inverse of a one-block supernode's diagonal block
+constexpr int kXLd = 260;      // right-hand-side rows of one pass (at most 256)
+constexpr int kZLd = 68;       // solved rows of a one-block supernode
+constexpr int kRowCap = 512;   // staged row indices
+
+// NG groups of 8 right-hand sides (1 or 2).
+template <int NG>
+struct SolveSmem {
+  double inv[kT * kInvLd];
+  double x[kXLd * 8 * NG];
+  double part[8 * 16 * 8 * NG];  // G: partial sums of the 8 warps
+  double z[8 * 20 * 8 * NG];     // solved rows: 64 of a block (ld kZLd) or 16 per warp (ld kWzLd)
+  int rows[kRowCap];
+};
+template <class T, int NG>
+constexpr int solve_min_blocks() { return NG == 1 && sizeof(T) == 4 ? 3 : 2; }
 
 __device__ __forceinline__ void report_status(Status* st, int code, int s, int col) {
   if (atomicCAS(&st->code, 0, code) == 0) {
@@ -59,282 +86,17 @@ __device__ __forceinline__ void red_release(int32_t* p, int v) {
 
 __device__ __forceinline__ int status_code(const Status* st) { return *(volatile const int32_t*)&st->code; }
 
-// Block-wide: wait until *flag >= target (thread 0 polls with acquire loads; the
-// barrier then orders every thread's later reads after the acquire).  False on
-// timeout or if another CTA has already recorded a failure.
-__device__ bool wait_geq(const int32_t* flag, int target, Status* st, int s, int* sh_ok, long long limit) {
-  if (threadIdx.x == 0) {
-    int good = 1;
-    if (ld_acquire(flag) < target) {
-      good = 0;
-      for (long long it = 0; it < limit; ++it) {
-        if (it >= 256) __nanosleep(128);  // short waits poll back to back (each poll is an L2 round trip)
-        if (ld_acquire(flag) >= target) {
-          good = 1;
-          break;
-        }
-        if (status_code(st) != 0) break;
-      }
-      if (!good && status_code(st) == 0) report_status(st, 3, s, target);
-    }
-    *sh_ok = good;
+// One thread: wait until *flag >= target.  False on timeout (recorded) or if another CTA
+// has already recorded a failure.
+__device__ __forceinline__ bool poll_geq(const int32_t* flag, int target, Status* st, int s, long long limit) {
+  if (ld_acquire(flag) >= target) return true;
+  for (long long it = 0; it < limit; ++it) {
+    if (it >= 256) __nanosleep(128);  // short waits poll back to back (each poll is an L2 round trip)
+    if (ld_acquire(flag) >= target) return true;
+    if (status_code(st) != 0) return false;
   }
-  __syncthreads();
-  int r = *sh_ok;
-  __syncthreads();
-  return r != 0;
-}
-
-// A 64 x 64 tile of T (column-major, leading dimension ld; rows < m and columns < kk
-// valid, zero elsewhere) held in registers, 16 entries per thread, so that the next
-// tile's loads are in flight while the current one is used.
-template <class T>
-struct TileRegs {
-  static constexpr int kPer = kT * kT / kThreads;
-  T v[kPer];
-  __device__ __forceinline__ void load(const T* P, int64_t ld, int m, int kk) {
-    if (m == kT && kk == kT) {
-#pragma unroll
-      for (int q = 0; q < kPer; ++q) {
-        const int idx = threadIdx.x + q * kThreads, k = idx >> 6, r = idx & 63;
-        v[q] = P[r + (int64_t)k * ld];
-      }
-      return;
-    }
-#pragma unroll
-    for (int q = 0; q < kPer; ++q) {
-      const int idx = threadIdx.x + q * kThreads, k = idx >> 6, r = idx & 63;
-      v[q] = (r < m && k < kk) ? P[r + (int64_t)k * ld] : T(0);
-    }
-  }
-  __device__ __forceinline__ void store(double* A) const {
-#pragma unroll
-    for (int q = 0; q < kPer; ++q) {
-      const int idx = threadIdx.x + q * kThreads, k = idx >> 6, r = idx & 63;
-      A[r + k * kPld] = (double)v[q];
-    }
-  }
-};
-
-// Stage L rows [r0, r0+m) x columns [c0, c0+kk) of a panel into A (ld kPld), widened to FP64.
-template <class T, int kLd = kPld>
-__device__ __forceinline__ void stage_block(double* A, const T* P, int64_t ld, int r0, int m, int c0, int kk) {
-  if (m == kT && kk == kT) {
-    T v[kT * kT / kThreads];
-#pragma unroll
-    for (int q = 0; q < kT * kT / kThreads; ++q) {
-      const int idx = threadIdx.x + q * kThreads, k = idx / kT, r = idx - k * kT;
-      v[q] = P[(r0 + r) + (int64_t)(c0 + k) * ld];
-    }
-#pragma unroll
-    for (int q = 0; q < kT * kT / kThreads; ++q) {
-      const int idx = threadIdx.x + q * kThreads, k = idx / kT, r = idx - k * kT;
-      A[r + k * kLd] = (double)v[q];
-    }
-    return;
-  }
-  for (int idx = threadIdx.x; idx < m * kk; idx += kThreads) {
-    int k = idx / m, r = idx - k * m;
-    A[r + k * kLd] = (double)P[(r0 + r) + (int64_t)(c0 + k) * ld];
-  }
-}
-
-// Stage X rows x0.. (contiguous) or rows rl[0..] (gathered) into B (leading dimension
-// ldb), through L2.
-__device__ __forceinline__ void stage_x(double* B, int ldb, const double* X, int64_t ldx, int x0, const int32_t* rl,
-                                        int m, int nr) {
-  for (int idx = threadIdx.x; idx < m * nr; idx += kThreads) {
-    int c = idx / m, r = idx - c * m;
-    int row = rl ? rl[r] : x0 + r;
-    B[r + c * ldb] = __ldcg(X + row + c * ldx);
-  }
-}
-
-// acc[i + c*kT] += sum_{k < kk} A(i, k) B[k + c*ldb]  for i < m, c < nr, with
-// A(i, k) = A[i + k*kPld] (kTrans false) or A[k + i*kPld] (kTrans true).  Few outputs
-// (one right-hand side): four threads per output and a shuffle reduction.
-template <bool kTrans>
-__device__ __forceinline__ void tile_gemv(double* acc, const double* A, const double* B, int ldb, int m, int kk,
-                                          int nr) {
-  if (m * nr * 4 <= kThreads) {
-    const int idx = threadIdx.x >> 2, part = threadIdx.x & 3;
-    const int c = idx / m, i = idx - c * m;
-    double s = 0.0;
-    if (idx < m * nr)
-      for (int k = part; k < kk; k += 4) s = fma(kTrans ? A[k + i * kPld] : A[i + k * kPld], B[k + c * ldb], s);
-    s += __shfl_xor_sync(0xffffffffu, s, 1);
-    s += __shfl_xor_sync(0xffffffffu, s, 2);
-    if (idx < m * nr && part == 0) acc[i + c * kT] += s;
-    return;
-  }
-  for (int idx = threadIdx.x; idx < m * nr; idx += kThreads) {
-    const int c = idx / m, i = idx - c * m;
-    double s = 0.0;
-    for (int k = 0; k < kk; ++k) s = fma(kTrans ? A[k + i * kPld] : A[i + k * kPld], B[k + c * ldb], s);
-    acc[i + c * kT] += s;
-  }
-}
-
-// X[x0 + i, c] (+/-)= sum_k A[i + k*lda] * B[k + c*kT] straight into global X with
-// atomics (i < m, c < nr, k < kk); A column-major with leading dimension lda.  With
-// rows, output i goes to X row x0 + rows[i] instead.
-template <bool kTrans>
-__device__ __forceinline__ void block_gemv_atomic(double* X, int64_t ldx, int x0, const double* A, int lda,
-                                                  const double* B, int m, int kk, int nr, double sign,
-                                                  const int32_t* rows = nullptr) {
-  if (m * nr * 4 <= kThreads) {  // few outputs (one or two right-hand sides): 4 threads per output
-    const int idx = threadIdx.x >> 2, part = threadIdx.x & 3;
-    const int c = idx / max(m, 1), i = idx - c * m;
-    double s = 0.0;
-    if (idx < m * nr) {
-      if (kTrans)
-        for (int k = part; k < kk; k += 4) s = fma(A[k + i * lda], B[k + c * kT], s);
-      else
-        for (int k = part; k < kk; k += 4) s = fma(A[i + k * lda], B[k + c * kT], s);
-    }
-    s += __shfl_xor_sync(0xffffffffu, s, 1);
-    s += __shfl_xor_sync(0xffffffffu, s, 2);
-    if (idx < m * nr && part == 0) atomicAdd(X + x0 + (rows ? rows[i] : i) + c * ldx, sign * s);
-    return;
-  }
-  for (int idx = threadIdx.x; idx < m * nr; idx += kThreads) {
-    int c = idx / m, i = idx - c * m;
-    double s = 0.0;
-    if (kTrans)
-      for (int k = 0; k < kk; ++k) s = fma(A[k + i * lda], B[k + c * kT], s);
-    else
-      for (int k = 0; k < kk; ++k) s = fma(A[i + k * lda], B[k + c * kT], s);
-    atomicAdd(X + x0 + (rows ? rows[i] : i) + c * ldx, sign * s);
-  }
-}
-
-// Lower-triangular solves of a kk x kk block held in A (ld lda) against the
-// right-hand sides acc (ld kT), one warp per right-hand side column; rinv holds
-// the reciprocals of the diagonal (computed off the dependency chain).
-// forward: acc <- D^-1 acc ; backward: acc <- D^-T acc.
-template <bool kForward>
-__device__ void block_trsv(double* acc, const double* A, const double* rinv, int kk, int nr, int lda = kPld) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = kThreads / 32;
-  for (int c = warp; c < nr; c += nw) {
-    double v0 = lane < kk ? acc[lane + c * kT] : 0.0;
-    double v1 = lane + 32 < kk ? acc[lane + 32 + c * kT] : 0.0;
-    for (int step = 0; step < kk; ++step) {
-      const int k = kForward ? step : kk - 1 - step;
-      const int owner = k & 31;
-      const bool hi = k >= 32;
-      double xk = __shfl_sync(0xffffffffu, hi ? v1 : v0, owner) * rinv[k];
-      if (lane == owner) {
-        if (hi) v1 = xk;
-        else v0 = xk;
-      }
-      if (kForward) {
-        // rows j > k: acc_j -= D[j][k] x_k
-        if (lane > k && lane < kk) v0 = fma(-A[lane + k * lda], xk, v0);
-        if (lane + 32 > k && lane + 32 < kk) v1 = fma(-A[lane + 32 + k * lda], xk, v1);
-      } else {
-        // rows j < k: acc_j -= D[k][j] x_k
-        if (lane < k) v0 = fma(-A[k + lane * lda], xk, v0);
-        if (lane + 32 < k) v1 = fma(-A[k + (lane + 32) * lda], xk, v1);
-      }
-    }
-    if (lane < kk) acc[lane + c * kT] = v0;
-    if (lane + 32 < kk) acc[lane + 32 + c * kT] = v1;
-  }
-}
-
-// Inverses of the eight 8 x 8 diagonal blocks of a full 64 x 64 lower block A (ld kPld),
-// written transposed into A's unused upper triangle: Inv_g[i][j] (i > j) at
-// A[(8g + j) + (8g + i) * kPld]; their diagonal is rinv.  Warp g inverts block g, lane j
-// its column j by substitution.  Computed before a chain task waits, off the chain.
-__device__ void invert_diag8(double* A, const double* rinv) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (warp >= 8 || lane >= 8) return;
-  const int b = 8 * warp, j = lane;
-  double z[8];
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    double t = 0.0;
-#pragma unroll
-    for (int k = 0; k < i; ++k)
-      if (k >= j) t = fma(A[(b + i) + (b + k) * kPld], z[k], t);
-    z[i] = i < j ? 0.0 : (i == j ? rinv[b + i] : -t * rinv[b + i]);
-  }
-#pragma unroll
-  for (int i = 1; i < 8; ++i)
-    if (i > j) A[(b + j) + (b + i) * kPld] = z[i];
-}
-
-// block_trsv for a full 64 x 64 block whose 8 x 8 diagonal inverses invert_diag8 stored:
-// eight groups of 8 rows, each solved by a product with its inverse (every lane computes
-// the group's 8 values from 8 shuffled inputs) and applied to the rows not yet solved.
-// forward: acc <- L^-1 acc ; backward: acc <- L^-T acc.  One warp per right-hand side.
-template <bool kForward>
-__device__ void block_trsv64(double* acc, const double* A, const double* rinv, int nr) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = kThreads / 32;
-  for (int c = warp; c < nr; c += nw) {
-    double v0 = acc[lane + c * kT], v1 = acc[lane + 32 + c * kT];
-#pragma unroll
-    for (int step = 0; step < 8; ++step) {
-      const int g = kForward ? step : 7 - step, b = 8 * g;
-      const bool hi = g >= 4;  // the group's rows are held in v1 of lanes b - 32 ..
-      double r[8], x[8];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) r[j] = __shfl_sync(0xffffffffu, hi ? v1 : v0, (b & 31) + j);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        double t = rinv[b + j] * r[j];
-        if (kForward) {
-#pragma unroll
-          for (int m = 0; m < j; ++m) t = fma(A[(b + m) + (b + j) * kPld], r[m], t);  // Inv[j][m]
-        } else {
-#pragma unroll
-          for (int m = j + 1; m < 8; ++m) t = fma(A[(b + j) + (b + m) * kPld], r[m], t);  // Inv[m][j]
-        }
-        x[j] = t;
-      }
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        if (!hi && lane == b + j) v0 = x[j];
-        if (hi && lane + 32 == b + j) v1 = x[j];
-      }
-      if (kForward) {  // rows below the group: v_r -= sum_j L[r][b + j] x_j
-        if (lane > b + 7) {
-#pragma unroll
-          for (int j = 0; j < 8; ++j) v0 = fma(-A[lane + (b + j) * kPld], x[j], v0);
-        }
-        if (lane + 32 > b + 7) {
-#pragma unroll
-          for (int j = 0; j < 8; ++j) v1 = fma(-A[lane + 32 + (b + j) * kPld], x[j], v1);
-        }
-      } else {  // rows above the group: v_k -= sum_j L[b + j][k] x_j
-        if (lane < b) {
-#pragma unroll
-          for (int j = 0; j < 8; ++j) v0 = fma(-A[(b + j) + lane * kPld], x[j], v0);
-        }
-        if (lane + 32 < b) {
-#pragma unroll
-          for (int j = 0; j < 8; ++j) v1 = fma(-A[(b + j) + (lane + 32) * kPld], x[j], v1);
-        }
-      }
-    }
-    acc[lane + c * kT] = v0;
-    acc[lane + 32 + c * kT] = v1;
-  }
-}
-
-// Next task of a persistent sweep; the whole block takes the same branch
-// (thread 0 alone reads the counter and the status word, a barrier reached by
-// only part of a block would hang).  -1 = no task left or a failure recorded.
-__device__ __forceinline__ int next_task(const PSolveArgs& a, int* sh_task, int* sh_stop) {
-  if (threadIdx.x == 0) {
-    *sh_task = atomicAdd(a.counter, 1);
-    *sh_stop = status_code(a.status) != 0;
-  }
-  __syncthreads();
-  const int tk = *sh_task;
-  const bool stop = *sh_stop != 0;
-  __syncthreads();
-  return (tk >= a.ntasks || stop) ? -1 : tk;
+  report_status(st, 3, s, target);
+  return false;
 }
 
 __device__ __forceinline__ unsigned long long now_ns() {
@@ -343,477 +105,669 @@ __device__ __forceinline__ unsigned long long now_ns() {
   return t;
 }
 
-// Task timeline for analysis (thread 0; trace may be null).
-__device__ __forceinline__ void trace_mark(const PSolveArgs& a, int tk, int slot, unsigned long long v) {
-  if (a.trace && threadIdx.x == 0) a.trace[4 * (size_t)tk + slot] = v;
+// Task timeline for analysis (of the first group of right-hand sides; trace may be null).
+__device__ __forceinline__ void trace_mark(unsigned long long* trace, const SolveRec& r, int slot) {
+  if (trace) trace[4 * (size_t)((unsigned)r.kind >> 3) + slot] = now_ns();
+}
+__device__ __forceinline__ void trace_start(unsigned long long* trace, const SolveRec& r) {
+  trace_mark(trace, r, 0);
+  if (trace) trace[4 * (size_t)((unsigned)r.kind >> 3) + 3] = ((unsigned long long)r.s << 8) | (unsigned)(r.kind & 7);
 }
 
-// Publish a block's writes, then bump a counter (thread 0).
-__device__ __forceinline__ void signal(int32_t* counter) {
-  __syncthreads();
-  if (threadIdx.x == 0) red_release(counter, 1);
+// D = A(16x4, row) * B(4x8, col) + D, FP64.  Fragment ownership (lane = 4*g + t):
+//   a0 = A[g][t], a1 = A[g+8][t], b0 = B[t][g],
+//   d0 = D[g][2t], d1 = D[g][2t+1], d2 = D[g+8][2t], d3 = D[g+8][2t+1].
+__device__ __forceinline__ void dmma(double (&d)[4], double a0, double a1, double b0) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};\n"
+      : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
+      : "d"(a0), "d"(a1), "d"(b0));
 }
 
-// Forward arrivals of one off-diagonal tile (panel rows r0 .. r1-1 of supernode s):
-// one per target supernode, i.e. per relative-index group the rows span (groups are
-// maximal runs of rows with the same target, numbered in row order), signalled in
-// parallel after the block's scatter.
-__device__ __forceinline__ void signal_arrivals(const PSolveArgs& a, const SnMeta& m, int r0, int r1) {
-  __syncthreads();
-  const int g0 = a.row_group[m.lidx + r0], g1 = a.row_group[m.lidx + r1 - 1];
-  for (int g = g0 + (int)threadIdx.x; g <= g1; g += kThreads) red_release(a.arrived + a.groups[g].t, 1);
-}
-
-// Shape of super-block p of a supernode of nblk 64-column blocks.
-struct SuperBlock {
-  int b0, nb;  // first block, blocks
-  __device__ SuperBlock(int p, int sb, int nblk) : b0(p * sb), nb(min(sb, nblk - p * sb)) {}
+// A 16 x 64 operand slab of one warp in fragment layout: element (m, k) lies at
+// p[m * sm + k * sk]; rows < mv and inner indices < kv are valid, the rest is zero.
+template <class T>
+struct Frag {
+  T a0[16], a1[16];
+  __device__ __forceinline__ void load(const T* p, int64_t sm, int64_t sk, int mv, int kv) {
+    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const T* q = p + g * sm + t * sk;
+    const bool v0 = g < mv, v1 = g + 8 < mv;
+    const int64_t s8 = 8 * sm, s4 = 4 * sk;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const bool kk = 4 * i + t < kv;
+      a0[i] = v0 && kk ? __ldg(q) : T(0);
+      a1[i] = v1 && kk ? __ldg(q + s8) : T(0);
+      q += s4;
+    }
+  }
 };
 
-// First element of tile (r, q) (r >= q) of the inverse of super-block p.
-template <class T>
-__device__ __forceinline__ const T* inv_tile(const PSolveArgs& a, const SnMeta& m, int p, int r, int q) {
-  const int64_t full = (int64_t)a.sb * (a.sb + 1) / 2;
-  return static_cast<const T*>(a.Inv) + m.ioff + ((int64_t)p * full + (int64_t)r * (r + 1) / 2 + q) * (kT * kT);
+// acc += A(16 x 64 slab) * B, B[k][c] = b[k + c * ldb] of NG groups of 8 columns.
+template <class T, int NG>
+__device__ __forceinline__ void slab_mma(double (&acc)[NG][4], const Frag<T>& f, const double* b, int ldb) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const double* q = b + t + g * ldb;
+#pragma unroll
+  for (int i = 0; i < 16; ++i)
+#pragma unroll
+    for (int n = 0; n < NG; ++n) dmma(acc[n], (double)f.a0[i], (double)f.a1[i], q[4 * i + n * 8 * ldb]);
 }
 
-// acc (64 x nr, ld kT) = sum_{j0 <= j < j1} tile_j (x) x_j, with the tile loads one
-// ahead in registers (the caller has issued tile j0's).  tile(j, regs) issues the
-// loads of tile j; xrow(j) gives the first X row of x_j, xlen(j) its valid rows;
-// kTrans applies the tiles transposed; m = valid outputs.  The x blocks are staged
-// all at once when they fit Bx.
-template <class T, bool kTrans, class TileFn, class XRow, class XLen>
-__device__ __forceinline__ void slab_product(double* acc, double* Ab, double* Bx, int j0, int j1, TileRegs<T>& regs,
-                                             TileFn tile, const double* X, int64_t ldx, XRow xrow, XLen xlen,
-                                             int m, int nr) {
-  const int nt = j1 - j0;
-  for (int idx = threadIdx.x; idx < kT * nr; idx += kThreads) acc[idx] = 0.0;
-  const bool all = nt * kT * nr <= kT * kT;
-  if (all)
-    for (int j = 0; j < nt; ++j) stage_x(Bx + j * kT, nt * kT, X, ldx, xrow(j0 + j), nullptr, xlen(j0 + j), nr);
-  for (int j = 0; j < nt; ++j) {
-    regs.store(Ab);
-    if (j + 1 < nt) tile(j0 + j + 1, regs);
-    if (!all) stage_x(Bx, kT, X, ldx, xrow(j0 + j), nullptr, xlen(j0 + j), nr);
-    __syncthreads();
-    if (all) tile_gemv<kTrans>(acc, Ab, Bx + j * kT, nt * kT, m, xlen(j0 + j), nr);
-    else tile_gemv<kTrans>(acc, Ab, Bx, kT, m, xlen(j0 + j), nr);
-    __syncthreads();
+// Rows of nc right-hand-side columns into b (ld ldb): row r < kr comes from X row
+// (rows ? rows[r] : x0 + r) when r < k and is zero otherwise.  kr: 64, 128 or 256.
+__device__ __forceinline__ void stage_x(double* b, int ldb, const double* X, int64_t ldx, int x0, const int* rows,
+                                        int k, int kr, int nc) {
+  const int r = threadIdx.x & (kr - 1);
+  const int row = r < k ? (rows ? rows[r] : x0 + r) : 0;
+  for (int c = threadIdx.x / kr; c < nc; c += kThreads / kr) {
+    const double v = r < k ? __ldcg(X + row + c * ldx) : 0.0;
+    b[r + c * ldb] = v;
   }
 }
 
-// out[x0 + i + c*ldx] += sign * acc[i + c*kT] for i < m, c < nr (atomic).
-__device__ __forceinline__ void add_out(double* out, int64_t ldx, int x0, const double* acc, int m, int nr,
-                                        double sign, const int32_t* rows = nullptr) {
-  for (int idx = threadIdx.x; idx < m * nr; idx += kThreads) {
-    int c = idx / m, i = idx - c * m;
-    atomicAdd(out + x0 + (rows ? rows[i] : i) + c * ldx, sign * acc[i + c * kT]);
+// out(row, c) += sign * acc for the tile rows below mv and columns below nc (atomic, fire
+// and forget): tile row r goes to out row (rows ? rows[r] : y0 + r).
+template <int NG>
+__device__ __forceinline__ void scatter(double* out, int64_t ldx, int y0, const int* rows, const double (&acc)[NG][4],
+                                        int mv, int nc, double sign) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int r = g + 8 * h;
+    if (r >= mv) continue;
+    double* o = out + (rows ? rows[r] : y0 + r);
+#pragma unroll
+    for (int n = 0; n < NG; ++n)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int c = n * 8 + 2 * t + e;
+        if (c < nc) atomicAdd(o + c * ldx, sign * acc[n][2 * h + e]);
+      }
   }
 }
 
-// Forward sweep of one tiny leaf supernode s (w <= kTinyMaxW columns, no arrivals to wait
-// for) by one thread: Z_0 <- L_00^-1 Y_0 by substitution (multiplying by the pivots'
-// reciprocals), then Y[ancestor rows] -= L_u0 Z_0 with atomic additions, then one arrival
-// per target group of its rows (the release orders the thread's own writes) and its
-// diagonal-done count.
+template <int NG>
+__device__ __forceinline__ void clear(double (&acc)[NG][4]) {
+#pragma unroll
+  for (int n = 0; n < NG; ++n)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) acc[n][e] = 0.0;
+}
+
+// Inverse of a one-block supernode's diagonal block (w x w lower triangle, ld w) into
+// shared memory, zero outside, up to the fragment sizes the products read.
+__device__ __forceinline__ void stage_inverse(double* s, const double* inv, int w) {
+  const int wr = (w + 15) & ~15;
+  for (int idx = threadIdx.x; idx < wr * kT; idx += kThreads) {
+    const int c = idx >> 6, r = idx & 63;
+    if (r < wr) s[r + c * kInvLd] = (r < w && c < w && r >= c) ? __ldg(inv + r + c * w) : 0.0;
+  }
+}
+
+// z = Inv y (kTrans false) or Inv^T y for the w rows of a one-block supernode, columns c0 ..
+// c0 + nc - 1 of it: y in shared memory (ld ldy, zero from row w on), result to global
+// (out, first row) and, when zs, to shared memory (ld kZLd, zero from row w on).
+template <int NG, bool kTrans>
+__device__ __forceinline__ void apply_inverse(double* out, int64_t ldx, double* zs, const double* inv, const double* y,
+                                              int ldy, int w, int nc) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+  const int mt = (w + 15) >> 4, ks = (w + 3) >> 2;
+  for (int pr = warp; pr < mt * NG; pr += kThreads / 32) {
+    const int im = pr / NG, in = pr % NG;
+    if (in * 8 >= nc) continue;
+    double d[4] = {0.0, 0.0, 0.0, 0.0}, d2[4] = {0.0, 0.0, 0.0, 0.0};
+    const double* b = y + t + (in * 8 + g) * ldy;
+    const double* p = kTrans ? inv + t + (im * 16 + g) * kInvLd : inv + im * 16 + g + t * kInvLd;
+    const int s1 = kTrans ? 8 * kInvLd : 8, sk = kTrans ? 4 : 4 * kInvLd;
+    const int i0 = kTrans ? 4 * im : 0, i1 = kTrans ? ks : min(ks, 4 * (im + 1));
+    int i = i0;
+    for (; i + 1 < i1; i += 2) {
+      dmma(d, p[i * sk], p[i * sk + s1], b[4 * i]);
+      dmma(d2, p[(i + 1) * sk], p[(i + 1) * sk + s1], b[4 * i + 4]);
+    }
+    if (i < i1) dmma(d, p[i * sk], p[i * sk + s1], b[4 * i]);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int r = im * 16 + g + 8 * (e >> 1), c = in * 8 + 2 * t + (e & 1);
+      const double v = d[e] + d2[e];
+      if (r < w && c < nc) out[r + c * ldx] = v;
+      if (zs) zs[r + c * kZLd] = v;  // rows from w on: zero rows of the inverse
+    }
+  }
+}
+
+// Forward sweep of one column of a tiny leaf supernode (w <= kTinyMaxW columns, no arrivals
+// to wait for) by one thread: Z_0 <- L_00^-1 Y_0 by substitution (multiplying by the pivots'
+// reciprocals), then Y[ancestor rows] -= L_u0 Z_0 with atomic additions.
 template <class T>
-__device__ void tiny_forward(const PSolveArgs& a, int s, int nr) {
-  const SnMeta m = a.meta[s];
+__device__ __forceinline__ void tiny_forward(const PSolveArgs& a, const SnMeta& m, int64_t xo) {
   const T* P = static_cast<const T*>(a.L) + m.off;
   const int32_t* rl = a.rows + m.lidx;
   const int w = m.w, h = m.h;
   const int64_t ld = m.ld;
-  double rinv[kTinyMaxW];
+  double y[kTinyMaxW];
 #pragma unroll
-  for (int j = 0; j < kTinyMaxW; ++j) rinv[j] = j < w ? 1.0 / (double)P[j + j * ld] : 0.0;
-  for (int c = 0; c < nr; ++c) {
-    const int64_t xo = (int64_t)c * a.ldx;
-    double y[kTinyMaxW];
-#pragma unroll
-    for (int j = 0; j < kTinyMaxW; ++j) {
-      if (j >= w) break;
-      double t = a.X[m.fc + j + xo];
+  for (int j = 0; j < kTinyMaxW; ++j) {
+    y[j] = 0.0;
+    if (j < w) {
+      double t = __ldcg(a.X + m.fc + j + xo);
 #pragma unroll
       for (int k = 0; k < j; ++k) t = fma(-(double)P[j + k * ld], y[k], t);
-      y[j] = t * rinv[j];
+      y[j] = t * (1.0 / (double)P[j + j * ld]);
       a.Z[m.fc + j + xo] = y[j];
     }
-    for (int r = w; r < h; ++r) {
-      double t = 0.0;
+  }
+  for (int r = w; r < h; ++r) {
+    double t = 0.0;
 #pragma unroll
-      for (int j = 0; j < kTinyMaxW; ++j)
-        if (j < w) t = fma((double)P[r + j * ld], y[j], t);
-      atomicAdd(a.X + rl[r] + xo, -t);
-    }
+    for (int j = 0; j < kTinyMaxW; ++j)
+      if (j < w) t = fma((double)P[r + j * ld], y[j], t);
+    atomicAdd(a.X + rl[r] + xo, -t);
   }
-  if (h > w) {
-    const int g0 = a.row_group[m.lidx + w], g1 = a.row_group[m.lidx + h - 1];
-    for (int g = g0; g <= g1; ++g) red_release(a.arrived + a.groups[g].t, 1);
-  }
-  red_release(a.blkdone + s, 1);
 }
 
-// Backward sweep of one tiny leaf supernode s by one thread, once its parent is done
-// (bounded wait, like wait_geq but per thread): Z_0 -= L_u0^T X[ancestor rows], then
-// X_0 <- L_00^-T Z_0 by substitution; then its diagonal-done count.
+// Backward sweep of one column of a tiny leaf supernode by one thread, its parent done:
+// Z_0 -= L_u0^T X[ancestor rows], then X_0 <- L_00^-T Z_0 by substitution.
 template <class T>
-__device__ void tiny_backward(const PSolveArgs& a, int s, int nr) {
-  const SnMeta m = a.meta[s];
-  const int par = a.sparent[s];
-  if (par >= 0) {
-    const int target = solve_done_count(a.meta[par].w, a.sb, a.tpt);
-    const int32_t* flag = a.blkdone + par;
-    if (ld_acquire(flag) < target) {
-      bool good = false;
-      for (long long it = 0; it < a.spin_limit; ++it) {
-        if (it >= 256) __nanosleep(128);
-        if (ld_acquire(flag) >= target) {
-          good = true;
-          break;
-        }
-        if (status_code(a.status) != 0) return;
-      }
-      if (!good) {
-        report_status(a.status, 3, s, target);
-        return;
-      }
-    }
-  }
+__device__ __forceinline__ void tiny_backward(const PSolveArgs& a, const SnMeta& m, int64_t xo) {
   const T* P = static_cast<const T*>(a.L) + m.off;
   const int32_t* rl = a.rows + m.lidx;
   const int w = m.w, h = m.h;
   const int64_t ld = m.ld;
-  double rinv[kTinyMaxW];
+  double z[kTinyMaxW];
 #pragma unroll
-  for (int j = 0; j < kTinyMaxW; ++j) rinv[j] = j < w ? 1.0 / (double)P[j + j * ld] : 0.0;
-  for (int c = 0; c < nr; ++c) {
-    const int64_t xo = (int64_t)c * a.ldx;
-    double z[kTinyMaxW];
+  for (int j = 0; j < kTinyMaxW; ++j) z[j] = j < w ? a.Z[m.fc + j + xo] : 0.0;
+  for (int r = w; r < h; ++r) {
+    const double xr = __ldcg(a.X + rl[r] + xo);
 #pragma unroll
-    for (int j = 0; j < kTinyMaxW; ++j) z[j] = j < w ? a.Z[m.fc + j + xo] : 0.0;
-    for (int r = w; r < h; ++r) {
-      const double xr = a.X[rl[r] + xo];
-#pragma unroll
-      for (int j = 0; j < kTinyMaxW; ++j)
-        if (j < w) z[j] = fma(-(double)P[r + j * ld], xr, z[j]);
-    }
-#pragma unroll
-    for (int j = kTinyMaxW - 1; j >= 0; --j) {
-      if (j >= w) continue;
-      double t = z[j];
-#pragma unroll
-      for (int k = j + 1; k < kTinyMaxW; ++k)
-        if (k < w) t = fma(-(double)P[k + j * ld], z[k], t);
-      z[j] = t * rinv[j];
-      a.X[m.fc + j + xo] = z[j];
-    }
+    for (int j = 0; j < kTinyMaxW; ++j)
+      if (j < w) z[j] = fma(-(double)P[r + j * ld], xr, z[j]);
   }
-  red_release(a.blkdone + s, 1);
+#pragma unroll
+  for (int j = kTinyMaxW - 1; j >= 0; --j) {
+    if (j >= w) continue;
+    double t = z[j];
+#pragma unroll
+    for (int k = j + 1; k < kTinyMaxW; ++k)
+      if (k < w) t = fma(-(double)P[k + j * ld], z[k], t);
+    z[j] = t * (1.0 / (double)P[j + j * ld]);
+    a.X[m.fc + j + xo] = z[j];
+  }
 }
 
-template <class T, int kR>
-__global__ void __launch_bounds__(kThreads, solve_min_blocks<kR>()) k_solve_forward(PSolveArgs a) {
-  extern __shared__ __align__(16) double sm[];
-  double* Ab = sm;                  // staged tile, ld kPld
-  double* Bx = sm + kT * kPld;      // staged right-hand-side rows
-  double* acc = Bx + kT * kT;       // accumulator, ld kT
-  __shared__ int sh_task, sh_stop, sh_ok;
-  __shared__ double sh_rinv[kT];
-  const int nr = a.nrhs;
-  TileRegs<T> regs;
-  for (;;) {
-    const int tk = next_task(a, &sh_task, &sh_stop);
-    if (tk < 0) return;
-    const SolveTask task = a.tasks[tk];
-    const int s = task.s;
-    trace_mark(a, tk, 0, now_ns());
-    trace_mark(a, tk, 3, ((unsigned long long)s << 8) | (unsigned)task.kind);
-    const SnMeta m = a.meta[s];
-    const T* P = static_cast<const T*>(a.L) + m.off;
-    const int32_t* rl = a.rows + m.lidx;
-    const int64_t ld = m.ld;
-    const int nblk = (m.w + kT - 1) / kT;
-    if (task.kind == 6) {
-      // T: tiny leaf supernodes, one per thread (nothing to wait for)
-      trace_mark(a, tk, 1, now_ns());
-      if ((int)threadIdx.x < task.t) tiny_forward<T>(a, a.tiny[task.i + threadIdx.x], nr);
-      __syncthreads();
-    } else if (task.kind == 5) {
-      // DI(p, r): Z[block r of p] += sum_{q <= r, this task's tiles} Inv_p(r, q) Y[block q of p]
-      const int p = task.i & 0xffffff, q0 = task.i >> 24, r = task.t;
-      const SuperBlock B(p, a.sb, nblk);
-      const int t = B.b0 + r, bt = min(kT, m.w - t * kT), q1 = min(r + 1, q0 + a.tpt);
-      auto tile = [&](int q, TileRegs<T>& R) { R.load(inv_tile<T>(a, m, p, r, q), kT, kT, kT); };
-      tile(q0, regs);  // the inverse is final: load before waiting
-      if (!wait_geq(a.arrived + s, a.expected[s], a.status, s, &sh_ok, a.spin_limit)) return;
-      if (!wait_geq(a.upd + m.sboff + p, p * B.nb * solve_ntask(a.sb, a.tpt), a.status, s, &sh_ok, a.spin_limit))
-        return;
-      trace_mark(a, tk, 1, now_ns());
-      slab_product<T, false>(
-          acc, Ab, Bx, q0, q1, regs, tile, a.X, a.ldx, [&](int q) { return m.fc + (B.b0 + q) * kT; },
-          [&](int q) { return min(kT, m.w - (B.b0 + q) * kT); }, bt, nr);
-      add_out(a.Z, a.ldx, m.fc + t * kT, acc, bt, nr, 1.0);
-      signal(a.blkdone + s);
-    } else if (task.kind == 1) {
-      // U(p, t): Y[block t] -= L(t, super-block p) Z[p] over this task's tiles
-      const int p = task.i & 0xffffff, q0 = task.i >> 24, t = task.t;
-      const SuperBlock B(p, a.sb, nblk);
-      const int r0 = t * kT, bt = min(kT, m.w - r0), q1 = min(B.nb, q0 + a.tpt);
-      auto tile = [&](int q, TileRegs<T>& R) {
-        const int c0 = (B.b0 + q) * kT;
-        R.load(P + r0 + (int64_t)c0 * ld, ld, bt, min(kT, m.w - c0));
-      };
-      tile(q0, regs);  // L is final: load before waiting
-      if (!wait_geq(a.blkdone + s, solve_di_range(nblk, a.sb, a.tpt, 0, p + 1), a.status, s, &sh_ok, a.spin_limit))
-        return;
-      trace_mark(a, tk, 1, now_ns());
-      slab_product<T, false>(
-          acc, Ab, Bx, q0, q1, regs, tile, a.Z, a.ldx, [&](int q) { return m.fc + (B.b0 + q) * kT; },
-          [&](int q) { return min(kT, m.w - (B.b0 + q) * kT); }, bt, nr);
-      add_out(a.X, a.ldx, m.fc + r0, acc, bt, nr, -1.0);
-      signal(a.upd + m.sboff + t / a.sb);
-    } else if (task.kind == 2) {
-      // O(p, u): Y[ancestor rows of tile u] -= L(u, super-block p) Z[p] over this task's tiles
-      const int p = task.i & 0xffffff, q0 = task.i >> 24, u = task.t, r0 = m.w + u * kT, bu = min(kT, m.h - r0);
-      const SuperBlock B(p, a.sb, nblk);
-      const int q1 = min(B.nb, q0 + a.tpt);
-      auto tile = [&](int q, TileRegs<T>& R) {
-        const int c0 = (B.b0 + q) * kT;
-        R.load(P + r0 + (int64_t)c0 * ld, ld, bu, min(kT, m.w - c0));
-      };
-      tile(q0, regs);
-      if (!wait_geq(a.blkdone + s, solve_di_range(nblk, a.sb, a.tpt, 0, p + 1), a.status, s, &sh_ok, a.spin_limit))
-        return;
-      trace_mark(a, tk, 1, now_ns());
-      slab_product<T, false>(
-          acc, Ab, Bx, q0, q1, regs, tile, a.Z, a.ldx, [&](int q) { return m.fc + (B.b0 + q) * kT; },
-          [&](int q) { return min(kT, m.w - (B.b0 + q) * kT); }, bu, nr);
-      add_out(a.X, a.ldx, 0, acc, bu, nr, -1.0, rl + r0);
-      signal_arrivals(a, m, r0, r0 + bu);
-      __syncthreads();
-    } else if (task.kind == 0) {
-      // D: one-block supernode, Z_0 <- L_00^-1 Y_0 (its off-diagonal tiles are O tasks)
-      const int w = m.w;
-      stage_block(Ab, P, ld, 0, w, 0, w);  // L is final: load before waiting
-      __syncthreads();
-      if (threadIdx.x < w) sh_rinv[threadIdx.x] = 1.0 / Ab[threadIdx.x * (kPld + 1)];
-      if (w == kT) {  // full block: 8 x 8 diagonal inverses, off the chain
-        __syncthreads();
-        invert_diag8(Ab, sh_rinv);
-      }
-      if (!wait_geq(a.arrived + s, a.expected[s], a.status, s, &sh_ok, a.spin_limit)) return;
-      trace_mark(a, tk, 1, now_ns());
-      stage_x(acc, kT, a.X, a.ldx, m.fc, nullptr, w, nr);
-      __syncthreads();
-      if (w == kT) block_trsv64<true>(acc, Ab, sh_rinv, nr);
-      else block_trsv<true>(acc, Ab, sh_rinv, w, nr);
-      __syncthreads();
-      for (int idx = threadIdx.x; idx < w * nr; idx += kThreads) {
-        int c = idx / w, i = idx - c * w;
-        a.Z[m.fc + i + c * a.ldx] = acc[i + c * kT];
-      }
-      signal(a.blkdone + s);
-    } else {
-      // F: one-block supernode whole: Z_0 <- L_00^-1 Y_0, then every off-diagonal tile's
-      // Y[ancestor rows] -= L_u0 Z_0
-      const int w = m.w, h = m.h, noff = (m.h - m.w + kT - 1) / kT;
-      // a panel that fits the two staging buffers is loaded whole (ld h) before waiting
-      const bool whole = h * w <= kT * kPld + kT * kT;
-      if (whole) {  // eight loads of a thread in flight at a time
-        for (int base = threadIdx.x; base < h * w; base += 8 * kThreads) {
-          T v[8];
+// Tiny leaf supernodes of one sweep, one thread per leaf and column (leaves fastest).
+template <class T, bool kFwd>
+__global__ void __launch_bounds__(128) k_solve_tiny(PSolveArgs a) {
+  if (status_code(a.status) != 0) return;
+  const int64_t total = (int64_t)a.ntiny * a.nrhs;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
+    const int c = (int)(i / a.ntiny), j = (int)(i - (int64_t)c * a.ntiny);
+    const SnMeta m = a.meta[a.tiny[j]];
+    unsigned long long* tr = a.trace && c == 0 && j % kTinyBatch == 0 ? a.trace + 4 * (a.tiny_task0 + j / kTinyBatch) : nullptr;
+    if (tr) {
+      tr[0] = tr[1] = now_ns();
+      tr[3] = ((unsigned long long)a.tiny[j] << 8) | 6;
+    }
+    if (kFwd) tiny_forward<T>(a, m, c * a.ldx);
+    else tiny_backward<T>(a, m, c * a.ldx);
+    if (tr) tr[2] = now_ns();
+  }
+}
+
+// ---- small one-block supernodes, one per warp ---------------------------------------------
+// w <= 16 columns: the inverse and four 16-row tiles of the off-diagonal part (backward: 64
+// of its rows) are the warp's fragments, the right-hand sides are loaded straight into
+// fragments too, and only the solved rows pass through the warp's 16 x 8 NG shared tile zs.
+// No block barrier.  False when the wait gave up.
+constexpr int kWzLd = 20;
+
+template <class T>
+__device__ __forceinline__ void frag_rows(Frag<T>& f, const T* A, int ld, int row0, int mrows, int w) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
 #pragma unroll
-          for (int q = 0; q < 8; ++q) {
-            const int idx = base + q * kThreads, c = idx / h, r = idx - c * h;
-            v[q] = idx < h * w ? P[r + (int64_t)c * ld] : T(0);
-          }
+  for (int i = 0; i < 16; ++i) {
+    const int row = row0 + (i >> 2) * 16 + g, col = 4 * (i & 3) + t;
+    const T* q = A + row + (int64_t)col * ld;
+    f.a0[i] = row < mrows && col < w ? __ldg(q) : T(0);
+    f.a1[i] = row + 8 < mrows && col < w ? __ldg(q + 8) : T(0);
+  }
+}
+
+// d = (4 fragment steps) * zs, to out rows r0 + g (+ 8) below w and, when kKeep, back to zs
+template <int NG>
+__device__ __forceinline__ void small_mma(double (&d)[NG][4], const double (&v0)[4], const double (&v1)[4],
+                                          const double* zs) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
 #pragma unroll
-          for (int q = 0; q < 8; ++q)
-            if (base + q * kThreads < h * w) Ab[base + q * kThreads] = (double)v[q];
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int n = 0; n < NG; ++n) dmma(d[n], v0[i], v1[i], zs[4 * i + t + (n * 8 + g) * kWzLd]);
+}
+
+template <class T, int NG>
+__device__ bool warp_forward(const PSolveArgs& a, const SolveRec& r, double* zs, double* X, double* Z, int32_t* sync,
+                             int nc, Frag<T>& f, unsigned long long* trace) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3, w = r.m;
+  const T* A = static_cast<const T*>(a.L) + r.a + w;
+  const double* inv = a.Inv1 + r.inv;
+  double v0[4], v1[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int k = 4 * i + t;
+    v0[i] = g < w && k < w ? __ldg(inv + g + k * w) : 0.0;
+    v1[i] = g + 8 < w && k < w ? __ldg(inv + g + 8 + k * w) : 0.0;
+  }
+  frag_rows<T>(f, A, r.ld, 0, r.k, w);
+  int tgt = 0, cnt = 0;  // this lane's arrival
+  if (lane < r.ng) {
+    const RelGroup gr = a.groups[r.g0 + lane];
+    const int lo = gr.j0 - w, hi = (lane + 1 < r.ng ? a.groups[r.g0 + lane + 1].j0 - w : r.k) - 1;
+    tgt = gr.t;
+    cnt = (hi >> 6) - (lo >> 6) + 1;
+  }
+  const int32_t* rows = a.rows + r.y0;
+  bool ok = true;
+  if (lane == 0) ok = poll_geq(sync + r.wait, a.expected[r.s], a.status, r.s, a.spin_limit);
+  ok = __shfl_sync(0xffffffffu, ok, 0);
+  __syncwarp();  // orders the warp's reads after lane 0's acquire
+  if (!ok) return false;
+  if (trace) trace_mark(trace, r, 1);
+  double d[NG][4];
+  clear<NG>(d);
+  {
+    double y[4][NG];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int n = 0; n < NG; ++n)
+        y[i][n] = 4 * i + t < w && n * 8 + g < nc ? __ldcg(X + r.x0 + 4 * i + t + (n * 8 + g) * a.ldx) : 0.0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int n = 0; n < NG; ++n) dmma(d[n], v0[i], v1[i], y[i][n]);
+  }
+#pragma unroll
+  for (int n = 0; n < NG; ++n)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int row = g + 8 * (e >> 1), c = n * 8 + 2 * t + (e & 1);
+      zs[row + c * kWzLd] = d[n][e];
+      if (row < w && c < nc) Z[r.x0 + row + c * a.ldx] = d[n][e];
+    }
+  __syncwarp();
+  for (int row0 = 0; row0 < r.k; row0 += 64) {
+    if (row0 > 0) frag_rows<T>(f, A, r.ld, row0, r.k, w);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      if (row0 + 16 * j >= r.k) break;
+      const double x0[4] = {(double)f.a0[4 * j], (double)f.a0[4 * j + 1], (double)f.a0[4 * j + 2], (double)f.a0[4 * j + 3]};
+      const double x1[4] = {(double)f.a1[4 * j], (double)f.a1[4 * j + 1], (double)f.a1[4 * j + 2], (double)f.a1[4 * j + 3]};
+      clear<NG>(d);
+      small_mma<NG>(d, x0, x1, zs);
+      scatter<NG>(X, a.ldx, 0, rows + row0 + 16 * j, d, r.k - row0 - 16 * j, nc, -1.0);
+    }
+  }
+  __syncwarp();
+  if (lane < r.ng) red_release(sync + 2 + tgt, cnt);
+  for (int q = lane + 32; q < r.ng; q += 32) {
+    const RelGroup gr = a.groups[r.g0 + q];
+    const int lo = gr.j0 - w, hi = (q + 1 < r.ng ? a.groups[r.g0 + q + 1].j0 - w : r.k) - 1;
+    red_release(sync + 2 + gr.t, (hi >> 6) - (lo >> 6) + 1);
+  }
+  return true;
+}
+
+template <class T, int NG>
+__device__ bool warp_backward(const PSolveArgs& a, const SolveRec& r, double* zs, double* X, const double* Z,
+                              int32_t* sync, int nc, Frag<T>& f, unsigned long long* trace) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3, w = r.m;
+  const T* A = static_cast<const T*>(a.L) + r.a + w;
+  const double* inv = a.Inv1 + r.inv;
+  double v0[4], v1[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int k = 4 * i + t;
+    v0[i] = g < w && k < w ? __ldg(inv + k + g * w) : 0.0;
+    v1[i] = g + 8 < w && k < w ? __ldg(inv + k + (g + 8) * w) : 0.0;
+  }
+  f.load(A, r.ld, 1, w, min(64, r.k));
+  const int32_t* rows = a.rows + r.y0;
+  int idx[16];
+#pragma unroll
+  for (int i = 0; i < 16; ++i) idx[i] = 4 * i + t < r.k ? rows[4 * i + t] : -1;
+  bool ok = true;
+  if (lane == 0 && r.wait >= 0) ok = poll_geq(sync + r.wait, r.target, a.status, r.s, a.spin_limit);
+  ok = __shfl_sync(0xffffffffu, ok, 0);
+  __syncwarp();  // orders the warp's reads after lane 0's acquire
+  if (!ok) return false;
+  if (trace) trace_mark(trace, r, 1);
+  double d[NG][4];
+#pragma unroll
+  for (int n = 0; n < NG; ++n)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int row = g + 8 * (e >> 1), c = n * 8 + 2 * t + (e & 1);
+      d[n][e] = row < w && c < nc ? -__ldcg(Z + r.x0 + row + c * a.ldx) : 0.0;  // d = L^T x - z
+    }
+  for (int row0 = 0; row0 < r.k; row0 += 64) {
+    if (row0 > 0) {
+      f.load(A + row0, r.ld, 1, w, min(64, r.k - row0));
+#pragma unroll
+      for (int i = 0; i < 16; ++i) idx[i] = row0 + 4 * i + t < r.k ? rows[row0 + 4 * i + t] : -1;
+    }
+#pragma unroll
+    for (int i0 = 0; i0 < 16; i0 += 8) {
+      if (row0 + 4 * i0 >= r.k) break;
+      double x[8][NG];
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int n = 0; n < NG; ++n)
+          x[i][n] = idx[i0 + i] >= 0 && n * 8 + g < nc ? __ldcg(X + idx[i0 + i] + (n * 8 + g) * a.ldx) : 0.0;
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int n = 0; n < NG; ++n) dmma(d[n], (double)f.a0[i0 + i], (double)f.a1[i0 + i], x[i][n]);
+    }
+  }
+#pragma unroll
+  for (int n = 0; n < NG; ++n)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) zs[g + 8 * (e >> 1) + (n * 8 + 2 * t + (e & 1)) * kWzLd] = -d[n][e];
+  __syncwarp();
+  clear<NG>(d);
+  small_mma<NG>(d, v0, v1, zs);
+#pragma unroll
+  for (int n = 0; n < NG; ++n)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int row = g + 8 * (e >> 1), c = n * 8 + 2 * t + (e & 1);
+      if (row < w && c < nc) X[r.x0 + row + c * a.ldx] = d[n][e];
+    }
+  __syncwarp();
+  if (lane == 0) red_release(sync + r.sig, 1);
+  return true;
+}
+
+// One persistent sweep.  Per task: the record, the operand's loads, the wait, then the
+// staged right-hand sides and the product.  A ticket is one task for one group of kSolveGroup
+// right-hand sides: the groups are independent solves with counters of their own whose
+// chains run side by side, and share the operand's tiles in L2.  The next ticket is drawn
+// while the last results are on their way.
+template <class T, int NG, bool kFwd>
+__global__ void __launch_bounds__(kThreads, solve_min_blocks<T, NG>()) k_solve(PSolveArgs a) {
+  extern __shared__ __align__(16) unsigned char sm_raw[];
+  SolveSmem<NG>& sm = *reinterpret_cast<SolveSmem<NG>*>(sm_raw);
+  __shared__ int sh_task[2], sh_ok;  // the ticket of a turn is drawn into the other slot during the turn before
+  const int tid = threadIdx.x, warp = tid >> 5;
+  constexpr int NC = 8 * NG;
+  const int ngrp = (a.nrhs + kSolveGroup - 1) / kSolveGroup, ntickets = a.ntasks * ngrp;
+  Frag<T> f;
+  if (tid == 0) sh_task[0] = status_code(a.status) != 0 ? ntickets : atomicAdd(a.counter, 1);
+  __syncthreads();
+  for (int turn = 0;; turn ^= 1) {
+    const int ticket = sh_task[turn];
+    if (ticket >= ntickets) return;
+    const int tk = ticket / ngrp, grp = ticket - tk * ngrp;
+    const SolveRec r = a.recs[tk];
+    int32_t* sync = a.sync + grp * a.sync_stride;
+    double* X = a.X + (int64_t)grp * kSolveGroup * a.ldx;
+    double* Z = a.Z + (int64_t)grp * kSolveGroup * a.ldx;
+    const int nc = min(kSolveGroup, a.nrhs - grp * kSolveGroup);
+    const int kind = r.kind & 7;
+    unsigned long long* trace = grp == 0 && tid == 0 && kind != 7 ? a.trace : nullptr;
+    if (trace) trace_start(trace, r);
+    const T* L = static_cast<const T*>(a.L);
+    int tgt = 0, cnt = 1;  // this thread's arrival (O, F)
+    if (kFwd && tid < r.ng) {
+      const RelGroup gr = a.groups[r.g0 + tid];
+      tgt = gr.t;
+      if (kind != 2) {  // F: one arrival per 64-row tile and target, as the plan counts them
+        const int lo = gr.j0 - r.m, hi = (tid + 1 < r.ng ? a.groups[r.g0 + tid + 1].j0 - r.m : r.k) - 1;
+        cnt = (hi >> 6) - (lo >> 6) + 1;
+      }
+    }
+
+    // ---- before the wait: the operand --------------------------------------------------
+    const bool one_block = kind == 4 || kind == 0;
+    int wm = warp & 3, wk = warp >> 2;  // row tile and inner half of this warp
+    // F / G: shapes of the off-diagonal part
+    int sh = 0, mtl = 1, ksp = 1, sc = 0;
+    if (kind == 7) {
+      bool ok = true;
+      if (warp < r.m) {
+        const SolveRec q = a.subs[r.x0 + warp];
+        double* zs = sm.z + warp * kWzLd * 8 * NG;
+        unsigned long long* wtrace = grp == 0 && (tid & 31) == 0 ? a.trace : nullptr;
+        if (wtrace) trace_start(wtrace, q);
+        if (kFwd) ok = warp_forward<T, NG>(a, q, zs, X, Z, sync, nc, f, wtrace);
+        else ok = warp_backward<T, NG>(a, q, zs, X, Z, sync, nc, f, wtrace);
+        if (wtrace) trace_mark(wtrace, q, 2);
+      }
+      if (tid == 0) sh_task[turn ^ 1] = atomicAdd(a.counter, 1);
+      if (!__syncthreads_and(ok)) return;
+      continue;
+    } else if (one_block) {
+      stage_inverse(sm.inv, a.Inv1 + r.inv, r.m);
+      for (int i = tid; i < min(r.k, kRowCap); i += kThreads) sm.rows[i] = a.rows[r.y0 + i];
+      const T* A = L + r.a + r.m;  // first off-diagonal row
+      if (kFwd) {
+        // m-tiles of 16 off-diagonal rows dealt to the warps; a warp's 16 fragment steps hold
+        // 4, 2 or 1 of them (w <= 16, 32, 64)
+        sh = r.m <= 16 ? 2 : r.m <= 32 ? 3 : 4;
+        sc = 128 << (4 - sh);  // rows per chunk
+        const int lane = tid & 31, g = lane >> 2, t = lane & 3;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          const int row = ((i >> sh) * 8 + warp) * 16 + g, col = 4 * (i & ((1 << sh) - 1)) + t;
+          const T* q = A + row + (int64_t)col * r.ld;
+          f.a0[i] = row < r.k && col < r.m ? __ldg(q) : T(0);
+          f.a1[i] = row + 8 < r.k && col < r.m ? __ldg(q + 8) : T(0);
         }
       } else {
-        stage_block(Ab, P, ld, 0, w, 0, w);  // L is final: load before waiting
+        // 16-column tiles x splits of the off-diagonal rows over the 8 warps
+        mtl = r.m <= 16 ? 1 : r.m <= 32 ? 2 : 4;
+        ksp = 8 / mtl;
+        sc = mtl <= 2 ? 256 : 128;
+        wm = warp & (mtl - 1);
+        wk = warp / mtl;
+        const int rw = sc / ksp;  // rows of a warp: 32 or 64
+        f.load(A + (int64_t)wm * 16 * r.ld + wk * rw, r.ld, 1, r.m - wm * 16, min(rw, r.k - wk * rw));
       }
-      const int lda = whole ? h : kPld;
-      __syncthreads();
-      if (threadIdx.x < w) sh_rinv[threadIdx.x] = 1.0 / Ab[threadIdx.x * (lda + 1)];
-      if (!wait_geq(a.arrived + s, a.expected[s], a.status, s, &sh_ok, a.spin_limit)) return;
-      trace_mark(a, tk, 1, now_ns());
-      stage_x(acc, kT, a.X, a.ldx, m.fc, nullptr, w, nr);
-      __syncthreads();
-      block_trsv<true>(acc, Ab, sh_rinv, w, nr, lda);
-      __syncthreads();
-      for (int idx = threadIdx.x; idx < w * nr; idx += kThreads) {
-        int c = idx / w, i = idx - c * w;
-        a.Z[m.fc + i + c * a.ldx] = acc[i + c * kT];
-      }
-      for (int u = 0; u < noff; ++u) {
-        const int r0 = w + u * kT, bu = min(kT, m.h - r0);
-        if (!whole) {
-          stage_block(Ab, P, ld, r0, bu, 0, w);
-          __syncthreads();
-        }
-        block_gemv_atomic<false>(a.X, a.ldx, 0, whole ? Ab + r0 : Ab, lda, acc, bu, w, nr, -1.0, rl + r0);
-        signal_arrivals(a, m, r0, r0 + bu);  // one per (tile, target), as the plan counts them
-        __syncthreads();
-      }
-      if (threadIdx.x == 0) red_release(a.blkdone + s, 1);
+    } else if (!kFwd && kind == 3) {  // W: one 16-column tile per warp
+      wm = warp;
+      wk = 0;
+      for (int i = tid; i < r.k; i += kThreads) sm.rows[i] = a.rows[r.x0 + i];
+      f.load(L + r.a + (int64_t)warp * 16 * r.ld, r.ld, 1, r.m - warp * 16, r.k);
+    } else if (!kFwd && kind == 5) {  // DI: this warp's tile of the inverse, transposed
+      const int R = r.g0 + wk;
+      f.load(static_cast<const T*>(a.Inv) + r.a + ((int64_t)R * (R + 1) / 2 + r.ng) * (kT * kT) + wm * 16 * kT, kT, 1,
+             r.m - wm * 16, min(kT, r.k - wk * kT));
+    } else if (!kFwd) {  // V
+      f.load(L + r.a + (int64_t)wm * 16 * r.ld + wk * kT, r.ld, 1, r.m - wm * 16, min(kT, r.k - wk * kT));
+    } else {  // DI, U, O
+      if (kind == 2)
+        for (int i = tid; i < r.m; i += kThreads) sm.rows[i] = a.rows[r.y0 + i];
+      const T* A = kind == 5 ? static_cast<const T*>(a.Inv) + r.a : L + r.a;
+      f.load(A + wm * 16 + (int64_t)wk * kT * r.ld, 1, r.ld, r.m - wm * 16, min(kT, r.k - wk * kT));
     }
-    trace_mark(a, tk, 2, now_ns());
-  }
-}
 
-template <class T, int kR>
-__global__ void __launch_bounds__(kThreads, solve_min_blocks<kR>()) k_solve_backward(PSolveArgs a) {
-  extern __shared__ __align__(16) double sm[];
-  double* Ab = sm;
-  double* Bx = sm + kT * kPld;
-  double* acc = Bx + kT * kT;
-  __shared__ int sh_task, sh_stop, sh_ok;
-  __shared__ double sh_rinv[kT];
-  const int nr = a.nrhs;
-  TileRegs<T> regs;
-  for (;;) {
-    const int tk = next_task(a, &sh_task, &sh_stop);
-    if (tk < 0) return;
-    const SolveTask task = a.tasks[tk];
-    const int s = task.s;
-    trace_mark(a, tk, 0, now_ns());
-    trace_mark(a, tk, 3, ((unsigned long long)s << 8) | (unsigned)task.kind);
-    const SnMeta m = a.meta[s];
-    const T* P = static_cast<const T*>(a.L) + m.off;
-    const int32_t* rl = a.rows + m.lidx;
-    const int64_t ld = m.ld;
-    const int nblk = (m.w + kT - 1) / kT, nsb = (nblk + a.sb - 1) / a.sb;
-    const int noff = (m.h - m.w + kT - 1) / kT;
-    if (task.kind == 6) {
-      // T: tiny leaf supernodes, one per thread (each waits for its parent)
-      trace_mark(a, tk, 1, now_ns());
-      if ((int)threadIdx.x < task.t) tiny_backward<T>(a, a.tiny[task.i + threadIdx.x], nr);
-      __syncthreads();
-      if (status_code(a.status) != 0) return;
-    } else if (task.kind == 5) {
-      // DI(p, r): X[block r of p] += sum_{q >= r, this task's tiles} Inv_p(q, r)^T Z[block q of p]
-      const int p = task.i & 0xffffff, j0 = task.i >> 24, r = task.t;
-      const SuperBlock B(p, a.sb, nblk);
-      const int t = B.b0 + r, bt = min(kT, m.w - t * kT), j1 = min(B.nb - r, j0 + a.tpt);
-      auto tile = [&](int j, TileRegs<T>& R) { R.load(inv_tile<T>(a, m, p, r + j, r), kT, kT, kT); };
-      tile(j0, regs);
-      // W tasks of every off-diagonal tile, V tasks of every later super-block into each block of p
-      const int nlast = nblk - (nsb - 1) * a.sb;
-      const int later = p < nsb - 1 ? (nsb - 2 - p) * solve_ntask(a.sb, a.tpt) + solve_ntask(nlast, a.tpt) : 0;
-      if (!wait_geq(a.upd + m.sboff + p, noff * solve_ntask(B.nb, a.tpt) + B.nb * later, a.status, s, &sh_ok,
-                    a.spin_limit))
-        return;
-      trace_mark(a, tk, 1, now_ns());
-      slab_product<T, true>(
-          acc, Ab, Bx, j0, j1, regs, tile, a.Z, a.ldx, [&](int j) { return m.fc + (t + j) * kT; },
-          [&](int j) { return min(kT, m.w - (t + j) * kT); }, bt, nr);
-      add_out(a.X, a.ldx, m.fc + t * kT, acc, bt, nr, 1.0);
-      signal(a.blkdone + s);
-    } else if (task.kind == 1) {
-      // V(p, t): Z[block t] -= L(super-block p, t)^T X[p] over this task's tiles
-      const int p = task.i & 0xffffff, q0 = task.i >> 24, t = task.t, c0 = t * kT, bt = min(kT, m.w - c0);
-      const SuperBlock B(p, a.sb, nblk);
-      const int q1 = min(B.nb, q0 + a.tpt);
-      auto tile = [&](int q, TileRegs<T>& R) {
-        const int r0 = (B.b0 + q) * kT;
-        R.load(P + r0 + (int64_t)c0 * ld, ld, min(kT, m.w - r0), bt);
-      };
-      tile(q0, regs);
-      if (!wait_geq(a.blkdone + s, solve_di_range(nblk, a.sb, a.tpt, p, nsb), a.status, s, &sh_ok, a.spin_limit))
-        return;
-      trace_mark(a, tk, 1, now_ns());
-      slab_product<T, true>(
-          acc, Ab, Bx, q0, q1, regs, tile, a.X, a.ldx, [&](int q) { return m.fc + (B.b0 + q) * kT; },
-          [&](int q) { return min(kT, m.w - (B.b0 + q) * kT); }, bt, nr);
-      add_out(a.Z, a.ldx, m.fc + c0, acc, bt, nr, -1.0);
-      signal(a.upd + m.sboff + t / a.sb);
-    } else if (task.kind == 3) {
-      // W(p, u): Z[p] -= L(u, super-block p)^T X[ancestor rows of tile u] over this task's
-      // tiles, final once the parent is done
-      const int p = task.i & 0xffffff, q0 = task.i >> 24, u = task.t, rr = m.w + u * kT, br = min(kT, m.h - rr);
-      const SuperBlock B(p, a.sb, nblk);
-      const int q1 = min(B.nb, q0 + a.tpt);
-      const int par = a.sparent[s];
-      regs.load(P + rr + (int64_t)(B.b0 + q0) * kT * ld, ld, br, min(kT, m.w - (B.b0 + q0) * kT));
-      if (par >= 0 &&
-          !wait_geq(a.blkdone + par, solve_done_count(a.meta[par].w, a.sb, a.tpt), a.status, s, &sh_ok, a.spin_limit))
-        return;
-      trace_mark(a, tk, 1, now_ns());
-      stage_x(Bx, kT, a.X, a.ldx, 0, rl + rr, br, nr);
-      for (int q = q0; q < q1; ++q) {
-        const int c0 = (B.b0 + q) * kT, bq = min(kT, m.w - c0);
-        regs.store(Ab);
-        if (q + 1 < q1) {
-          const int c1 = c0 + kT;
-          regs.load(P + rr + (int64_t)c1 * ld, ld, br, min(kT, m.w - c1));
-        }
-        __syncthreads();
-        block_gemv_atomic<true>(a.Z, a.ldx, m.fc + c0, Ab, kPld, Bx, bq, br, nr, -1.0);
-        __syncthreads();
-      }
-      if (threadIdx.x == 0) red_release(a.upd + m.sboff + p, 1);
-    } else if (task.kind == 0) {
-      // B: one-block supernode, X_0 <- L_00^-T Z_0 once its W updates landed
-      const int w = m.w;
-      stage_block(Ab, P, ld, 0, w, 0, w);  // L is final: load before waiting
-      __syncthreads();
-      if (threadIdx.x < w) sh_rinv[threadIdx.x] = 1.0 / Ab[threadIdx.x * (kPld + 1)];
-      if (w == kT) {  // full block: 8 x 8 diagonal inverses, off the chain
-        __syncthreads();
-        invert_diag8(Ab, sh_rinv);
-      }
-      if (!wait_geq(a.upd + m.sboff, noff, a.status, s, &sh_ok, a.spin_limit)) return;
-      trace_mark(a, tk, 1, now_ns());
-      stage_x(acc, kT, a.Z, a.ldx, m.fc, nullptr, w, nr);
-      __syncthreads();
-      if (w == kT) block_trsv64<false>(acc, Ab, sh_rinv, nr);
-      else block_trsv<false>(acc, Ab, sh_rinv, w, nr);
-      __syncthreads();
-      for (int idx = threadIdx.x; idx < w * nr; idx += kThreads) {
-        int c = idx / w, i = idx - c * w;
-        a.X[m.fc + i + c * a.ldx] = acc[i + c * kT];
-      }
-      signal(a.blkdone + s);
-    } else {
-      // G: one-block supernode whole: Z_0 -= L_u0^T X_u for every off-diagonal tile
-      // (ancestor rows, final once the parent is done), then X_0 <- L_00^-T Z_0
-      const int w = m.w;
-      const int par = a.sparent[s];
-      if (par >= 0 &&
-          !wait_geq(a.blkdone + par, solve_done_count(a.meta[par].w, a.sb, a.tpt), a.status, s, &sh_ok, a.spin_limit))
-        return;
-      trace_mark(a, tk, 1, now_ns());
-      stage_x(acc, kT, a.Z, a.ldx, m.fc, nullptr, w, nr);
-      for (int u = 0; u < noff; ++u) {
-        const int r0 = w + u * kT, bu = min(kT, m.h - r0);
-        __syncthreads();
-        stage_block(Ab, P, ld, r0, bu, 0, w);
-        stage_x(Bx, kT, a.X, a.ldx, 0, rl + r0, bu, nr);
-        __syncthreads();
-        for (int idx = threadIdx.x; idx < w * nr; idx += kThreads) {  // acc_k -= sum_r L_rk x_r
-          const int c = idx / w, k = idx - c * w;
-          double t = 0.0;
-          for (int r = 0; r < bu; ++r) t = fma(Ab[r + k * kPld], Bx[r + c * kT], t);
-          acc[k + c * kT] -= t;
-        }
-      }
-      __syncthreads();
-      stage_block(Ab, P, ld, 0, w, 0, w);
-      __syncthreads();
-      if (threadIdx.x < w) sh_rinv[threadIdx.x] = 1.0 / Ab[threadIdx.x * (kPld + 1)];
-      __syncthreads();
-      block_trsv<false>(acc, Ab, sh_rinv, w, nr);
-      __syncthreads();
-      for (int idx = threadIdx.x; idx < w * nr; idx += kThreads) {
-        int c = idx / w, i = idx - c * w;
-        a.X[m.fc + i + c * a.ldx] = acc[i + c * kT];
-      }
-      __syncthreads();
-      if (threadIdx.x == 0) red_release(a.blkdone + s, 1);
+    // ---- the wait ----------------------------------------------------------------------
+    if (tid == 0) {
+      bool ok = true;
+      if (kFwd && (one_block || kind == 5)) ok = poll_geq(sync + 2 + r.s, a.expected[r.s], a.status, r.s, a.spin_limit);
+      if (ok && r.wait >= 0 && !(kFwd && one_block)) ok = poll_geq(sync + r.wait, r.target, a.status, r.s, a.spin_limit);
+      sh_ok = ok;
     }
-    trace_mark(a, tk, 2, now_ns());
+    __syncthreads();
+    if (!sh_ok) return;
+    if (trace) trace_mark(trace, r, 1);
+
+    // ---- the product -------------------------------------------------------------------
+    if (one_block) {
+      const int w = r.m;
+      const T* A = L + r.a + w;
+      const int nch = (r.k + sc - 1) / sc;
+      {
+        if (kFwd) {
+          // F, D: Z_0 <- L_00^-1 Y_0, then every off-diagonal row's Y[ancestor row] -= L_u0 Z_0
+          stage_x(sm.x, kXLd, X, a.ldx, r.x0, nullptr, w, kT, nc);
+          __syncthreads();
+          apply_inverse<NG, false>(Z + r.x0, a.ldx, sm.z, sm.inv, sm.x, kXLd, w, nc);
+          __syncthreads();
+          const int lane = tid & 31, g = lane >> 2, t = lane & 3;
+          for (int ch = 0; ch < nch; ++ch) {
+            const int rb = ch * sc;
+            if (ch > 0) {  // this chunk's fragments
+#pragma unroll
+              for (int i = 0; i < 16; ++i) {
+                const int row = rb + ((i >> sh) * 8 + warp) * 16 + g, col = 4 * (i & ((1 << sh) - 1)) + t;
+                const T* q = A + row + (int64_t)col * r.ld;
+                f.a0[i] = row < r.k && col < w ? __ldg(q) : T(0);
+                f.a1[i] = row + 8 < r.k && col < w ? __ldg(q + 8) : T(0);
+              }
+            }
+            double acc[NG][4];
+            clear<NG>(acc);
+            const double* b = sm.z + t + g * kZLd;
+#pragma unroll
+            for (int q4 = 0; q4 < 4; ++q4) {  // quarters of the fragment steps; a tile ends after 1, 2 or 4
+              const int kb = 16 * (q4 & ((1 << (sh - 2)) - 1));
+              if (kb < w) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                  for (int n = 0; n < NG; ++n)
+                    dmma(acc[n], (double)f.a0[4 * q4 + i], (double)f.a1[4 * q4 + i], b[kb + 4 * i + n * 8 * kZLd]);
+              }
+              if (((q4 + 1) & ((1 << (sh - 2)) - 1)) == 0) {
+                const int row0 = rb + ((4 * q4 >> sh) * 8 + warp) * 16;
+                if (row0 < r.k) {
+                  if (row0 + 16 <= kRowCap) scatter<NG>(X, a.ldx, 0, sm.rows + row0, acc, r.k - row0, nc, -1.0);
+                  else scatter<NG>(X, a.ldx, 0, a.rows + r.y0 + row0, acc, r.k - row0, nc, -1.0);
+                }
+                clear<NG>(acc);
+              }
+            }
+          }
+        } else {
+          // G, B: Z_0 -= L_u0^T X[ancestor rows], then X_0 <- L_00^-T Z_0
+          double zv[2 * NG];
+          const int zi = tid & 63, zc = tid >> 6;
+#pragma unroll
+          for (int q = 0; q < 2 * NG; ++q) zv[q] = zi < w && zc + 4 * q < nc ? __ldcg(Z + r.x0 + zi + (zc + 4 * q) * a.ldx) : 0.0;
+          double acc[NG][4];
+          clear<NG>(acc);
+          const int rw = sc / ksp;
+          for (int ch = 0; ch < nch; ++ch) {
+            const int rb = ch * sc, kc = min(sc, r.k - rb);
+            if (ch > 0) __syncthreads();
+            stage_x(sm.x, kXLd, X, a.ldx, 0, rb + sc <= kRowCap ? sm.rows + rb : a.rows + r.y0 + rb, kc, sc, nc);
+            if (ch > 0)
+              f.load(A + (int64_t)wm * 16 * r.ld + rb + wk * rw, r.ld, 1, w - wm * 16, min(rw, kc - wk * rw));
+            __syncthreads();
+            if (wk * rw < kc) {
+              const int lane = tid & 31, g = lane >> 2, t = lane & 3;
+              const double* b = sm.x + wk * rw + t + g * kXLd;
+#pragma unroll
+              for (int i = 0; i < 16; ++i)
+                if (i < 8 || rw > 32)
+#pragma unroll
+                  for (int n = 0; n < NG; ++n) dmma(acc[n], (double)f.a0[i], (double)f.a1[i], b[4 * i + n * 8 * kXLd]);
+            }
+          }
+          {
+            const int lane = tid & 31, g = lane >> 2, t = lane & 3;
+#pragma unroll
+            for (int n = 0; n < NG; ++n)
+#pragma unroll
+              for (int e = 0; e < 4; ++e)
+                sm.part[((warp * NC) + n * 8 + 2 * t + (e & 1)) * 16 + g + 8 * (e >> 1)] = acc[n][e];
+          }
+          __syncthreads();
+#pragma unroll
+          for (int q = 0; q < 2 * NG; ++q) {
+            const int c = zc + 4 * q;
+            if (c < nc) {
+              double v = zv[q];
+              if (zi < w && nch > 0)
+                for (int k = 0; k < ksp; ++k) v -= sm.part[(((k * mtl + (zi >> 4)) * NC) + c) * 16 + (zi & 15)];
+              sm.z[zi + c * kZLd] = v;
+            }
+          }
+          __syncthreads();
+          apply_inverse<NG, true>(X + r.x0, a.ldx, nullptr, sm.inv, sm.z, kZLd, w, nc);
+        }
+      }
+    } else {
+      // wide supernodes: one operand of up to tpt tiles, two at a time
+      const bool W = !kFwd && kind == 3;
+      const int nch = ((W ? r.m : r.k) + 127) / 128;
+      // forward: DI reads Y into Z, U and O read Z into Y; backward: DI reads Z into X, V and W read X into Z
+      const bool to_z = kFwd == (kind == 5);
+      const double sign = kind == 5 ? 1.0 : -1.0;
+      {
+        const double* src = to_z ? X : Z;
+        double* dst = to_z ? Z : X;
+        double acc[NG][4];
+        clear<NG>(acc);
+        for (int ch = 0; ch < nch; ++ch) {
+          if (ch > 0 && !W) __syncthreads();
+          if (W) {
+            if (ch == 0) stage_x(sm.x, kXLd, src, a.ldx, 0, sm.rows, r.k, kT, nc);
+          } else {
+            stage_x(sm.x, kXLd, src, a.ldx, r.x0 + ch * 128, nullptr, r.k - ch * 128, 128, nc);
+          }
+          if (ch > 0) {  // further tiles of the task
+            const int kv = min(kT, r.k - ch * 128 - wk * kT);
+            if (W) {
+              f.load(L + r.a + (int64_t)(ch * 128 + warp * 16) * r.ld, r.ld, 1, r.m - ch * 128 - warp * 16, r.k);
+            } else if (!kFwd && kind == 5) {
+              const int R = r.g0 + 2 * ch + wk;
+              f.load(static_cast<const T*>(a.Inv) + r.a + ((int64_t)R * (R + 1) / 2 + r.ng) * (kT * kT) + wm * 16 * kT,
+                     kT, 1, r.m - wm * 16, kv);
+            } else if (!kFwd) {
+              f.load(L + r.a + (int64_t)wm * 16 * r.ld + ch * 128 + wk * kT, r.ld, 1, r.m - wm * 16, kv);
+            } else {
+              const T* A = kind == 5 ? static_cast<const T*>(a.Inv) + r.a : L + r.a;
+              f.load(A + wm * 16 + (int64_t)(ch * 128 + wk * kT) * r.ld, 1, r.ld, r.m - wm * 16, kv);
+            }
+          }
+          if (!W || ch == 0) __syncthreads();
+          const int mv = W ? r.m - ch * 128 - wm * 16 : r.m - wm * 16;
+          if (mv > 0 && (W || ch * 128 + wk * kT < r.k)) slab_mma<T, NG>(acc, f, sm.x + wk * kT, kXLd);
+          if (W) {
+            if (mv > 0) scatter<NG>(dst, a.ldx, r.y0 + ch * 128 + wm * 16, nullptr, acc, mv, nc, sign);
+            clear<NG>(acc);
+          }
+        }
+        const int mv = r.m - wm * 16;
+        if (!W && mv > 0) {
+          if (kFwd && kind == 2) scatter<NG>(dst, a.ldx, 0, sm.rows + wm * 16, acc, mv, nc, sign);
+          else scatter<NG>(dst, a.ldx, r.y0 + wm * 16, nullptr, acc, mv, nc, sign);
+        }
+      }
+    }
+
+    // ---- next ticket, signals ------------------------------------------------------------
+    if (tid == 0) {
+      const int stop = status_code(a.status);
+      const int nx = atomicAdd(a.counter, 1);
+      sh_task[turn ^ 1] = stop != 0 ? ntickets : nx;
+    }
+    __syncthreads();
+    if (r.sig >= 0 && tid == 0) red_release(sync + r.sig, 1);
+    if (kFwd && (kind == 2 || one_block)) {
+      if (tid < r.ng) red_release(sync + 2 + tgt, cnt);
+      for (int g = tid + kThreads; g < r.ng; g += kThreads) {  // F with more targets than threads
+        const RelGroup gr = a.groups[r.g0 + g];
+        const int lo = gr.j0 - r.m, hi = (g + 1 < r.ng ? a.groups[r.g0 + g + 1].j0 - r.m : r.k) - 1;
+        red_release(sync + 2 + gr.t, (hi >> 6) - (lo >> 6) + 1);
+      }
+    }
+    if (trace) trace_mark(trace, r, 2);
   }
 }
 
@@ -929,29 +883,97 @@ __global__ void __launch_bounds__(kInvThreads, 2) k_sb_inverse(const T* __restri
   }
 }
 
+// ---- inverses of one-block supernodes' diagonal blocks ------------------------------------
+// One warp per block of at most 32 columns (kW = 32) or one block of 64 threads per wider one:
+// thread c substitutes down column c, x_i = (delta_ic - sum_{k<i} L_ik x_k) / L_ii, the block
+// and the columns in shared memory (FP64).
+template <class T, int kW>
+__global__ void __launch_bounds__(128) k_diag_inverse(const T* __restrict__ L, double* __restrict__ Inv,
+                                                      const Inv1Item* __restrict__ items, int count) {
+  constexpr int kLd = kW + 1, kGroup = kW, kPer = kW == 32 ? 4 : 1;
+  extern __shared__ __align__(16) double smd[];
+  const int grp = threadIdx.x / kGroup, c = threadIdx.x % kGroup;
+  const int i0 = blockIdx.x * kPer + grp;
+  double* A = smd + (size_t)grp * 2 * kW * kLd;
+  double* X = A + kW * kLd;
+  auto sync = [&]() {
+    if constexpr (kW == 32) __syncwarp();
+    else __syncthreads();
+  };
+  if (i0 >= count) return;
+  const Inv1Item it = items[i0];
+  const int w = it.w;
+  for (int idx = c; idx < w * w; idx += kGroup) {
+    const int k = idx / w, i = idx - k * w;
+    if (i >= k) A[i * kLd + k] = (double)L[it.a + i + (int64_t)k * it.ld];
+  }
+  sync();
+  if (c < w) {
+    for (int i = 0; i < c; ++i) X[i * kLd + c] = 0.0;
+    for (int i = c; i < w; ++i) {
+      double s0 = 0.0, s1 = 0.0;
+      int k = c;
+      for (; k + 1 < i; k += 2) {
+        s0 = fma(A[i * kLd + k], X[k * kLd + c], s0);
+        s1 = fma(A[i * kLd + k + 1], X[(k + 1) * kLd + c], s1);
+      }
+      if (k < i) s0 = fma(A[i * kLd + k], X[k * kLd + c], s0);
+      X[i * kLd + c] = ((i == c ? 1.0 : 0.0) - (s0 + s1)) / A[i * kLd + i];
+    }
+  }
+  sync();
+  for (int idx = c; idx < w * w; idx += kGroup) {
+    const int k = idx / w, i = idx - k * w;
+    Inv[it.inv + idx] = X[i * kLd + k];
+  }
+}
+
+constexpr size_t kDiagInvSmem32 = (size_t)4 * 2 * 32 * 33 * sizeof(double);
+constexpr size_t kDiagInvSmem64 = (size_t)2 * 64 * 65 * sizeof(double);
+
+int g_solve_grid[2][2] = {};  // resident CTAs of the sweeps: [FP32][NG - 1]
+
+template <class T, int NG>
+void init_sweeps(int fp32, int sms) {
+  int per = 0;
+  cudaFuncSetAttribute(k_solve<T, NG, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SolveSmem<NG>));
+  cudaFuncSetAttribute(k_solve<T, NG, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SolveSmem<NG>));
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_solve<T, NG, true>, kThreads, sizeof(SolveSmem<NG>));
+  g_solve_grid[fp32][NG - 1] = sms * (per > 0 ? per : 1);
+}
+
+template <class T, int NG>
+void run_sweep(cudaStream_t st, const PSolveArgs& a, bool forward) {
+  const int64_t tickets = (int64_t)a.ntasks * ((a.nrhs + kSolveGroup - 1) / kSolveGroup);
+  const int cap = g_solve_grid[std::is_same<T, float>::value][NG - 1], grid = cap < tickets ? cap : (int)tickets;
+  const int64_t pairs = (int64_t)a.ntiny * a.nrhs;
+  const int tiny = pairs > 148 * 16 * 128 ? 148 * 16 : (int)((pairs + 127) / 128);
+  if (forward) {
+    if (tiny > 0) k_solve_tiny<T, true><<<tiny, 128, 0, st>>>(a);
+    if (grid > 0) k_solve<T, NG, true><<<grid, kThreads, sizeof(SolveSmem<NG>), st>>>(a);
+  } else {
+    if (grid > 0) k_solve<T, NG, false><<<grid, kThreads, sizeof(SolveSmem<NG>), st>>>(a);
+    if (tiny > 0) k_solve_tiny<T, false><<<tiny, 128, 0, st>>>(a);
+  }
+}
+
 }  // namespace
 
-int g_solve_grid = 0;    // CTAs of the persistent sweeps (resident CTAs of the device)
-int g_solve_grid16 = 0;  // CTAs of the persistent sweeps for <= 16 right-hand sides
-
 void init_solve_attributes() {
-  for (auto f : {k_solve_forward<double, 64>, k_solve_backward<double, 64>, k_solve_forward<float, 64>,
-                 k_solve_backward<float, 64>})
-    cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)solve_smem<64>());
-  for (auto f : {k_solve_forward<double, 16>, k_solve_backward<double, 16>, k_solve_forward<float, 16>,
-                 k_solve_backward<float, 16>})
-    cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)solve_smem<16>());
-  cudaFuncSetAttribute(k_sb_inverse<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kInvSmem);
-  cudaFuncSetAttribute(k_sb_inverse<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kInvSmem);
-  int dev = 0, sms = 0, per = 0, per16 = 0;
+  int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_solve_forward<double, 64>, kThreads, solve_smem<64>());
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per16, k_solve_forward<double, 16>, kThreads, solve_smem<16>());
-  g_solve_grid = sms * (per > 0 ? per : 1);
-  if (g_solve_grid <= 0) g_solve_grid = 148;
-  g_solve_grid16 = sms * (per16 > 0 ? per16 : 1);
-  if (g_solve_grid16 <= 0) g_solve_grid16 = g_solve_grid;
+  if (sms <= 0) sms = 148;
+  init_sweeps<double, 1>(0, sms);
+  init_sweeps<double, 2>(0, sms);
+  init_sweeps<float, 1>(1, sms);
+  init_sweeps<float, 2>(1, sms);
+  cudaFuncSetAttribute(k_sb_inverse<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kInvSmem);
+  cudaFuncSetAttribute(k_sb_inverse<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kInvSmem);
+  cudaFuncSetAttribute(k_diag_inverse<double, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDiagInvSmem32);
+  cudaFuncSetAttribute(k_diag_inverse<float, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDiagInvSmem32);
+  cudaFuncSetAttribute(k_diag_inverse<double, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDiagInvSmem64);
+  cudaFuncSetAttribute(k_diag_inverse<float, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDiagInvSmem64);
 }
 
 void launch_sb_inverse(cudaStream_t st, const void* L, void* Inv, bool fp32, const SnMeta* meta,
@@ -965,29 +987,25 @@ void launch_sb_inverse(cudaStream_t st, const void* L, void* Inv, bool fp32, con
                                                                static_cast<double*>(Inv), meta, items, sb);
 }
 
+void launch_diag_inverse(cudaStream_t st, const void* L, double* Inv, bool fp32, const Inv1Item* items, int narrow,
+                         int count) {
+  auto run = [&](auto* l) {
+    using T = typename std::remove_const<typename std::remove_pointer<decltype(l)>::type>::type;
+    if (narrow > 0) k_diag_inverse<T, 32><<<(narrow + 3) / 4, 128, kDiagInvSmem32, st>>>(l, Inv, items, narrow);
+    if (count > narrow) k_diag_inverse<T, 64><<<count - narrow, 64, kDiagInvSmem64, st>>>(l, Inv, items + narrow, count - narrow);
+  };
+  if (fp32) run(static_cast<const float*>(L));
+  else run(static_cast<const double*>(L));
+}
+
 void launch_solve_persistent(cudaStream_t st, const PSolveArgs& a, bool forward) {
-  if (a.ntasks <= 0 || a.spin_limit <= 0) return;
-  const bool small = a.nrhs <= 16;
-  const int cap = small ? g_solve_grid16 : g_solve_grid;
-  const int grid = cap < a.ntasks ? cap : a.ntasks;
-  if (small) {
-    const size_t sm = solve_smem<16>();
-    if (a.fp32) {
-      if (forward) k_solve_forward<float, 16><<<grid, kThreads, sm, st>>>(a);
-      else k_solve_backward<float, 16><<<grid, kThreads, sm, st>>>(a);
-    } else {
-      if (forward) k_solve_forward<double, 16><<<grid, kThreads, sm, st>>>(a);
-      else k_solve_backward<double, 16><<<grid, kThreads, sm, st>>>(a);
-    }
-    return;
-  }
-  const size_t sm = solve_smem<64>();
+  if (a.ntasks + a.ntiny <= 0 || a.spin_limit <= 0) return;
   if (a.fp32) {
-    if (forward) k_solve_forward<float, 64><<<grid, kThreads, sm, st>>>(a);
-    else k_solve_backward<float, 64><<<grid, kThreads, sm, st>>>(a);
+    if (a.nrhs <= 8) run_sweep<float, 1>(st, a, forward);
+    else run_sweep<float, 2>(st, a, forward);
   } else {
-    if (forward) k_solve_forward<double, 64><<<grid, kThreads, sm, st>>>(a);
-    else k_solve_backward<double, 64><<<grid, kThreads, sm, st>>>(a);
+    if (a.nrhs <= 8) run_sweep<double, 1>(st, a, forward);
+    else run_sweep<double, 2>(st, a, forward);
   }
 }
 

@@ -1,0 +1,78 @@
+"""Solve sweeps at the edges of their task shapes: one-block supernodes of every width class
+(a warp's 16 columns, 32, 64) over off-diagonal parts below and above what a warp and the
+staged row list hold, right-hand-side counts around the 8-column fragments, the 16-column
+groups and the 64-column passes, and tasks of one and of several tile pairs, in FP64 and
+LDL^T.  Answers agree with the CPU oracle's substitution to 1e-12 (the
+other GPU tests' bound: the matrices are diagonally dominant, condition below 1e3, so
+rounding differences stay near 1e-14)."""
+import os
+
+import numpy as np
+import pytest
+
+from oracle import numeric
+from sympack_b200 import DistSparseMatrix, RelaxationParameters, generators as G, symPACKMatrix2D, symPACKOptions
+
+pytestmark = pytest.mark.gpu
+TOL = 1e-12
+
+
+def bordered(widths, border, seed):
+    """Dense diagonal blocks of the given widths, each coupled to every row of a dense border."""
+    rng = np.random.default_rng(seed)
+    n = sum(widths) + border
+    starts = np.concatenate([[0], np.cumsum(widths)])
+    i, j = [], []
+    for b, w in enumerate(widths):
+        rows = np.concatenate([starts[b] + np.arange(w), np.arange(n - border, n)])
+        c = starts[b] + np.arange(w)
+        r, cc = np.meshgrid(rows, c, indexing="ij")
+        keep = r > cc
+        i.append(cc[keep])
+        j.append(r[keep])
+    r, cc = np.meshgrid(np.arange(n - border, n), np.arange(n - border, n), indexing="ij")
+    keep = r > cc
+    i.append(cc[keep])
+    j.append(r[keep])
+    i, j = np.concatenate(i), np.concatenate(j)
+    return G._dominant(n, i, j, -rng.uniform(0.05, 1.0, len(i)), 1e-2)
+
+
+def solver(A, **opt):
+    M = symPACKMatrix2D()
+    M.Init(symPACKOptions(device=0, orderingStr="NATURAL", relax=RelaxationParameters(0, 0, 0, 0, 0.0, 0.0, 0.0), **opt))
+    M.SymbolicFactorization(A)
+    M.DistributeMatrix(A)
+    M.Factorize()
+    return M
+
+
+def oracle_for(M, A, ldl=False):
+    _, invp = M.GetOrdering()
+    xl, li = M.GetStructure()
+    sym = dict(xsuper=M.GetSupernodalPartition(), xlindx=xl, lindx=li, supmember=M.GetSupMembership(), invp=invp)
+    f = numeric.OracleFactor(A.size, sym, threads=os.cpu_count(), ldl=ldl)
+    f.distribute(A.colptr, A.rowind, A.nzvalLocal)
+    f.factorize()
+    return f
+
+
+WIDTHS = [1, 3, 5, 15, 16, 17, 31, 32, 33, 63, 64, 2, 7, 64, 16]
+
+
+@pytest.mark.parametrize("tiles", [1, 2, 5])
+@pytest.mark.parametrize("border", [1, 63, 65, 128, 129, 300, 530, 1100])
+@pytest.mark.parametrize("dec", ["LL", "LDL"])
+def test_one_block_supernodes_match_the_oracle(dec, border, tiles):
+    A = DistSparseMatrix.from_lower_csc(*bordered(WIDTHS, border, border))
+    M = solver(A, decomposition=dec, plan_solve_tiles=tiles)
+    w = np.diff(M.GetSupernodalPartition())
+    assert set(WIDTHS) & set(w.tolist()) >= {5, 16, 17, 32, 33, 64}  # the blocks stay supernodes of their own
+    f = oracle_for(M, A, dec == "LDL")
+    rng = np.random.default_rng(1)
+    for nrhs in (1, 8, 9, 16, 17, 64, 81):
+        b = rng.standard_normal((A.size, nrhs))
+        M.Solve(b)
+        x, xo = M.GetSolution(nrhs=nrhs), f.solve(b)
+        assert np.max(np.abs(x - xo)) <= TOL * np.max(np.abs(xo)), nrhs
+    M.close()
