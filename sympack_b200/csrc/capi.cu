@@ -103,8 +103,6 @@ struct spb_handle {
   double* d_norms = nullptr;
   std::vector<int32_t> seg_off{};  // systems of a batch (0-based row offsets); empty = one system
   int32_t* d_rowseg = nullptr;     // system of each row (batches only)
-  double* dR = nullptr;       // residual / correction right-hand side (original order)
-  double* dD = nullptr;       // correction (original order)
   double* dXo = nullptr;      // refined solution (original order)
   int ir_iterations = 0;
   double backward_error = -1.0;
@@ -177,7 +175,7 @@ void release_device(spb_handle* h) {
   h->device_bytes = 0;
   h->dL = nullptr;
   h->dW = nullptr;
-  h->dX = h->dZ = h->dB = h->dR = h->dD = h->dXo = nullptr;
+  h->dX = h->dZ = h->dB = h->dXo = nullptr;
   h->dInv = h->dInvB = nullptr;
   h->dInv1 = h->dInv1B = nullptr;
   h->dsplit = nullptr;
@@ -398,7 +396,7 @@ int ensure_rhs_capacity(spb_handle* h, int nrhs) {
   }
   int64_t need = (int64_t)h->sym.n * nrhs;
   if (need <= h->x_cap) return SPB_OK;
-  for (double** p : {&h->dX, &h->dZ, &h->dB, &h->dR, &h->dD, &h->dXo}) {
+  for (double** p : {&h->dX, &h->dZ, &h->dB, &h->dXo}) {
     if (*p) {
       auto it = std::find(h->allocs.begin(), h->allocs.end(), (void*)*p);
       if (it != h->allocs.end()) h->allocs.erase(it);
@@ -412,11 +410,7 @@ int ensure_rhs_capacity(spb_handle* h, int nrhs) {
   SPB_CK(h, dalloc(h, &h->dX, need));
   SPB_CK(h, dalloc(h, &h->dZ, need));
   SPB_CK(h, dalloc(h, &h->dB, need));
-  if (h->fp32) {
-    SPB_CK(h, dalloc(h, &h->dR, need));
-    SPB_CK(h, dalloc(h, &h->dD, need));
-    SPB_CK(h, dalloc(h, &h->dXo, need));
-  }
+  if (h->fp32) SPB_CK(h, dalloc(h, &h->dXo, need));
   h->x_cap = need;
   SPB_CK(h, cudaStreamSynchronize(h->own_stream));  // allocations usable from any stream
   return SPB_OK;
@@ -593,11 +587,11 @@ int ir_solve(spb_handle* h, const double* d_b, int64_t ldb, double* d_x, int64_t
     double eta = 0.0, eta_prev = 1e300;
     int it = 0;
     for (;;) {
-      spb::dev::launch_residual(h->stream, h->d_rowptr, h->d_col, h->d_val, x, b, h->dR, n, nr, ldx);
       SPB_CK(h, cudaMemsetAsync(xmax, 0, sizeof(double) * 128 * (size_t)nseg, h->stream));
       SPB_CK(h, cudaMemsetAsync(h->d_norms, 0, sizeof(double), h->stream));
-      spb::dev::launch_segmax(h->stream, x, n, nr, ldx, h->d_rowseg, xmax);
-      spb::dev::launch_segmax(h->stream, h->dR, n, nr, ldx, h->d_rowseg, rmax);
+      // the residual goes where a correction solve reads its right-hand sides
+      spb::dev::launch_residual(h->stream, h->d_rowptr, h->d_col, h->d_val, x, ldx, b, ldb, h->dX, h->dinvp0, n, nr,
+                                h->d_rowseg, xmax, rmax);
       spb::dev::launch_eta(h->stream, anorm, bmax, xmax, rmax, nseg, nr, h->d_norms);
       SPB_CK(h, cudaMemcpyAsync(&eta, h->d_norms, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
       int rc = check_solve_status(h);  // synchronizes
@@ -612,8 +606,8 @@ int ir_solve(spb_handle* h, const double* d_b, int64_t ldb, double* d_x, int64_t
         return fail(h, SPB_ERR_NOT_CONVERGED, msg);
       }
       eta_prev = eta;
-      plain_solve(h, h->dR, ldx, h->dD, ldx, nr);
-      spb::dev::launch_axpy(h->stream, x, h->dD, n, nr, ldx);
+      enqueue_solve(h, nr);
+      spb::dev::launch_permute_add(h->stream, x, ldx, h->dX, n, h->dinvp0, n, nr);
       ++it;
     }
     iters_all = std::max(iters_all, it);
@@ -908,7 +902,7 @@ int64_t predict_bytes(const spb_handle* h, bool fp32, int nrhs) {
     const int nmaps = tile_map_index(P, of);
     t += b(split_layout(P, of, off), sizeof(float)) + b(ns, 8) + b(nmaps, sizeof(CUtensorMap)) + b(ns, 4);
   }
-  if (nrhs > 0) t += (fp32 ? 6 : 3) * b(n * nrhs, 8);
+  if (nrhs > 0) t += (fp32 ? 4 : 3) * b(n * nrhs, 8);
   return t;
 }
 

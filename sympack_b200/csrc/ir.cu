@@ -6,6 +6,8 @@
 // system by system, with that system's own norms), solves A d = r with the FP32 factor and updates x += d in FP64.
 // A is held as full symmetric CSR in the original ordering; its values are
 // gathered from the lower-triangle input on every DistributeMatrix.
+#include <type_traits>
+
 #include "kernels.cuh"
 
 namespace spb {
@@ -30,23 +32,6 @@ __device__ __forceinline__ void atomic_max_nonneg(double* addr, double v) {
   atomicMax(reinterpret_cast<unsigned long long*>(addr), (unsigned long long)__double_as_longlong(v));
 }
 
-// r = b - A x, one warp per row and right-hand side column.
-__global__ void k_residual(const int64_t* __restrict__ rowptr, const int32_t* __restrict__ col,
-                           const double* __restrict__ val, const double* __restrict__ x, const double* __restrict__ b,
-                           double* __restrict__ r, int n, int nrhs, int64_t ld) {
-  const int lane = threadIdx.x & 31;
-  const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-  for (int64_t w = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5); w < (int64_t)n * nrhs; w += warps) {
-    const int c = (int)(w / n), i = (int)(w - (int64_t)c * n);
-    const double* xc = x + c * ld;
-    double s = 0.0;
-    for (int64_t p = rowptr[i] + lane; p < rowptr[i + 1]; p += 32) s = fma(val[p], xc[col[p]], s);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (lane == 0) r[i + c * ld] = b[i + c * ld] - s;
-  }
-}
-
 // Per-system maxima.  Rows are grouped into systems (segments) given by
 // rowseg[i] (nullptr: one system); out[seg * 64 + c] = max |v[i + c*ld]| over
 // the rows i of that system.  Each CTA takes a contiguous chunk of rows, each
@@ -67,11 +52,12 @@ __device__ __forceinline__ void flush_segmax(double* out, int seg, double m) {
   }
 }
 
-__global__ void k_segmax(const double* __restrict__ v, int n, int nrhs, int64_t ld, const int32_t* __restrict__ rowseg,
+__global__ void k_segmax(const double* __restrict__ v, int n, int64_t ld, const int32_t* __restrict__ rowseg,
                          double* __restrict__ out) {
   const int64_t r0 = (int64_t)blockIdx.x * kChunk;
   const int64_t r1 = min((int64_t)n, r0 + kChunk);
-  for (int c = 0; c < nrhs; ++c) {
+  {
+    const int c = blockIdx.y;
     int seg = -1;
     double m = 0.0;
     for (int64_t i = r0 + threadIdx.x; i < r1; i += blockDim.x) {
@@ -84,6 +70,99 @@ __global__ void k_segmax(const double* __restrict__ v, int n, int nrhs, int64_t 
       m = fmax(m, fabs(v[i + c * ld]));
     }
     flush_segmax(out + c, seg, m);
+  }
+}
+
+// One refinement step's view of the current x: r = b - A x, stored permuted (R[invp[i] + c n],
+// the right-hand side of the correction solve), with max |x| and max |r| per system and
+// column (xmax, rmax; layout as in k_segmax) taken on the way.  Bound by the reads of A: four
+// lanes share a row, so that a load of val takes whole sectors, and CB columns share each
+// entry of A, so that A is read ceil(nrhs / CB) times.  A block takes a contiguous run of rows
+// and keeps its maxima in registers to the end of the run (or of a system).  27-point 36^3, 50
+// columns: the warp-per-entry kernel and the two passes for the maxima took 0.73 ms a step.
+constexpr int kResThreads = 256;
+template <int CB>
+__global__ void __launch_bounds__(kResThreads) k_residual(const int64_t* __restrict__ rowptr, const int32_t* __restrict__ col,
+                                                          const double* __restrict__ val, const double* __restrict__ x,
+                                                          int64_t ldx, const double* __restrict__ b, int64_t ldb,
+                                                          double* __restrict__ R, const int32_t* __restrict__ invp0,
+                                                          int n, int nrhs, const int32_t* __restrict__ rowseg,
+                                                          double* __restrict__ xmax, double* __restrict__ rmax) {
+  __shared__ unsigned long long smax[2][CB];
+  const int c0 = blockIdx.y * CB, nc = min(CB, nrhs - c0), q = threadIdx.x & 3;
+  if (threadIdx.x < 2 * CB) smax[threadIdx.x / CB][threadIdx.x % CB] = 0;
+  __syncthreads();
+  const int64_t chunk = ((n + gridDim.x - 1) / gridDim.x + 63) / 64 * 64;
+  const int64_t r0 = blockIdx.x * chunk, r1 = min((int64_t)n, r0 + chunk);
+  double mr[CB], mx[CB];
+#pragma unroll
+  for (int c = 0; c < CB; ++c) mr[c] = mx[c] = 0.0;
+  int seg = -1;
+  for (int64_t base = r0; base < r1; base += kResThreads / 4) {
+    const int64_t i = base + (threadIdx.x >> 2);
+    const bool in = i < r1;
+    double s[CB];
+#pragma unroll
+    for (int c = 0; c < CB; ++c) s[c] = 0.0;
+    if (in) {
+      const int64_t p1 = rowptr[i + 1];
+      for (int64_t p = rowptr[i] + q; p < p1; p += 4) {
+        const double v = val[p];
+        const double* xj = x + col[p] + c0 * ldx;
+#pragma unroll
+        for (int c = 0; c < CB; ++c)
+          if (c < nc) s[c] = fma(v, xj[c * ldx], s[c]);
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < CB; ++c) {
+      s[c] += __shfl_xor_sync(0xffffffffu, s[c], 1);
+      s[c] += __shfl_xor_sync(0xffffffffu, s[c], 2);
+    }
+    if (!in) continue;
+    if (rowseg && rowseg[i] != seg) {
+      if (seg >= 0) {
+#pragma unroll
+        for (int c = 0; c < CB; ++c) {
+          if ((c & 3) != q || c >= nc) continue;
+          atomic_max_nonneg(rmax + seg * 64 + c0 + c, mr[c]);
+          atomic_max_nonneg(xmax + seg * 64 + c0 + c, mx[c]);
+          mr[c] = mx[c] = 0.0;
+        }
+      }
+      seg = rowseg[i];
+    }
+    const int64_t pr = invp0[i];
+#pragma unroll
+    for (int c = 0; c < CB; ++c) {
+      if ((c & 3) != q || c >= nc) continue;
+      const double r = b[i + (c0 + c) * ldb] - s[c];
+      R[pr + (int64_t)(c0 + c) * n] = r;
+      mr[c] = fmax(mr[c], fabs(r));
+      mx[c] = fmax(mx[c], fabs(x[i + (c0 + c) * ldx]));
+    }
+  }
+  if (rowseg) {
+    if (seg >= 0) {
+#pragma unroll
+      for (int c = 0; c < CB; ++c) {
+        if ((c & 3) != q || c >= nc) continue;
+        atomic_max_nonneg(rmax + seg * 64 + c0 + c, mr[c]);
+        atomic_max_nonneg(xmax + seg * 64 + c0 + c, mx[c]);
+      }
+    }
+    return;
+  }
+#pragma unroll
+  for (int c = 0; c < CB; ++c) {
+    if ((c & 3) != q || c >= nc) continue;
+    atomicMax(&smax[0][c], (unsigned long long)__double_as_longlong(mr[c]));
+    atomicMax(&smax[1][c], (unsigned long long)__double_as_longlong(mx[c]));
+  }
+  __syncthreads();
+  if (threadIdx.x < nc) {
+    atomicMax(reinterpret_cast<unsigned long long*>(rmax + c0 + threadIdx.x), smax[0][threadIdx.x]);
+    atomicMax(reinterpret_cast<unsigned long long*>(xmax + c0 + threadIdx.x), smax[1][threadIdx.x]);
   }
 }
 
@@ -133,14 +212,6 @@ __global__ void k_eta(const double* __restrict__ anorm, const double* __restrict
   if ((threadIdx.x & 31) == 0) atomic_max_nonneg(eta, e);
 }
 
-__global__ void k_axpy(double* __restrict__ x, const double* __restrict__ d, int n, int nrhs, int64_t ld) {
-  const int64_t total = (int64_t)n * nrhs;
-  for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < total; k += (int64_t)gridDim.x * blockDim.x) {
-    const int c = (int)(k / n), i = (int)(k - (int64_t)c * n);
-    x[i + c * ld] += d[i + c * ld];
-  }
-}
-
 }  // namespace
 
 void launch_gather(cudaStream_t st, double* dst, const double* src, const int64_t* idx, int64_t n) {
@@ -148,13 +219,22 @@ void launch_gather(cudaStream_t st, double* dst, const double* src, const int64_
 }
 
 void launch_residual(cudaStream_t st, const int64_t* rowptr, const int32_t* col, const double* val, const double* x,
-                     const double* b, double* r, int n, int nrhs, int64_t ld) {
-  k_residual<<<grid_for((int64_t)n * nrhs * 32, 256), 256, 0, st>>>(rowptr, col, val, x, b, r, n, nrhs, ld);
+                     int64_t ldx, const double* b, int64_t ldb, double* R, const int32_t* invp0, int n, int nrhs,
+                     const int32_t* rowseg, double* xmax, double* rmax) {
+  auto run = [&](auto cb) {
+    constexpr int CB = decltype(cb)::value;
+    const int by = (nrhs + CB - 1) / CB, rows = (n + 63) / 64, cap = (148 * 8 + by - 1) / by;
+    k_residual<CB><<<dim3(rows < cap ? rows : cap, by), kResThreads, 0, st>>>(rowptr, col, val, x, ldx, b, ldb, R, invp0,
+                                                                              n, nrhs, rowseg, xmax, rmax);
+  };
+  if (nrhs == 1) run(std::integral_constant<int, 1>());
+  else if (nrhs <= 4) run(std::integral_constant<int, 4>());
+  else run(std::integral_constant<int, 8>());
 }
 
 void launch_segmax(cudaStream_t st, const double* v, int n, int nrhs, int64_t ld, const int32_t* rowseg,
                    double* out) {
-  k_segmax<<<(n + kChunk - 1) / kChunk, 256, 0, st>>>(v, n, nrhs, ld, rowseg, out);
+  k_segmax<<<dim3((n + kChunk - 1) / kChunk, nrhs), 256, 0, st>>>(v, n, ld, rowseg, out);
 }
 
 void launch_rowsum_segmax(cudaStream_t st, const int64_t* rowptr, const double* val, int n, const int32_t* rowseg,
@@ -165,10 +245,6 @@ void launch_rowsum_segmax(cudaStream_t st, const int64_t* rowptr, const double* 
 void launch_eta(cudaStream_t st, const double* anorm, const double* bmax, const double* xmax, const double* rmax,
                 int nseg, int nrhs, double* eta) {
   k_eta<<<grid_for((int64_t)nseg * nrhs, 256), 256, 0, st>>>(anorm, bmax, xmax, rmax, nseg, nrhs, eta);
-}
-
-void launch_axpy(cudaStream_t st, double* x, const double* d, int n, int nrhs, int64_t ld) {
-  k_axpy<<<grid_for((int64_t)n * nrhs, 256), 256, 0, st>>>(x, d, n, nrhs, ld);
 }
 
 }  // namespace dev

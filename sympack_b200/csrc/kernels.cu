@@ -67,12 +67,14 @@ __global__ void k_permute_in(double* X, int64_t ldx, const double* B, int64_t ld
   }
 }
 
+template <bool kAdd>
 __global__ void k_permute_out(double* B, int64_t ldb, const double* X, int64_t ldx, const int32_t* invp0, int n,
                               int nrhs) {
   int64_t total = (int64_t)n * nrhs;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
     int c = (int)(i / n), r = (int)(i - (int64_t)c * n);
-    B[r + c * ldb] = X[invp0[r] + c * ldx];
+    if (kAdd) B[r + c * ldb] += X[invp0[r] + c * ldx];
+    else B[r + c * ldb] = X[invp0[r] + c * ldx];
   }
 }
 
@@ -129,7 +131,12 @@ void launch_permute_in(cudaStream_t st, double* X, int64_t ldx, const double* B,
 
 void launch_permute_out(cudaStream_t st, double* B, int64_t ldb, const double* X, int64_t ldx,
                         const int32_t* invp0, int n, int nrhs) {
-  k_permute_out<<<grid_for((int64_t)n * nrhs, 256), 256, 0, st>>>(B, ldb, X, ldx, invp0, n, nrhs);
+  k_permute_out<false><<<grid_for((int64_t)n * nrhs, 256), 256, 0, st>>>(B, ldb, X, ldx, invp0, n, nrhs);
+}
+
+void launch_permute_add(cudaStream_t st, double* B, int64_t ldb, const double* X, int64_t ldx,
+                        const int32_t* invp0, int n, int nrhs) {
+  k_permute_out<true><<<grid_for((int64_t)n * nrhs, 256), 256, 0, st>>>(B, ldb, X, ldx, invp0, n, nrhs);
 }
 
 }  // namespace dev

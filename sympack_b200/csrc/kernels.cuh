@@ -125,23 +125,25 @@ void launch_sb_inverse(cudaStream_t st, const void* L, void* Inv, bool fp32, con
 void launch_diag_inverse(cudaStream_t st, const void* L, double* Inv, bool fp32, const Inv1Item* items, int narrow,
                          int count);
 
-// Precision form (FP64 refinement): gather CSR values, residual r = b - A x,
-// per-column max |v| (out zeroed by the caller), max row sum of |A|, x += d.
+// Precision form (FP64 refinement): gather CSR values, permuted residual R of b - A x with
+// per-system, per-column max |x| and max |r| (zeroed by the caller), max |v|, max row sum of |A|.
 void launch_gather(cudaStream_t st, double* dst, const double* src, const int64_t* idx, int64_t n);
 void launch_residual(cudaStream_t st, const int64_t* rowptr, const int32_t* col, const double* val, const double* x,
-                     const double* b, double* r, int n, int nrhs, int64_t ld);
+                     int64_t ldx, const double* b, int64_t ldb, double* R, const int32_t* invp0, int n, int nrhs,
+                     const int32_t* rowseg, double* xmax, double* rmax);
 void launch_segmax(cudaStream_t st, const double* v, int n, int nrhs, int64_t ld, const int32_t* rowseg,
                    double* out);
 void launch_rowsum_segmax(cudaStream_t st, const int64_t* rowptr, const double* val, int n, const int32_t* rowseg,
                           double* anorm);
 void launch_eta(cudaStream_t st, const double* anorm, const double* bmax, const double* xmax, const double* rmax,
                 int nseg, int nrhs, double* eta);
-void launch_axpy(cudaStream_t st, double* x, const double* d, int n, int nrhs, int64_t ld);
 
-// X[invp[i], c] = B[i, c]   and   B[i, c] = X[invp[i], c]
+// X[invp[i], c] = B[i, c],   B[i, c] = X[invp[i], c]   and   B[i, c] += X[invp[i], c]
 void launch_permute_in(cudaStream_t st, double* X, int64_t ldx, const double* B, int64_t ldb,
                        const int32_t* invp0, int n, int nrhs);
 void launch_permute_out(cudaStream_t st, double* B, int64_t ldb, const double* X, int64_t ldx,
+                        const int32_t* invp0, int n, int nrhs);
+void launch_permute_add(cudaStream_t st, double* B, int64_t ldb, const double* X, int64_t ldx,
                         const int32_t* invp0, int n, int nrhs);
 
 }  // namespace dev

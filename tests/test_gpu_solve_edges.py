@@ -1,8 +1,8 @@
 """Solve sweeps at the edges of their task shapes: one-block supernodes of every width class
 (a warp's 16 columns, 32, 64) over off-diagonal parts below and above what a warp and the
 staged row list hold, right-hand-side counts around the 8-column fragments, the 16-column
-groups and the 64-column passes, and tasks of one and of several tile pairs, in FP64 and
-LDL^T.  Answers agree with the CPU oracle's substitution to 1e-12 (the
+groups and the 64-column passes, and tasks of one and of several tile pairs, in FP64, LDL^T
+and FP32 + refinement.  FP64 answers agree with the CPU oracle's substitution to 1e-12 (the
 other GPU tests' bound: the matrices are diagonally dominant, condition below 1e3, so
 rounding differences stay near 1e-14)."""
 import os
@@ -75,4 +75,31 @@ def test_one_block_supernodes_match_the_oracle(dec, border, tiles):
         M.Solve(b)
         x, xo = M.GetSolution(nrhs=nrhs), f.solve(b)
         assert np.max(np.abs(x - xo)) <= TOL * np.max(np.abs(xo)), nrhs
+    M.close()
+
+
+@pytest.mark.parametrize("border", [65, 530])
+def test_refined_solves_with_a_padded_leading_dimension(border):
+    """FP32 + refinement through device pointers whose leading dimension exceeds n."""
+    import torch
+    A = DistSparseMatrix.from_lower_csc(*bordered(WIDTHS, border, 3))
+    M = solver(A, precision="FP32_IR")
+    n, ld = A.size, A.size + 13
+    for nrhs in (1, 4, 5, 20, 70):
+        b = torch.full((nrhs, ld), float("nan"), dtype=torch.float64, device="cuda")
+        b[:, :n] = torch.from_numpy(np.random.default_rng(nrhs).standard_normal((nrhs, n)))
+        x = torch.full_like(b, 7.0)
+        torch.cuda.synchronize()
+        M.SolveDevice(b.data_ptr(), x.data_ptr(), nrhs, ld)
+        assert M.info().backward_error <= 1e-12
+        xh, bh = x.cpu().numpy(), b.cpu().numpy()
+        assert np.all(xh[:, n:] == 7.0)
+        r = A.matvec(np.ascontiguousarray(xh[:, :n].T)) - bh[:, :n].T
+        s = np.zeros(n)  # row sums of |A|
+        np.add.at(s, A.rowind - 1, np.abs(A.nzvalLocal))
+        cols = np.repeat(np.arange(n), np.diff(A.colptr))
+        off = A.rowind - 1 != cols
+        np.add.at(s, cols[off], np.abs(A.nzvalLocal[off]))
+        eta = np.max(np.abs(r), axis=0) / (s.max() * np.max(np.abs(xh[:, :n]), axis=1) + np.max(np.abs(bh[:, :n]), axis=1))
+        assert eta.max() <= 1.01e-12
     M.close()
