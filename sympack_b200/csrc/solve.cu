@@ -772,6 +772,7 @@ __global__ void __launch_bounds__(kThreads, solve_min_blocks<T, NG>()) k_solve(P
 }
 
 // ---- diagonal super-block inverses ---------------------------------------------------
+// Super-blocks of more than kStripBlocks blocks, whose strips do not fit in shared memory.
 // One CTA per (super-block p, column block j): the tiles Inv(i, j), i = j .. nb - 1, of
 // Inv_p = L_pp^-1 by block substitution down column j:
 //   Inv(j, j) = L_jj^-1,   Inv(i, j) = -L_ii^-1 sum_{k=j}^{i-1} L_ik Inv(k, j),
@@ -883,6 +884,140 @@ __global__ void __launch_bounds__(kInvThreads, 2) k_sb_inverse(const T* __restri
   }
 }
 
+// ---- super-blocks of at most kStripBlocks blocks: strips of 16 columns ------------------
+// A CTA takes 16 columns of column block j of Inv_p and carries them, transposed (16 rows),
+// through the block rows i = j .. nb - 1 in shared memory:
+//   R_i = (E_i - sum_{k=j}^{i-1} R_k L_ik^T) L_ii^-T.
+// The sums run on the FP64 tensor pipe, warp v taking rows 8v .. of block i, its fragments of
+// L_ik loaded straight from the panel one tile ahead; the triangular solve is one warp's, by
+// 8-column pieces as the panel TRSM's.  Bound by that chain, 28 tile products and 8 solves for
+// the first column of a full super-block; four strips share a column block so that a product
+// takes a quarter of the time, and all CTAs of a launch are independent.  The one-CTA-per-
+// column kernel above (products with scalar FMAs, every tile re-read through L2, a 64-step
+// inverse per tile) took 0.58 ms on the 60^3 Laplacian and about 0.45 ms on any matrix with
+// one full super-block.
+constexpr int kStripBlocks = 16;
+constexpr int kXs = 16;  // X[k][m] at k * 16 + (m ^ 4 (k & 3)): conflict-free fragment reads
+__host__ __device__ constexpr size_t strip_smem(int nb) {
+  return ((size_t)nb * kT * kXs + kT * 68 + kT) * sizeof(double);
+}
+__device__ __forceinline__ int xs(int k, int m) { return k * kXs + (m ^ (4 * (k & 3))); }
+
+template <class T>
+__global__ void __launch_bounds__(256, 2) k_sb_inverse_strips(const T* __restrict__ L, T* __restrict__ Inv,
+                                                              const SnMeta* __restrict__ meta,
+                                                              const InvItem* __restrict__ items, int sb) {
+  constexpr int kLd = 68;
+  extern __shared__ __align__(16) double smx[];
+  const InvItem it = items[blockIdx.x >> 2];
+  const int col0 = (blockIdx.x & 3) * 16;
+  const SnMeta m = meta[it.s];
+  const int nblk = (m.w + kT - 1) / kT, b0 = it.p * sb, nb = min(sb, nblk - b0), j = it.j;
+  double* D = smx;
+  double* Rinv = D + kT * kLd;
+  double* X = Rinv + kT;
+  T* base = Inv + m.ioff + (int64_t)it.p * ((int64_t)sb * (sb + 1) / 2) * (kT * kT);
+  const T* P = L + m.off;
+  const int64_t ld = m.ld;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+  for (int i = j; i < nb; ++i) {
+    const int ci = (b0 + i) * kT, bi = min(kT, m.w - ci);
+    // L_ii, identity beyond bi
+    T dv[16];
+#pragma unroll
+    for (int q = 0; q < 16; ++q) {
+      const int idx = tid + q * 256, c = idx >> 6, r = idx & 63;
+      dv[q] = r < bi && c <= r ? P[ci + r + (int64_t)(ci + c) * ld] : T(r == c ? 1 : 0);
+    }
+    const T* row = P + ci + 8 * warp + g + (int64_t)(b0 + j) * kT * ld;
+    const bool ok = 8 * warp + g < bi;
+    double acc[2][4] = {};
+    T f[16];
+    auto load = [&](int k) {
+#pragma unroll
+      for (int q = 0; q < 16; ++q) f[q] = ok ? row[(int64_t)((k - j) * kT + 4 * q + t) * ld] : T(0);
+    };
+    if (i > j) load(j);
+    for (int k = j; k < i; ++k) {
+      double b[16];
+#pragma unroll
+      for (int q = 0; q < 16; ++q) b[q] = (double)f[q];
+      if (k + 1 < i) load(k + 1);
+      const int k0 = (k - j) * kT;
+#pragma unroll
+      for (int q = 0; q < 16; ++q) {
+        const int kk = k0 + 4 * q + t;
+        dmma(acc[q & 1], X[xs(kk, g)], X[xs(kk, g + 8)], b[q]);
+      }
+    }
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int n = 8 * warp + 2 * t + (e & 1), mm = g + 8 * (e >> 1);
+      X[xs((i - j) * kT + n, mm)] = (i == j && n < bi && n == col0 + mm ? 1.0 : 0.0) - acc[0][e] - acc[1][e];
+    }
+#pragma unroll
+    for (int q = 0; q < 16; ++q) {
+      const int idx = tid + q * 256, c = idx >> 6, r = idx & 63;
+      D[r + c * kLd] = (double)dv[q];
+      if (r == c) Rinv[r] = 1.0 / (double)dv[q];
+    }
+    __syncthreads();
+    if (warp == 0) {
+      double* R = X + (i - j) * kT * kXs;  // xs() of whole 4-row groups: local rows count alike
+      double v[8][4];
+#pragma unroll
+      for (int n = 0; n < 8; ++n)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) v[n][e] = R[xs(8 * n + 2 * t + (e & 1), g + 8 * (e >> 1))];
+      const int mm = lane & 15;
+#pragma unroll 1
+      for (int p = 0; p < 8; ++p) {  // v[n] holds column tile p + n
+        const int kb = 8 * p;
+        if (p > 0) {
+#pragma unroll
+          for (int e = 0; e < 4; ++e) R[xs(kb + 2 * t + (e & 1), g + 8 * (e >> 1))] = v[0][e];
+          __syncwarp();
+        }
+        double x[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) x[q] = R[xs(kb + q, mm)];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          x[q] *= Rinv[kb + q];
+#pragma unroll
+          for (int k = q + 1; k < 8; ++k) x[k] = fma(-x[q], D[kb + k + (kb + q) * kLd], x[k]);
+          if (q & 1) asm volatile("" ::: "memory");
+        }
+        __syncwarp();
+        if (lane < 16) {
+#pragma unroll
+          for (int q = 0; q < 8; ++q) R[xs(kb + q, mm)] = x[q];
+        }
+        __syncwarp();
+        const double a0 = -R[xs(kb + t, g)], a1 = -R[xs(kb + t, g + 8)];
+        const double a2 = -R[xs(kb + 4 + t, g)], a3 = -R[xs(kb + 4 + t, g + 8)];
+        const double* b = D + g + kb + 8 + (kb + t) * kLd;
+#pragma unroll
+        for (int n = 1; n < 8; ++n) {
+          if (p + n < 8) {
+            dmma(v[n], a0, a1, b[8 * (n - 1)]);
+            dmma(v[n], a2, a3, b[8 * (n - 1) + 4 * kLd]);
+          }
+#pragma unroll
+          for (int e = 0; e < 4; ++e) v[n - 1][e] = v[n][e];
+        }
+      }
+    }
+    __syncthreads();
+    T* dst = base + ((int64_t)i * (i + 1) / 2 + j) * (kT * kT) + col0 * kT;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int idx = tid + q * 256, r = idx & 63, mm = idx >> 6;
+      dst[r + mm * kT] = (T)X[xs((i - j) * kT + r, mm)];
+    }
+  }
+}
+
 // ---- inverses of one-block supernodes' diagonal blocks ------------------------------------
 // One warp per block of at most 32 columns (kW = 32) or one block of 64 threads per wider one:
 // thread c substitutes down column c, x_i = (delta_ic - sum_{k<i} L_ik x_k) / L_ii, the block
@@ -968,6 +1103,8 @@ void init_solve_attributes() {
   init_sweeps<double, 2>(0, sms);
   init_sweeps<float, 1>(1, sms);
   init_sweeps<float, 2>(1, sms);
+  cudaFuncSetAttribute(k_sb_inverse_strips<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)strip_smem(kStripBlocks));
+  cudaFuncSetAttribute(k_sb_inverse_strips<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)strip_smem(kStripBlocks));
   cudaFuncSetAttribute(k_sb_inverse<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kInvSmem);
   cudaFuncSetAttribute(k_sb_inverse<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kInvSmem);
   cudaFuncSetAttribute(k_diag_inverse<double, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDiagInvSmem32);
@@ -979,6 +1116,15 @@ void init_solve_attributes() {
 void launch_sb_inverse(cudaStream_t st, const void* L, void* Inv, bool fp32, const SnMeta* meta,
                        const InvItem* items, int count, int sb) {
   if (count <= 0) return;
+  if (sb <= kStripBlocks) {
+    if (fp32)
+      k_sb_inverse_strips<float><<<4 * count, 256, strip_smem(sb), st>>>(static_cast<const float*>(L),
+                                                                         static_cast<float*>(Inv), meta, items, sb);
+    else
+      k_sb_inverse_strips<double><<<4 * count, 256, strip_smem(sb), st>>>(static_cast<const double*>(L),
+                                                                          static_cast<double*>(Inv), meta, items, sb);
+    return;
+  }
   if (fp32)
     k_sb_inverse<float><<<count, kInvThreads, kInvSmem, st>>>(static_cast<const float*>(L), static_cast<float*>(Inv),
                                                               meta, items, sb);
