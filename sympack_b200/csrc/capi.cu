@@ -208,6 +208,7 @@ spb::dev::FactorArgs factor_args(spb_handle* h) {
   a.groups = h->dgroups;
   a.rel = h->drel;
   a.fp32 = h->fp32;
+  a.big_rows = h->plan.big_tile_rows;
   a.engine = h->opt.fp32_engine;
   a.split = h->dsplit;
   a.split_off = h->dsplit_off;

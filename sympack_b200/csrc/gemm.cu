@@ -45,7 +45,7 @@ template <int BM, int BN, int NT, class T, class CT>
 __device__ void tile_epilogue(const FactorArgs& a, const TileItem& it, const SnMeta& m, const CT* Cs, int ldc,
                               int64_t* Cbase, int64_t* Crel) {
   static_assert(NT % BM == 0, "one row per thread");
-  const int tid = threadIdx.x, i = tid % BM, c0 = tid / BM;
+  const int tid = ftask::thread_id(), i = tid % BM, c0 = tid / BM;
   constexpr int kStep = NT / BM;
   T* L = static_cast<T*>(a.L);
   const int jr = it.a_row0 + i;
@@ -179,22 +179,22 @@ __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void* src, uint32_t
 // Stage barriers of the DMMA tile, kept across the tiles a persistent CTA runs: g counts the
 // stages this CTA has consumed, so stage q of its life uses buffer q % kDStages and phase
 // (q / kDStages) & 1 of that buffer's barriers.
+// The barriers sit above the stages: full[i], copies landed (one arrival with the byte count
+// + transaction bytes), then empty[i], read by all 8 warps.
 struct DmPipe {
-  uint64_t* full;   // copies landed: one arrival (with the byte count) + transaction bytes
-  uint64_t* empty;  // read by all 8 warps
   uint32_t g;
 };
 
 template <int BN>
 __device__ __forceinline__ void dm_setup(DmPipe& P, unsigned char* smem_raw) {
   using D = DTile<BN>;
-  P.full = reinterpret_cast<uint64_t*>(smem_raw + D::kMainBytes + D::kIntsBytes);
-  P.empty = P.full + kDStages;
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem_raw + D::kMainBytes + D::kIntsBytes);
+  uint64_t* empty = full + kDStages;
   P.g = 0;
   if (threadIdx.x == 0) {
     for (int i = 0; i < kDStages; ++i) {
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(P.full + i)) : "memory");
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(P.empty + i)), "r"(kDThreads / 32)
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(full + i)) : "memory");
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(empty + i)), "r"(kDThreads / 32)
                    : "memory");
     }
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
@@ -212,11 +212,13 @@ __device__ bool dmma_tile_task(const FactorArgs& a, const TileItem& it, unsigned
   double* pipe = reinterpret_cast<double*>(smem_raw);
   double* Cs = reinterpret_cast<double*>(smem_raw);  // reused once the main loop is done
   int* ints = reinterpret_cast<int*>(smem_raw + D::kMainBytes);
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem_raw + D::kMainBytes + D::kIntsBytes);
+  uint64_t* empty = full + kDStages;
   const SnMeta m = a.meta[it.s];
   const double* g = static_cast<const double*>(a.L) + m.off;
   const double* gb = a.ldl ? a.W + m.off : g;  // second operand: L, or L D for LDL^T
   const int64_t ld = m.ld;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = ftask::thread_id(), lane = tid & 31, warp = tid >> 5;
   const int wm = warp % D::kWarpsM, wn = warp / D::kWarpsM;
   const int gq = lane >> 2, tq = lane & 3;
   const int a0 = it.a_row0 & ~1, b0 = it.b_row0 & ~1;
@@ -246,7 +248,7 @@ __device__ bool dmma_tile_task(const FactorArgs& a, const TileItem& it, unsigned
       if (o < kDLds) As[l * kDLds + o] = 0.0;
       else Bs[l * D::kLdb + o - kDLds] = 0.0;
     }
-    const uint32_t bar = smem_u32(P.full + q % kDStages);
+    const uint32_t bar = smem_u32(full + q % kDStages);
     __syncwarp();
     if (lane == 0)
       asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar),
@@ -274,7 +276,7 @@ __device__ bool dmma_tile_task(const FactorArgs& a, const TileItem& it, unsigned
   for (int kt = 0; kt < nk; ++kt) {
     const uint32_t q = g0 + kt;
     const int st = q % kDStages;
-    if (!mbar_wait(smem_u32(P.full + st), (q / kDStages) & 1, kDWaitLimit)) {
+    if (!mbar_wait(smem_u32(full + st), (q / kDStages) & 1, kDWaitLimit)) {
       ok = false;
       break;
     }
@@ -298,12 +300,12 @@ __device__ bool dmma_tile_task(const FactorArgs& a, const TileItem& it, unsigned
       }
     }
     __syncwarp();
-    if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(smem_u32(P.empty + st)) : "memory");
+    if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(smem_u32(empty + st)) : "memory");
     // warp 0 refills the buffer of the previous stage once every warp has read it
     const int pk = kt - 1;
     if (warp == 0 && pk >= 0 && pk + kDStages < nk) {
       const uint32_t pq = g0 + pk;
-      if (!mbar_wait(smem_u32(P.empty + pq % kDStages), (pq / kDStages) & 1, kDWaitLimit)) {
+      if (!mbar_wait(smem_u32(empty + pq % kDStages), (pq / kDStages) & 1, kDWaitLimit)) {
         ok = false;
         break;
       }
@@ -316,7 +318,7 @@ __device__ bool dmma_tile_task(const FactorArgs& a, const TileItem& it, unsigned
     if (warp == 0 && lane == 0) {  // let this CTA's copies in flight land (bounded)
       for (int kt = 0; kt < issued; ++kt) {
         const uint32_t q = g0 + kt;
-        mbar_wait(smem_u32(P.full + q % kDStages), (q / kDStages) & 1, kDWaitLimit);
+        mbar_wait(smem_u32(full + q % kDStages), (q / kDStages) & 1, kDWaitLimit);
       }
       report_status(a.status, 3, it.s, -1);
     }
@@ -356,7 +358,7 @@ constexpr size_t kSSmemBytes = kSCBytes + 4 * 64 * sizeof(int);
 
 // One 64 x 64 FMA tile (256 threads, kSSmemBytes of shared memory).
 template <class T>
-__device__ __noinline__ void simt_tile_task(const FactorArgs& a, const TileItem& it, unsigned char* smem_raw) {
+__device__ __forceinline__ void simt_tile_task(const FactorArgs& a, const TileItem& it, unsigned char* smem_raw) {
   T(*As)[64] = reinterpret_cast<T(*)[64]>(smem_raw);
   T(*Bs)[64] = reinterpret_cast<T(*)[64]>(smem_raw + 16 * 64 * sizeof(T));
   T* Cs = reinterpret_cast<T*>(smem_raw);
@@ -366,7 +368,7 @@ __device__ __noinline__ void simt_tile_task(const FactorArgs& a, const TileItem&
   // second operand: L, or L D for LDL^T (FP64 only, so W is read only when T is double)
   const T* gb = a.ldl ? reinterpret_cast<const T*>(a.W + m.off) : g;
   const int64_t ld = m.ld;
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  const int tid = ftask::thread_id(), tx = tid & 15, ty = tid >> 4;
   T acc[4][4];
 #pragma unroll
   for (int i = 0; i < 4; ++i)
@@ -1566,15 +1568,16 @@ __device__ __forceinline__ unsigned smid() {
 // The largest task body: the DMMA tile (FP64), the TMA-fed tcgen05 tile (FP32), whose
 // stages and barriers sit above every other body's shared memory (at most 96 KB).
 constexpr size_t kFSmemBytes = kDSmemBytes;  // the DMMA pipe and its barriers (above every other body's)
-static_assert(kFSmemBytes >= 96 * 1024 + DTile<kDTileN>::kIntsBytes + 2 * kDStages * sizeof(uint64_t),
-              "small panels (96 KB) stay below the DMMA stage barriers");
+// what a small-panel task may use: everything below the DMMA stage barriers
+constexpr int kFSmallCap = (int)((kFSmemBytes - 2 * kDStages * sizeof(uint64_t)) / sizeof(double));
+static_assert(kFSmallCap >= 96 * 1024 / 8 + ftask::kSmallHeadDoubles, "small panels (96 KB) fit");
 constexpr size_t kFSmemBytes32 = kVSmemBytes;
-static_assert(kFSmemBytes32 >= 96 * 1024 + 1024, "FP32 persistent shared memory");
+static_assert(kFSmemBytes32 >= kFSmallCap * sizeof(double) + 1024, "FP32 persistent shared memory");
 
 // FP64: two CTAs per SM (128 x 64 DMMA tiles); FP32: one (the TMA-fed tile's 193 KB).
-template <class T>
+template <class T, bool kLdl>
 __global__ void __launch_bounds__(256, std::is_same<T, float>::value ? 1 : 2)
-    k_factor_persistent(FactorArgs a, FactorSched f) {
+    k_factor_persistent(const __grid_constant__ FactorArgs a, const __grid_constant__ FactorSched f) {
   constexpr bool kF32 = std::is_same<T, float>::value;
   extern __shared__ __align__(16) unsigned char smem_f[];
   __shared__ int sh_task, sh_go;
@@ -1621,11 +1624,10 @@ __global__ void __launch_bounds__(256, std::is_same<T, float>::value ? 1 : 2)
     const FTask t = f.tasks[tk];
     switch (t.kind) {
       case 0:
-        ftask::factor_small_task<T>(a, f.small_items[t.item], reinterpret_cast<double*>(smem_f));
+        ftask::factor_small_task<T, kLdl>(a, f.small_items[t.item], reinterpret_cast<double*>(smem_f), kFSmallCap);
         break;
       case 1:
-        if (!kF32 && a.ldl) ftask::ldl_diag_task<T>(a, f.panel[t.item], f.winv, reinterpret_cast<double*>(smem_f));
-        else ftask::potrf_diag_task<T>(a, f.panel[t.item], f.winv, reinterpret_cast<double*>(smem_f));
+        ftask::diag_task<T, kLdl>(a, f.panel[t.item], f.winv, reinterpret_cast<double*>(smem_f));
         break;
       case 2:
         ftask::trsm_rows_task<T>(a, f.panel[t.item], f.winv, reinterpret_cast<double*>(smem_f));
@@ -1653,8 +1655,9 @@ void launch_factor_persistent(cudaStream_t st, const FactorArgs& a, const Factor
   // so the grid size is a matter of speed, not of progress)
   const int fit = (a.fp32 ? g_fper32 : g_fper64) * g_sms;
   const int grid = fit < f.ntasks ? fit : f.ntasks;
-  if (a.fp32) k_factor_persistent<float><<<grid, 256, kFSmemBytes32, st>>>(a, f);
-  else k_factor_persistent<double><<<grid, 256, kFSmemBytes, st>>>(a, f);
+  if (a.fp32) k_factor_persistent<float, false><<<grid, 256, kFSmemBytes32, st>>>(a, f);
+  else if (a.ldl) k_factor_persistent<double, true><<<grid, 256, kFSmemBytes, st>>>(a, f);
+  else k_factor_persistent<double, false><<<grid, 256, kFSmemBytes, st>>>(a, f);
 }
 
 void init_gemm_attributes() {
@@ -1666,14 +1669,15 @@ void init_gemm_attributes() {
   cudaFuncSetAttribute(k_gemm_tc32w, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWSmemBytes);
   cudaFuncSetAttribute(k_gemm_tc32p, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPSmemBytes);
   cudaFuncSetAttribute(k_gemm_dmma, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDSmemBytes);
-  cudaFuncSetAttribute(k_factor_persistent<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFSmemBytes);
-  cudaFuncSetAttribute(k_factor_persistent<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFSmemBytes32);
+  cudaFuncSetAttribute(k_factor_persistent<double, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFSmemBytes);
+  cudaFuncSetAttribute(k_factor_persistent<double, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFSmemBytes);
+  cudaFuncSetAttribute(k_factor_persistent<float, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFSmemBytes32);
   int nb = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_factor_persistent<double>, 256, kFSmemBytes) ==
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_factor_persistent<double, true>, 256, kFSmemBytes) ==
           cudaSuccess &&
       nb > 0)
     g_fper64 = nb;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_factor_persistent<float>, 256, kFSmemBytes32) ==
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_factor_persistent<float, false>, 256, kFSmemBytes32) ==
           cudaSuccess &&
       nb > 0)
     g_fper32 = nb;

@@ -31,24 +31,24 @@ __global__ void k_assemble(T* __restrict__ L, const int64_t* __restrict__ dst, c
     L[dst[i]] = (T)vals[i];
 }
 
-template <class T>
-__global__ void __launch_bounds__(128) k_factor_small(FactorArgs a, const int32_t* __restrict__ items) {
+template <class T, bool kLdl>
+__global__ void __launch_bounds__(kThreads) k_factor_small(FactorArgs a, const int32_t* __restrict__ items, int cap) {
   extern __shared__ double sm_small[];
-  factor_small_task<T>(a, items[blockIdx.x], sm_small);
+  factor_small_task<T, kLdl>(a, items[blockIdx.x], sm_small, cap);
 }
 
 template <class T>
 __global__ void __launch_bounds__(kThreads, 1) k_potrf_diag(FactorArgs a, const PanelItem* __restrict__ items,
                                                          double* __restrict__ winv) {
   extern __shared__ double sm_diag[];
-  potrf_diag_task<T>(a, items[blockIdx.x], winv, sm_diag);
+  diag_task<T, false>(a, items[blockIdx.x], winv, sm_diag);
 }
 
 template <class T>
 __global__ void __launch_bounds__(kThreads, 1) k_ldl_diag(FactorArgs a, const PanelItem* __restrict__ items,
                                                        double* __restrict__ winv) {
   extern __shared__ double sm_ldl[];
-  ldl_diag_task<T>(a, items[blockIdx.x], winv, sm_ldl);
+  diag_task<T, true>(a, items[blockIdx.x], winv, sm_ldl);
 }
 
 template <class T>
@@ -78,6 +78,9 @@ __global__ void k_permute_out(double* B, int64_t ldb, const double* X, int64_t l
   }
 }
 
+// shared memory of the largest small panel (96 KB) and what its task keeps before it
+constexpr int kSmallSmemMax = 96 * 1024 + kSmallHeadDoubles * 8;
+
 int grid_for(int64_t work, int threads) {
   int64_t g = (work + threads - 1) / threads;
   if (g > 148 * 16) g = 148 * 16;
@@ -94,8 +97,9 @@ void launch_assemble(cudaStream_t st, double* L, const int64_t* dst, const doubl
 void init_kernel_attributes() {
   for (auto f : {k_trsm_rows<double>, k_trsm_rows<float>})
     cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, kTrsmSmemDoubles * (int)sizeof(double));
-  for (auto f : {k_factor_small<double>, k_factor_small<float>})
-    cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
+  cudaFuncSetAttribute(k_factor_small<double, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmallSmemMax);
+  cudaFuncSetAttribute(k_factor_small<double, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmallSmemMax);
+  cudaFuncSetAttribute(k_factor_small<float, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmallSmemMax);
   init_gemm_attributes();
   init_solve_attributes();
 }
@@ -106,9 +110,14 @@ void launch_assemble(cudaStream_t st, void* L, bool fp32, const int64_t* dst, co
   else k_assemble<double><<<grid_for(nnz, 256), 256, 0, st>>>(static_cast<double*>(L), dst, vals, nnz);
 }
 
-void launch_factor_small(cudaStream_t st, const FactorArgs& a, const int32_t* items, int count, int smem_bytes) {
-  if (a.fp32) k_factor_small<float><<<count, 128, smem_bytes, st>>>(a, items);
-  else k_factor_small<double><<<count, 128, smem_bytes, st>>>(a, items);
+// panel_bytes: the largest panel of the launch; with room for its padded leading dimension
+void launch_factor_small(cudaStream_t st, const FactorArgs& a, const int32_t* items, int count, int panel_bytes) {
+  int smem = panel_bytes + panel_bytes / 4 + 15 * 32 * 8 + kSmallHeadDoubles * 8;
+  if (smem > kSmallSmemMax) smem = kSmallSmemMax;
+  const int cap = smem / 8;
+  if (a.ldl) k_factor_small<double, true><<<count, kThreads, smem, st>>>(a, items, cap);
+  else if (a.fp32) k_factor_small<float, false><<<count, kThreads, smem, st>>>(a, items, cap);
+  else k_factor_small<double, false><<<count, kThreads, smem, st>>>(a, items, cap);
 }
 
 void launch_potrf_diag(cudaStream_t st, const FactorArgs& a, const PanelItem* items, int count, double* winv) {

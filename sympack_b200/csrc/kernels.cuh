@@ -27,6 +27,7 @@ struct FactorArgs {
   const RelGroup* groups;
   const int32_t* rel;        // positions of update rows in their targets' row lists
   bool fp32;                 // FP32 factor storage (precision form)
+  int big_rows;              // products with at least this many rows have tensor-core tiles of their own
   int engine;                // FP32 128 x 128 tiles: 0 tcgen05 per tile, 1 mma.sync, 2 persistent tcgen05,
                              // 3 tcgen05 fed by TMA
   // engine 3: split copies of the FP32 panels that have 128 x 128 tiles (per supernode

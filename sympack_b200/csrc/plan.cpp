@@ -21,6 +21,7 @@ Plan build_plan(const Symbolic& sym, const PlanParams& prm) {
   Plan P;
   P.n = sym.n;
   P.nsuper = sym.nsuper();
+  P.big_tile_rows = prm.big_tile_rows;
   const int ns = P.nsuper;
   P.meta.resize(ns);
   P.rows.resize(sym.lindx.size());
@@ -219,6 +220,7 @@ Plan build_plan(const Symbolic& sym, const PlanParams& prm) {
     for (int s : sns) {
       const SnMeta& m = P.meta[s];
       int rows = m.h - m.w;
+      if (!P.is_big[s] && fuses_update(m, prm.big_tile_rows)) continue;  // done by the panel's own task
       if (rows > 0) push_tiles(pick(rows), tile_of(rows), s, 1, m.w, m.h, m.w, m.h, 0, m.w);
     }
     flush_gemm(Lane::Join, 0);
@@ -293,6 +295,7 @@ Plan build_plan(const Symbolic& sym, const PlanParams& prm) {
         const SnMeta& m = P.meta[P.small_items[i]];
         double w = m.w, mm = m.h - m.w;
         f += w * w * w / 3.0 + mm * w * w;
+        if (fuses_update(m, prm.big_tile_rows)) f += mm * (mm + 1.0) * w;
       } else if (st.kind == StepKind::PotrfDiag) {
         double nb = P.panel_items[i].nb;
         f += nb * nb * nb / 3.0;
@@ -697,7 +700,18 @@ static void build_factor_dag(Plan& P, const PlanParams& prm, const std::vector<d
         r.s = s;
         sigv.push_back(SDONE + s);
         const double w = m.w, mm = m.h - m.w;
-        r.us = 2.2 + 13.0 * (w * w * w / 3.0 + mm * w * w) / 20e3;
+        r.us = 3.0 + 0.9 * ((m.w + 7) / 8) + mm * w * w / 25e3;
+        if (fuses_update(m, prm.big_tile_rows)) {  // its external update lands with the panel
+          r.us += 0.7 + mm * mm * (0.5 * w + 8.0) / 25e3;
+          for (int j = m.w, last = -1; j < m.h; ++j) {
+            const int tgt = P.groups[P.row_group[m.lidx + j]].t;
+            if (tgt != last) {
+              sigv.push_back(EXT + tgt);
+              e_ext[tgt] += 1;
+            }
+            last = tgt;
+          }
+        }
         e_sdone[s] += 1;
       } else if (st.kind == StepKind::PotrfDiag || st.kind == StepKind::TrsmRows) {
         const PanelItem& it = P.panel_items[i];

@@ -52,6 +52,16 @@ struct TileItem {
   int32_t ncols;  // valid columns in this tile (<= tile width)
 };
 
+// A small panel (factored whole in shared memory) scatters its external update itself when
+// its product has too few rows for a tensor-core tile of its own, at most kFuseRows.
+constexpr int kFuseRows = 128;
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+inline bool fuses_update(const SnMeta& m, int big_tile_rows) {
+  return m.h - m.w <= kFuseRows && m.h - m.w < big_tile_rows;
+}
+
 // One launch of the factorization sequence.
 enum class StepKind : int32_t {
   FactorSmall = 0,   // fused POTRF + TRSM of whole panels in shared memory (items = supernode ids)
@@ -70,7 +80,7 @@ struct Step {
   StepKind kind;
   int32_t begin;  // range into the matching item array
   int32_t count;
-  int32_t arg;    // PotrfDiag/TrsmRows: column block start c0; FactorSmall: shared-memory bytes
+  int32_t arg;    // PotrfDiag/TrsmRows: column block start c0; FactorSmall: largest panel (h w doubles, bytes)
   int32_t tile;   // Gemm: tile edge (64 or 128)
   Lane lane = Lane::Join;
   int32_t blk = 0;  // Chain / Side: column block index k = c0 / 64
@@ -246,6 +256,7 @@ struct Plan {
   std::vector<TileItem> tile_items;
   std::vector<Step> steps;
   int32_t max_diag_slots = 0;      // scratch slots of the diagonal blocks (one per diagonal block)
+  int32_t big_tile_rows = 128;     // PlanParams::big_tile_rows of this plan
   // persistent factorization: tasks in dispatch order (topological), their waits and signals
   std::vector<FTask> ftasks;
   std::vector<FWait> fwaits;

@@ -1,0 +1,43 @@
+"""Factorization tasks at the edges of their shapes: small panels whose width is not a multiple
+of the 8-column pieces, with off-diagonal parts around what a warp (24 rows), a block (192
+rows) and the fused external update (128 rows) take; diagonal blocks narrower than 64 and row
+tiles that end inside a warp's 16 rows; both schedules, Cholesky and LDL^T.  Factor and
+solution agree with the CPU oracle to 1e-12, the other GPU tests' bound (condition below 1e3)."""
+import numpy as np
+import pytest
+
+from sympack_b200 import DistSparseMatrix
+from test_gpu_solve_edges import bordered, oracle_for, solver
+
+pytestmark = pytest.mark.gpu
+TOL = 1e-12
+WIDTHS = [1, 7, 8, 9, 17, 24, 31, 32, 33, 40, 65, 100]
+
+
+@pytest.mark.parametrize("schedule", ["persistent", "steps"])
+@pytest.mark.parametrize("dec", ["LL", "LDL"])
+@pytest.mark.parametrize("border", [2, 15, 25, 127, 128, 129, 210, 400])
+def test_panel_tasks_match_the_oracle(border, dec, schedule):
+    A = DistSparseMatrix.from_lower_csc(*bordered(WIDTHS, border, border + 1))
+    M = solver(A, decomposition=dec, factor_schedule=schedule)
+    w = np.diff(M.GetSupernodalPartition())
+    assert set(w.tolist()) >= {7, 9, 17, 31, 33, 65}
+    f = oracle_for(M, A, dec == "LDL")
+    Lo = f.factor()
+    assert np.max(np.abs(M.GetFactor() - Lo)) <= TOL * np.max(np.abs(Lo))
+    b = np.random.default_rng(2).standard_normal((A.size, 3))
+    M.Solve(b)
+    x, xo = M.GetSolution(nrhs=3), f.solve(b)
+    assert np.max(np.abs(x - xo)) <= TOL * np.max(np.abs(xo))
+    M.close()
+
+
+@pytest.mark.parametrize("column", [0, 5, 12, 40])
+def test_a_bad_pivot_is_reported_where_it_is(column):
+    """The first non-positive pivot's column, in a piece's interior and beyond the first piece."""
+    from sympack_b200.solver import NotSPDError
+    n, cp, ri, v = bordered([60, 20], 30, 4)
+    v = v.copy()
+    v[cp[column] - 1] = -1.0  # the diagonal entry (first of its column)
+    with pytest.raises(NotSPDError, match=f"column {column + 1}$"):
+        solver(DistSparseMatrix.from_lower_csc(n, cp, ri, v))
