@@ -84,25 +84,21 @@ template <bool kLdl>
 __device__ __forceinline__ void piece_rows(double (&x)[kPiece], double (&rs)[kPiece], bool who, int valid,
                                            Status* status, int s, int col) {
   const int lane = thread_id() & 31;
+  double own = x[0];  // lane k: its pivot, kept ahead of the row's other entries
 #pragma unroll
   for (int k = 0; k < kPiece; ++k) {
-    double d = __shfl_sync(0xffffffffu, x[k], k);
+    const double d = __shfl_sync(0xffffffffu, own, k);
+    rs[k] = kLdl ? 1.0 / d : rsqrt(d);
     if (kLdl ? !(fabs(d) > 0.0) : !(d > 0.0)) {
       if (who && lane == k && k < valid) report(status, 1, s, col + k);
-      d = 1.0;
+      rs[k] = 1.0;
       if (lane == k) x[k] = 1.0;
     }
-    if constexpr (kLdl) {
-      rs[k] = 1.0 / d;
-      const double y = x[k] * rs[k];
+    const double y = x[k] * rs[k];  // the row's entry of L
+    if constexpr (!kLdl) x[k] = y;
+    if (k + 1 < kPiece) own = fma(-x[k], y, x[k + 1]);
 #pragma unroll
-      for (int j = k + 1; j < kPiece; ++j) x[j] = fma(-x[k], __shfl_sync(0xffffffffu, y, j), x[j]);
-    } else {
-      rs[k] = rsqrt(d);
-      x[k] *= rs[k];
-#pragma unroll
-      for (int j = k + 1; j < kPiece; ++j) x[j] = fma(-x[k], __shfl_sync(0xffffffffu, x[k], j), x[j]);
-    }
+    for (int j = k + 1; j < kPiece; ++j) x[j] = fma(-x[k], __shfl_sync(0xffffffffu, y, j), x[j]);
   }
 }
 
@@ -118,8 +114,8 @@ __device__ __forceinline__ void piece_rows(double (&x)[kPiece], double (&rs)[kPi
 constexpr int kSmallHeadDoubles = 64 + 2 * kFuseRows;
 
 template <class T, bool kLdl>
-__device__ __forceinline__ void factor_small_task(const FactorArgs& a, int s, double* sm, int cap) {
-  const SnMeta m = a.meta[s];
+__device__ __forceinline__ void factor_small_task(const FactorArgs& a, int s, const SnMeta& meta, double* sm, int cap) {
+  const SnMeta m = meta;
   const int h = m.h, w = m.w, M = h - w;
   double* Dk = sm;
   int64_t* cbase = reinterpret_cast<int64_t*>(sm + 64);
@@ -168,19 +164,23 @@ __device__ __forceinline__ void factor_small_task(const FactorArgs& a, int s, do
     }
     __syncthreads();  // every warp has the piece before its rows are overwritten
     if (active) {
+      // entries above the diagonal of the piece are written too; nothing reads them
       auto put = [&](const double (&v)[kPiece], int row) {
 #pragma unroll
         for (int j = 0; j < kPiece; ++j)
-          if (j < pw && row >= kb + j) {
-            if constexpr (kLdl) {
-              if (row == kb + j) Dk[row] = v[j];
-              P[row + (kb + j) * ldp] = row == kb + j ? 1.0 : v[j] * rs[j];
-            } else {
-              P[row + (kb + j) * ldp] = v[j];
-            }
-          }
+          if (j < pw) P[row + (kb + j) * ldp] = kLdl ? v[j] * rs[j] : v[j];
       };
       if (lane < kPiece ? warp == 0 && lane < pw : r < h) put(x, r);
+      if constexpr (kLdl) {
+        if (warp == 0) {
+#pragma unroll
+          for (int j = 0; j < kPiece; ++j)
+            if (lane == j && j < pw) {
+              Dk[kb + j] = x[j];
+              P[kb + j + (kb + j) * ldp] = 1.0;
+            }
+        }
+      }
       for (int r0 = kb + pw + 24 * (warp + nw); r0 < h; r0 += 24 * nw) {
         r = r0 + lane - kPiece;
         const bool in = lane >= kPiece && r < h;
@@ -283,23 +283,42 @@ constexpr int kDiagSmemDoubles = kNB * kDL + 2 * kNB + 2 * kPiece * kDL;
 // Warps 3-7 hold the block's columns as tensor-core accumulators, 8 columns a tile.  For a
 // piece the tile's warp lays its columns in shared memory, warps 0-2 factor it and solve the
 // rows below (piece_rows), then every later tile takes the solved columns off with 2 MMA
-// steps per 16 rows, the next piece's tile first.  The solving warps wait for that tile only.
+// steps per 16 rows, the next piece's tile first.  The solving warps wait for that tile only;
+// finished columns and the pieces' inverses are written out beside the next pieces.
 // The scratch slot gets the factored block (FP64) with the inverses of its 8 x 8 diagonal
 // pieces transposed into their upper triangles, 1/L_kk (1 for LDL^T, whose TRSM then computes
 // W's rows) and 1/D_kk.  LDL^T: L takes the unit block, W the block times D (its diagonal is
 // D).  A block narrower than 64 is padded with the identity.
 template <class T, bool kLdl>
-__device__ __forceinline__ void diag_task(const FactorArgs& a, const PanelItem& it, double* __restrict__ winv, double* sm) {
+__device__ __forceinline__ void diag_task(const FactorArgs& a, const PanelItem& it, const SnMeta& meta,
+                                         double* __restrict__ winv, double* sm) {
   double* D = sm;
   double* Rinv = sm + kNB * kDL;  // 1 / L_kk (LDL^T: 1)
   double* Dk = Rinv + kNB;        // LDL^T: D_kk
   double* Wp = Dk + kNB;          // LDL^T: the columns of L D of this piece and the one before, ld kDL
-  const SnMeta m = a.meta[it.s];
+  const SnMeta m = meta;
   T* gl = static_cast<T*>(a.L) + m.off;
   const int nb = it.nb, c0 = it.c0;
   const int64_t ld = m.ld;
   const int tid = thread_id(), lane = tid & 31, warp = tid >> 5;
   constexpr int kPieces = kNB / kPiece;
+  double* W = winv ? winv + (size_t)it.slot * kSlot : nullptr;
+  // inverse of piece p, lane j its column j, into the upper triangle of the scratch slot's piece
+  auto invert = [&](int p) {
+    if (!W || lane >= kPiece) return;
+    const int kb = kPiece * p;
+    double z[kPiece];
+#pragma unroll
+    for (int i = 0; i < kPiece; ++i) {
+      double v = 0.0;
+#pragma unroll
+      for (int k = 0; k < i; ++k) v = fma(D[kb + i + (kb + k) * kDL], z[k], v);  // z[k] = 0 for k < lane
+      z[i] = i < lane ? 0.0 : i == lane ? Rinv[kb + i] : -v * Rinv[kb + i];
+    }
+#pragma unroll
+    for (int i = 1; i < kPiece; ++i)
+      if (i > lane) W[kb + lane + (kb + i) * kNB] = z[i];
+  };
   // barriers: 1 the solving warps, 2 they and the next piece's owner, 3 everybody
   if (warp < 3) {
 #pragma unroll 1
@@ -313,27 +332,33 @@ __device__ __forceinline__ void diag_task(const FactorArgs& a, const PanelItem& 
 #pragma unroll
         for (int j = 0; j < kPiece; ++j) x[j] = row < kNB ? D[row + (kb + j) * kDL] : 0.0;
         piece_rows<kLdl>(x, rs, warp == 0, nb - kb, a.status, it.s, m.fc + c0 + kb);
+      } else if (warp == 2) {  // no rows left for it: the piece before's inverse
+        invert(p - 1);
       }
       asm volatile("bar.sync 1, 96;\n" ::: "memory");  // all have the piece before its rows change
-      if (active && (lane < kPiece ? warp == 0 : row < kNB)) {
+      if (active && (lane < kPiece ? warp == 0 : row < kNB)) {  // the piece's upper entries too; nothing reads them
 #pragma unroll
         for (int j = 0; j < kPiece; ++j) {
-          if (row < kb + j) continue;
-          if constexpr (kLdl) {
-            Wp[(p & 1) * kPiece * kDL + row + j * kDL] = x[j];
-            D[row + (kb + j) * kDL] = row == kb + j ? 1.0 : x[j] * rs[j];
-            if (row == kb + j) {
-              Rinv[row] = 1.0;
-              Dk[row] = x[j];
-            }
-          } else {
-            D[row + (kb + j) * kDL] = x[j];
-            if (row == kb + j) Rinv[row] = rs[j];
-          }
+          if constexpr (kLdl) Wp[(p & 1) * kPiece * kDL + row + j * kDL] = x[j];
+          D[row + (kb + j) * kDL] = kLdl ? x[j] * rs[j] : x[j];
+        }
+      }
+      if (warp == 0 && lane < kPiece) {
+        double mine = 0.0;
+#pragma unroll
+        for (int j = 0; j < kPiece; ++j)
+          if (lane == j) mine = kLdl ? x[j] : rs[j];
+        if constexpr (kLdl) {
+          Rinv[kb + lane] = 1.0;
+          Dk[kb + lane] = mine;
+          D[kb + lane + (kb + lane) * kDL] = 1.0;
+        } else {
+          Rinv[kb + lane] = mine;
         }
       }
       asm volatile("bar.sync 3, 256;\n" ::: "memory");
     }
+    if (warp == 2) invert(kPieces - 1);
   } else {
     const int g = lane >> 2, t = lane & 3;
     const T* gsrc = gl + c0 + (int64_t)c0 * ld;
@@ -393,40 +418,25 @@ __device__ __forceinline__ void diag_task(const FactorArgs& a, const PanelItem& 
           asm volatile("bar.arrive 2, 128;\n" ::: "memory");
         }
       }
+      if (warp >= 6) {  // the finished columns go out while the next piece is factored
+        const int r = 32 * (warp - 6) + lane;
+#pragma unroll
+        for (int j = 0; j < kPiece; ++j) {
+          const int c = kb + j;
+          if (r < c) continue;
+          const double l = D[r + c * kDL];
+          if (r < nb && c < nb) {
+            gl[(c0 + r) + (int64_t)(c0 + c) * ld] = (T)l;
+            if constexpr (kLdl) a.W[m.off + (c0 + r) + (int64_t)(c0 + c) * ld] = l * Dk[c];
+          }
+          if (W) W[r + c * kNB] = l;
+        }
+        if (W && (r >> 3) == p) {
+          W[kNB * kNB + r] = Rinv[r];
+          if constexpr (kLdl) W[kNB * kNB + kNB + r] = 1.0 / Dk[r];
+        }
+      }
     }
-  }
-  __syncthreads();
-  if (lane < kPiece) {  // warp p inverts piece p, lane j its column j, into the upper triangle
-    const int kb = kPiece * warp;
-    double z[kPiece];
-#pragma unroll
-    for (int i = 0; i < kPiece; ++i) {
-      double v = 0.0;
-#pragma unroll
-      for (int k = 0; k < i; ++k)
-        if (k >= lane) v = fma(D[kb + i + (kb + k) * kDL], z[k], v);
-      z[i] = i < lane ? 0.0 : i == lane ? Rinv[kb + i] : -v * Rinv[kb + i];
-    }
-#pragma unroll
-    for (int i = 1; i < kPiece; ++i)
-      if (i > lane) D[kb + lane + (kb + i) * kDL] = z[i];
-  }
-  __syncthreads();
-  double* W = winv ? winv + (size_t)it.slot * kSlot : nullptr;
-  double* gw = kLdl ? a.W + m.off + c0 + (int64_t)c0 * ld : nullptr;
-#pragma unroll
-  for (int q = 0; q < kNB * kNB / kThreads; ++q) {
-    const int idx = tid + q * kThreads, c = idx / kNB, r = idx - c * kNB;
-    const double l = D[r + c * kDL];
-    if (r < nb && c < nb && r >= c) {
-      gl[(c0 + r) + (int64_t)(c0 + c) * ld] = (T)l;
-      if constexpr (kLdl) gw[r + (int64_t)c * ld] = l * Dk[c];
-    }
-    if (W && (r >> 3) >= (c >> 3)) W[idx] = l;
-  }
-  if (W && tid < kNB) {
-    W[kNB * kNB + tid] = Rinv[tid];
-    if constexpr (kLdl) W[kNB * kNB + kNB + tid] = 1.0 / Dk[tid];
   }
 }
 
@@ -443,12 +453,12 @@ __device__ __forceinline__ void diag_task(const FactorArgs& a, const PanelItem& 
 constexpr int kTrsmSmemDoubles = 2 * kNB * kDL + kNB;
 
 template <class T>
-__device__ __forceinline__ void trsm_rows_task(const FactorArgs& a, const PanelItem& it, const double* __restrict__ winv,
-                               double* sm) {
+__device__ __forceinline__ void trsm_rows_task(const FactorArgs& a, const PanelItem& it, const SnMeta& meta,
+                                              const double* __restrict__ winv, double* sm) {
   double* R = sm;                // R[r + k*kDL]
   double* D = sm + kNB * kDL;    // D[i + j*kDL] = L11[i][j]
   double* Rinv = sm + 2 * kNB * kDL;
-  const SnMeta m = a.meta[it.s];
+  const SnMeta m = meta;
   T* g = static_cast<T*>(a.L) + m.off;
   const int nb = it.nb, c0 = it.c0;
   const int64_t ld = m.ld;

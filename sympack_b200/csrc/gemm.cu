@@ -206,15 +206,18 @@ __device__ __forceinline__ void dm_setup(DmPipe& P, unsigned char* smem_raw) {
 // Returns false, after recording status 3, when a barrier wait gave up (the copies in
 // flight have then been waited for, bounded).
 template <int BN>
-__device__ bool dmma_tile_task(const FactorArgs& a, const TileItem& it, unsigned char* smem_raw, DmPipe& P) {
+__device__ bool dmma_tile_task(const FactorArgs& a, const TileItem& item, const SnMeta& meta, unsigned char* smem_raw,
+                               DmPipe& P) {
   using D = DTile<BN>;
   __shared__ int sh_abort;
   double* pipe = reinterpret_cast<double*>(smem_raw);
-  double* Cs = reinterpret_cast<double*>(smem_raw);  // reused once the main loop is done
-  int* ints = reinterpret_cast<int*>(smem_raw + D::kMainBytes);
+  // mode 1: per accumulator column its target column's base and its group's offset
+  int64_t* cbase = reinterpret_cast<int64_t*>(smem_raw + D::kMainBytes);
+  int64_t* crel = cbase + 128;
   uint64_t* full = reinterpret_cast<uint64_t*>(smem_raw + D::kMainBytes + D::kIntsBytes);
   uint64_t* empty = full + kDStages;
-  const SnMeta m = a.meta[it.s];
+  const TileItem it = item;
+  const SnMeta m = meta;
   const double* g = static_cast<const double*>(a.L) + m.off;
   const double* gb = a.ldl ? a.W + m.off : g;  // second operand: L, or L D for LDL^T
   const int64_t ld = m.ld;
@@ -222,7 +225,6 @@ __device__ bool dmma_tile_task(const FactorArgs& a, const TileItem& it, unsigned
   const int wm = warp % D::kWarpsM, wn = warp / D::kWarpsM;
   const int gq = lane >> 2, tq = lane & 3;
   const int a0 = it.a_row0 & ~1, b0 = it.b_row0 & ~1;
-  const int ashift = it.a_row0 - a0, bshift = it.b_row0 - b0;
   // rows copied per column: the tile's rows, within the column's padded storage (ld, a
   // multiple of 4, so the count is even and the copy a multiple of 16 bytes)
   const int nra = (int)min((int64_t)kDM, ld - a0), nrb = (int)min((int64_t)BN, ld - b0);
@@ -263,6 +265,15 @@ __device__ bool dmma_tile_task(const FactorArgs& a, const TileItem& it, unsigned
   };
   if (warp == 0)
     for (int kt = 0; kt < nk && kt < kDStages; ++kt) issue(kt);
+  if (it.mode == 1 && warp >= 8 - BN / 32) {  // the last warps fetch the column table meanwhile
+    const int c = tid - (kDThreads - BN), jc = b0 + c;
+    if (jc >= it.b_row0 && jc < it.b_row0 + it.ncols) {
+      const RelGroup gr = a.groups[a.row_group[m.lidx + jc]];
+      const SnMeta mt = a.meta[gr.t];
+      cbase[c] = mt.off + (int64_t)(a.rows[m.lidx + jc] - mt.fc) * mt.ld;
+      crel[c] = gr.rel_off - gr.j0;
+    }
+  }
 
   double acc[D::kMI][4][4];
 #pragma unroll
@@ -327,20 +338,41 @@ __device__ bool dmma_tile_task(const FactorArgs& a, const TileItem& it, unsigned
     return false;
   }
   P.g = g0 + nk;
-  // accumulator row r / column c are panel rows a0 + r / b0 + c; Cs holds the tile from
-  // a_row0 / b_row0
+  // accumulator row r / column c are panel rows a0 + r / b0 + c.  Straight from the
+  // accumulators: a warp's reduction covers four columns of 8 consecutive rows, as many
+  // sectors as 32 rows of one column, and no warp waits for another (through a shared-memory
+  // copy of the tile, with its two barriers and the column table fetched in between, a tile
+  // cost about 11 us beside its flops).  A row's place in a target is loaded once per group.
+  double* L = static_cast<double*>(a.L);
+  const int jr0 = a0 + wm * (16 * D::kMI) + gq, rend = it.a_row0 + it.mrows;
+  int64_t last = INT64_MIN;  // group offsets (rel_off - j0) can be negative
+  int pos[2 * D::kMI];
 #pragma unroll
-  for (int mi = 0; mi < D::kMI; ++mi)
+  for (int ni = 0; ni < 4; ++ni)
 #pragma unroll
-    for (int ni = 0; ni < 4; ++ni) {
-      const int r0 = wm * (16 * D::kMI) + mi * 16 + gq - ashift, c0 = wn * 32 + ni * 8 + 2 * tq - bshift;
-      if (r0 >= 0 && c0 >= 0) Cs[r0 + c0 * kDLdc] = acc[mi][ni][0];
-      if (r0 >= 0 && c0 + 1 >= 0) Cs[r0 + (c0 + 1) * kDLdc] = acc[mi][ni][1];
-      if (c0 >= 0) Cs[r0 + 8 + c0 * kDLdc] = acc[mi][ni][2];
-      if (c0 + 1 >= 0) Cs[r0 + 8 + (c0 + 1) * kDLdc] = acc[mi][ni][3];
+    for (int e = 0; e < 2; ++e) {
+      const int c = wn * 32 + ni * 8 + 2 * tq + e, jc = b0 + c;
+      if (jc < it.b_row0 || jc >= it.b_row0 + it.ncols) continue;
+      double* out = L + m.off + (int64_t)jc * ld;
+      if (it.mode == 1) {
+        const int64_t cr = crel[c];
+        if (cr != last) {
+          last = cr;
+#pragma unroll
+          for (int q = 0; q < 2 * D::kMI; ++q) {
+            const int jr = jr0 + 8 * q;
+            pos[q] = jr >= jc && jr < rend ? a.rel[cr + jr] : 0;
+          }
+        }
+        out = L + cbase[c];
+      }
+#pragma unroll
+      for (int q = 0; q < 2 * D::kMI; ++q) {
+        const int jr = jr0 + 8 * q;
+        if (jr >= it.a_row0 && jr >= jc && jr < rend)
+          atomicAdd(out + (it.mode == 1 ? pos[q] : jr), -acc[q >> 1][ni][2 * (q & 1) + e]);
+      }
     }
-  __syncthreads();
-  tile_epilogue<kDM, BN, kDThreads, double, double>(a, it, m, Cs, kDLdc, (int64_t*)ints, (int64_t*)ints + 128);
   return true;
 }
 
@@ -348,7 +380,7 @@ __global__ void __launch_bounds__(kDThreads, 2) k_gemm_dmma(FactorArgs a, const 
   extern __shared__ __align__(16) unsigned char smem_dmma[];
   DmPipe P;
   dm_setup<kDTileN>(P, smem_dmma);
-  dmma_tile_task<kDTileN>(a, items[blockIdx.x], smem_dmma, P);
+  dmma_tile_task<kDTileN>(a, items[blockIdx.x], a.meta[items[blockIdx.x].s], smem_dmma, P);
 }
 
 // ---- 64 x 64 FP64 FMA tile --------------------------------------------------------
@@ -358,12 +390,14 @@ constexpr size_t kSSmemBytes = kSCBytes + 4 * 64 * sizeof(int);
 
 // One 64 x 64 FMA tile (256 threads, kSSmemBytes of shared memory).
 template <class T>
-__device__ __forceinline__ void simt_tile_task(const FactorArgs& a, const TileItem& it, unsigned char* smem_raw) {
+__device__ __forceinline__ void simt_tile_task(const FactorArgs& a, const TileItem& item, const SnMeta& meta,
+                                              unsigned char* smem_raw) {
+  const TileItem it = item;
   T(*As)[64] = reinterpret_cast<T(*)[64]>(smem_raw);
   T(*Bs)[64] = reinterpret_cast<T(*)[64]>(smem_raw + 16 * 64 * sizeof(T));
   T* Cs = reinterpret_cast<T*>(smem_raw);
   int* ints = reinterpret_cast<int*>(smem_raw + kSCBytes);
-  const SnMeta m = a.meta[it.s];
+  const SnMeta m = meta;
   const T* g = static_cast<const T*>(a.L) + m.off;
   // second operand: L, or L D for LDL^T (FP64 only, so W is read only when T is double)
   const T* gb = a.ldl ? reinterpret_cast<const T*>(a.W + m.off) : g;
@@ -408,7 +442,7 @@ __device__ __forceinline__ void simt_tile_task(const FactorArgs& a, const TileIt
 template <class T>
 __global__ void __launch_bounds__(256) k_gemm_simt(FactorArgs a, const TileItem* __restrict__ items) {
   extern __shared__ __align__(16) unsigned char smem_simt[];
-  simt_tile_task<T>(a, items[blockIdx.x], smem_simt);
+  simt_tile_task<T>(a, items[blockIdx.x], a.meta[items[blockIdx.x].s], smem_simt);
 }
 
 // ---- 128 x 128 split-precision 3xTF32 tensor-core tile (FP32 storage) -------------
@@ -1574,75 +1608,117 @@ static_assert(kFSmallCap >= 96 * 1024 / 8 + ftask::kSmallHeadDoubles, "small pan
 constexpr size_t kFSmemBytes32 = kVSmemBytes;
 static_assert(kFSmemBytes32 >= kFSmallCap * sizeof(double) + 1024, "FP32 persistent shared memory");
 
-// FP64: two CTAs per SM (128 x 64 DMMA tiles); FP32: one (the TMA-fed tile's 193 KB).
-template <class T, bool kLdl>
-__global__ void __launch_bounds__(256, std::is_same<T, float>::value ? 1 : 2)
-    k_factor_persistent(const __grid_constant__ FactorArgs a, const __grid_constant__ FactorSched f) {
-  constexpr bool kF32 = std::is_same<T, float>::value;
-  extern __shared__ __align__(16) unsigned char smem_f[];
-  __shared__ int sh_task, sh_go;
-  TcTile tc;
-  DmPipe dp;
-  if constexpr (kF32) tc_setup(tc, smem_f);  // tensor memory and stage barriers for the whole launch
-  else dm_setup<kDTileN>(dp, smem_f);
-  for (;;) {
-    if (threadIdx.x == 0) {
-      int tk = atomicAdd(f.counter, 1);
-      int go = tk < f.ntasks && status_of(a.status) == 0;
-      if (go && f.trace) f.trace[4 * (size_t)tk] = global_ns();
-      if (go) {
-        const FTask t = f.tasks[tk];
-        for (int w = 0; w < t.nwait && go; ++w) {
-          const FWait fw = w == 0 ? FWait{t.w0_ctr, t.w0_target} : f.waits[t.wait0 + w];
-          const int32_t* c = f.ctr + fw.ctr;
-          if (ld_acquire_i(c) >= fw.target) continue;
-          go = 0;
-          for (long long it = 0; it < f.spin_limit; ++it) {
-            if (it >= 256) __nanosleep(128);
-            if (ld_acquire_i(c) >= fw.target) {
-              go = 1;
-              break;
-            }
-            if (status_of(a.status) != 0) break;
+// The task a CTA runs next: its record, item and supernode, brought to shared memory by warp
+// 1 while warp 0 publishes the task before it (a release waits for the block's outstanding
+// reductions, about a microsecond), so that no other warp starts with a chain of dependent
+// loads.
+struct alignas(16) NextTask {
+  FTask t;
+  SnMeta m;
+  int32_t item[8];  // TileItem, PanelItem or the small panel's supernode
+  int32_t tk, go;
+};
+
+// One warp: fetch task tk and wait until its dependencies are met (bounded).
+__device__ __forceinline__ void next_task(const FactorArgs& a, const FactorSched& f, int tk, NextTask& nx) {
+  const int lane = threadIdx.x & 31;
+  constexpr unsigned kAll = 0xffffffffu;
+  int go = tk < f.ntasks && status_of(a.status) == 0;
+  go = __shfl_sync(kAll, go, 0);
+  if (go) {
+    if (f.trace && lane == 0) f.trace[4 * (size_t)tk] = global_ns();
+    const int w = lane < 8 ? reinterpret_cast<const int32_t*>(f.tasks + tk)[lane] : 0;
+    const int kind = __shfl_sync(kAll, w, 0), item = __shfl_sync(kAll, w, 1);
+    const int wait0 = __shfl_sync(kAll, w, 2), nwait = __shfl_sync(kAll, w, 3);
+    const int ctr0 = __shfl_sync(kAll, w, 6), target0 = __shfl_sync(kAll, w, 7);
+    const int32_t* src = kind == 0 ? f.small_items + item
+                                   : kind <= 2 ? reinterpret_cast<const int32_t*>(f.panel + item)
+                                               : reinterpret_cast<const int32_t*>(f.tiles + item);
+    const int ni = kind == 0 ? 1 : kind <= 2 ? (int)(sizeof(PanelItem) / 4) : (int)(sizeof(TileItem) / 4);
+    const int v = lane < ni ? src[lane] : 0;
+    const int s = __shfl_sync(kAll, v, 0);
+    const int mv = lane < (int)(sizeof(SnMeta) / 4) ? reinterpret_cast<const int32_t*>(a.meta + s)[lane] : 0;
+    if (lane < 8) reinterpret_cast<int32_t*>(&nx.t)[lane] = w;
+    if (lane < 8) nx.item[lane] = v;
+    if (lane == 0) {
+      for (int q = 0; q < nwait && go; ++q) {
+        const FWait fw = q == 0 ? FWait{ctr0, target0} : f.waits[wait0 + q];
+        const int32_t* c = f.ctr + fw.ctr;
+        if (ld_acquire_i(c) >= fw.target) continue;
+        go = 0;
+        for (long long it = 0; it < f.spin_limit; ++it) {
+          if (it >= 256) __nanosleep(128);
+          if (ld_acquire_i(c) >= fw.target) {
+            go = 1;
+            break;
           }
-          if (!go && atomicCAS(&a.status->code, 0, 3) == 0) {  // a wait expired
-            a.status->supernode = -1;
-            a.status->column = fw.ctr;
-          }
+          if (status_of(a.status) != 0) break;
+        }
+        if (!go && atomicCAS(&a.status->code, 0, 3) == 0) {  // a wait expired
+          a.status->supernode = -1;
+          a.status->column = fw.ctr;
         }
       }
       if (go && f.trace) {
         f.trace[4 * (size_t)tk + 1] = global_ns();
         f.trace[4 * (size_t)tk + 3] = smid();
       }
-      sh_task = tk;
-      sh_go = go;
     }
+    if (lane < (int)(sizeof(SnMeta) / 4)) reinterpret_cast<int32_t*>(&nx.m)[lane] = mv;
+  }
+  if (lane == 0) {
+    nx.tk = tk;
+    nx.go = go;
+  }
+}
+
+// FP64: two CTAs per SM (128 x 64 DMMA tiles); FP32: one (the TMA-fed tile's 193 KB).
+template <class T, bool kLdl>
+__global__ void __launch_bounds__(256, std::is_same<T, float>::value ? 1 : 2)
+    k_factor_persistent(const __grid_constant__ FactorArgs a, const __grid_constant__ FactorSched f) {
+  constexpr bool kF32 = std::is_same<T, float>::value;
+  extern __shared__ __align__(16) unsigned char smem_f[];
+  __shared__ NextTask nx;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  TcTile tc;
+  DmPipe dp;
+  if constexpr (kF32) tc_setup(tc, smem_f);  // tensor memory and stage barriers for the whole launch
+  else dm_setup<kDTileN>(dp, smem_f);
+  int ticket = 0;  // warp 1, lane 0
+  if (warp == 1 && lane == 0) ticket = atomicAdd(f.counter, 1);
+  for (;;) {
+    if (warp == 1) next_task(a, f, __shfl_sync(0xffffffffu, ticket, 0), nx);
     __syncthreads();
-    const int tk = sh_task;
-    if (!sh_go) break;
-    const FTask t = f.tasks[tk];
-    switch (t.kind) {
+    if (!nx.go) break;
+    const int kind = nx.t.kind, nsig = nx.t.nsig, sig0 = nx.t.sig0;
+    int sig = warp == 0 && lane < nsig ? f.sigs[sig0 + lane] : -1;
+    switch (kind) {
       case 0:
-        ftask::factor_small_task<T, kLdl>(a, f.small_items[t.item], reinterpret_cast<double*>(smem_f), kFSmallCap);
+        ftask::factor_small_task<T, kLdl>(a, nx.item[0], nx.m, reinterpret_cast<double*>(smem_f), kFSmallCap);
         break;
       case 1:
-        ftask::diag_task<T, kLdl>(a, f.panel[t.item], f.winv, reinterpret_cast<double*>(smem_f));
+        ftask::diag_task<T, kLdl>(a, *reinterpret_cast<const PanelItem*>(nx.item), nx.m, f.winv,
+                                  reinterpret_cast<double*>(smem_f));
         break;
       case 2:
-        ftask::trsm_rows_task<T>(a, f.panel[t.item], f.winv, reinterpret_cast<double*>(smem_f));
+        ftask::trsm_rows_task<T>(a, *reinterpret_cast<const PanelItem*>(nx.item), nx.m, f.winv,
+                                 reinterpret_cast<double*>(smem_f));
         break;
       case 3:
-        simt_tile_task<T>(a, f.tiles[t.item], smem_f);
+        simt_tile_task<T>(a, *reinterpret_cast<const TileItem*>(nx.item), nx.m, smem_f);
         break;
       default:
-        if constexpr (kF32) tc32t_tile_task(a, f.tiles[t.item], tc);  // a failure records status 3
-        else dmma_tile_task<kDTileN>(a, f.tiles[t.item], smem_f, dp);
+        if constexpr (kF32) tc32t_tile_task(a, *reinterpret_cast<const TileItem*>(nx.item), tc);  // a failure records status 3
+        else dmma_tile_task<kDTileN>(a, *reinterpret_cast<const TileItem*>(nx.item), nx.m, smem_f, dp);
         break;
     }
+    if (warp == 1 && lane == 0) ticket = atomicAdd(f.counter, 1);
+    const int tk = nx.tk;
     __syncthreads();
     if (f.trace && threadIdx.x == 0) f.trace[4 * (size_t)tk + 2] = global_ns();
-    for (int i = threadIdx.x; i < t.nsig; i += blockDim.x) red_release_i(f.ctr + f.sigs[t.sig0 + i], 1);
+    if (sig >= 0) red_release_i(f.ctr + sig, 1);
+    if (warp == 0)
+      for (int i = lane + 32; i < nsig; i += 32) red_release_i(f.ctr + f.sigs[sig0 + i], 1);
   }
   if constexpr (kF32) tc_teardown(tc);
 }

@@ -34,28 +34,29 @@ __global__ void k_assemble(T* __restrict__ L, const int64_t* __restrict__ dst, c
 template <class T, bool kLdl>
 __global__ void __launch_bounds__(kThreads) k_factor_small(FactorArgs a, const int32_t* __restrict__ items, int cap) {
   extern __shared__ double sm_small[];
-  factor_small_task<T, kLdl>(a, items[blockIdx.x], sm_small, cap);
+  const int s = items[blockIdx.x];
+  factor_small_task<T, kLdl>(a, s, a.meta[s], sm_small, cap);
 }
 
 template <class T>
 __global__ void __launch_bounds__(kThreads, 1) k_potrf_diag(FactorArgs a, const PanelItem* __restrict__ items,
                                                          double* __restrict__ winv) {
   extern __shared__ double sm_diag[];
-  diag_task<T, false>(a, items[blockIdx.x], winv, sm_diag);
+  diag_task<T, false>(a, items[blockIdx.x], a.meta[items[blockIdx.x].s], winv, sm_diag);
 }
 
 template <class T>
 __global__ void __launch_bounds__(kThreads, 1) k_ldl_diag(FactorArgs a, const PanelItem* __restrict__ items,
                                                        double* __restrict__ winv) {
   extern __shared__ double sm_ldl[];
-  diag_task<T, true>(a, items[blockIdx.x], winv, sm_ldl);
+  diag_task<T, true>(a, items[blockIdx.x], a.meta[items[blockIdx.x].s], winv, sm_ldl);
 }
 
 template <class T>
 __global__ void __launch_bounds__(kThreads, 2) k_trsm_rows(FactorArgs a, const PanelItem* __restrict__ items,
                                                         const double* __restrict__ winv) {
   extern __shared__ double sm_trsm[];
-  trsm_rows_task<T>(a, items[blockIdx.x], winv, sm_trsm);
+  trsm_rows_task<T>(a, items[blockIdx.x], a.meta[items[blockIdx.x].s], winv, sm_trsm);
 }
 
 __global__ void k_permute_in(double* X, int64_t ldx, const double* B, int64_t ldb, const int32_t* invp0, int n,
