@@ -903,6 +903,55 @@ __host__ __device__ constexpr size_t strip_smem(int nb) {
 }
 __device__ __forceinline__ int xs(int k, int m) { return k * kXs + (m ^ (4 * (k & 3))); }
 
+// One warp: R <- R D^-T for a strip R of 16 rows x 64 (element (m, k) at xs(k, m)), D lower
+// triangular with leading dimension ld and reciprocal diagonal Rinv, by 8-column pieces.
+__device__ __forceinline__ void strip_solve(double* R, const double* D, const double* Rinv, int kLd) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  double v[8][4];
+#pragma unroll
+  for (int n = 0; n < 8; ++n)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) v[n][e] = R[xs(8 * n + 2 * t + (e & 1), g + 8 * (e >> 1))];
+  const int mm = lane & 15;
+#pragma unroll 1
+  for (int p = 0; p < 8; ++p) {  // v[n] holds column tile p + n
+    const int kb = 8 * p;
+    if (p > 0) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) R[xs(kb + 2 * t + (e & 1), g + 8 * (e >> 1))] = v[0][e];
+      __syncwarp();
+    }
+    double x[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) x[q] = R[xs(kb + q, mm)];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      x[q] *= Rinv[kb + q];
+#pragma unroll
+      for (int k = q + 1; k < 8; ++k) x[k] = fma(-x[q], D[kb + k + (kb + q) * kLd], x[k]);
+      if (q & 1) asm volatile("" ::: "memory");
+    }
+    __syncwarp();
+    if (lane < 16) {
+#pragma unroll
+      for (int q = 0; q < 8; ++q) R[xs(kb + q, mm)] = x[q];
+    }
+    __syncwarp();
+    const double a0 = -R[xs(kb + t, g)], a1 = -R[xs(kb + t, g + 8)];
+    const double a2 = -R[xs(kb + 4 + t, g)], a3 = -R[xs(kb + 4 + t, g + 8)];
+    const double* b = D + g + kb + 8 + (kb + t) * kLd;
+#pragma unroll
+    for (int n = 1; n < 8; ++n) {
+      if (p + n < 8) {
+        dmma(v[n], a0, a1, b[8 * (n - 1)]);
+        dmma(v[n], a2, a3, b[8 * (n - 1) + 4 * kLd]);
+      }
+#pragma unroll
+      for (int e = 0; e < 4; ++e) v[n - 1][e] = v[n][e];
+    }
+  }
+}
+
 template <class T>
 __global__ void __launch_bounds__(256, 2) k_sb_inverse_strips(const T* __restrict__ L, T* __restrict__ Inv,
                                                               const SnMeta* __restrict__ meta,
@@ -963,50 +1012,7 @@ __global__ void __launch_bounds__(256, 2) k_sb_inverse_strips(const T* __restric
     }
     __syncthreads();
     if (warp == 0) {
-      double* R = X + (i - j) * kT * kXs;  // xs() of whole 4-row groups: local rows count alike
-      double v[8][4];
-#pragma unroll
-      for (int n = 0; n < 8; ++n)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) v[n][e] = R[xs(8 * n + 2 * t + (e & 1), g + 8 * (e >> 1))];
-      const int mm = lane & 15;
-#pragma unroll 1
-      for (int p = 0; p < 8; ++p) {  // v[n] holds column tile p + n
-        const int kb = 8 * p;
-        if (p > 0) {
-#pragma unroll
-          for (int e = 0; e < 4; ++e) R[xs(kb + 2 * t + (e & 1), g + 8 * (e >> 1))] = v[0][e];
-          __syncwarp();
-        }
-        double x[8];
-#pragma unroll
-        for (int q = 0; q < 8; ++q) x[q] = R[xs(kb + q, mm)];
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          x[q] *= Rinv[kb + q];
-#pragma unroll
-          for (int k = q + 1; k < 8; ++k) x[k] = fma(-x[q], D[kb + k + (kb + q) * kLd], x[k]);
-          if (q & 1) asm volatile("" ::: "memory");
-        }
-        __syncwarp();
-        if (lane < 16) {
-#pragma unroll
-          for (int q = 0; q < 8; ++q) R[xs(kb + q, mm)] = x[q];
-        }
-        __syncwarp();
-        const double a0 = -R[xs(kb + t, g)], a1 = -R[xs(kb + t, g + 8)];
-        const double a2 = -R[xs(kb + 4 + t, g)], a3 = -R[xs(kb + 4 + t, g + 8)];
-        const double* b = D + g + kb + 8 + (kb + t) * kLd;
-#pragma unroll
-        for (int n = 1; n < 8; ++n) {
-          if (p + n < 8) {
-            dmma(v[n], a0, a1, b[8 * (n - 1)]);
-            dmma(v[n], a2, a3, b[8 * (n - 1) + 4 * kLd]);
-          }
-#pragma unroll
-          for (int e = 0; e < 4; ++e) v[n - 1][e] = v[n][e];
-        }
-      }
+      strip_solve(X + (i - j) * kT * kXs, D, Rinv, kLd);  // whole 4-row groups: local rows count alike in xs()
     }
     __syncthreads();
     T* dst = base + ((int64_t)i * (i + 1) / 2 + j) * (kT * kT) + col0 * kT;
@@ -1019,52 +1025,81 @@ __global__ void __launch_bounds__(256, 2) k_sb_inverse_strips(const T* __restric
 }
 
 // ---- inverses of one-block supernodes' diagonal blocks ------------------------------------
-// One warp per block of at most 32 columns (kW = 32) or one block of 64 threads per wider one:
-// thread c substitutes down column c, x_i = (delta_ic - sum_{k<i} L_ik x_k) / L_ii, the block
-// and the columns in shared memory (FP64).
-template <class T, int kW>
-__global__ void __launch_bounds__(128) k_diag_inverse(const T* __restrict__ L, double* __restrict__ Inv,
-                                                      const Inv1Item* __restrict__ items, int count) {
-  constexpr int kLd = kW + 1, kGroup = kW, kPer = kW == 32 ? 4 : 1;
-  extern __shared__ __align__(16) double smd[];
-  const int grp = threadIdx.x / kGroup, c = threadIdx.x % kGroup;
-  const int i0 = blockIdx.x * kPer + grp;
-  double* A = smd + (size_t)grp * 2 * kW * kLd;
-  double* X = A + kW * kLd;
-  auto sync = [&]() {
-    if constexpr (kW == 32) __syncwarp();
-    else __syncthreads();
-  };
+// At most 32 columns: one warp per block, lane c substitutes down column c with the column in
+// registers, x_i = (delta_ic - sum_{k<i} L_ik x_k) / L_ii, rows of L broadcast from shared
+// memory, four sums at a time against the latency of a chain of FMAs.  (Columns in shared
+// memory, two reads per FMA: 113 us on the 463 x 467 grid.)
+constexpr int kDiagWarps = 4;
+template <class T>
+__global__ void __launch_bounds__(32 * kDiagWarps) k_diag_inverse(const T* __restrict__ L, double* __restrict__ Inv,
+                                                                  const Inv1Item* __restrict__ items, int count) {
+  constexpr int kW = kInv1Narrow, kLd = kW + 2;
+  __shared__ __align__(16) double sh[kDiagWarps][kW * kLd];
+  __shared__ double shr[kDiagWarps][kW];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int i0 = blockIdx.x * kDiagWarps + warp;
   if (i0 >= count) return;
   const Inv1Item it = items[i0];
   const int w = it.w;
-  for (int idx = c; idx < w * w; idx += kGroup) {
-    const int k = idx / w, i = idx - k * w;
-    if (i >= k) A[i * kLd + k] = (double)L[it.a + i + (int64_t)k * it.ld];
-  }
-  sync();
-  if (c < w) {
-    for (int i = 0; i < c; ++i) X[i * kLd + c] = 0.0;
-    for (int i = c; i < w; ++i) {
-      double s0 = 0.0, s1 = 0.0;
-      int k = c;
-      for (; k + 1 < i; k += 2) {
-        s0 = fma(A[i * kLd + k], X[k * kLd + c], s0);
-        s1 = fma(A[i * kLd + k + 1], X[(k + 1) * kLd + c], s1);
+  double* A = sh[warp];   // row i at i * kLd
+  for (int k = 0; k < w; ++k)
+    if (lane < w && lane >= k) A[lane * kLd + k] = (double)L[it.a + lane + (int64_t)k * it.ld];
+  if (lane < w) shr[warp][lane] = 1.0 / A[lane * kLd + lane];
+  __syncwarp();
+  double x[kW];
+#pragma unroll
+  for (int i = 0; i < kW; ++i) {
+    x[i] = 0.0;
+    if (i < w) {
+      double s[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+      for (int k = 0; k + 1 < i; k += 2) {
+        const double2 l = *reinterpret_cast<const double2*>(A + i * kLd + k);
+        s[k & 2] = fma(l.x, x[k], s[k & 2]);
+        s[(k & 2) + 1] = fma(l.y, x[k + 1], s[(k & 2) + 1]);
       }
-      if (k < i) s0 = fma(A[i * kLd + k], X[k * kLd + c], s0);
-      X[i * kLd + c] = ((i == c ? 1.0 : 0.0) - (s0 + s1)) / A[i * kLd + i];
+      if (i & 1) s[0] = fma(A[i * kLd + i - 1], x[i - 1], s[0]);
+      // x_k = 0 for k < c, so columns right of row i stay zero
+      x[i] = i < lane ? 0.0 : ((i == lane ? 1.0 : 0.0) - ((s[0] + s[1]) + (s[2] + s[3]))) * shr[warp][i];
     }
   }
-  sync();
-  for (int idx = c; idx < w * w; idx += kGroup) {
-    const int k = idx / w, i = idx - k * w;
-    Inv[it.inv + idx] = X[i * kLd + k];
-  }
+  __syncwarp();
+#pragma unroll
+  for (int i = 0; i < kW; ++i)
+    if (lane < w && i < w) A[i * kLd + lane] = x[i];
+  __syncwarp();
+  for (int k = 0; k < w; ++k)
+    if (lane < w) Inv[it.inv + (int64_t)k * w + lane] = A[lane * kLd + k];
 }
 
-constexpr size_t kDiagInvSmem32 = (size_t)4 * 2 * 32 * 33 * sizeof(double);
-constexpr size_t kDiagInvSmem64 = (size_t)2 * 64 * 65 * sizeof(double);
+// Wider blocks: a warp per strip of 16 columns, solved as a strip of a super-block is.
+template <class T>
+__global__ void __launch_bounds__(128) k_diag_inverse_wide(const T* __restrict__ L, double* __restrict__ Inv,
+                                                           const Inv1Item* __restrict__ items) {
+  constexpr int kLd = 68;
+  __shared__ __align__(16) double D[kT * kLd];
+  __shared__ double Rinv[kT];
+  extern __shared__ __align__(16) double smw[];  // a strip per warp
+  const Inv1Item it = items[blockIdx.x];
+  const int w = it.w, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, col0 = 16 * warp;
+  for (int idx = threadIdx.x; idx < kT * kT; idx += 128) {
+    const int c = idx >> 6, r = idx & 63;
+    const double v = r < w && c <= r ? (double)L[it.a + r + (int64_t)c * it.ld] : (r == c ? 1.0 : 0.0);
+    D[r + c * kLd] = v;
+    if (r == c) Rinv[r] = 1.0 / v;
+  }
+  double* X = smw + warp * kT * kXs;
+  for (int idx = lane; idx < kT * 16; idx += 32) {
+    const int k = idx >> 4, m = idx & 15;
+    X[xs(k, m)] = k < w && k == col0 + m ? 1.0 : 0.0;
+  }
+  __syncthreads();
+  if (col0 >= w) return;
+  strip_solve(X, D, Rinv, kLd);
+  __syncwarp();
+  for (int m = 0; m < 16 && col0 + m < w; ++m)
+    for (int r = lane; r < w; r += 32) Inv[it.inv + r + (int64_t)(col0 + m) * w] = X[xs(r, m)];
+}
 
 int g_solve_grid[2][2] = {};  // resident CTAs of the sweeps: [FP32][NG - 1]
 
@@ -1103,14 +1138,12 @@ void init_solve_attributes() {
   init_sweeps<double, 2>(0, sms);
   init_sweeps<float, 1>(1, sms);
   init_sweeps<float, 2>(1, sms);
+  cudaFuncSetAttribute(k_diag_inverse_wide<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * kT * kXs * (int)sizeof(double));
+  cudaFuncSetAttribute(k_diag_inverse_wide<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * kT * kXs * (int)sizeof(double));
   cudaFuncSetAttribute(k_sb_inverse_strips<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)strip_smem(kStripBlocks));
   cudaFuncSetAttribute(k_sb_inverse_strips<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)strip_smem(kStripBlocks));
   cudaFuncSetAttribute(k_sb_inverse<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kInvSmem);
   cudaFuncSetAttribute(k_sb_inverse<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kInvSmem);
-  cudaFuncSetAttribute(k_diag_inverse<double, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDiagInvSmem32);
-  cudaFuncSetAttribute(k_diag_inverse<float, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDiagInvSmem32);
-  cudaFuncSetAttribute(k_diag_inverse<double, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDiagInvSmem64);
-  cudaFuncSetAttribute(k_diag_inverse<float, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDiagInvSmem64);
 }
 
 void launch_sb_inverse(cudaStream_t st, const void* L, void* Inv, bool fp32, const SnMeta* meta,
@@ -1137,8 +1170,10 @@ void launch_diag_inverse(cudaStream_t st, const void* L, double* Inv, bool fp32,
                          int count) {
   auto run = [&](auto* l) {
     using T = typename std::remove_const<typename std::remove_pointer<decltype(l)>::type>::type;
-    if (narrow > 0) k_diag_inverse<T, 32><<<(narrow + 3) / 4, 128, kDiagInvSmem32, st>>>(l, Inv, items, narrow);
-    if (count > narrow) k_diag_inverse<T, 64><<<count - narrow, 64, kDiagInvSmem64, st>>>(l, Inv, items + narrow, count - narrow);
+    if (narrow > 0)
+      k_diag_inverse<T><<<(narrow + kDiagWarps - 1) / kDiagWarps, 32 * kDiagWarps, 0, st>>>(l, Inv, items, narrow);
+    if (count > narrow)
+      k_diag_inverse_wide<T><<<count - narrow, 128, 4 * kT * kXs * sizeof(double), st>>>(l, Inv, items + narrow);
   };
   if (fp32) run(static_cast<const float*>(L));
   else run(static_cast<const double*>(L));
