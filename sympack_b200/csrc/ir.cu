@@ -38,7 +38,7 @@ __device__ __forceinline__ void atomic_max_nonneg(double* addr, double v) {
 // thread keeps a running maximum while its rows stay in one system, and a warp
 // whose lanes end in the same system merges before the atomic.  out zeroed by
 // the caller.
-constexpr int kChunk = 4096;
+constexpr int kChunk = 1024;
 
 __device__ __forceinline__ void flush_segmax(double* out, int seg, double m) {
   const unsigned full = 0xffffffffu;
@@ -88,30 +88,41 @@ __global__ void __launch_bounds__(kResThreads) k_residual(const int64_t* __restr
                                                           double* __restrict__ R, const int32_t* __restrict__ invp0,
                                                           int n, int nrhs, const int32_t* __restrict__ rowseg,
                                                           double* __restrict__ xmax, double* __restrict__ rmax) {
+  constexpr int kOwn = (CB + 3) / 4;  // columns whose sums a lane finishes
   __shared__ unsigned long long smax[2][CB];
   const int c0 = blockIdx.y * CB, nc = min(CB, nrhs - c0), q = threadIdx.x & 3;
   if (threadIdx.x < 2 * CB) smax[threadIdx.x / CB][threadIdx.x % CB] = 0;
   __syncthreads();
   const int64_t chunk = ((n + gridDim.x - 1) / gridDim.x + 63) / 64 * 64;
   const int64_t r0 = blockIdx.x * chunk, r1 = min((int64_t)n, r0 + chunk);
-  double mr[CB], mx[CB];
+  double mr[kOwn], mx[kOwn];
 #pragma unroll
-  for (int c = 0; c < CB; ++c) mr[c] = mx[c] = 0.0;
+  for (int o = 0; o < kOwn; ++o) mr[o] = mx[o] = 0.0;
   int seg = -1;
   for (int64_t base = r0; base < r1; base += kResThreads / 4) {
     const int64_t i = base + (threadIdx.x >> 2);
     const bool in = i < r1;
-    double s[CB];
+    double s[CB], bv[kOwn], xv[kOwn];
+    int64_t pr = 0;
 #pragma unroll
     for (int c = 0; c < CB; ++c) s[c] = 0.0;
-    if (in) {
-      const int64_t p1 = rowptr[i + 1];
-      for (int64_t p = rowptr[i] + q; p < p1; p += 4) {
-        const double v = val[p];
-        const double* xj = x + col[p] + c0 * ldx;
+    if (in) {  // everything that does not depend on the row's entries first
+      const int64_t p1 = rowptr[i + 1], p0 = rowptr[i] + q;
+      pr = invp0[i];
+#pragma unroll
+      for (int o = 0; o < kOwn; ++o) {
+        const int c = 4 * o + q;
+        bv[o] = c < nc ? b[i + (c0 + c) * ldb] : 0.0;
+        xv[o] = c < nc ? x[i + (c0 + c) * ldx] : 0.0;
+      }
+      for (int64_t p = p0; p < p1; p += 8) {  // two of the lane's entries at a time
+        const bool two = p + 4 < p1;
+        const double v0 = val[p], v1 = two ? val[p + 4] : 0.0;
+        const double* x0 = x + col[p] + c0 * ldx;
+        const double* x1 = two ? x + col[p + 4] + c0 * ldx : x0;
 #pragma unroll
         for (int c = 0; c < CB; ++c)
-          if (c < nc) s[c] = fma(v, xj[c * ldx], s[c]);
+          if (c < nc) s[c] = fma(v1, two ? x1[c * ldx] : 0.0, fma(v0, x0[c * ldx], s[c]));
       }
     }
 #pragma unroll
@@ -123,41 +134,48 @@ __global__ void __launch_bounds__(kResThreads) k_residual(const int64_t* __restr
     if (rowseg && rowseg[i] != seg) {
       if (seg >= 0) {
 #pragma unroll
-        for (int c = 0; c < CB; ++c) {
-          if ((c & 3) != q || c >= nc) continue;
-          atomic_max_nonneg(rmax + seg * 64 + c0 + c, mr[c]);
-          atomic_max_nonneg(xmax + seg * 64 + c0 + c, mx[c]);
-          mr[c] = mx[c] = 0.0;
+        for (int o = 0; o < kOwn; ++o) {
+          const int c = 4 * o + q;
+          if (c >= nc) continue;
+          atomic_max_nonneg(rmax + seg * 64 + c0 + c, mr[o]);
+          atomic_max_nonneg(xmax + seg * 64 + c0 + c, mx[o]);
+          mr[o] = mx[o] = 0.0;
         }
       }
       seg = rowseg[i];
     }
-    const int64_t pr = invp0[i];
 #pragma unroll
-    for (int c = 0; c < CB; ++c) {
-      if ((c & 3) != q || c >= nc) continue;
-      const double r = b[i + (c0 + c) * ldb] - s[c];
+    for (int o = 0; o < kOwn; ++o) {
+      const int c = 4 * o + q;
+      if (c >= nc) continue;
+      double sum = s[4 * o];
+#pragma unroll
+      for (int e = 1; e < 4; ++e)
+        if (4 * o + e < CB && q == e) sum = s[4 * o + e];
+      const double r = bv[o] - sum;
       R[pr + (int64_t)(c0 + c) * n] = r;
-      mr[c] = fmax(mr[c], fabs(r));
-      mx[c] = fmax(mx[c], fabs(x[i + (c0 + c) * ldx]));
+      mr[o] = fmax(mr[o], fabs(r));
+      mx[o] = fmax(mx[o], fabs(xv[o]));
     }
   }
   if (rowseg) {
     if (seg >= 0) {
 #pragma unroll
-      for (int c = 0; c < CB; ++c) {
-        if ((c & 3) != q || c >= nc) continue;
-        atomic_max_nonneg(rmax + seg * 64 + c0 + c, mr[c]);
-        atomic_max_nonneg(xmax + seg * 64 + c0 + c, mx[c]);
+      for (int o = 0; o < kOwn; ++o) {
+        const int c = 4 * o + q;
+        if (c >= nc) continue;
+        atomic_max_nonneg(rmax + seg * 64 + c0 + c, mr[o]);
+        atomic_max_nonneg(xmax + seg * 64 + c0 + c, mx[o]);
       }
     }
     return;
   }
 #pragma unroll
-  for (int c = 0; c < CB; ++c) {
-    if ((c & 3) != q || c >= nc) continue;
-    atomicMax(&smax[0][c], (unsigned long long)__double_as_longlong(mr[c]));
-    atomicMax(&smax[1][c], (unsigned long long)__double_as_longlong(mx[c]));
+  for (int o = 0; o < kOwn; ++o) {
+    const int c = 4 * o + q;
+    if (c >= nc) continue;
+    atomicMax(&smax[0][c], (unsigned long long)__double_as_longlong(mr[o]));
+    atomicMax(&smax[1][c], (unsigned long long)__double_as_longlong(mx[o]));
   }
   __syncthreads();
   if (threadIdx.x < nc) {
@@ -223,7 +241,7 @@ void launch_residual(cudaStream_t st, const int64_t* rowptr, const int32_t* col,
                      const int32_t* rowseg, double* xmax, double* rmax) {
   auto run = [&](auto cb) {
     constexpr int CB = decltype(cb)::value;
-    const int by = (nrhs + CB - 1) / CB, rows = (n + 63) / 64, cap = (148 * 8 + by - 1) / by;
+    const int by = (nrhs + CB - 1) / CB, rows = (n + 63) / 64, cap = (148 * 16 + by - 1) / by;
     k_residual<CB><<<dim3(rows < cap ? rows : cap, by), kResThreads, 0, st>>>(rowptr, col, val, x, ldx, b, ldb, R, invp0,
                                                                               n, nrhs, rowseg, xmax, rmax);
   };
