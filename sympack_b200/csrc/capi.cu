@@ -188,14 +188,22 @@ void release_device(spb_handle* h) {
   h->x_cap = 0;
 }
 
-// The persistent factorization runs FP64 handles (unless the steps are asked for) and
-// FP32 handles that ask for it and whose 128 x 128 tiles use the TMA-fed tcgen05 engine
-// (the one with a task body for the persistent kernel).
-bool persistent_schedule(const spb_options& o) {
+// The persistent factorization runs FP64 handles (unless the steps are asked for) and FP32
+// handles whose 128 x 128 tiles use the TMA-fed tcgen05 engine (the one with a task body for
+// the persistent kernel) when they ask for it or leave the choice and the factorization is
+// short: below kFp32PersistentFlops the step sequence is bound by its launches (463 x 463
+// grid 2.75 ms against 2.22 persistent, 27-point 28^3 2.84 / 2.49, 46^3 (2.4e11 flops) 9.40 /
+// 8.33, 50 systems of up to 6,000 rows 9.12 / 4.81), the two meet near 7e11 flops (54^3 17.8 /
+// 17.4 ms), and above, the tiles bind and the sequence's warp-specialised kernel is the
+// better engine (60^3 26.9 / 31.3, 80^3 107.7 / 156.1).
+constexpr double kFp32PersistentFlops = 5e11;
+bool persistent_schedule(const spb_options& o, double flops) {
   if (o.precision == SPB_PRECISION_FP64) return o.factor_schedule != SPB_FACTOR_STEPS;
-  return o.factor_schedule == SPB_FACTOR_PERSISTENT && o.fp32_engine == 3;
+  if (o.fp32_engine != 3) return false;
+  return o.factor_schedule == SPB_FACTOR_PERSISTENT ||
+         (o.factor_schedule == SPB_FACTOR_AUTO && flops < kFp32PersistentFlops);
 }
-bool persistent_factor(const spb_handle* h) { return persistent_schedule(h->opt); }
+bool persistent_factor(const spb_handle* h) { return persistent_schedule(h->opt, h->sym.flops_stat); }
 
 spb::dev::FactorArgs factor_args(spb_handle* h) {
   spb::dev::FactorArgs a;
@@ -730,7 +738,7 @@ spb::RelaxParams relax_of(const spb_options& o) {
   return rp;
 }
 
-spb::PlanParams plan_params_of(const spb_options& o) {
+spb::PlanParams plan_params_of(const spb_options& o, const spb::Symbolic& sym) {
   spb::PlanParams pp;
   if (o.device >= 0) {
     int sms = 0;
@@ -741,7 +749,7 @@ spb::PlanParams plan_params_of(const spb_options& o) {
   if (o.plan_outer_nb > 0) pp.outer_nb = o.plan_outer_nb;
   if (o.plan_solve_chunk > 0) pp.solve_sb = o.plan_solve_chunk;
   if (o.plan_solve_tiles > 0) pp.solve_tpt = o.plan_solve_tiles;
-  pp.factor_dag = persistent_schedule(o);
+  pp.factor_dag = persistent_schedule(o, sym.flops_stat);
   pp.fp32 = o.precision == SPB_PRECISION_FP32_IR;
   return pp;
 }
@@ -856,9 +864,9 @@ int install_device(spb_handle* h);
 int64_t predict_bytes(const spb_handle* h, bool fp32, int nrhs) {
   spb_options o = h->opt;
   o.precision = fp32 ? SPB_PRECISION_FP32_IR : SPB_PRECISION_FP64;
-  const spb::PlanParams want = plan_params_of(o);
+  const spb::PlanParams want = plan_params_of(o, h->sym);
   const spb::Plan* plan = &h->plan;
-  if (!(want == plan_params_of(h->opt))) {
+  if (!(want == plan_params_of(h->opt, h->sym))) {
     std::lock_guard<std::mutex> lock(h->pred_mu);
     std::unique_ptr<spb::Plan>& c = h->pred_plan[fp32 ? 1 : 0];
     if (!c || !(h->pred_prm[fp32 ? 1 : 0] == want)) {
@@ -909,7 +917,7 @@ int64_t predict_bytes(const spb_handle* h, bool fp32, int nrhs) {
 
 int install_symbolic(spb_handle* h, int32_t n, const int64_t* colptr, const int32_t* rowind) {
   try {
-    h->plan = spb::build_plan(h->sym, plan_params_of(h->opt));
+    h->plan = spb::build_plan(h->sym, plan_params_of(h->opt, h->sym));
     h->amap = spb::build_assembly_map(h->sym, h->plan, colptr, rowind);
   } catch (const std::bad_alloc&) {
     return fail(h, SPB_ERR_OOM, "symbolic: host allocation failed");
@@ -1124,11 +1132,11 @@ int spb_symbolic_from(spb_handle* h, const spb_handle* src) {
     h->nnz_a = src->nnz_a;
     h->colptr = src->colptr;
     h->rowind = src->rowind;
-    if (plan_params_of(h->opt) == plan_params_of(src->opt)) {  // same tunables: the same plan
+    if (plan_params_of(h->opt, h->sym) == plan_params_of(src->opt, src->sym)) {  // same tunables: the same plan
       h->plan = src->plan;
       h->amap = src->amap;
     } else {
-      h->plan = spb::build_plan(h->sym, plan_params_of(h->opt));
+      h->plan = spb::build_plan(h->sym, plan_params_of(h->opt, h->sym));
       h->amap = spb::build_assembly_map(h->sym, h->plan, h->colptr.data(), h->rowind.data());
     }
   } catch (const std::bad_alloc&) {
@@ -1598,7 +1606,7 @@ int spb_reorder_factor_from_trace(spb_handle* h) {
     us[i] = done > met ? (double)(done - met) * 1e-3 : 0.0;
   }
   try {
-    spb::reorder_factor_tasks(P, plan_params_of(h->opt), us);
+    spb::reorder_factor_tasks(P, plan_params_of(h->opt, h->sym), us);
   } catch (const std::exception& e) {
     return fail(h, SPB_ERR_INVALID, e.what());
   }

@@ -98,7 +98,7 @@ class symPACKOptions:
     plan_solve_chunk: int = 0      # 64-column blocks per solve super-block (0 = library default 8)
     plan_solve_tiles: int = 0      # 64 x 64 tiles per super-block solve task (0 = library default 2)
     factor_schedule: str = "auto"  # "persistent" (one launch; FP64, or FP32_IR with tcgen05-tma), "steps",
-                                   # or "auto" (persistent for FP64, steps for FP32_IR)
+                                   # or "auto" (persistent for FP64 and short FP32_IR factorizations)
 
     def to_c(self) -> N.spb_options:
         if self.orderingStr not in N.ORDERINGS:
