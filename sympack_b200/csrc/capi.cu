@@ -80,7 +80,7 @@ struct spb_handle {
   spb::SolveRec* dfsubs = nullptr;
   spb::SolveRec* dbsubs = nullptr;
   int32_t* dexpected = nullptr;
-  int32_t* dtiny = nullptr;        // leaf supernodes of the forward sweep's T tasks
+  spb::TinyRec* dtiny = nullptr;   // tiny leaf supernodes
   int32_t* dsparent = nullptr;
   int32_t* dsync = nullptr;  // solve counters (spb::solve_sync_ints)
   void* dInv = nullptr;      // diagonal super-block inverses of the forward operand (L, or L D for LDL^T)
@@ -446,14 +446,15 @@ void ensure_inverses(spb_handle* h) {
 // Forward and backward persistent sweeps on the permuted right-hand sides X (n x nrhs,
 // ld n; the solution replaces them), with Z (same shape) between the sweeps and the
 // counters of `groups` groups of kSolveGroup right-hand sides in sync; that many groups per
-// pass.  prof: record the per-pass events.
+// pass.  Z and the counters are zero at entry (launch_permute_in, launch_residual).  prof:
+// record the per-pass events.
 void enqueue_sweeps(spb_handle* h, double* X, double* Z, int32_t* sync, int groups, int nrhs, bool prof) {
   const spb::Plan& P = h->plan;
   const size_t ints = spb::solve_sync_ints(P);
   const int step = spb::kSolveGroup * groups;
   for (int c0 = 0, pass = 0; c0 < nrhs; c0 += step, ++pass) {
-    // counters must start at zero
-    cudaMemsetAsync(sync, 0, sizeof(int32_t) * ints * groups, h->stream);
+    // counters must start at zero; what filled X cleared them for the first pass, and Z
+    if (pass > 0) cudaMemsetAsync(sync, 0, sizeof(int32_t) * ints * groups, h->stream);
     spb::dev::PSolveArgs a{};
     // LDL^T: the forward sweep solves with L D (diagonal D), the backward one with unit L
     a.L = h->ldl ? (void*)h->dW : h->dL;
@@ -485,7 +486,6 @@ void enqueue_sweeps(spb_handle* h, double* X, double* Z, int32_t* sync, int grou
     a.trace = prof ? h->dtrace : nullptr;
     const size_t pass_bytes = sizeof(double) * (size_t)h->sym.n * a.nrhs;
     if (prof) cudaEventRecord(h->events[e0], h->stream);
-    cudaMemsetAsync(a.Z, 0, pass_bytes, h->stream);  // DI tasks of wide supernodes add into Z
     spb::dev::launch_solve_persistent(h->stream, a, true);
     if (prof) cudaEventRecord(h->events[e0 + 1], h->stream);
     a.L = h->dL;
@@ -503,6 +503,9 @@ void enqueue_sweeps(spb_handle* h, double* X, double* Z, int32_t* sync, int grou
     if (prof) cudaEventRecord(h->events[e0 + 3], h->stream);
   }
 }
+
+// Counters to clear for a solve on the handle's own workspace.
+int64_t sync_ints(const spb_handle* h) { return (int64_t)spb::solve_sync_ints(h->plan) * spb::kSolveGroups; }
 
 // Both sweeps on the handle's workspace h->dX (n x nrhs, ld n), inverses first if stale.
 void enqueue_solve(spb_handle* h, int nrhs) {
@@ -567,7 +570,7 @@ int check_solve_status(spb_handle* h) {
 // Solve with the factor as it is: b (ld ldb) -> x (ld ldx), through the permuted workspace.
 void plain_solve(spb_handle* h, const double* b, int64_t ldb, double* x, int64_t ldx, int nrhs) {
   const int n = h->sym.n;
-  spb::dev::launch_permute_in(h->stream, h->dX, n, b, ldb, h->dinvp0, n, nrhs);
+  spb::dev::launch_permute_in(h->stream, h->dX, n, b, ldb, h->dinvp0, n, nrhs, h->dZ, h->dsync, sync_ints(h));
   enqueue_solve(h, nrhs);
   spb::dev::launch_permute_out(h->stream, x, ldx, h->dX, n, h->dinvp0, n, nrhs);
 }
@@ -600,7 +603,7 @@ int ir_solve(spb_handle* h, const double* d_b, int64_t ldb, double* d_x, int64_t
       SPB_CK(h, cudaMemsetAsync(h->d_norms, 0, sizeof(double), h->stream));
       // the residual goes where a correction solve reads its right-hand sides
       spb::dev::launch_residual(h->stream, h->d_rowptr, h->d_col, h->d_val, x, ldx, b, ldb, h->dX, h->dinvp0, n, nr,
-                                h->d_rowseg, xmax, rmax);
+                                h->d_rowseg, xmax, rmax, h->dZ, h->dsync, sync_ints(h));
       spb::dev::launch_eta(h->stream, anorm, bmax, xmax, rmax, nseg, nr, h->d_norms);
       SPB_CK(h, cudaMemcpyAsync(&eta, h->d_norms, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
       int rc = check_solve_status(h);  // synchronizes
@@ -888,7 +891,7 @@ int64_t predict_bytes(const spb_handle* h, bool fp32, int nrhs) {
   t += b(P.tile_items.size(), sizeof(spb::TileItem)) + b(n, 4) + b(ns, 4);
   t += b(P.fwd_recs.size(), sizeof(spb::SolveRec)) + b(P.bwd_recs.size(), sizeof(spb::SolveRec));
   t += b(P.fwd_subs.size(), sizeof(spb::SolveRec)) + b(P.bwd_subs.size(), sizeof(spb::SolveRec));
-  t += b(P.fwd_wait.size(), 4) + b(P.tiny.size(), 4) + b(P.sparent.size(), 4) +
+  t += b(P.fwd_wait.size(), 4) + b(P.tiny_recs.size(), sizeof(spb::TinyRec)) + b(P.sparent.size(), 4) +
        b((int64_t)spb::solve_sync_ints(P) * spb::kSolveGroups, 4);
   t += b(P.inv_elems, fp32 ? sizeof(float) : sizeof(double)) + b(P.inv_items.size(), sizeof(spb::InvItem));
   t += b(P.inv1_elems, sizeof(double)) + b(P.inv1_items.size(), sizeof(spb::Inv1Item));
@@ -981,7 +984,7 @@ int install_device(spb_handle* h) {
   SPB_CK(h, dalloc(h, &h->dfsubs, P.fwd_subs.size()));
   SPB_CK(h, dalloc(h, &h->dbsubs, P.bwd_subs.size()));
   SPB_CK(h, dalloc(h, &h->dexpected, P.fwd_wait.size()));
-  SPB_CK(h, dalloc(h, &h->dtiny, P.tiny.size()));
+  SPB_CK(h, dalloc(h, &h->dtiny, P.tiny_recs.size()));
   SPB_CK(h, dalloc(h, &h->dsparent, P.sparent.size()));
   SPB_CK(h, dalloc(h, &h->dsync, spb::solve_sync_ints(P) * spb::kSolveGroups));
   {
@@ -1028,7 +1031,7 @@ int install_device(spb_handle* h) {
   SPB_CK(h, up(h->dfsubs, P.fwd_subs.data(), P.fwd_subs.size() * sizeof(spb::SolveRec)));
   SPB_CK(h, up(h->dbsubs, P.bwd_subs.data(), P.bwd_subs.size() * sizeof(spb::SolveRec)));
   SPB_CK(h, up(h->dexpected, P.fwd_wait.data(), P.fwd_wait.size() * 4));
-  SPB_CK(h, up(h->dtiny, P.tiny.data(), P.tiny.size() * 4));
+  SPB_CK(h, up(h->dtiny, P.tiny_recs.data(), P.tiny_recs.size() * sizeof(spb::TinyRec)));
   SPB_CK(h, up(h->dsparent, P.sparent.data(), P.sparent.size() * 4));
   SPB_CK(h, up(h->dinvitems, P.inv_items.data(), P.inv_items.size() * sizeof(spb::InvItem)));
   SPB_CK(h, up(h->dinv1items, P.inv1_items.data(), P.inv1_items.size() * sizeof(spb::Inv1Item)));
@@ -1349,7 +1352,7 @@ int spb_solve_device(spb_handle* h, const double* d_rhs, double* d_x, int32_t nr
   if (rc) return rc;
   if (h->fp32) return ir_solve(h, d_rhs, ld, d_x, ld, nrhs);
   if (h->profiling) SPB_CK(h, ensure_events(h, 4 * (size_t)((nrhs + 63) / 64) + 2));
-  spb::dev::launch_permute_in(h->stream, h->dX, n, d_rhs, ld, h->dinvp0, n, nrhs);
+  spb::dev::launch_permute_in(h->stream, h->dX, n, d_rhs, ld, h->dinvp0, n, nrhs, h->dZ, h->dsync, sync_ints(h));
   enqueue_solve(h, nrhs);
   rc = collect_solve_profile(h, nrhs);
   if (rc) return rc;
@@ -1377,7 +1380,7 @@ int spb_solve(spb_handle* h, const double* rhs, int32_t nrhs, int64_t ldb) {
     return SPB_OK;
   }
   if (h->profiling) SPB_CK(h, ensure_events(h, 4 * (size_t)((nrhs + 63) / 64)));
-  spb::dev::launch_permute_in(h->stream, h->dX, n, h->dB, n, h->dinvp0, n, nrhs);
+  spb::dev::launch_permute_in(h->stream, h->dX, n, h->dB, n, h->dinvp0, n, nrhs, h->dZ, h->dsync, sync_ints(h));
   enqueue_solve(h, nrhs);
   rc = collect_solve_profile(h, nrhs);
   if (rc) return rc;
@@ -1763,10 +1766,10 @@ extern "C" int spb_solve_device_noalloc(spb_handle* h, const double* d_rhs, doub
   double* X = reinterpret_cast<double*>(base);
   double* Z = reinterpret_cast<double*>(base + kNoAllocXBytes);
   int32_t* sync = reinterpret_cast<int32_t*>(base + 2 * kNoAllocXBytes);
-  spb::dev::launch_permute_in(h->stream, X, n, d_rhs, ld, h->dinvp0, n, nrhs);
   ensure_inverses(h);  // the first solve after a factorization computes them (arena of the analysis)
   const size_t ints = spb::solve_sync_ints(h->plan) * sizeof(int32_t);  // as many groups as the counters have room for
   const int groups = (int)std::min<size_t>(spb::kSolveGroups, kNoAllocSyncBytes / ints);
+  spb::dev::launch_permute_in(h->stream, X, n, d_rhs, ld, h->dinvp0, n, nrhs, Z, sync, (int64_t)(ints / 4) * groups);
   enqueue_sweeps(h, X, Z, sync, groups, nrhs, false);
   spb::dev::launch_permute_out(h->stream, d_x, ld, X, n, h->dinvp0, n, nrhs);
   SPB_CK(h, cudaGetLastError());

@@ -75,7 +75,8 @@ __global__ void k_segmax(const double* __restrict__ v, int n, int64_t ld, const 
 
 // One refinement step's view of the current x: r = b - A x, stored permuted (R[invp[i] + c n],
 // the right-hand side of the correction solve), with max |x| and max |r| per system and
-// column (xmax, rmax; layout as in k_segmax) taken on the way.  Bound by the reads of A: four
+// column (xmax, rmax; layout as in k_segmax) taken on the way and Z and the counters cleared
+// for the correction's sweeps.  Bound by the reads of A: four
 // lanes share a row, so that a load of val takes whole sectors, and CB columns share each
 // entry of A, so that A is read ceil(nrhs / CB) times.  A block takes a contiguous run of rows
 // and keeps its maxima in registers to the end of the run (or of a system).  27-point 36^3, 50
@@ -87,10 +88,15 @@ __global__ void __launch_bounds__(kResThreads) k_residual(const int64_t* __restr
                                                           int64_t ldx, const double* __restrict__ b, int64_t ldb,
                                                           double* __restrict__ R, const int32_t* __restrict__ invp0,
                                                           int n, int nrhs, const int32_t* __restrict__ rowseg,
-                                                          double* __restrict__ xmax, double* __restrict__ rmax) {
+                                                          double* __restrict__ xmax, double* __restrict__ rmax,
+                                                          double* __restrict__ Z, int32_t* __restrict__ sync,
+                                                          int64_t nsync) {
   constexpr int kOwn = (CB + 3) / 4;  // columns whose sums a lane finishes
   __shared__ unsigned long long smax[2][CB];
   const int c0 = blockIdx.y * CB, nc = min(CB, nrhs - c0), q = threadIdx.x & 3;
+  for (int64_t i = (blockIdx.y * (int64_t)gridDim.x + blockIdx.x) * kResThreads + threadIdx.x; i < nsync;
+       i += (int64_t)gridDim.x * gridDim.y * kResThreads)
+    sync[i] = 0;
   if (threadIdx.x < 2 * CB) smax[threadIdx.x / CB][threadIdx.x % CB] = 0;
   __syncthreads();
   const int64_t chunk = ((n + gridDim.x - 1) / gridDim.x + 63) / 64 * 64;
@@ -154,6 +160,7 @@ __global__ void __launch_bounds__(kResThreads) k_residual(const int64_t* __restr
         if (4 * o + e < CB && q == e) sum = s[4 * o + e];
       const double r = bv[o] - sum;
       R[pr + (int64_t)(c0 + c) * n] = r;
+      Z[i + (int64_t)(c0 + c) * n] = 0.0;
       mr[o] = fmax(mr[o], fabs(r));
       mx[o] = fmax(mx[o], fabs(xv[o]));
     }
@@ -238,12 +245,12 @@ void launch_gather(cudaStream_t st, double* dst, const double* src, const int64_
 
 void launch_residual(cudaStream_t st, const int64_t* rowptr, const int32_t* col, const double* val, const double* x,
                      int64_t ldx, const double* b, int64_t ldb, double* R, const int32_t* invp0, int n, int nrhs,
-                     const int32_t* rowseg, double* xmax, double* rmax) {
+                     const int32_t* rowseg, double* xmax, double* rmax, double* Z, int32_t* sync, int64_t nsync) {
   auto run = [&](auto cb) {
     constexpr int CB = decltype(cb)::value;
     const int by = (nrhs + CB - 1) / CB, rows = (n + 63) / 64, cap = (148 * 16 + by - 1) / by;
     k_residual<CB><<<dim3(rows < cap ? rows : cap, by), kResThreads, 0, st>>>(rowptr, col, val, x, ldx, b, ldb, R, invp0,
-                                                                              n, nrhs, rowseg, xmax, rmax);
+                                                                              n, nrhs, rowseg, xmax, rmax, Z, sync, nsync);
   };
   if (nrhs == 1) run(std::integral_constant<int, 1>());
   else if (nrhs <= 4) run(std::integral_constant<int, 4>());

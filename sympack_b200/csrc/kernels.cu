@@ -60,11 +60,14 @@ __global__ void __launch_bounds__(kThreads, 2) k_trsm_rows(FactorArgs a, const P
 }
 
 __global__ void k_permute_in(double* X, int64_t ldx, const double* B, int64_t ldb, const int32_t* invp0, int n,
-                             int nrhs) {
+                             int nrhs, double* __restrict__ Z, int32_t* __restrict__ sync, int64_t nsync) {
   int64_t total = (int64_t)n * nrhs;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nsync; i += (int64_t)gridDim.x * blockDim.x)
+    sync[i] = 0;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
     int c = (int)(i / n), r = (int)(i - (int64_t)c * n);
     X[invp0[r] + c * ldx] = B[r + c * ldb];
+    Z[i] = 0.0;
   }
 }
 
@@ -135,8 +138,8 @@ void launch_trsm_rows(cudaStream_t st, const FactorArgs& a, const PanelItem* ite
 }
 
 void launch_permute_in(cudaStream_t st, double* X, int64_t ldx, const double* B, int64_t ldb,
-                       const int32_t* invp0, int n, int nrhs) {
-  k_permute_in<<<grid_for((int64_t)n * nrhs, 256), 256, 0, st>>>(X, ldx, B, ldb, invp0, n, nrhs);
+                       const int32_t* invp0, int n, int nrhs, double* Z, int32_t* sync, int64_t nsync) {
+  k_permute_in<<<grid_for((int64_t)n * nrhs, 256), 256, 0, st>>>(X, ldx, B, ldb, invp0, n, nrhs, Z, sync, nsync);
 }
 
 void launch_permute_out(cudaStream_t st, double* B, int64_t ldb, const double* X, int64_t ldx,

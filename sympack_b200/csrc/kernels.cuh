@@ -104,7 +104,7 @@ struct PSolveArgs {
   const SolveRec* recs;
   const SolveRec* subs;
   int ntasks;
-  const int32_t* tiny;  // tiny leaf supernodes (Plan::tiny)
+  const TinyRec* tiny;  // tiny leaf supernodes (Plan::tiny_recs)
   int ntiny;
   int64_t tiny_task0;   // place of their first batch in the task list (trace)
   int32_t* counter;
@@ -131,7 +131,7 @@ void launch_diag_inverse(cudaStream_t st, const void* L, double* Inv, bool fp32,
 void launch_gather(cudaStream_t st, double* dst, const double* src, const int64_t* idx, int64_t n);
 void launch_residual(cudaStream_t st, const int64_t* rowptr, const int32_t* col, const double* val, const double* x,
                      int64_t ldx, const double* b, int64_t ldb, double* R, const int32_t* invp0, int n, int nrhs,
-                     const int32_t* rowseg, double* xmax, double* rmax);
+                     const int32_t* rowseg, double* xmax, double* rmax, double* Z, int32_t* sync, int64_t nsync);
 void launch_segmax(cudaStream_t st, const double* v, int n, int nrhs, int64_t ld, const int32_t* rowseg,
                    double* out);
 void launch_rowsum_segmax(cudaStream_t st, const int64_t* rowptr, const double* val, int n, const int32_t* rowseg,
@@ -139,9 +139,10 @@ void launch_rowsum_segmax(cudaStream_t st, const int64_t* rowptr, const double* 
 void launch_eta(cudaStream_t st, const double* anorm, const double* bmax, const double* xmax, const double* rmax,
                 int nseg, int nrhs, double* eta);
 
-// X[invp[i], c] = B[i, c],   B[i, c] = X[invp[i], c]   and   B[i, c] += X[invp[i], c]
+// X[invp[i], c] = B[i, c],   B[i, c] = X[invp[i], c]   and   B[i, c] += X[invp[i], c].  What
+// fills X also clears Z (n x nrhs, ld n) and the first nsync counters for the sweeps.
 void launch_permute_in(cudaStream_t st, double* X, int64_t ldx, const double* B, int64_t ldb,
-                       const int32_t* invp0, int n, int nrhs);
+                       const int32_t* invp0, int n, int nrhs, double* Z, int32_t* sync, int64_t nsync);
 void launch_permute_out(cudaStream_t st, double* B, int64_t ldb, const double* X, int64_t ldx,
                         const int32_t* invp0, int n, int nrhs);
 void launch_permute_add(cudaStream_t st, double* B, int64_t ldb, const double* X, int64_t ldx,

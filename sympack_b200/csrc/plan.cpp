@@ -603,6 +603,11 @@ static void build_solve_recs(Plan& P) {
   };
   fill(P.fwd_tasks, true, P.fwd_recs, P.fwd_subs);
   fill(P.bwd_tasks, false, P.bwd_recs, P.bwd_subs);
+  P.tiny_recs.resize(P.tiny.size());
+  for (size_t i = 0; i < P.tiny.size(); ++i) {
+    const SnMeta& m = P.meta[P.tiny[i]];
+    P.tiny_recs[i] = TinyRec{m.off, (int32_t)m.lidx, m.fc, m.ld, m.w, m.h, P.tiny[i]};
+  }
   P.fwd_wait = P.fwd_pending;
   for (int32_t s : P.tiny) {
     const SnMeta& m = P.meta[s];
@@ -731,9 +736,11 @@ static void build_factor_dag(Plan& P, const PlanParams& prm, const std::vector<d
         const double fl = 2.0 * t.mrows * t.ncols * t.kn;
         // fixed cost + per-CTA rate (FP64 128 x 64 tiles at two CTAs per SM, FP32 3xTF32
         // tiles at one).  The FP64 figures, like the small-panel, diagonal-block and TRSM
-        // times above, fit the per-kind duration quantiles of the task timeline of a traced
-        // 60^3 Laplacian factorization (spb_get_factor_trace): a 128 x 64 tile costs about
-        // 11 us before its first flop (pipeline fill, dependency reads, atomic epilogue)
+        // times above, were fitted to the per-kind duration quantiles of the task timeline of
+        // a traced 60^3 Laplacian factorization (spb_get_factor_trace).  The tasks have become
+        // faster since, but today's medians in their place (17 us a diagonal block, 9 a row
+        // tile, 7.5 us + flops / 100 GFLOP/s a 128 x 64 tile) ordered the tasks no better: 60^3
+        // 30.28 -> 30.38 ms, 27-point 60^3 73.97 -> 74.18, 463 x 467 grid 3.43 -> 3.38
         r.us = st.tile == 128 ? (prm.fp32 ? 3.0 + fl / 600e3 : 11.0 + fl / 105e3) : 5.0 + fl / 16.7e3;
         if (t.mode == 0) {
           for (int c = t.b_row0 / 64; c <= (t.b_row0 + t.ncols - 1) / 64; ++c) {

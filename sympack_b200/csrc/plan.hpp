@@ -203,6 +203,16 @@ SPB_HD inline int solve_done_count(int w, int sb, int tpt) {
   return nblk == 1 ? 1 : solve_di_range(nblk, sb, tpt, 0, (nblk + sb - 1) / sb);
 }
 
+// A tiny leaf supernode as its kernels read it (one load before everything else).
+struct alignas(16) TinyRec {
+  int64_t off;   // its panel
+  int32_t lidx;  // its row list
+  int32_t fc;
+  int32_t ld;
+  int32_t w, h;
+  int32_t s;
+};
+
 // One CTA of the super-block inverse kernel: column block j of Inv_p of supernode s
 // (tiles (i, j), i = j .. nb_p - 1).
 struct InvItem {
@@ -275,6 +285,7 @@ struct Plan {
   std::vector<SolveRec> fwd_subs, bwd_subs;  // the records of their batches
   std::vector<int32_t> fwd_wait;             // arrivals the forward sweep waits for (without the tiny leaves')
   std::vector<int32_t> tiny;  // leaf supernodes of the forward T tasks
+  std::vector<TinyRec> tiny_recs;  // the same as device records
   int32_t nblk_total = 0;  // 64-column blocks over all supernodes
   int32_t nsb_total = 0;   // solve super-blocks over all supernodes (per-super-block counters)
   int32_t solve_sb = 8;    // 64-column blocks per solve super-block

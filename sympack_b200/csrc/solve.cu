@@ -242,7 +242,7 @@ __device__ __forceinline__ void apply_inverse(double* out, int64_t ldx, double* 
 // to wait for) by one thread: Z_0 <- L_00^-1 Y_0 by substitution (multiplying by the pivots'
 // reciprocals), then Y[ancestor rows] -= L_u0 Z_0 with atomic additions.
 template <class T>
-__device__ __forceinline__ void tiny_forward(const PSolveArgs& a, const SnMeta& m, int64_t xo) {
+__device__ __forceinline__ void tiny_forward(const PSolveArgs& a, const TinyRec& m, int64_t xo) {
   const T* P = static_cast<const T*>(a.L) + m.off;
   const int32_t* rl = a.rows + m.lidx;
   const int w = m.w, h = m.h;
@@ -271,7 +271,7 @@ __device__ __forceinline__ void tiny_forward(const PSolveArgs& a, const SnMeta& 
 // Backward sweep of one column of a tiny leaf supernode by one thread, its parent done:
 // Z_0 -= L_u0^T X[ancestor rows], then X_0 <- L_00^-T Z_0 by substitution.
 template <class T>
-__device__ __forceinline__ void tiny_backward(const PSolveArgs& a, const SnMeta& m, int64_t xo) {
+__device__ __forceinline__ void tiny_backward(const PSolveArgs& a, const TinyRec& m, int64_t xo) {
   const T* P = static_cast<const T*>(a.L) + m.off;
   const int32_t* rl = a.rows + m.lidx;
   const int w = m.w, h = m.h;
@@ -300,15 +300,16 @@ __device__ __forceinline__ void tiny_backward(const PSolveArgs& a, const SnMeta&
 // Tiny leaf supernodes of one sweep, one thread per leaf and column (leaves fastest).
 template <class T, bool kFwd>
 __global__ void __launch_bounds__(128) k_solve_tiny(PSolveArgs a) {
-  if (status_code(a.status) != 0) return;
+  const int st = status_code(a.status);  // in flight beside the first record
   const int64_t total = (int64_t)a.ntiny * a.nrhs;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
     const int c = (int)(i / a.ntiny), j = (int)(i - (int64_t)c * a.ntiny);
-    const SnMeta m = a.meta[a.tiny[j]];
+    const TinyRec m = a.tiny[j];
+    if (st != 0) return;
     unsigned long long* tr = a.trace && c == 0 && j % kTinyBatch == 0 ? a.trace + 4 * (a.tiny_task0 + j / kTinyBatch) : nullptr;
     if (tr) {
       tr[0] = tr[1] = now_ns();
-      tr[3] = ((unsigned long long)a.tiny[j] << 8) | 6;
+      tr[3] = ((unsigned long long)m.s << 8) | 6;
     }
     if (kFwd) tiny_forward<T>(a, m, c * a.ldx);
     else tiny_backward<T>(a, m, c * a.ldx);
