@@ -791,9 +791,8 @@ def run_ours(args):
 
     K = args.steps
     # per step: assemble, the factorization (one persistent launch), then two solves (permute in,
-    # forward, backward, permute out), the first one after the factorization also computing the
-    # diagonal super-block inverses
-    # assembly, factorization, two solves (permutations, tiny leaves and sweeps), block inverses
+    # tiny leaves, forward, backward, tiny leaves, permute out), the first one after the
+    # factorization also computing the super-block and diagonal block inverses
     launches_per_step = 1 + info.factor_launches + 6 + 6 + (3 if info.inverse_bytes else 0)
     if rank == 0:
         line = {

@@ -109,7 +109,8 @@ __device__ __forceinline__ void piece_rows(double (&x)[kPiece], double (&rs)[kPi
 // the panel by a warp per column; the update's 16 x 8 tiles on the FP64 tensor pipe, in FP64
 // for FP32 panels too, scattered from the accumulators through the relative indices, whose
 // column tables are fetched while the panel is loaded.  Bound by latency: global round trips
-// and the chain of pivots.  sm: kSmallHeadDoubles doubles (D of LDL^T, column tables), then
+// and the chain of pivots.  463 x 467 grid: 5.9 us a panel with its update; the panel by
+// single columns took 6.1 us and the separate 64 x 64 update task 5.4 us and a dispatch.  sm: kSmallHeadDoubles doubles (D of LDL^T, column tables), then
 // the panel; cap = doubles of shared memory.
 constexpr int kSmallHeadDoubles = 64 + 2 * kFuseRows;
 
@@ -287,7 +288,8 @@ constexpr int kDiagSmemDoubles = kNB * kDL + 2 * kNB + 2 * kPiece * kDL;
 // finished columns and the pieces' inverses are written out beside the next pieces.
 // The scratch slot gets the factored block (FP64) with the inverses of its 8 x 8 diagonal
 // pieces transposed into their upper triangles, 1/L_kk (1 for LDL^T, whose TRSM then computes
-// W's rows) and 1/D_kk.  LDL^T: L takes the unit block, W the block times D (its diagonal is
+// W's rows) and 1/D_kk.  11 us a block measured alone, 13 to 18 us beside other tasks; the
+// scalar version (the trailing triangle as a chain of shared-memory FMAs) took 19 to 25 us.  LDL^T: L takes the unit block, W the block times D (its diagonal is
 // D).  A block narrower than 64 is padded with the identity.
 template <class T, bool kLdl>
 __device__ __forceinline__ void diag_task(const FactorArgs& a, const PanelItem& it, const SnMeta& meta,
@@ -447,8 +449,8 @@ __device__ __forceinline__ void diag_task(const FactorArgs& a, const PanelItem& 
 // 8-column tiles, the other the odd ones); a piece's 16 x 8 tile is multiplied by the piece's
 // inverse (2 MMA steps) by the warp that has it, and the solved columns are applied to the
 // later tiles (2 steps each) by both, through the pair's rows in shared memory.  Bound by that chain; no scalar FP64 instruction is on it, since each would
-// queue behind the update tiles that share the SM in the persistent factorization (a thread
-// per row substituting took 9.8 us a tile there, 12.8 us beside update tiles).
+// queue behind the update tiles that share the SM in the persistent factorization (8 to 9 us
+// a tile there; a thread per row substituting took 9.8 us, 12.8 us beside update tiles).
 // Shared memory (doubles) of trsm_rows_task.
 constexpr int kTrsmSmemDoubles = 2 * kNB * kDL + kNB;
 

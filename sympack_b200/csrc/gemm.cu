@@ -6,15 +6,16 @@
 //   then the src_to_tgt_offset / colindx scatter of 2D.hpp:1395-1466), fused so
 //   that C never leaves the SM.
 //
-// Tile engines (one shared epilogue for the tiles staged in shared memory):
+// Tile engines:
 //   k_gemm_dmma   128 x 64 FP64 tiles on the FP64 tensor pipe (mma.sync m16n8k4 .f64),
-//                 3-stage cp.async pipeline, 8 warps of 32 x 32, two CTAs per SM
+//                 bulk-copy pipeline, 8 warps of 32 x 32, two CTAs per SM, subtracted from
+//                 the accumulators
 //   k_gemm_simt   64 x 64 tiles with FMA, for narrow updates
 //   k_gemm_tc32   128 x 128 FP32 tiles, 3xTF32 on tcgen05, operands staged by cp.async
 //   k_gemm_tc32w  the same on TMA-loaded split copies, persistent and warp-specialised
 //                 (tc32t_tile_task: one such tile, a task of the persistent FP32 factorization)
 //   k_gemm_tc32p, k_gemm_tf32x3   a persistent tcgen05 variant and an mma.sync one
-// The epilogue stages C in shared memory and walks it column by column, so
+// Tiles staged in shared memory share an epilogue that walks C column by column, so
 // consecutive threads touch consecutive target rows (coalesced atomics).
 #include <climits>
 #include <type_traits>
@@ -134,7 +135,7 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, long lo
 // refills it.  No block-wide barrier in the K loop.  Copies start on 16-byte boundaries,
 // so an operand's rows are counted from the even row at or below its first row: accumulator
 // row i is panel row (a_row0 & ~1) + i (the plan cuts these tiles so that they fit).
-constexpr int kDM = 128, kDK = 16, kDStages = 4, kDLds = 132, kDLdc = 130, kDThreads = 256;
+constexpr int kDM = 128, kDK = 16, kDStages = 4, kDLds = 132, kDThreads = 256;
 constexpr int kDTileN = 64;  // FP64 update tiles are 128 x 64
 template <int BN>
 struct DTile {
@@ -143,8 +144,7 @@ struct DTile {
   static constexpr int kMI = kDM / kWarpsM / 16;  // 16-row MMA tiles per warp
   static constexpr int kStageElems = kDK * (kDLds + kLdb);
   static constexpr size_t kPipeBytes = (size_t)kDStages * kStageElems * sizeof(double);
-  static constexpr size_t kCBytes = (size_t)BN * kDLdc * sizeof(double);
-  static constexpr size_t kMainBytes = kPipeBytes > kCBytes ? kPipeBytes : kCBytes;
+  static constexpr size_t kMainBytes = kPipeBytes;
   static constexpr size_t kIntsBytes = 4 * 128 * sizeof(int);
   static constexpr size_t kSmemBytes = kMainBytes + kIntsBytes + 2 * kDStages * sizeof(uint64_t);
   static_assert((kDLds * 8) % 16 == 0 && (kLdb * 8) % 16 == 0 && (kStageElems * 8) % 16 == 0,
@@ -342,7 +342,7 @@ __device__ bool dmma_tile_task(const FactorArgs& a, const TileItem& item, const 
   // accumulators: a warp's reduction covers four columns of 8 consecutive rows, as many
   // sectors as 32 rows of one column, and no warp waits for another (through a shared-memory
   // copy of the tile, with its two barriers and the column table fetched in between, a tile
-  // cost about 11 us beside its flops).  A row's place in a target is loaded once per group.
+  // cost about 11 us beside its flops; about 7.5 us now).  A row's place in a target is loaded once per group.
   double* L = static_cast<double*>(a.L);
   const int jr0 = a0 + wm * (16 * D::kMI) + gq, rend = it.a_row0 + it.mrows;
   int64_t last = INT64_MIN;  // group offsets (rel_off - j0) can be negative

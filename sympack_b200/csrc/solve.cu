@@ -32,7 +32,9 @@
 // the wait only the right-hand sides pass through shared memory.  The products run
 // on the FP64 tensor pipe for one right-hand side too: an 8-column group costs no
 // more issue slots than scalar FMAs with their shared-memory reads would.
-// FP32 factors are widened as they enter a product.
+// FP32 factors are widened as they enter a product.  60^3 Laplacian, FP64: 1 right-hand side
+// 2.16 -> 1.20 ms, 16 right-hand sides 4.85 -> 2.09 ms against tasks that staged their tiles
+// in shared memory and multiplied with scalar FMAs (0.34 ms by the bytes of both sweeps).
 #include <type_traits>
 
 #include "kernels.cuh"
@@ -62,6 +64,8 @@ struct SolveSmem {
   double z[8 * 20 * 8 * NG];     // solved rows: 64 of a block (ld kZLd) or 16 per warp (ld kWzLd)
   int rows[kRowCap];
 };
+// Three CTAs per SM where the fragments of a pair of tiles leave room in 80 registers (FP32, one
+// group); FP64 fragments spill there (60^3, 1 right-hand side: 1.22 -> 1.69 ms).
 template <class T, int NG>
 constexpr int solve_min_blocks() { return NG == 1 && sizeof(T) == 4 ? 3 : 2; }
 
