@@ -1672,6 +1672,19 @@ __device__ __forceinline__ void next_task(const FactorArgs& a, const FactorSched
   }
 }
 
+// LDL^T's small panels and diagonal blocks as calls: with both bodies inlined that instance
+// spills in its tiles (quasi-definite 50^3 step 22.30 ms inlined, 22.07 called; the Cholesky
+// instance the other way round, 64-system batch 109.6 against 110.7 ms).
+template <class T>
+__device__ __noinline__ void small_ldl_call(const FactorArgs& a, int s, const SnMeta& m, double* sm) {
+  ftask::factor_small_task<T, true>(a, s, m, sm, kFSmallCap);
+}
+template <class T>
+__device__ __noinline__ void diag_ldl_call(const FactorArgs& a, const PanelItem& it, const SnMeta& m, double* winv,
+                                           double* sm) {
+  ftask::diag_task<T, true>(a, it, m, winv, sm);
+}
+
 // FP64: two CTAs per SM (128 x 64 DMMA tiles); FP32: one (the TMA-fed tile's 193 KB).
 template <class T, bool kLdl>
 __global__ void __launch_bounds__(256, std::is_same<T, float>::value ? 1 : 2)
@@ -1694,11 +1707,16 @@ __global__ void __launch_bounds__(256, std::is_same<T, float>::value ? 1 : 2)
     int sig = warp == 0 && lane < nsig ? f.sigs[sig0 + lane] : -1;
     switch (kind) {
       case 0:
-        ftask::factor_small_task<T, kLdl>(a, nx.item[0], nx.m, reinterpret_cast<double*>(smem_f), kFSmallCap);
+        if constexpr (kLdl) small_ldl_call<T>(a, nx.item[0], nx.m, reinterpret_cast<double*>(smem_f));
+        else ftask::factor_small_task<T, false>(a, nx.item[0], nx.m, reinterpret_cast<double*>(smem_f), kFSmallCap);
         break;
       case 1:
-        ftask::diag_task<T, kLdl>(a, *reinterpret_cast<const PanelItem*>(nx.item), nx.m, f.winv,
-                                  reinterpret_cast<double*>(smem_f));
+        if constexpr (kLdl)
+          diag_ldl_call<T>(a, *reinterpret_cast<const PanelItem*>(nx.item), nx.m, f.winv,
+                           reinterpret_cast<double*>(smem_f));
+        else
+          ftask::diag_task<T, false>(a, *reinterpret_cast<const PanelItem*>(nx.item), nx.m, f.winv,
+                                     reinterpret_cast<double*>(smem_f));
         break;
       case 2:
         ftask::trsm_rows_task<T>(a, *reinterpret_cast<const PanelItem*>(nx.item), nx.m, f.winv,
