@@ -80,7 +80,8 @@ typedef struct spb_options {
   double ir_tolerance;     /* backward-error target of refinement (1e-12) */
   int ir_max_iter;         /* refinement iteration cap */
   int verbose;
-  int plan_small_max_w;    /* widest supernode factored whole in shared memory (0 = default 32) */
+  int plan_small_max_w;    /* widest supernode factored whole in shared memory (0 = default 32); panels of
+                              more than 96 KB of doubles never are, so 110 columns is the widest */
   int plan_big_tile_rows;  /* products with this many rows use 128 x 128 tensor-core tiles (0 = default 128) */
   int fp32_engine;         /* FP32_IR 128 x 128 update tiles: 3 = tcgen05 with its operands loaded by
                               TMA from split (hi / lo) copies of the panels, one tensor map per panel

@@ -110,16 +110,15 @@ __device__ __forceinline__ void piece_rows(double (&x)[kPiece], double (&rs)[kPi
 // for FP32 panels too, scattered from the accumulators through the relative indices, whose
 // column tables are fetched while the panel is loaded.  Bound by latency: global round trips
 // and the chain of pivots.  463 x 467 grid: 5.9 us a panel with its update; the panel by
-// single columns took 6.1 us and the separate 64 x 64 update task 5.4 us and a dispatch.  sm: kSmallHeadDoubles doubles (D of LDL^T, column tables), then
-// the panel; cap = doubles of shared memory.
-constexpr int kSmallHeadDoubles = 64 + 2 * kFuseRows;
-
+// single columns took 6.1 us and the separate 64 x 64 update task 5.4 us and a dispatch.
+// sm: kSmallHeadDoubles doubles (D of LDL^T, column tables), then the panel; cap = doubles of
+// shared memory.
 template <class T, bool kLdl>
 __device__ __forceinline__ void factor_small_task(const FactorArgs& a, int s, const SnMeta& meta, double* sm, int cap) {
   const SnMeta m = meta;
   const int h = m.h, w = m.w, M = h - w;
   double* Dk = sm;
-  int64_t* cbase = reinterpret_cast<int64_t*>(sm + 64);
+  int64_t* cbase = reinterpret_cast<int64_t*>(sm + kSmallDEntries);
   int64_t* crel = cbase + kFuseRows;
   double* P = sm + kSmallHeadDoubles;
   const int pad = (h + 11) / 16 * 16 + 4;  // 4 mod 16: conflict-free fragment reads

@@ -1604,7 +1604,7 @@ __device__ __forceinline__ unsigned smid() {
 constexpr size_t kFSmemBytes = kDSmemBytes;  // the DMMA pipe and its barriers (above every other body's)
 // what a small-panel task may use: everything below the DMMA stage barriers
 constexpr int kFSmallCap = (int)((kFSmemBytes - 2 * kDStages * sizeof(uint64_t)) / sizeof(double));
-static_assert(kFSmallCap >= 96 * 1024 / 8 + ftask::kSmallHeadDoubles, "small panels (96 KB) fit");
+static_assert(kFSmallCap >= kSmallPanelBytes / 8 + kSmallHeadDoubles, "small panels (96 KB) fit");
 constexpr size_t kFSmemBytes32 = kVSmemBytes;
 static_assert(kFSmemBytes32 >= kFSmallCap * sizeof(double) + 1024, "FP32 persistent shared memory");
 

@@ -83,7 +83,7 @@ __global__ void k_permute_out(double* B, int64_t ldb, const double* X, int64_t l
 }
 
 // shared memory of the largest small panel (96 KB) and what its task keeps before it
-constexpr int kSmallSmemMax = 96 * 1024 + kSmallHeadDoubles * 8;
+constexpr int kSmallSmemMax = kSmallPanelBytes + kSmallHeadDoubles * 8;
 
 int grid_for(int64_t work, int threads) {
   int64_t g = (work + threads - 1) / threads;

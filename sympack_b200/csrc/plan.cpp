@@ -66,7 +66,7 @@ Plan build_plan(const Symbolic& sym, const PlanParams& prm) {
   P.is_big.assign(ns, 0);
   for (int s = 0; s < ns; ++s) {
     const SnMeta& m = P.meta[s];
-    bool small = m.w <= prm.small_max_w && (int64_t)m.h * m.w * 8 <= prm.small_max_bytes;
+    bool small = m.w <= prm.small_max_w && (int64_t)m.h * m.w * 8 <= std::min(prm.small_max_bytes, kSmallPanelBytes);
     P.is_big[s] = small ? 0 : 1;
     double w = m.w, mm = m.h - m.w;
     P.exec_flops += w * w * w / 3.0 + mm * w * w + mm * mm * w;

@@ -55,6 +55,15 @@ struct TileItem {
 // A small panel (factored whole in shared memory) scatters its external update itself when
 // its product has too few rows for a tensor-core tile of its own, at most kFuseRows.
 constexpr int kFuseRows = 128;
+// Largest small panel (doubles in shared memory), whatever width is asked for, and the widest
+// that size allows: a panel has at least as many rows as columns.  The panel's task keeps
+// kSmallHeadDoubles in front of it: D of LDL^T, an entry per column, and two column tables.
+constexpr int kSmallPanelBytes = 96 * 1024;
+constexpr int kSmallMaxW = 110;
+static_assert((kSmallMaxW + 1) * (kSmallMaxW + 1) * 8 > kSmallPanelBytes, "no small panel is wider");
+constexpr int kSmallDEntries = 112;
+static_assert(kSmallDEntries >= kSmallMaxW && kSmallDEntries % 2 == 0, "D of the widest small panel");
+constexpr int kSmallHeadDoubles = kSmallDEntries + 2 * kFuseRows;
 #ifdef __CUDACC__
 __host__ __device__
 #endif
@@ -317,7 +326,7 @@ constexpr int kTinyMaxW = 4, kTinyMaxElems = 64, kTinyBatch = 128;
 // Tunables of the plan.
 struct PlanParams {
   int small_max_w = 32;          // widest panel handled by the fused small-panel kernel
-  int small_max_bytes = 96 * 1024;
+  int small_max_bytes = kSmallPanelBytes;  // at most kSmallPanelBytes
   int nb = 64;                   // column block of the blocked panel factorization
   int outer_nb = 256;            // outer block: the trailing columns are updated once per outer block
   int big_tile_rows = 128;       // products with at least this many rows use 128 x 128 tensor-core tiles

@@ -73,6 +73,7 @@ static void path_matrix(int n, std::vector<int64_t>& cp, std::vector<int32_t>& r
 }
 
 static long long n_rel = 0;
+static int widest_small = 0;
 
 static void check_plan(const Symbolic& sym, const PlanParams& prm, const char* what) {
   const Plan P = build_plan(sym, prm);
@@ -104,6 +105,15 @@ static void check_plan(const Symbolic& sym, const PlanParams& prm, const char* w
       }
     }
     CHECK(!bad, "%s: relative indices differ from a merge of the row lists", what);
+  }
+  // small panels: what their task keeps in shared memory holds D of the widest one, however
+  // wide the caller lets them be
+  for (int s = 0; s < P.nsuper; ++s) {
+    const SnMeta& m = P.meta[s];
+    if (P.is_big[s]) continue;
+    widest_small = std::max(widest_small, m.w);
+    CHECK(m.w <= kSmallDEntries, "%s: small panel %d has %d columns", what, s, m.w);
+    CHECK(m.w <= prm.small_max_w && (int64_t)m.h * m.w * 8 <= kSmallPanelBytes, "%s: small panel %d x %d", what, m.h, m.w);
   }
   // tiles
   for (const Step& st : P.steps) {
@@ -462,6 +472,23 @@ int main() {
     small.solve_sb = 3;
     small.solve_tpt = 1;
     check_plan(forest, small, "batch FP64 small blocks");
+  }
+  // small panels of any width that fits in shared memory: dense blocks of 140, 111 and 110
+  // columns, of which only the last one is small enough
+  {
+    std::vector<Symbolic> parts;
+    std::vector<int64_t> cp;
+    std::vector<int32_t> ri;
+    for (int n : {140, 111, 110}) {
+      dense_matrix(n, cp, ri);
+      parts.push_back(symbolic_factorization(n, cp.data(), ri.data(), OrderingKind::NATURAL, RelaxParams()));
+    }
+    PlanParams wide;
+    wide.factor_dag = true;
+    wide.small_max_w = 4096;
+    wide.small_max_bytes = 1 << 20;
+    check_plan(merge_symbolic(parts), wide, "wide small panels");
+    CHECK(widest_small == kSmallMaxW, "widest small panel %d", widest_small);
   }
   if (fails) {
     std::fprintf(stderr, "%d violations\n", fails);

@@ -32,6 +32,25 @@ def test_panel_tasks_match_the_oracle(border, dec, schedule):
     M.close()
 
 
+@pytest.mark.parametrize("schedule", ["persistent", "steps"])
+@pytest.mark.parametrize("dec", ["LL", "LDL"])
+@pytest.mark.parametrize("width,border", [(65, 60), (65, 123), (80, 60), (96, 32), (110, 1)])
+def test_small_panels_wider_than_64_columns(width, border, dec, schedule):
+    """plan_small_max_w above 64: panels up to the widest that fit in shared memory (110 columns,
+    96 KB), D of LDL^T kept beside the column tables of the fused update."""
+    A = DistSparseMatrix.from_lower_csc(*bordered([width, width], border, width + border))
+    M = solver(A, decomposition=dec, factor_schedule=schedule, plan_small_max_w=4096)
+    assert width in np.diff(M.GetSupernodalPartition())
+    f = oracle_for(M, A, dec == "LDL")
+    Lo = f.factor()
+    assert np.max(np.abs(M.GetFactor() - Lo)) <= TOL * np.max(np.abs(Lo))
+    b = np.random.default_rng(3).standard_normal((A.size, 2))
+    M.Solve(b)
+    x, xo = M.GetSolution(nrhs=2), f.solve(b)
+    assert np.max(np.abs(x - xo)) <= TOL * np.max(np.abs(xo))
+    M.close()
+
+
 @pytest.mark.parametrize("column", [0, 5, 12, 40])
 def test_a_bad_pivot_is_reported_where_it_is(column):
     """The first non-positive pivot's column, in a piece's interior and beyond the first piece."""
