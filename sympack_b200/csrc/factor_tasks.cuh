@@ -45,9 +45,10 @@ __device__ __forceinline__ void split_store(const FactorArgs& a, const SnMeta& m
   p[0] = __uint_as_float(hi);
   p[(int64_t)m.h * pitch] = __uint_as_float(lo);
 }
-// The copy's writes come before the TMA loads (async proxy) of the tasks that wait for
-// this one's counters.
-__device__ __forceinline__ void split_fence() { asm volatile("fence.proxy.async.global;" ::: "memory"); }
+// A panel task's writes that update tiles read through the async proxy (the split copies by
+// TMA, FP64 panels by bulk copies) come before the copies of the tiles that wait for this
+// task's counters: executed by the threads that wrote, before the barrier of the release.
+__device__ __forceinline__ void async_fence() { asm volatile("fence.proxy.async.global;" ::: "memory"); }
 
 constexpr int kNB = 64;
 constexpr int kThreads = 256;  // threads of the POTRF and TRSM kernels
@@ -224,6 +225,9 @@ __device__ __forceinline__ void factor_small_task(const FactorArgs& a, int s, co
     gl[r + (int64_t)c * m.ld] = (T)v;
     if constexpr (kLdl) gw[r + (int64_t)c * m.ld] = v * Dk[c];
   }
+  if constexpr (std::is_same<T, double>::value) {
+    if (!fuse) async_fence();  // a fused panel has no update tiles
+  }
   if constexpr (std::is_same<T, float>::value) {
     const int64_t off = a.split ? a.split_off[s] : -1;
     if (off >= 0) {  // off-diagonal rows, row by row (consecutive threads take consecutive columns)
@@ -231,7 +235,7 @@ __device__ __forceinline__ void factor_small_task(const FactorArgs& a, int s, co
         const int r = w + idx / w, c = idx % w;
         split_store(a, m, off, r, c, (float)P[r + c * ldp]);
       }
-      split_fence();
+      async_fence();
     }
   }
   if (!fuse) return;
@@ -542,6 +546,7 @@ __device__ __forceinline__ void trsm_rows_task(const FactorArgs& a, const PanelI
         gw[(it.row0 + r) + (int64_t)(c0 + k) * ld] = v;
       }
     }
+    async_fence();
     return;
   }
 #pragma unroll
@@ -549,7 +554,9 @@ __device__ __forceinline__ void trsm_rows_task(const FactorArgs& a, const PanelI
     const int idx = tid + q * kThreads, k = idx / kNB, r = idx - k * kNB;
     if (r < rows && k < nb) g[(it.row0 + r) + (int64_t)(c0 + k) * ld] = (T)R[r + k * kDL];
   }
-  if constexpr (std::is_same<T, float>::value) {
+  if constexpr (std::is_same<T, double>::value) {
+    async_fence();
+  } else {
     const int64_t off = a.split ? a.split_off[it.s] : -1;
     if (off >= 0) {  // the tile's rows, row by row (consecutive threads take consecutive columns)
 #pragma unroll
@@ -557,7 +564,7 @@ __device__ __forceinline__ void trsm_rows_task(const FactorArgs& a, const PanelI
         const int idx = tid + q * kThreads, r = idx / kNB, k = idx - r * kNB;
         if (r < rows && k < nb) split_store(a, m, off, it.row0 + r, c0 + k, (float)R[r + k * kDL]);
       }
-      split_fence();
+      async_fence();
     }
   }
 }

@@ -263,8 +263,12 @@ __device__ bool dmma_tile_task(const FactorArgs& a, const TileItem& item, const 
       bulk_g2s(smem_u32(Bs + (lane - 16) * D::kLdb), gb + b0 + (k + lane - 16) * ld, (uint32_t)nrb * 8, bar);
     ++issued;
   };
-  if (warp == 0)
+  if (warp == 0) {
+    // the operands' rows were written by other CTAs of this launch (generic proxy, a panel
+    // task) before the counters this tile waited for were released
+    asm volatile("fence.proxy.async.global;\n" ::: "memory");
     for (int kt = 0; kt < nk && kt < kDStages; ++kt) issue(kt);
+  }
   if (it.mode == 1 && warp >= 8 - BN / 32) {  // the last warps fetch the column table meanwhile
     const int c = tid - (kDThreads - BN), jc = b0 + c;
     if (jc >= it.b_row0 && jc < it.b_row0 + it.ncols) {

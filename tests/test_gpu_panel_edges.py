@@ -6,7 +6,7 @@ solution agree with the CPU oracle to 1e-12, the other GPU tests' bound (conditi
 import numpy as np
 import pytest
 
-from sympack_b200 import DistSparseMatrix
+from sympack_b200 import DistSparseMatrix, generators as G
 from test_gpu_solve_edges import bordered, oracle_for, solver
 
 pytestmark = pytest.mark.gpu
@@ -49,6 +49,21 @@ def test_small_panels_wider_than_64_columns(width, border, dec, schedule):
     x, xo = M.GetSolution(nrhs=2), f.solve(b)
     assert np.max(np.abs(x - xo)) <= TOL * np.max(np.abs(xo))
     M.close()
+
+
+@pytest.mark.parametrize("dec", ["LL", "LDL"])
+def test_update_tiles_see_the_panels_finished_before_them(dec):
+    """Bulk copies of the update tiles read panels that other blocks of the same launch have just
+    stored; the step sequence, a launch per step, has no such hand-over.  Both agree every time."""
+    A = DistSparseMatrix.from_lower_csc(*(G.stencil27(16, 16, 16, 1e-2) if dec == "LL" else G.quasi_definite_3d(16, 16, 16)))
+    M, S = (solver(A, decomposition=dec, factor_schedule=k) for k in ("persistent", "steps"))
+    Ls = S.GetFactor()
+    for _ in range(20):
+        M.DistributeMatrix(A)
+        M.Factorize()
+        assert np.max(np.abs(M.GetFactor() - Ls)) <= TOL * np.max(np.abs(Ls))
+    M.close()
+    S.close()
 
 
 @pytest.mark.parametrize("column", [0, 5, 12, 40])
