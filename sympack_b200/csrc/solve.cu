@@ -19,7 +19,8 @@
 // of a wide supernode has two steps per super-block (its DI products, then the
 // updates of the next super-block) instead of one per 64 columns.  The diagonal
 // block of a one-block supernode is applied through its inverse too
-// (k_diag_inverse).  The forward sweep reads the permuted right-hand sides Y
+// (k_diag_inverse), in FP64 with one correction by its residual (solve_block), without which
+// the residual would grow with the block's condition.  The forward sweep reads the permuted right-hand sides Y
 // (accumulating the descendants' contributions there) and writes its solution
 // to Z; the backward sweep accumulates into Z and writes the final solution X.
 //
@@ -33,7 +34,7 @@
 // on the FP64 tensor pipe for one right-hand side too: an 8-column group costs no
 // more issue slots than scalar FMAs with their shared-memory reads would.
 // FP32 factors are widened as they enter a product.  60^3 Laplacian, FP64: 1 right-hand side
-// 2.16 -> 1.20 ms, 16 right-hand sides 4.85 -> 2.09 ms against tasks that staged their tiles
+// 2.16 -> 1.25 ms, 16 right-hand sides 4.85 -> 2.16 ms against tasks that staged their tiles
 // in shared memory and multiplied with scalar FMAs (0.34 ms by the bytes of both sweeps).
 #include <type_traits>
 
@@ -62,6 +63,7 @@ struct SolveSmem {
   double x[kXLd * 8 * NG];
   double part[8 * 16 * 8 * NG];  // G: partial sums of the 8 warps
   double z[8 * 20 * 8 * NG];     // solved rows: 64 of a block (ld kZLd) or 16 per warp (ld kWzLd)
+  double ldiag[kT];              // diagonal of a one-block supernode's diagonal block
   int rows[kRowCap];
 };
 // Three CTAs per SM where the fragments of a pair of tiles leave room in 80 registers (FP32, one
@@ -200,45 +202,122 @@ __device__ __forceinline__ void clear(double (&acc)[NG][4]) {
     for (int e = 0; e < 4; ++e) acc[n][e] = 0.0;
 }
 
-// Inverse of a one-block supernode's diagonal block (w x w lower triangle, ld w) into
-// shared memory, zero outside, up to the fragment sizes the products read.
-__device__ __forceinline__ void stage_inverse(double* s, const double* inv, int w) {
+// FP64 factors: the product with a diagonal block's inverse is corrected once by its residual
+// (z += Inv (y - L z)), which brings it to the accuracy of a substitution.  The product alone
+// leaves a residual that grows with the block's condition: dense 24 x 24 blocks of condition
+// 1e12, residual against |L||L^T||x|: 1.9e-16 alone, 2.0e-17 corrected, 1.2e-17 by
+// substitution.  FP32 factors need none: their own rounding is 1e9 times that, and refinement
+// recomputes the residual.  Costs two more products and barriers a task: 60^3 Laplacian 1.20 ->
+// 1.25 ms, 16 right-hand sides 2.09 -> 2.16, 27-point 17^3 0.168 -> 0.181.
+template <class T>
+constexpr bool kCorrect = std::is_same<T, double>::value;
+
+// Inverse of a one-block supernode's diagonal block L (w x w lower triangle, ld w) into
+// the lower triangle of s, zero outside, up to the fragment sizes the products read.  When
+// corrected, L's strict lower triangle goes to the upper one, transposed, and its diagonal to
+// ldiag.
+template <class T>
+__device__ __forceinline__ void stage_inverse(double* s, double* ldiag, const double* inv, const T* L, int64_t ld, int w) {
   const int wr = (w + 15) & ~15;
   for (int idx = threadIdx.x; idx < wr * kT; idx += kThreads) {
     const int c = idx >> 6, r = idx & 63;
-    if (r < wr) s[r + c * kInvLd] = (r < w && c < w && r >= c) ? __ldg(inv + r + c * w) : 0.0;
+    if (r >= wr || (kCorrect<T> && r < c)) continue;
+    const bool in = r < w && c < w && r >= c;
+    s[r + c * kInvLd] = in ? __ldg(inv + r + c * w) : 0.0;
+    if constexpr (kCorrect<T>) {
+      const double l = in ? (double)__ldg(L + r + c * ld) : 0.0;
+      if (r > c) s[c + r * kInvLd] = l;
+      else ldiag[r] = l;
+    }
   }
 }
 
-// z = Inv y (kTrans false) or Inv^T y for the w rows of a one-block supernode, columns c0 ..
-// c0 + nc - 1 of it: y in shared memory (ld ldy, zero from row w on), result to global
-// (out, first row) and, when zs, to shared memory (ld kZLd, zero from row w on).
-template <int NG, bool kTrans>
-__device__ __forceinline__ void apply_inverse(double* out, int64_t ldx, double* zs, const double* inv, const double* y,
-                                              int ldy, int w, int nc) {
+// d + d2 += Op B for rows 16 im .. of the staged triangle, B[k][c] = b[k] of this lane's column:
+// Op = Inv or L (kL), transposed with kTrans.  Entries on the other side of the diagonal belong
+// to the other operand (kMask) or are zero.
+template <bool kTrans, bool kL, bool kMask>
+__device__ __forceinline__ void tri_mma(double (&d)[4], double (&d2)[4], const double* s, const double* ldiag,
+                                        const double* b, int im, int ks) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3, row = im * 16 + g;
+  constexpr bool kDown = kTrans != kL;  // the inner index runs down a column of s
+  const double* p = kDown ? s + t + row * kInvLd : s + row + t * kInvLd;
+  constexpr int s1 = kDown ? 8 * kInvLd : 8, sk = kDown ? 4 : 4 * kInvLd;
+  int i = kTrans ? 4 * im + 4 : 0;
+  const int e = kTrans ? ks : min(ks, 4 * im);
+  for (; i + 1 < e; i += 2) {
+    dmma(d, p[i * sk], p[i * sk + s1], b[4 * i]);
+    dmma(d2, p[(i + 1) * sk], p[(i + 1) * sk + s1], b[4 * i + 4]);
+  }
+  if (i < e) dmma(d, p[i * sk], p[i * sk + s1], b[4 * i]);
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {  // the 16 x 16 tile on the diagonal
+    i = 4 * im + q;
+    if (i >= ks) break;
+    double a0 = p[i * sk], a1 = p[i * sk + s1];
+    if (kMask) {
+      const int k = 4 * q + t;  // against local rows g, g + 8
+      if (kL) {
+        const double l = ldiag[4 * i + t];
+        if (k == g) a0 = l;
+        if (k == g + 8) a1 = l;
+      }
+      if (kTrans ? k < g : k > g) a0 = 0.0;
+      if (kTrans ? k < g + 8 : k > g + 8) a1 = 0.0;
+    }
+    if (q & 1) dmma(d2, a0, a1, b[4 * i]);
+    else dmma(d, a0, a1, b[4 * i]);
+  }
+}
+
+// z = L^-1 y (kTrans false) or L^-T y for the w rows of a one-block supernode, nc columns, by
+// the whole block: y in shared memory (ld ldy, zero from row w on; overwritten when corrected),
+// result to global (out, first row) and to zs (ld kZLd, zero from row w on).  A warp has at
+// most one 16 x 8 tile.  Ends without a barrier.
+template <class T, int NG, bool kTrans>
+__device__ __forceinline__ void solve_block(double* out, int64_t ldx, double* zs, const double* inv,
+                                            const double* ldiag, double* y, int ldy, int w, int nc) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
   const int mt = (w + 15) >> 4, ks = (w + 3) >> 2;
-  for (int pr = warp; pr < mt * NG; pr += kThreads / 32) {
-    const int im = pr / NG, in = pr % NG;
-    if (in * 8 >= nc) continue;
-    double d[4] = {0.0, 0.0, 0.0, 0.0}, d2[4] = {0.0, 0.0, 0.0, 0.0};
-    const double* b = y + t + (in * 8 + g) * ldy;
-    const double* p = kTrans ? inv + t + (im * 16 + g) * kInvLd : inv + im * 16 + g + t * kInvLd;
-    const int s1 = kTrans ? 8 * kInvLd : 8, sk = kTrans ? 4 : 4 * kInvLd;
-    const int i0 = kTrans ? 4 * im : 0, i1 = kTrans ? ks : min(ks, 4 * (im + 1));
-    int i = i0;
-    for (; i + 1 < i1; i += 2) {
-      dmma(d, p[i * sk], p[i * sk + s1], b[4 * i]);
-      dmma(d2, p[(i + 1) * sk], p[(i + 1) * sk + s1], b[4 * i + 4]);
-    }
-    if (i < i1) dmma(d, p[i * sk], p[i * sk + s1], b[4 * i]);
+  static_assert(kT / 16 * NG <= kThreads / 32, "a tile per warp");
+  const int im = warp / NG, in = warp % NG;
+  const bool mine = warp < mt * NG && in * 8 < nc;
+  const int row = im * 16 + g, col = in * 8 + 2 * t;  // accumulators: rows row, row + 8 x columns col, col + 1
+  double d[4] = {0.0, 0.0, 0.0, 0.0}, d2[4] = {0.0, 0.0, 0.0, 0.0};
+  if (mine) {
+    tri_mma<kTrans, false, kCorrect<T>>(d, d2, inv, nullptr, y + t + (in * 8 + g) * ldy, im, ks);
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const int r = im * 16 + g + 8 * (e >> 1), c = in * 8 + 2 * t + (e & 1);
-      const double v = d[e] + d2[e];
-      if (r < w && c < nc) out[r + c * ldx] = v;
-      if (zs) zs[r + c * kZLd] = v;  // rows from w on: zero rows of the inverse
+    for (int e = 0; e < 4; ++e) d[e] += d2[e];
+  }
+  if constexpr (kCorrect<T>) {
+    double r[4], r2[4] = {0.0, 0.0, 0.0, 0.0};
+    if (mine) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        zs[row + 8 * (e >> 1) + (col + (e & 1)) * kZLd] = d[e];
+        r[e] = -y[row + 8 * (e >> 1) + (col + (e & 1)) * ldy];
+      }
     }
+    __syncthreads();
+    if (mine) {
+      tri_mma<kTrans, true, true>(r, r2, inv, ldiag, zs + t + (in * 8 + g) * kZLd, im, ks);  // L z - y
+#pragma unroll
+      for (int e = 0; e < 4; ++e) y[row + 8 * (e >> 1) + (col + (e & 1)) * ldy] = -(r[e] + r2[e]);
+    }
+    __syncthreads();
+    if (mine) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) r[e] = r2[e] = 0.0;
+      tri_mma<kTrans, false, true>(r, r2, inv, nullptr, y + t + (in * 8 + g) * ldy, im, ks);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) d[e] += r[e] + r2[e];
+    }
+  }
+  if (!mine) return;
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const int r = row + 8 * (e >> 1), c = col + (e & 1);
+    if (r < w && c < nc) out[r + c * ldx] = d[e];
+    zs[r + c * kZLd] = d[e];  // rows from w on: zero rows of the inverse
   }
 }
 
@@ -340,19 +419,70 @@ __device__ __forceinline__ void frag_rows(Frag<T>& f, const T* A, int ld, int ro
   }
 }
 
-// d = (4 fragment steps) * zs, to out rows r0 + g (+ 8) below w and, when kKeep, back to zs
+// d += (4 fragment steps, zero from inner index w on) * zs
 template <int NG>
 __device__ __forceinline__ void small_mma(double (&d)[NG][4], const double (&v0)[4], const double (&v1)[4],
-                                          const double* zs) {
+                                          const double* zs, int w) {
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < 4; ++i) {
+    if (4 * i >= w) break;
 #pragma unroll
     for (int n = 0; n < NG; ++n) dmma(d[n], v0[i], v1[i], zs[4 * i + t + (n * 8 + g) * kWzLd]);
+  }
+}
+
+// FP64: the diagonal block's lower triangle into the warp's Ls (16 x 16, ld kWzLd), for the
+// correction by the residual.
+__device__ __forceinline__ void stage_small(double* Ls, const double* L, int64_t ld, int w) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    const int c = 2 * q + (lane >> 4), r = lane & 15;
+    Ls[r + c * kWzLd] = r < w && c <= r ? __ldg(L + r + c * ld) : 0.0;
+  }
+}
+
+// d <- d + Inv (y - L d), Inv in the fragments v0, v1, L in Ls (kTrans: both transposed), y the
+// 16 x 8 NG tile ys (overwritten); zs: the warp's other tile.
+template <int NG, bool kTrans>
+__device__ __forceinline__ void correct_small(double (&d)[NG][4], const double (&v0)[4], const double (&v1)[4],
+                                              const double* Ls, double* zs, double* ys, int w) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  double r[NG][4];
+#pragma unroll
+  for (int n = 0; n < NG; ++n)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int o = g + 8 * (e >> 1) + (n * 8 + 2 * t + (e & 1)) * kWzLd;
+      zs[o] = d[n][e];
+      r[n][e] = -ys[o];
+    }
+  __syncwarp();
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {  // L d - y
+    if (4 * i >= w) break;
+    const int k = 4 * i + t;
+    const double l0 = kTrans ? Ls[k + g * kWzLd] : Ls[g + k * kWzLd];
+    const double l1 = kTrans ? Ls[k + (g + 8) * kWzLd] : Ls[g + 8 + k * kWzLd];
+#pragma unroll
+    for (int n = 0; n < NG; ++n) dmma(r[n], l0, l1, zs[k + (n * 8 + g) * kWzLd]);
+  }
+#pragma unroll
+  for (int n = 0; n < NG; ++n)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) ys[g + 8 * (e >> 1) + (n * 8 + 2 * t + (e & 1)) * kWzLd] = -r[n][e];
+  __syncwarp();
+  clear<NG>(r);
+  small_mma<NG>(r, v0, v1, ys, w);
+#pragma unroll
+  for (int n = 0; n < NG; ++n)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) d[n][e] += r[n][e];
 }
 
 template <class T, int NG>
-__device__ bool warp_forward(const PSolveArgs& a, const SolveRec& r, double* zs, double* X, double* Z, int32_t* sync,
+__device__ bool warp_forward(const PSolveArgs& a, const SolveRec& r, double* zs, double* ys, double* Ls, double* X, double* Z, int32_t* sync,
                              int nc, Frag<T>& f, unsigned long long* trace) {
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3, w = r.m;
   const T* A = static_cast<const T*>(a.L) + r.a + w;
@@ -365,6 +495,7 @@ __device__ bool warp_forward(const PSolveArgs& a, const SolveRec& r, double* zs,
     v1[i] = g + 8 < w && k < w ? __ldg(inv + g + 8 + k * w) : 0.0;
   }
   frag_rows<T>(f, A, r.ld, 0, r.k, w);
+  if constexpr (kCorrect<T>) stage_small(Ls, A - w, r.ld, w);
   int tgt = 0, cnt = 0;  // this lane's arrival
   if (lane < r.ng) {
     const RelGroup gr = a.groups[r.g0 + lane];
@@ -391,7 +522,14 @@ __device__ bool warp_forward(const PSolveArgs& a, const SolveRec& r, double* zs,
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
-      for (int n = 0; n < NG; ++n) dmma(d[n], v0[i], v1[i], y[i][n]);
+      for (int n = 0; n < NG; ++n) {
+        if constexpr (kCorrect<T>) ys[4 * i + t + (n * 8 + g) * kWzLd] = y[i][n];
+        dmma(d[n], v0[i], v1[i], y[i][n]);
+      }
+  }
+  if constexpr (kCorrect<T>) {
+    __syncwarp();
+    correct_small<NG, false>(d, v0, v1, Ls, zs, ys, w);
   }
 #pragma unroll
   for (int n = 0; n < NG; ++n)
@@ -410,7 +548,7 @@ __device__ bool warp_forward(const PSolveArgs& a, const SolveRec& r, double* zs,
       const double x0[4] = {(double)f.a0[4 * j], (double)f.a0[4 * j + 1], (double)f.a0[4 * j + 2], (double)f.a0[4 * j + 3]};
       const double x1[4] = {(double)f.a1[4 * j], (double)f.a1[4 * j + 1], (double)f.a1[4 * j + 2], (double)f.a1[4 * j + 3]};
       clear<NG>(d);
-      small_mma<NG>(d, x0, x1, zs);
+      small_mma<NG>(d, x0, x1, zs, w);
       scatter<NG>(X, a.ldx, 0, rows + row0 + 16 * j, d, r.k - row0 - 16 * j, nc, -1.0);
     }
   }
@@ -425,8 +563,8 @@ __device__ bool warp_forward(const PSolveArgs& a, const SolveRec& r, double* zs,
 }
 
 template <class T, int NG>
-__device__ bool warp_backward(const PSolveArgs& a, const SolveRec& r, double* zs, double* X, const double* Z,
-                              int32_t* sync, int nc, Frag<T>& f, unsigned long long* trace) {
+__device__ bool warp_backward(const PSolveArgs& a, const SolveRec& r, double* zs, double* ys, double* Ls, double* X,
+                              const double* Z, int32_t* sync, int nc, Frag<T>& f, unsigned long long* trace) {
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3, w = r.m;
   const T* A = static_cast<const T*>(a.L) + r.a + w;
   const double* inv = a.Inv1 + r.inv;
@@ -438,6 +576,7 @@ __device__ bool warp_backward(const PSolveArgs& a, const SolveRec& r, double* zs
     v1[i] = g + 8 < w && k < w ? __ldg(inv + k + (g + 8) * w) : 0.0;
   }
   f.load(A, r.ld, 1, w, min(64, r.k));
+  if constexpr (kCorrect<T>) stage_small(Ls, A - w, r.ld, w);
   const int32_t* rows = a.rows + r.y0;
   int idx[16];
 #pragma unroll
@@ -483,7 +622,8 @@ __device__ bool warp_backward(const PSolveArgs& a, const SolveRec& r, double* zs
     for (int e = 0; e < 4; ++e) zs[g + 8 * (e >> 1) + (n * 8 + 2 * t + (e & 1)) * kWzLd] = -d[n][e];
   __syncwarp();
   clear<NG>(d);
-  small_mma<NG>(d, v0, v1, zs);
+  small_mma<NG>(d, v0, v1, zs, w);
+  if constexpr (kCorrect<T>) correct_small<NG, true>(d, v0, v1, Ls, ys, zs, w);
 #pragma unroll
   for (int n = 0; n < NG; ++n)
 #pragma unroll
@@ -545,17 +685,20 @@ __global__ void __launch_bounds__(kThreads, solve_min_blocks<T, NG>()) k_solve(P
       if (warp < r.m) {
         const SolveRec q = a.subs[r.x0 + warp];
         double* zs = sm.z + warp * kWzLd * 8 * NG;
+        double* ys = sm.x + warp * kXLd * NG;           // a second tile and the diagonal block
+        double* Ls = sm.inv + warp * (kT * kInvLd / 8);
+        static_assert(kXLd * NG >= kWzLd * 8 * NG && kT * kInvLd / 8 >= 16 * kWzLd, "a warp's tiles");
         unsigned long long* wtrace = grp == 0 && (tid & 31) == 0 ? a.trace : nullptr;
         if (wtrace) trace_start(wtrace, q);
-        if (kFwd) ok = warp_forward<T, NG>(a, q, zs, X, Z, sync, nc, f, wtrace);
-        else ok = warp_backward<T, NG>(a, q, zs, X, Z, sync, nc, f, wtrace);
+        if (kFwd) ok = warp_forward<T, NG>(a, q, zs, ys, Ls, X, Z, sync, nc, f, wtrace);
+        else ok = warp_backward<T, NG>(a, q, zs, ys, Ls, X, Z, sync, nc, f, wtrace);
         if (wtrace) trace_mark(wtrace, q, 2);
       }
       if (tid == 0) sh_task[turn ^ 1] = atomicAdd(a.counter, 1);
       if (!__syncthreads_and(ok)) return;
       continue;
     } else if (one_block) {
-      stage_inverse(sm.inv, a.Inv1 + r.inv, r.m);
+      stage_inverse<T>(sm.inv, sm.ldiag, a.Inv1 + r.inv, L + r.a, r.ld, r.m);
       for (int i = tid; i < min(r.k, kRowCap); i += kThreads) sm.rows[i] = a.rows[r.y0 + i];
       const T* A = L + r.a + r.m;  // first off-diagonal row
       if (kFwd) {
@@ -620,7 +763,7 @@ __global__ void __launch_bounds__(kThreads, solve_min_blocks<T, NG>()) k_solve(P
           // F, D: Z_0 <- L_00^-1 Y_0, then every off-diagonal row's Y[ancestor row] -= L_u0 Z_0
           stage_x(sm.x, kXLd, X, a.ldx, r.x0, nullptr, w, kT, nc);
           __syncthreads();
-          apply_inverse<NG, false>(Z + r.x0, a.ldx, sm.z, sm.inv, sm.x, kXLd, w, nc);
+          solve_block<T, NG, false>(Z + r.x0, a.ldx, sm.z, sm.inv, sm.ldiag, sm.x, kXLd, w, nc);
           __syncthreads();
           const int lane = tid & 31, g = lane >> 2, t = lane & 3;
           for (int ch = 0; ch < nch; ++ch) {
@@ -703,7 +846,7 @@ __global__ void __launch_bounds__(kThreads, solve_min_blocks<T, NG>()) k_solve(P
             }
           }
           __syncthreads();
-          apply_inverse<NG, true>(X + r.x0, a.ldx, nullptr, sm.inv, sm.z, kZLd, w, nc);
+          solve_block<T, NG, true>(X + r.x0, a.ldx, sm.x, sm.inv, sm.ldiag, sm.z, kZLd, w, nc);
         }
       }
     } else {
