@@ -77,8 +77,10 @@ constexpr int kPiece = 8;
 // column's entries from their lanes by shuffles, so that every lane issues the same 28 FMAs:
 // a warp issues an FP64 instruction every 8 cycles or so, which is what the chain of pivots
 // costs (the piece factored redundantly by every lane, 120 FMAs, took 1.2 us a piece).
-// Cholesky: rs = 1 / L_kk, x becomes row L^-T; a pivot not > 0 is reported (who: this warp
-// reports) and replaced by 1.  LDL^T (Potf2_LDL, lapack.hpp:206-270, lower triangle): d_k =
+// Cholesky: rs = 1 / L_kk, x becomes row L^-T, and lane k keeps the pivot d_k as x[k] for its
+// consumer to take sqrt of beside the chain (L_kk = d_k rs would round d_k's root twice over,
+// and L_kk^2 twice that: residual of the factor 18 % larger on a 100 x 103 grid); a pivot not
+// > 0 is reported (who: this warp reports) and replaced by 1.  LDL^T (Potf2_LDL, lapack.hpp:206-270, lower triangle): d_k =
 // A_kk, |d_k| > 0 or reported; rs = 1 / d_k, x becomes the row's entries of L D.  Reported
 // pivots: column col + k of supernode s, k < valid.
 template <bool kLdl>
@@ -95,11 +97,12 @@ __device__ __forceinline__ void piece_rows(double (&x)[kPiece], double (&rs)[kPi
       rs[k] = 1.0;
       if (lane == k) x[k] = 1.0;
     }
-    const double y = x[k] * rs[k];  // the row's entry of L
-    if constexpr (!kLdl) x[k] = y;
-    if (k + 1 < kPiece) own = fma(-x[k], y, x[k + 1]);
+    const double y = x[k] * rs[k];          // the row's entry of L
+    const double l = kLdl ? x[k] : y;
+    if (k + 1 < kPiece) own = fma(-l, y, x[k + 1]);
 #pragma unroll
-    for (int j = k + 1; j < kPiece; ++j) x[j] = fma(-x[k], __shfl_sync(0xffffffffu, y, j), x[j]);
+    for (int j = k + 1; j < kPiece; ++j) x[j] = fma(-l, __shfl_sync(0xffffffffu, y, j), x[j]);
+    if constexpr (!kLdl) x[k] = lane == k ? (d > 0.0 ? d : 1.0) : y;
   }
 }
 
@@ -220,10 +223,14 @@ __device__ __forceinline__ void factor_small_task(const FactorArgs& a, int s, co
   double* gw = kLdl ? a.W + m.off : nullptr;
   for (int idx = tid; idx < h * w; idx += nthr) {
     const int c = (int)((idx + 0.5f) * rh), r = idx - c * h;
-    if (r < c) continue;
+    if (kLdl ? r < c : r <= c) continue;
     const double v = P[r + c * ldp];
     gl[r + (int64_t)c * m.ld] = (T)v;
     if constexpr (kLdl) gw[r + (int64_t)c * m.ld] = v * Dk[c];
+  }
+  if constexpr (!kLdl) {  // the last warp: the diagonal, from the pivots
+    if (warp == nw - 1)
+      for (int c = lane; c < w; c += 32) gl[c + (int64_t)c * m.ld] = (T)sqrt(P[c + c * ldp]);
   }
   if constexpr (std::is_same<T, double>::value) {
     if (!fuse) async_fence();  // a fused panel has no update tiles
@@ -425,11 +432,13 @@ __device__ __forceinline__ void diag_task(const FactorArgs& a, const PanelItem& 
       }
       if (warp >= 6) {  // the finished columns go out while the next piece is factored
         const int r = 32 * (warp - 6) + lane;
+        double lrr = 1.0;  // Cholesky: the row's diagonal entry, from its pivot
+        if (!kLdl && (r >> 3) == p) lrr = sqrt(D[r + r * kDL]);
 #pragma unroll
         for (int j = 0; j < kPiece; ++j) {
           const int c = kb + j;
           if (r < c) continue;
-          const double l = D[r + c * kDL];
+          const double l = !kLdl && r == c ? lrr : D[r + c * kDL];
           if (r < nb && c < nb) {
             gl[(c0 + r) + (int64_t)(c0 + c) * ld] = (T)l;
             if constexpr (kLdl) a.W[m.off + (c0 + r) + (int64_t)(c0 + c) * ld] = l * Dk[c];

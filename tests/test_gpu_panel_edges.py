@@ -75,3 +75,26 @@ def test_a_bad_pivot_is_reported_where_it_is(column):
     v[cp[column] - 1] = -1.0  # the diagonal entry (first of its column)
     with pytest.raises(NotSPDError, match=f"column {column + 1}$"):
         solver(DistSparseMatrix.from_lower_csc(n, cp, ri, v))
+
+
+@pytest.mark.parametrize("schedule", ["persistent", "steps"])
+def test_diagonal_entries_are_the_rounded_square_roots(schedule):
+    """Pivots that no update touches: diagonal matrices (one-column panels) and the first column
+    of dense 64-column and wider blocks.  L_kk is sqrt's result, bit for bit."""
+    d = np.random.default_rng(5).uniform(1e-3, 1e3, 2000)
+    n = len(d)
+    M = solver(DistSparseMatrix.from_lower_csc(n, np.arange(1, n + 2), np.arange(1, n + 1, dtype=np.int32), d),
+               factor_schedule=schedule)
+    assert np.array_equal(M.GetFactor()[M.GetOrdering()[1] - 1], np.sqrt(d))
+    M.close()
+    for seed in range(20):
+        n, cp, ri, v = bordered([40, 70], 30, seed)
+        M = solver(DistSparseMatrix.from_lower_csc(n, cp, ri, v), factor_schedule=schedule)
+        L, pos = M.GetFactor(), 0
+        xs, (xl, li), perm = M.GetSupernodalPartition(), M.GetStructure(), M.GetOrdering()[0]
+        for s in range(len(xs) - 1):
+            c = perm[xs[s] - 1]
+            if c in (1, 41):  # the first column of each block
+                assert L[pos] == np.sqrt(v[cp[c - 1] - 1])
+            pos += (xs[s + 1] - xs[s]) * (xl[s + 1] - xl[s])
+        M.close()
