@@ -294,13 +294,16 @@ constexpr int kDiagSmemDoubles = kNB * kDL + 2 * kNB + 2 * kPiece * kDL;
 // Warps 3-7 hold the block's columns as tensor-core accumulators, 8 columns a tile.  For a
 // piece the tile's warp lays its columns in shared memory, warps 0-2 factor it and solve the
 // rows below (piece_rows), then every later tile takes the solved columns off with 2 MMA
-// steps per 16 rows, the next piece's tile first.  The solving warps wait for that tile only;
+// steps per 16 rows, the next piece's tile first: the second step from zero and added, five
+// roundings of an entry a piece instead of eight (residual of the factor, 27-point 17^3 6.4e-17
+// -> 5.9e-17; the scalar version split its sums alike).  The solving warps wait for that tile only;
 // finished columns and the pieces' inverses are written out beside the next pieces.
 // The scratch slot gets the factored block (FP64) with the inverses of its 8 x 8 diagonal
 // pieces transposed into their upper triangles, 1/L_kk (1 for LDL^T, whose TRSM then computes
 // W's rows) and 1/D_kk.  11 us a block measured alone, 13 to 18 us beside other tasks; the
-// scalar version (the trailing triangle as a chain of shared-memory FMAs) took 19 to 25 us.  LDL^T: L takes the unit block, W the block times D (its diagonal is
-// D).  A block narrower than 64 is padded with the identity.
+// scalar version (the trailing triangle as a chain of shared-memory FMAs) took 19 to 25 us.
+// LDL^T: L takes the unit block, W the block times D (its diagonal is D).  A block narrower
+// than 64 is padded with the identity.
 template <class T, bool kLdl>
 __device__ __forceinline__ void diag_task(const FactorArgs& a, const PanelItem& it, const SnMeta& meta,
                                          double* __restrict__ winv, double* sm) {
@@ -414,8 +417,11 @@ __device__ __forceinline__ void diag_task(const FactorArgs& a, const PanelItem& 
         for (int i = 0; i < 4; ++i)
           if (i >= n0 / 2) {
             const double* v = A + 16 * i;
+            double h[4] = {0.0, 0.0, 0.0, 0.0};
+            dmma(h, -v[4 * kDL], -v[4 * kDL + 8], b1);
             dmma(acc[i], -v[0], -v[8], b0);
-            dmma(acc[i], -v[4 * kDL], -v[4 * kDL + 8], b1);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[i][e] += h[e];
             if (n0 == p + 1) lay(acc[i], n0, i);
           }
         if (n0 == p + 1) asm volatile("bar.arrive 2, 128;\n" ::: "memory");
@@ -423,8 +429,11 @@ __device__ __forceinline__ void diag_task(const FactorArgs& a, const PanelItem& 
       if (n1 < kPieces && n1 > p) {
         const double* B = D + 8 * n1 + g + (kb + t) * kDL;
         const double* v = A + 48;
+        double h[4] = {0.0, 0.0, 0.0, 0.0};
+        dmma(h, -v[4 * kDL], -v[4 * kDL + 8], B[4 * kDL]);
         dmma(last, -v[0], -v[8], B[0]);
-        dmma(last, -v[4 * kDL], -v[4 * kDL + 8], B[4 * kDL]);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) last[e] += h[e];
         if (n1 == p + 1) {
           lay(last, n1, 3);
           asm volatile("bar.arrive 2, 128;\n" ::: "memory");
