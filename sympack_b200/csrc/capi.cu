@@ -10,6 +10,7 @@
 #include <cstdio>
 #include <cstring>
 #include <exception>
+#include <limits>
 #include <memory>
 #include <atomic>
 #include <mutex>
@@ -590,25 +591,37 @@ int ir_solve(spb_handle* h, const double* d_b, int64_t ldb, double* d_x, int64_t
     double* x = d_x + (int64_t)c0 * ldx;
     plain_solve(h, b, ldb, x, ldx, nr);
     const int nseg = num_segments(h);
-    double* anorm = h->d_norms + 1;
+    double* anorm = h->d_norms + 2;
     double* bmax = anorm + nseg;
     double* xmax = bmax + (size_t)nseg * 64;
     double* rmax = xmax + (size_t)nseg * 64;
     SPB_CK(h, cudaMemsetAsync(bmax, 0, sizeof(double) * 64 * (size_t)nseg, h->stream));
     spb::dev::launch_segmax(h->stream, b, n, nr, ldb, h->d_rowseg, bmax);
-    double eta = 0.0, eta_prev = 1e300;
+    // backward error of the systems and right-hand sides whose norms are finite, and whether all
+    // are; the finite ones are refined to the end before the others fail the call
+    double measured[2] = {0.0, 0.0}, eta_prev = 1e300;
     int it = 0;
     for (;;) {
       SPB_CK(h, cudaMemsetAsync(xmax, 0, sizeof(double) * 128 * (size_t)nseg, h->stream));
-      SPB_CK(h, cudaMemsetAsync(h->d_norms, 0, sizeof(double), h->stream));
+      SPB_CK(h, cudaMemsetAsync(h->d_norms, 0, 2 * sizeof(double), h->stream));
       // the residual goes where a correction solve reads its right-hand sides
       spb::dev::launch_residual(h->stream, h->d_rowptr, h->d_col, h->d_val, x, ldx, b, ldb, h->dX, h->dinvp0, n, nr,
                                 h->d_rowseg, xmax, rmax, h->dZ, h->dsync, sync_ints(h));
       spb::dev::launch_eta(h->stream, anorm, bmax, xmax, rmax, nseg, nr, h->d_norms);
-      SPB_CK(h, cudaMemcpyAsync(&eta, h->d_norms, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+      SPB_CK(h, cudaMemcpyAsync(measured, h->d_norms, sizeof(measured), cudaMemcpyDeviceToHost, h->stream));
       int rc = check_solve_status(h);  // synchronizes
       if (rc) return rc;
-      if (eta <= tol) break;
+      const bool finite = measured[1] == 0.0;
+      double eta = measured[0];
+      if (eta <= tol && finite) {
+        eta_all = std::max(eta_all, eta);
+        break;
+      }
+      if (!finite && (eta <= tol || it >= maxit || (it >= 4 && eta > 0.9 * eta_prev))) {
+        h->ir_iterations = std::max(iters_all, it);
+        h->backward_error = std::numeric_limits<double>::infinity();
+        return fail(h, SPB_ERR_NOT_CONVERGED, "refinement: a right-hand side, its solution or its residual is not finite");
+      }
       if (it >= maxit || (it >= 4 && eta > 0.9 * eta_prev)) {
         h->ir_iterations = std::max(iters_all, it);
         h->backward_error = std::max(eta_all, eta);
@@ -623,7 +636,6 @@ int ir_solve(spb_handle* h, const double* d_b, int64_t ldb, double* d_x, int64_t
       ++it;
     }
     iters_all = std::max(iters_all, it);
-    eta_all = std::max(eta_all, eta);
   }
   h->ir_iterations = iters_all;
   h->backward_error = eta_all;
@@ -905,7 +917,7 @@ int64_t predict_bytes(const spb_handle* h, bool fp32, int nrhs) {
       for (int64_t p = h->colptr[c - 1]; p < h->colptr[c]; ++p) offdiag += h->rowind[p - 1] != c;
     const int64_t nnz_full = h->nnz_a + offdiag;
     t += b(n + 1, 8) + b(nnz_full, 4) + b(nnz_full, 8) + b(nnz_full, 8);
-    t += b(1 + (int64_t)num_segments(h) * (1 + 3 * 64), 8);
+    t += b(2 + (int64_t)num_segments(h) * (1 + 3 * 64), 8);
     if (!h->seg_off.empty()) t += b(n, 4);
   }
   if (fp32 && o.fp32_engine == 3) {
@@ -1074,7 +1086,7 @@ int install_device(spb_handle* h) {
     SPB_CK(h, dalloc(h, &h->d_col, h->csr_col.size()));
     SPB_CK(h, dalloc(h, &h->d_csrsrc, h->csr_src.size()));
     SPB_CK(h, dalloc(h, &h->d_val, h->csr_col.size()));
-    SPB_CK(h, dalloc(h, &h->d_norms, 1 + (size_t)num_segments(h) * (1 + 3 * 64)));
+    SPB_CK(h, dalloc(h, &h->d_norms, 2 + (size_t)num_segments(h) * (1 + 3 * 64)));
     if (!h->seg_off.empty()) {
       std::vector<int32_t> rowseg(n);
       for (size_t k = 0; k + 1 < h->seg_off.size(); ++k)
@@ -1252,8 +1264,8 @@ static int distribute_common(spb_handle* h) {
   spb::dev::launch_assemble(h->stream, h->dL, h->fp32, h->damap, h->dA, h->nnz_a);
   if (h->fp32) {  // FP64 copy of A for the refinement residuals, and ||A||_inf
     spb::dev::launch_gather(h->stream, h->d_val, h->dA, h->d_csrsrc, (int64_t)h->csr_col.size());
-    SPB_CK(h, cudaMemsetAsync(h->d_norms + 1, 0, sizeof(double) * num_segments(h), h->stream));
-    spb::dev::launch_rowsum_segmax(h->stream, h->d_rowptr, h->d_val, h->sym.n, h->d_rowseg, h->d_norms + 1);
+    SPB_CK(h, cudaMemsetAsync(h->d_norms + 2, 0, sizeof(double) * num_segments(h), h->stream));
+    spb::dev::launch_rowsum_segmax(h->stream, h->d_rowptr, h->d_val, h->sym.n, h->d_rowseg, h->d_norms + 2);
   }
   SPB_CK(h, cudaGetLastError());
   if (h->profiling) SPB_CK(h, cudaEventRecord(h->events[1], h->stream));

@@ -27,7 +27,11 @@ __global__ void k_gather(double* __restrict__ dst, const double* __restrict__ sr
     dst[i] = src[idx[i]];
 }
 
-// Non-negative doubles order like their bit patterns: max through 64-bit integer atomics.
+// Non-negative doubles order like their bit patterns, a NaN above infinity: maxima through
+// 64-bit integers keep it, where fmax would drop it.
+__device__ __forceinline__ double max_nonneg(double a, double b) {
+  return __longlong_as_double(max(__double_as_longlong(a), __double_as_longlong(b)));
+}
 __device__ __forceinline__ void atomic_max_nonneg(double* addr, double v) {
   atomicMax(reinterpret_cast<unsigned long long*>(addr), (unsigned long long)__double_as_longlong(v));
 }
@@ -45,7 +49,7 @@ __device__ __forceinline__ void flush_segmax(double* out, int seg, double m) {
   const int seg0 = __shfl_sync(full, seg, 0);
   if (__all_sync(full, seg == seg0)) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(full, m, o));
+    for (int o = 16; o > 0; o >>= 1) m = max_nonneg(m, __shfl_xor_sync(full, m, o));
     if ((threadIdx.x & 31) == 0 && seg0 >= 0) atomic_max_nonneg(out + seg0 * 64, m);
   } else if (seg >= 0) {
     atomic_max_nonneg(out + seg * 64, m);
@@ -67,7 +71,7 @@ __global__ void k_segmax(const double* __restrict__ v, int n, int64_t ld, const 
         seg = si;
         m = 0.0;
       }
-      m = fmax(m, fabs(v[i + c * ld]));
+      m = max_nonneg(m, fabs(v[i + c * ld]));
     }
     flush_segmax(out + c, seg, m);
   }
@@ -161,8 +165,8 @@ __global__ void __launch_bounds__(kResThreads) k_residual(const int64_t* __restr
       const double r = bv[o] - sum;
       R[pr + (int64_t)(c0 + c) * n] = r;
       Z[i + (int64_t)(c0 + c) * n] = 0.0;
-      mr[o] = fmax(mr[o], fabs(r));
-      mx[o] = fmax(mx[o], fabs(xv[o]));
+      mr[o] = max_nonneg(mr[o], fabs(r));
+      mx[o] = max_nonneg(mx[o], fabs(xv[o]));
     }
   }
   if (rowseg) {
@@ -207,34 +211,44 @@ __global__ void k_rowsum_segmax(const int64_t* __restrict__ rowptr, const double
     }
     double s = 0.0;
     for (int64_t p = rowptr[i]; p < rowptr[i + 1]; ++p) s += fabs(val[p]);
-    m = fmax(m, s);
+    m = max_nonneg(m, s);
   }
   const unsigned full = 0xffffffffu;
   const int seg0 = __shfl_sync(full, seg, 0);
   if (__all_sync(full, seg == seg0)) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(full, m, o));
+    for (int o = 16; o > 0; o >>= 1) m = max_nonneg(m, __shfl_xor_sync(full, m, o));
     if ((threadIdx.x & 31) == 0 && seg0 >= 0) atomic_max_nonneg(anorm + seg0, m);
   } else if (seg >= 0) {
     atomic_max_nonneg(anorm + seg, m);
   }
 }
 
-// eta = max over systems and right-hand sides of rmax / (anorm * xmax + bmax):
-// the normwise backward error of every system by itself.
+// eta[0] = max over systems and right-hand sides of rmax / (anorm * xmax + bmax), the normwise
+// backward error of every system by itself, over those where all four are finite; eta[1] = 1
+// when there are others.
 __global__ void k_eta(const double* __restrict__ anorm, const double* __restrict__ bmax,
                       const double* __restrict__ xmax, const double* __restrict__ rmax, int nseg, int nrhs,
                       double* __restrict__ eta) {
   double e = 0.0;
+  bool bad = false;
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nseg * nrhs; k += gridDim.x * blockDim.x) {
     const int seg = k / nrhs, c = k - seg * nrhs;
-    const double r = rmax[seg * 64 + c];
-    const double den = anorm[seg] * xmax[seg * 64 + c] + bmax[seg * 64 + c];
-    e = fmax(e, den > 0.0 ? r / den : (r > 0.0 ? 1e300 : 0.0));
+    const double an = anorm[seg], b = bmax[seg * 64 + c], x = xmax[seg * 64 + c], r = rmax[seg * 64 + c];
+    if (!isfinite(an) || !isfinite(b) || !isfinite(x) || !isfinite(r)) {
+      bad = true;
+      continue;
+    }
+    const double den = an * x + b;
+    e = max_nonneg(e, den > 0.0 ? r / den : (r > 0.0 ? 1e300 : 0.0));
   }
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) e = fmax(e, __shfl_xor_sync(0xffffffffu, e, o));
-  if ((threadIdx.x & 31) == 0) atomic_max_nonneg(eta, e);
+  for (int o = 16; o > 0; o >>= 1) e = max_nonneg(e, __shfl_xor_sync(0xffffffffu, e, o));
+  bad = __any_sync(0xffffffffu, bad);
+  if ((threadIdx.x & 31) == 0) {
+    atomic_max_nonneg(eta, e);
+    if (bad) atomic_max_nonneg(eta + 1, 1.0);
+  }
 }
 
 }  // namespace

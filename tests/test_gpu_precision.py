@@ -131,3 +131,57 @@ def test_profiling_turned_on_between_refined_solves():
     M.SetProfiling(False)
     assert backward_error(A, x1, b) <= 1e-12
     assert np.max(np.abs(x1 - x0)) <= 1e-10 * np.max(np.abs(x0))
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+@pytest.mark.parametrize("batch", [False, True])
+def test_a_right_hand_side_that_is_not_finite_fails_and_the_others_are_refined(bad, batch):
+    """A NaN must not pass as a backward error of zero: the call fails, backward_error is
+    infinite, and the other right-hand sides still reach the tolerance."""
+    import torch
+    mats = [G.laplacian_2d(20, 20), G.stencil27(6, 6, 6, 1e-2)]
+    n, cp, ri, v, *offsets = G.block_diagonal(mats) if batch else mats[0]
+    A = DistSparseMatrix.from_lower_csc(n, cp, ri, v)
+    M = symPACKMatrix2D()
+    M.Init(symPACKOptions(device=0, precision="FP32_IR"))
+    if batch:
+        M.SymbolicFactorizationBatch(A, offsets[0])
+    else:
+        M.SymbolicFactorization(A)
+    M.DistributeMatrix(A)
+    M.Factorize()
+    b = np.random.default_rng(1).standard_normal((3, n))
+    b[1, 7] = bad
+    bd, xd = torch.from_numpy(b).cuda(), torch.zeros((3, n), dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    with pytest.raises(SymPACKError, match="not finite"):
+        M.SolveDevice(bd.data_ptr(), xd.data_ptr(), 3, n)
+    assert M.info().backward_error == float("inf")
+    x = xd.cpu().numpy()
+    for k in (0, 2):
+        r = A.matvec(np.ascontiguousarray(x[k][:, None]))[:, 0] - b[k]
+        assert np.max(np.abs(r)) <= 1e-12 * (40 * np.max(np.abs(x[k])) + np.max(np.abs(b[k])))
+    b[1, 7] = 1.0  # the handle stays usable
+    bd.copy_(torch.from_numpy(b))
+    torch.cuda.synchronize()
+    M.SolveDevice(bd.data_ptr(), xd.data_ptr(), 3, n)
+    assert M.info().backward_error <= 1e-12
+    M.close()
+
+
+@pytest.mark.parametrize("schedule", ["persistent", "steps"])
+def test_a_diagonal_entry_beyond_fp32_is_not_reported_as_solved(schedule):
+    """1e39 is infinite in the FP32 factor: its unknown comes out as 0, not NaN, and the
+    refinement says that it did not converge."""
+    d = np.ones(40)
+    d[11] = 1e39
+    A = DistSparseMatrix.from_lower_csc(40, np.arange(1, 42), np.arange(1, 41, dtype=np.int32), d)
+    M = symPACKMatrix2D()
+    M.Init(symPACKOptions(device=0, precision="FP32_IR", factor_schedule=schedule))
+    M.SymbolicFactorization(A)
+    M.DistributeMatrix(A)
+    M.Factorize()
+    with pytest.raises(SymPACKError, match="refinement"):
+        M.Solve(d * 2.0)
+    assert 0 < M.info().backward_error < float("inf")
+    M.close()
