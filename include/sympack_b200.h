@@ -102,8 +102,8 @@ typedef struct spb_options {
                               form with fp32_engine 3); SPB_FACTOR_STEPS runs the level-ordered launch
                               sequence replayed from a CUDA graph (the FP32 form with engines 0-2
                               always does); SPB_FACTOR_AUTO (0, the default) is persistent for FP64
-                              and, with fp32_engine 3, for FP32 factorizations below 5e11 flops,
-                              else steps */
+                              and, with fp32_engine 3, for FP32 factorizations below 5e11 flops
+                              whose elimination tree is not very wide, else steps */
 } spb_options;
 
 #define SPB_FACTOR_AUTO 0

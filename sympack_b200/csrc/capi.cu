@@ -196,7 +196,8 @@ void release_device(spb_handle* h) {
 // grid 2.75 ms against 2.22 persistent, 27-point 28^3 2.84 / 2.49, 46^3 (2.4e11 flops) 9.40 /
 // 8.33, 50 systems of up to 6,000 rows 9.12 / 4.81), the two meet near 7e11 flops (54^3 17.8 /
 // 17.4 ms), and above, the tiles bind and the sequence's warp-specialised kernel is the
-// better engine (60^3 26.9 / 31.3, 80^3 107.7 / 156.1).
+// better engine (60^3 26.9 / 31.3, 80^3 107.7 / 156.1).  The flops are the whole handle's: a
+// batch above the line keeps the sequence, although each of its systems is short.
 constexpr double kFp32PersistentFlops = 5e11;
 bool persistent_schedule(const spb_options& o, double flops) {
   if (o.precision == SPB_PRECISION_FP64) return o.factor_schedule != SPB_FACTOR_STEPS;
@@ -204,7 +205,8 @@ bool persistent_schedule(const spb_options& o, double flops) {
   return o.factor_schedule == SPB_FACTOR_PERSISTENT ||
          (o.factor_schedule == SPB_FACTOR_AUTO && flops < kFp32PersistentFlops);
 }
-bool persistent_factor(const spb_handle* h) { return persistent_schedule(h->opt, h->sym.flops_stat); }
+// The plan has the last word: wide FP32 trees keep the sequence (kWideSupernodesPerStep).
+bool persistent_factor(const spb_handle* h) { return h->plan.persistent; }
 
 spb::dev::FactorArgs factor_args(spb_handle* h) {
   spb::dev::FactorArgs a;
@@ -765,6 +767,7 @@ spb::PlanParams plan_params_of(const spb_options& o, const spb::Symbolic& sym) {
   if (o.plan_solve_chunk > 0) pp.solve_sb = o.plan_solve_chunk;
   if (o.plan_solve_tiles > 0) pp.solve_tpt = o.plan_solve_tiles;
   pp.factor_dag = persistent_schedule(o, sym.flops_stat);
+  pp.dag_unless_wide = o.precision != SPB_PRECISION_FP64 && o.factor_schedule == SPB_FACTOR_AUTO;
   pp.fp32 = o.precision == SPB_PRECISION_FP32_IR;
   return pp;
 }

@@ -317,7 +317,9 @@ Plan build_plan(const Symbolic& sym, const PlanParams& prm) {
     P.step_flops[k] = f;
   }
   for (const SnMeta& m : P.meta) P.solve_sweep_bytes += 8.0 * m.h * m.w;
-  if (prm.factor_dag) build_factor_dag(P, prm);
+  P.persistent = prm.factor_dag &&
+                 !(prm.dag_unless_wide && P.nsuper > (int64_t)kWideSupernodesPerStep * (int64_t)P.steps.size());
+  if (P.persistent) build_factor_dag(P, prm);
 
   // Solve super-blocks: per supernode, its first super-block counter and (for
   // supernodes wider than one block) the offset of its inverse tiles.

@@ -276,6 +276,7 @@ struct Plan {
   std::vector<Step> steps;
   int32_t max_diag_slots = 0;      // scratch slots of the diagonal blocks (one per diagonal block)
   int32_t big_tile_rows = 128;     // PlanParams::big_tile_rows of this plan
+  bool persistent = false;         // the factorization runs as the tasks below, not as the steps
   // persistent factorization: tasks in dispatch order (topological), their waits and signals
   std::vector<FTask> ftasks;
   std::vector<FWait> fwaits;
@@ -323,6 +324,15 @@ constexpr int kWarpMaxW = 16, kWarpMaxOff = 128;
 constexpr int kSolveGroup = 16, kSolveGroups = 4;
 constexpr int kTinyMaxW = 4, kTinyMaxElems = 64, kTinyBatch = 128;
 
+// FP32 factorizations left to the automatic schedule: supernodes per step of the level-ordered
+// sequence above which the sequence is kept.  A launch of it costs about 13 us, however many
+// supernodes it takes; the persistent launch has one block per SM (the tensor-core tile's
+// shared memory) and takes about 8 us a supernode and block, 230 of them in 13 us on 148 SMs.
+// Measured, persistent / steps in ms: 800 x 800 grid (193 supernodes a step) 5.76 / 5.99,
+// 1000 x 1000 (259) 8.65 / 7.68, 1400 x 1400 (392) 16.4 / 11.8; 300 30 x 30 grids (2,400) 1.88 /
+// 0.72, 2,000 6^3 grids (6,333) 2.24 / 0.77; 200 systems of 500 to 700 rows (72) 1.36 / 2.21.
+constexpr int kWideSupernodesPerStep = 230;
+
 // Tunables of the plan.
 struct PlanParams {
   int small_max_w = 32;          // widest panel handled by the fused small-panel kernel
@@ -334,13 +344,15 @@ struct PlanParams {
   int solve_tpt = 2;             // 64 x 64 tiles per DI / U / V / O / W solve task (>= 1)
   int sms = 148;                 // SMs of the device: a launch with too few tiles to fill them
                                  // splits its tiles' K range (partial products add atomically)
-  bool factor_dag = true;        // build the persistent factorization's task graph (FP64 handles)
+  bool factor_dag = true;        // build the persistent factorization's task graph
+  bool dag_unless_wide = false;  // only when the tree is not too wide for it (kWideSupernodesPerStep)
   bool fp32 = false;             // FP32 factor (precision form): 128 x 128 tensor-core tiles, one CTA
                                  // per SM; FP64: 128 x 64 tiles at two CTAs per SM
   bool operator==(const PlanParams& o) const {
     return small_max_w == o.small_max_w && small_max_bytes == o.small_max_bytes && nb == o.nb &&
            outer_nb == o.outer_nb && big_tile_rows == o.big_tile_rows && solve_sb == o.solve_sb &&
-           solve_tpt == o.solve_tpt && sms == o.sms && factor_dag == o.factor_dag && fp32 == o.fp32;
+           solve_tpt == o.solve_tpt && sms == o.sms && factor_dag == o.factor_dag && dag_unless_wide == o.dag_unless_wide &&
+           fp32 == o.fp32;
   }
 };
 
