@@ -607,8 +607,8 @@ int ir_solve(spb_handle* h, const double* d_b, int64_t ldb, double* d_x, int64_t
       SPB_CK(h, cudaMemsetAsync(xmax, 0, sizeof(double) * 128 * (size_t)nseg, h->stream));
       SPB_CK(h, cudaMemsetAsync(h->d_norms, 0, 2 * sizeof(double), h->stream));
       // the residual goes where a correction solve reads its right-hand sides
-      spb::dev::launch_residual(h->stream, h->d_rowptr, h->d_col, h->d_val, x, ldx, b, ldb, h->dX, h->dinvp0, n, nr,
-                                h->d_rowseg, xmax, rmax, h->dZ, h->dsync, sync_ints(h));
+      spb::dev::launch_residual(h->stream, h->d_rowptr, h->d_col, h->d_val, x, ldx, b, ldb, h->dX, h->dinvp0, n,
+                                (int64_t)h->csr_col.size(), nr, h->d_rowseg, xmax, rmax, h->dZ, h->dsync, sync_ints(h));
       spb::dev::launch_eta(h->stream, anorm, bmax, xmax, rmax, nseg, nr, h->d_norms);
       SPB_CK(h, cudaMemcpyAsync(measured, h->d_norms, sizeof(measured), cudaMemcpyDeviceToHost, h->stream));
       int rc = check_solve_status(h);  // synchronizes

@@ -80,13 +80,18 @@ __global__ void k_segmax(const double* __restrict__ v, int n, int64_t ld, const 
 // One refinement step's view of the current x: r = b - A x, stored permuted (R[invp[i] + c n],
 // the right-hand side of the correction solve), with max |x| and max |r| per system and
 // column (xmax, rmax; layout as in k_segmax) taken on the way and Z and the counters cleared
-// for the correction's sweeps.  Bound by the reads of A: four
-// lanes share a row, so that a load of val takes whole sectors, and CB columns share each
+// for the correction's sweeps.  Bound by the reads of A: LPR lanes
+// share a row, so that a load of val takes whole sectors, and CB columns share each
 // entry of A, so that A is read ceil(nrhs / CB) times.  A block takes a contiguous run of rows
 // and keeps its maxima in registers to the end of the run (or of a system).  27-point 36^3, 50
 // columns: the warp-per-entry kernel and the two passes for the maxima took 0.73 ms a step.
+// Four lanes share a short row, a warp the rows of matrices with more than kWarpRow entries a
+// row on average (refined solve of one right-hand side, dense n = 1,000: 297 us with 4 lanes,
+// 177 with 32; 42 entries a row: equal).  Rows beyond kLongRow entries are left to the whole
+// block at the end (n = 50,000 with one full row: 6.58 ms with 4 lanes on it, 0.38 so).
+constexpr int kLongRow = 1024, kLongRows = 64, kWarpRow = 64;
 constexpr int kResThreads = 256;
-template <int CB>
+template <int CB, int LPR>
 __global__ void __launch_bounds__(kResThreads) k_residual(const int64_t* __restrict__ rowptr, const int32_t* __restrict__ col,
                                                           const double* __restrict__ val, const double* __restrict__ x,
                                                           int64_t ldx, const double* __restrict__ b, int64_t ldb,
@@ -95,57 +100,72 @@ __global__ void __launch_bounds__(kResThreads) k_residual(const int64_t* __restr
                                                           double* __restrict__ xmax, double* __restrict__ rmax,
                                                           double* __restrict__ Z, int32_t* __restrict__ sync,
                                                           int64_t nsync) {
-  constexpr int kOwn = (CB + 3) / 4;  // columns whose sums a lane finishes
+  constexpr int kOwn = (CB + LPR - 1) / LPR;  // columns whose sums a lane finishes
   __shared__ unsigned long long smax[2][CB];
-  const int c0 = blockIdx.y * CB, nc = min(CB, nrhs - c0), q = threadIdx.x & 3;
+  __shared__ double part[kResThreads / 32][CB];
+  __shared__ int nlong, longs[kLongRows];
+  const int c0 = blockIdx.y * CB, nc = min(CB, nrhs - c0), q = threadIdx.x & (LPR - 1);
   for (int64_t i = (blockIdx.y * (int64_t)gridDim.x + blockIdx.x) * kResThreads + threadIdx.x; i < nsync;
        i += (int64_t)gridDim.x * gridDim.y * kResThreads)
     sync[i] = 0;
   if (threadIdx.x < 2 * CB) smax[threadIdx.x / CB][threadIdx.x % CB] = 0;
+  if (threadIdx.x == 0) nlong = 0;
   __syncthreads();
-  const int64_t chunk = ((n + gridDim.x - 1) / gridDim.x + 63) / 64 * 64;
+  constexpr int kRows = kResThreads / LPR;
+  const int64_t chunk = ((n + gridDim.x - 1) / gridDim.x + kRows - 1) / kRows * kRows;
   const int64_t r0 = blockIdx.x * chunk, r1 = min((int64_t)n, r0 + chunk);
   double mr[kOwn], mx[kOwn];
 #pragma unroll
   for (int o = 0; o < kOwn; ++o) mr[o] = mx[o] = 0.0;
   int seg = -1;
-  for (int64_t base = r0; base < r1; base += kResThreads / 4) {
-    const int64_t i = base + (threadIdx.x >> 2);
-    const bool in = i < r1;
+  for (int64_t base = r0; base < r1; base += kRows) {
+    const int64_t i = base + threadIdx.x / LPR;
+    bool in = i < r1;
     double s[CB], bv[kOwn], xv[kOwn];
-    int64_t pr = 0;
+    int64_t pr = 0, p0 = 0, p1 = 0;
 #pragma unroll
     for (int c = 0; c < CB; ++c) s[c] = 0.0;
+    if (in) {
+      p1 = rowptr[i + 1], p0 = rowptr[i] + q;
+      if (p1 - p0 + q > kLongRow) {  // to the list, while it has room
+        const unsigned group = 0xffffffffu >> (32 - LPR) << (threadIdx.x & 31 & ~(LPR - 1));
+        int at = q == 0 ? atomicAdd(&nlong, 1) : 0;
+        at = __shfl_sync(group, at, 0, LPR);
+        if (at < kLongRows) {
+          if (q == 0) longs[at] = (int)i;
+          in = false;
+        }
+      }
+    }
     if (in) {  // everything that does not depend on the row's entries first
-      const int64_t p1 = rowptr[i + 1], p0 = rowptr[i] + q;
       pr = invp0[i];
 #pragma unroll
       for (int o = 0; o < kOwn; ++o) {
-        const int c = 4 * o + q;
+        const int c = LPR * o + q;
         bv[o] = c < nc ? b[i + (c0 + c) * ldb] : 0.0;
         xv[o] = c < nc ? x[i + (c0 + c) * ldx] : 0.0;
       }
-      for (int64_t p = p0; p < p1; p += 8) {  // two of the lane's entries at a time
-        const bool two = p + 4 < p1;
-        const double v0 = val[p], v1 = two ? val[p + 4] : 0.0;
+      for (int64_t p = p0; p < p1; p += 2 * LPR) {  // two of the lane's entries at a time
+        const bool two = p + LPR < p1;
+        const double v0 = val[p], v1 = two ? val[p + LPR] : 0.0;
         const double* x0 = x + col[p] + c0 * ldx;
-        const double* x1 = two ? x + col[p + 4] + c0 * ldx : x0;
+        const double* x1 = two ? x + col[p + LPR] + c0 * ldx : x0;
 #pragma unroll
         for (int c = 0; c < CB; ++c)
           if (c < nc) s[c] = fma(v1, two ? x1[c * ldx] : 0.0, fma(v0, x0[c * ldx], s[c]));
       }
     }
+    __syncwarp();
 #pragma unroll
-    for (int c = 0; c < CB; ++c) {
-      s[c] += __shfl_xor_sync(0xffffffffu, s[c], 1);
-      s[c] += __shfl_xor_sync(0xffffffffu, s[c], 2);
-    }
+    for (int c = 0; c < CB; ++c)
+#pragma unroll
+      for (int o = 1; o < LPR; o *= 2) s[c] += __shfl_xor_sync(0xffffffffu, s[c], o);
     if (!in) continue;
     if (rowseg && rowseg[i] != seg) {
       if (seg >= 0) {
 #pragma unroll
         for (int o = 0; o < kOwn; ++o) {
-          const int c = 4 * o + q;
+          const int c = LPR * o + q;
           if (c >= nc) continue;
           atomic_max_nonneg(rmax + seg * 64 + c0 + c, mr[o]);
           atomic_max_nonneg(xmax + seg * 64 + c0 + c, mx[o]);
@@ -156,12 +176,12 @@ __global__ void __launch_bounds__(kResThreads) k_residual(const int64_t* __restr
     }
 #pragma unroll
     for (int o = 0; o < kOwn; ++o) {
-      const int c = 4 * o + q;
+      const int c = LPR * o + q;
       if (c >= nc) continue;
-      double sum = s[4 * o];
+      double sum = s[0];
 #pragma unroll
-      for (int e = 1; e < 4; ++e)
-        if (4 * o + e < CB && q == e) sum = s[4 * o + e];
+      for (int e = 1; e < CB; ++e)
+        if (e / LPR == o && c == e) sum = s[e];
       const double r = bv[o] - sum;
       R[pr + (int64_t)(c0 + c) * n] = r;
       Z[i + (int64_t)(c0 + c) * n] = 0.0;
@@ -169,11 +189,47 @@ __global__ void __launch_bounds__(kResThreads) k_residual(const int64_t* __restr
       mx[o] = max_nonneg(mx[o], fabs(xv[o]));
     }
   }
+  __syncthreads();
+  const int listed = min(nlong, kLongRows);
+  for (int k = 0; k < listed; ++k) {  // a long row: every thread its share, summed over the block
+    const int64_t i = longs[k], p1 = rowptr[i + 1];
+    double s[CB];
+#pragma unroll
+    for (int c = 0; c < CB; ++c) s[c] = 0.0;
+#pragma unroll 2
+    for (int64_t p = rowptr[i] + threadIdx.x; p < p1; p += kResThreads) {
+      const double v = val[p];
+      const double* xp = x + col[p] + c0 * ldx;
+#pragma unroll
+      for (int c = 0; c < CB; ++c)
+        if (c < nc) s[c] = fma(v, xp[c * ldx], s[c]);
+    }
+#pragma unroll
+    for (int c = 0; c < CB; ++c) {
+#pragma unroll
+      for (int o = 1; o < 32; o *= 2) s[c] += __shfl_xor_sync(0xffffffffu, s[c], o);
+      if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5][c] = s[c];
+    }
+    __syncthreads();
+    if (threadIdx.x < nc) {
+      const int c = threadIdx.x;
+      double sum = 0.0;
+#pragma unroll
+      for (int w = 0; w < kResThreads / 32; ++w) sum += part[w][c];
+      const double r = b[i + (c0 + c) * ldb] - sum, xi = fabs(x[i + (c0 + c) * ldx]);
+      R[invp0[i] + (int64_t)(c0 + c) * n] = r;
+      Z[i + (int64_t)(c0 + c) * n] = 0.0;
+      const int sg = rowseg ? rowseg[i] : 0;
+      atomic_max_nonneg(rmax + sg * 64 + c0 + c, fabs(r));
+      atomic_max_nonneg(xmax + sg * 64 + c0 + c, xi);
+    }
+    __syncthreads();
+  }
   if (rowseg) {
     if (seg >= 0) {
 #pragma unroll
       for (int o = 0; o < kOwn; ++o) {
-        const int c = 4 * o + q;
+        const int c = LPR * o + q;
         if (c >= nc) continue;
         atomic_max_nonneg(rmax + seg * 64 + c0 + c, mr[o]);
         atomic_max_nonneg(xmax + seg * 64 + c0 + c, mx[o]);
@@ -183,7 +239,7 @@ __global__ void __launch_bounds__(kResThreads) k_residual(const int64_t* __restr
   }
 #pragma unroll
   for (int o = 0; o < kOwn; ++o) {
-    const int c = 4 * o + q;
+    const int c = LPR * o + q;
     if (c >= nc) continue;
     atomicMax(&smax[0][c], (unsigned long long)__double_as_longlong(mr[o]));
     atomicMax(&smax[1][c], (unsigned long long)__double_as_longlong(mx[o]));
@@ -258,17 +314,22 @@ void launch_gather(cudaStream_t st, double* dst, const double* src, const int64_
 }
 
 void launch_residual(cudaStream_t st, const int64_t* rowptr, const int32_t* col, const double* val, const double* x,
-                     int64_t ldx, const double* b, int64_t ldb, double* R, const int32_t* invp0, int n, int nrhs,
-                     const int32_t* rowseg, double* xmax, double* rmax, double* Z, int32_t* sync, int64_t nsync) {
-  auto run = [&](auto cb) {
-    constexpr int CB = decltype(cb)::value;
-    const int by = (nrhs + CB - 1) / CB, rows = (n + 63) / 64, cap = (148 * 16 + by - 1) / by;
-    k_residual<CB><<<dim3(rows < cap ? rows : cap, by), kResThreads, 0, st>>>(rowptr, col, val, x, ldx, b, ldb, R, invp0,
-                                                                              n, nrhs, rowseg, xmax, rmax, Z, sync, nsync);
+                     int64_t ldx, const double* b, int64_t ldb, double* R, const int32_t* invp0, int n, int64_t nnz,
+                     int nrhs, const int32_t* rowseg, double* xmax, double* rmax, double* Z, int32_t* sync,
+                     int64_t nsync) {
+  auto run = [&](auto cb, auto lpr) {
+    constexpr int CB = decltype(cb)::value, LPR = decltype(lpr)::value, kRows = kResThreads / LPR;
+    const int by = (nrhs + CB - 1) / CB, rows = (n + kRows - 1) / kRows, cap = (148 * 16 + by - 1) / by;
+    k_residual<CB, LPR><<<dim3(rows < cap ? rows : cap, by), kResThreads, 0, st>>>(
+        rowptr, col, val, x, ldx, b, ldb, R, invp0, n, nrhs, rowseg, xmax, rmax, Z, sync, nsync);
   };
-  if (nrhs == 1) run(std::integral_constant<int, 1>());
-  else if (nrhs <= 4) run(std::integral_constant<int, 4>());
-  else run(std::integral_constant<int, 8>());
+  auto lanes = [&](auto cb) {
+    if (nnz > kWarpRow * (int64_t)n) run(cb, std::integral_constant<int, 32>());
+    else run(cb, std::integral_constant<int, 4>());
+  };
+  if (nrhs == 1) lanes(std::integral_constant<int, 1>());
+  else if (nrhs <= 4) lanes(std::integral_constant<int, 4>());
+  else lanes(std::integral_constant<int, 8>());
 }
 
 void launch_segmax(cudaStream_t st, const double* v, int n, int nrhs, int64_t ld, const int32_t* rowseg,

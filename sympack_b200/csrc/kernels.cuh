@@ -130,8 +130,9 @@ void launch_diag_inverse(cudaStream_t st, const void* L, double* Inv, bool fp32,
 // per-system, per-column max |x| and max |r| (zeroed by the caller), max |v|, max row sum of |A|.
 void launch_gather(cudaStream_t st, double* dst, const double* src, const int64_t* idx, int64_t n);
 void launch_residual(cudaStream_t st, const int64_t* rowptr, const int32_t* col, const double* val, const double* x,
-                     int64_t ldx, const double* b, int64_t ldb, double* R, const int32_t* invp0, int n, int nrhs,
-                     const int32_t* rowseg, double* xmax, double* rmax, double* Z, int32_t* sync, int64_t nsync);
+                     int64_t ldx, const double* b, int64_t ldb, double* R, const int32_t* invp0, int n, int64_t nnz,
+                     int nrhs, const int32_t* rowseg, double* xmax, double* rmax, double* Z, int32_t* sync,
+                     int64_t nsync);
 void launch_segmax(cudaStream_t st, const double* v, int n, int nrhs, int64_t ld, const int32_t* rowseg,
                    double* out);
 void launch_rowsum_segmax(cudaStream_t st, const int64_t* rowptr, const double* val, int n, const int32_t* rowseg,

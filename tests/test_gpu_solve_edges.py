@@ -105,6 +105,53 @@ def test_refined_solves_with_a_padded_leading_dimension(border):
     M.close()
 
 
+def long_rows(n, rows, entries, seed):
+    """n unknowns coupled only to the last `rows` ones, each of those to `entries` others."""
+    rng = np.random.default_rng(seed)
+    i = np.concatenate([np.sort(rng.choice(n - rows, entries, replace=False)) for _ in range(rows)])
+    j = np.repeat(np.arange(n - rows, n), entries)
+    return G._dominant(n, i, j, -rng.uniform(0.05, 1.0, len(i)), 1e-2)
+
+
+@pytest.mark.parametrize("n,rows,entries,batch", [
+    (3000, 1, 1024, False), (3000, 1, 1025, False), (30000, 2, 20000, False), (3000, 2, 2000, True),
+    (40000, 100, 1100, False),  # more long rows in one block than its list holds (64 columns)
+    (1200, 1100, 64, False),    # rows of more than 64 entries on average: a warp each
+    (2000, 1900, 90, True),
+])
+def test_residuals_of_long_rows(n, rows, entries, batch):
+    """Rows of A around and beyond what four lanes, a warp and a block of the residual kernel take."""
+    mats = [long_rows(n, rows, entries, 1)]
+    if batch:
+        mats += [G.laplacian_2d(9, 7, 0.1), long_rows(n + 500, rows, entries, 2)]
+    a = G.block_diagonal(mats) if batch else mats[0]
+    A = DistSparseMatrix.from_lower_csc(*a[:4])
+    M = symPACKMatrix2D()
+    M.Init(symPACKOptions(device=0, orderingStr="NATURAL", precision="FP32_IR", relax=RelaxationParameters(0, 0, 0, 0, 0.0, 0.0, 0.0)))
+    if batch:
+        M.SymbolicFactorizationBatch(A, a[4])
+    else:
+        M.SymbolicFactorization(A)
+    M.DistributeMatrix(A)
+    M.Factorize()
+    offsets = a[4] if batch else [0, n]
+    cols = np.repeat(np.arange(A.size), np.diff(A.colptr))
+    off = A.rowind - 1 != cols
+    s = np.zeros(A.size)
+    np.add.at(s, A.rowind - 1, np.abs(A.nzvalLocal))
+    np.add.at(s, cols[off], np.abs(A.nzvalLocal[off]))
+    for nrhs in (1, 3, 9, 64):
+        b = np.random.default_rng(nrhs).standard_normal((A.size, nrhs))
+        M.Solve(b)
+        x = M.GetSolution(nrhs=nrhs)
+        r = np.abs(A.matvec(x) - b)
+        for lo, hi in zip(offsets[:-1], offsets[1:]):  # every system by itself
+            den = s[lo:hi].max() * np.abs(x[lo:hi]).max(axis=0) + np.abs(b[lo:hi]).max(axis=0)
+            assert (r[lo:hi].max(axis=0) / den).max() <= 1.01e-12
+        assert M.info().backward_error <= 1e-12
+    M.close()
+
+
 def dense_spd(n, cond, seed):
     rng = np.random.default_rng(seed)
     q, _ = np.linalg.qr(rng.standard_normal((n, n)))
