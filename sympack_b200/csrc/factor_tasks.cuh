@@ -83,13 +83,18 @@ constexpr int kPiece = 8;
 // > 0 is reported (who: this warp reports) and replaced by 1.  LDL^T (Potf2_LDL, lapack.hpp:206-270, lower triangle): d_k =
 // A_kk, |d_k| > 0 or reported; rs = 1 / d_k, x becomes the row's entries of L D.  Reported
 // pivots: column col + k of supernode s, k < valid.
-template <bool kLdl>
+// kShort: a piece of fewer than 8 columns ends there (valid of them), else its padding is factored too.
+template <bool kLdl, bool kShort>
 __device__ __forceinline__ void piece_rows(double (&x)[kPiece], double (&rs)[kPiece], bool who, int valid,
                                            Status* status, int s, int col) {
   const int lane = thread_id() & 31;
   double own = x[0];  // lane k: its pivot, kept ahead of the row's other entries
 #pragma unroll
   for (int k = 0; k < kPiece; ++k) {
+    if (kShort && k >= valid) {
+      rs[k] = 1.0;
+      continue;
+    }
     const double d = __shfl_sync(0xffffffffu, own, k);
     rs[k] = kLdl ? 1.0 / d : rsqrt(d);
     if (kLdl ? !(fabs(d) > 0.0) : !(d > 0.0)) {
@@ -164,7 +169,7 @@ __device__ __forceinline__ void factor_small_task(const FactorArgs& a, int s, co
 #pragma unroll
       for (int j = 0; j < kPiece; ++j)
         x[j] = r < h && j < pw && (lane < pw || lane >= kPiece) ? P[r + (kb + j) * ldp] : (lane == j ? 1.0 : 0.0);
-      piece_rows<kLdl>(x, rs, warp == 0, pw, a.status, s, m.fc + kb);
+      piece_rows<kLdl, true>(x, rs, warp == 0, pw, a.status, s, m.fc + kb);
     }
     __syncthreads();  // every warp has the piece before its rows are overwritten
     if (active) {
@@ -346,7 +351,7 @@ __device__ __forceinline__ void diag_task(const FactorArgs& a, const PanelItem& 
       if (active) {
 #pragma unroll
         for (int j = 0; j < kPiece; ++j) x[j] = row < kNB ? D[row + (kb + j) * kDL] : 0.0;
-        piece_rows<kLdl>(x, rs, warp == 0, nb - kb, a.status, it.s, m.fc + c0 + kb);
+        piece_rows<kLdl, false>(x, rs, warp == 0, nb - kb, a.status, it.s, m.fc + c0 + kb);
       } else if (warp == 2) {  // no rows left for it: the piece before's inverse
         invert(p - 1);
       }

@@ -66,6 +66,20 @@ def test_update_tiles_see_the_panels_finished_before_them(dec):
     S.close()
 
 
+@pytest.mark.parametrize("schedule", ["persistent", "steps"])
+@pytest.mark.parametrize("dec", ["LL", "LDL"])
+@pytest.mark.parametrize("widths,border", [([1] * 70, 1), ([1] * 40, 31), ([3, 4] * 20, 4), ([5, 7] * 15, 9), ([12] * 9, 30), ([30] * 5, 20)])
+def test_launches_of_tiny_panels(widths, border, dec, schedule):
+    """Panels of up to 32, 256 and 1,024 entries, the sizes up to which a launch of them takes 32,
+    64 and 128 threads a panel; pieces that end before their eighth column."""
+    A = DistSparseMatrix.from_lower_csc(*bordered(widths, border, len(widths)))
+    M = solver(A, decomposition=dec, factor_schedule=schedule)
+    f = oracle_for(M, A, dec == "LDL")
+    Lo = f.factor()
+    assert np.max(np.abs(M.GetFactor() - Lo)) <= TOL * np.max(np.abs(Lo))
+    M.close()
+
+
 @pytest.mark.parametrize("column", [0, 5, 12, 40])
 def test_a_bad_pivot_is_reported_where_it_is(column):
     """The first non-positive pivot's column, in a piece's interior and beyond the first piece."""
