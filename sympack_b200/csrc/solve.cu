@@ -34,7 +34,7 @@
 // on the FP64 tensor pipe for one right-hand side too: an 8-column group costs no
 // more issue slots than scalar FMAs with their shared-memory reads would.
 // FP32 factors are widened as they enter a product.  60^3 Laplacian, FP64: 1 right-hand side
-// 2.16 -> 1.25 ms, 16 right-hand sides 4.85 -> 2.16 ms against tasks that staged their tiles
+// 2.16 -> 1.22 ms, 16 right-hand sides 4.85 -> 2.16 ms against tasks that staged their tiles
 // in shared memory and multiplied with scalar FMAs (0.34 ms by the bytes of both sweeps).
 #include <type_traits>
 
@@ -208,7 +208,7 @@ __device__ __forceinline__ void clear(double (&acc)[NG][4]) {
 // 1e12, residual against |L||L^T||x|: 1.9e-16 alone, 2.0e-17 corrected, 1.2e-17 by
 // substitution.  FP32 factors need none: their own rounding is 1e9 times that, and refinement
 // recomputes the residual.  Costs two more products and barriers a task: 60^3 Laplacian 1.20 ->
-// 1.25 ms, 16 right-hand sides 2.09 -> 2.16, 27-point 17^3 0.168 -> 0.181.
+// 1.22 ms, 16 right-hand sides 2.09 -> 2.16, 27-point 17^3 0.168 -> 0.182.
 template <class T>
 constexpr bool kCorrect = std::is_same<T, double>::value;
 
@@ -218,16 +218,26 @@ constexpr bool kCorrect = std::is_same<T, double>::value;
 // ldiag.
 template <class T>
 __device__ __forceinline__ void stage_inverse(double* s, double* ldiag, const double* inv, const T* L, int64_t ld, int w) {
-  const int wr = (w + 15) & ~15;
-  for (int idx = threadIdx.x; idx < wr * kT; idx += kThreads) {
-    const int c = idx >> 6, r = idx & 63;
-    if (r >= wr || (kCorrect<T> && r < c)) continue;
-    const bool in = r < w && c < w && r >= c;
-    s[r + c * kInvLd] = in ? __ldg(inv + r + c * w) : 0.0;
-    if constexpr (kCorrect<T>) {
-      const double l = in ? (double)__ldg(L + r + c * ld) : 0.0;
-      if (r > c) s[c + r * kInvLd] = l;
-      else ldiag[r] = l;
+  const int wr = (w + 15) & ~15, r = threadIdx.x & 63;
+  if (r >= wr) return;
+  for (int c0 = threadIdx.x >> 6; c0 < wr; c0 += 16) {  // four columns' loads in flight
+    double v[4], l[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int c = c0 + 4 * q;
+      const bool in = r < w && c < w && r >= c;
+      v[q] = in ? __ldg(inv + r + c * w) : 0.0;
+      if constexpr (kCorrect<T>) l[q] = in ? (double)__ldg(L + r + c * ld) : 0.0;
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int c = c0 + 4 * q;
+      if (kCorrect<T> ? r < c : c >= wr) continue;
+      s[r + c * kInvLd] = v[q];
+      if constexpr (kCorrect<T>) {
+        if (r > c) s[c + r * kInvLd] = l[q];
+        else ldiag[r] = l[q];
+      }
     }
   }
 }
