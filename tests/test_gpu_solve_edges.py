@@ -105,6 +105,23 @@ def test_refined_solves_with_a_padded_leading_dimension(border):
     M.close()
 
 
+@pytest.mark.parametrize("dec", ["LL", "LDL"])
+@pytest.mark.parametrize("leaves", [31, 32, 33, 64, 200])
+@pytest.mark.parametrize("border", [1, 3])
+def test_tiny_leaves_that_share_their_rows(leaves, border, dec):
+    """One-column leaves on the same few rows, in and beyond whole warps, with right-hand-side
+    counts whose columns start inside a warp."""
+    A = DistSparseMatrix.from_lower_csc(*bordered([1] * leaves, border, leaves))
+    M = solver(A, decomposition=dec)
+    f = oracle_for(M, A, dec == "LDL")
+    for nrhs in (1, 3, 16, 17):
+        b = np.random.default_rng(nrhs).standard_normal((A.size, nrhs))
+        M.Solve(b)
+        x, xo = M.GetSolution(nrhs=nrhs), f.solve(b)
+        assert np.max(np.abs(x - xo)) <= TOL * np.max(np.abs(xo))
+    M.close()
+
+
 def long_rows(n, rows, entries, seed):
     """n unknowns coupled only to the last `rows` ones, each of those to `entries` others."""
     rng = np.random.default_rng(seed)
