@@ -454,6 +454,9 @@ void ensure_inverses(spb_handle* h) {
 void enqueue_sweeps(spb_handle* h, double* X, double* Z, int32_t* sync, int groups, int nrhs, bool prof) {
   const spb::Plan& P = h->plan;
   const size_t ints = spb::solve_sync_ints(P);
+  // tickets (a task for a group of right-hand sides) count in 32 bits
+  const int64_t most = std::max(P.fwd_recs.size(), P.bwd_recs.size());
+  groups = (int)std::min<int64_t>(groups, std::max<int64_t>(1, (INT32_MAX - 65536) / std::max<int64_t>(1, most)));
   const int step = spb::kSolveGroup * groups;
   for (int c0 = 0, pass = 0; c0 < nrhs; c0 += step, ++pass) {
     // counters must start at zero; what filled X cleared them for the first pass, and Z
@@ -479,6 +482,7 @@ void enqueue_sweeps(spb_handle* h, double* X, double* Z, int32_t* sync, int grou
     a.ntiny = (int)P.tiny.size();
     a.sync = sync;
     a.sync_stride = (int64_t)ints;
+    a.row_unit = P.row_unit;
     a.status = h->dstatus;
     a.spin_limit = h->wait_limit;
     const size_t e0 = 4 * (size_t)pass;

@@ -103,6 +103,7 @@ struct PSolveArgs {
   int nrhs;  // <= kSolveGroup * kSolveGroups
   const SolveRec* recs;
   const SolveRec* subs;
+  int row_unit;      // Plan::row_unit of the records
   int ntasks;
   const TinyRec* tiny;  // tiny leaf supernodes (Plan::tiny_recs)
   int ntiny;

@@ -2,7 +2,6 @@
 
 #include <algorithm>
 #include <atomic>
-#include <climits>
 #include <cstdint>
 #include <queue>
 #include <stdexcept>
@@ -24,13 +23,11 @@ Plan build_plan(const Symbolic& sym, const PlanParams& prm) {
   P.big_tile_rows = prm.big_tile_rows;
   const int ns = P.nsuper;
   P.meta.resize(ns);
-  P.rows.resize(sym.lindx.size());
-  for (size_t k = 0; k < sym.lindx.size(); ++k) P.rows[k] = sym.lindx[k] - 1;
   P.lindx_total = (int64_t)sym.lindx.size();
   P.supmember0.resize(sym.n);
   for (int i = 0; i < sym.n; ++i) P.supmember0[i] = sym.supmember[i] - 1;
 
-  int64_t off = 0;
+  int64_t off = 0, lend = 0;
   for (int s = 0; s < ns; ++s) {
     SnMeta& m = P.meta[s];
     m.fc = sym.xsuper[s] - 1;
@@ -38,7 +35,8 @@ Plan build_plan(const Symbolic& sym, const PlanParams& prm) {
     m.h = (int32_t)(sym.xlindx[s + 1] - sym.xlindx[s]);
     m.ld = (int32_t)round_up(m.h, 4);
     m.off = off;
-    m.lidx = sym.xlindx[s] - 1;
+    m.lidx = round_up(lend + m.w, kRowUnit) - m.w;
+    lend = m.lidx + m.h;
     m.boff = P.nblk_total;
     m.sboff = 0;
     m.ioff = -1;
@@ -46,6 +44,9 @@ Plan build_plan(const Symbolic& sym, const PlanParams& prm) {
     off += round_up((int64_t)m.ld * m.w, 32);
   }
   P.arena_elems = off;
+  P.rows.assign(lend, 0);
+  for (int s = 0; s < ns; ++s)
+    for (int r = 0; r < P.meta[s].h; ++r) P.rows[P.meta[s].lidx + r] = sym.lindx[sym.xlindx[s] - 1 + r] - 1;
 
   // supernodal elimination tree and height levels
   P.sparent.assign(ns, -1);
@@ -436,6 +437,7 @@ Plan build_plan(const Symbolic& sym, const PlanParams& prm) {
   for (size_t i = 0; i < P.tiny.size(); i += kTinyBatch)  // the tiny leaves last
     P.bwd_tasks.push_back(SolveTask{P.tiny[i], 6, (int32_t)i,
                                     (int32_t)std::min<size_t>(kTinyBatch, P.tiny.size() - i)});
+  P.row_unit = prm.wide_rows || P.rows.size() > (size_t)INT32_MAX ? kRowUnit : 1;
   build_solve_recs(P);
   return P;
 }
@@ -443,9 +445,6 @@ Plan build_plan(const Symbolic& sym, const PlanParams& prm) {
 // Device records of the solve tasks, and the places of the one-block supernodes' inverses.
 static void build_solve_recs(Plan& P) {
   const int ns = P.nsuper, SB = P.solve_sb, TPT = P.solve_tpt;
-  if (std::max(P.fwd_tasks.size(), P.bwd_tasks.size()) >= ((size_t)1 << 28))
-    throw std::runtime_error("plan: more than 2^28 solve tasks");
-  if (P.rows.size() > (size_t)INT32_MAX) throw std::runtime_error("plan: row lists beyond 2^31 entries");
   std::vector<uint8_t> tiny(ns, 0);
   for (int32_t s : P.tiny) tiny[s] = 1;
   std::vector<int64_t> inv(ns, -1);
@@ -485,7 +484,7 @@ static void build_solve_recs(Plan& P) {
       r.m = m.w;
       r.k = kind == 4 ? m.h - m.w : 0;
       r.x0 = m.fc;
-      r.y0 = (int32_t)(m.lidx + m.w);
+      r.y0 = (int32_t)((m.lidx + m.w) / P.row_unit);
       if (fwd) {
         r.wait = arrived + s;  // the target is read from the expected counts
         if (kind == 0) r.sig = done_f + s;
@@ -544,7 +543,7 @@ static void build_solve_recs(Plan& P) {
         r.m = br;
         r.k = cols;
         r.x0 = m.fc + col0;
-        r.y0 = (int32_t)(m.lidx + r0);
+        r.y0 = (int32_t)((m.lidx + r0) / P.row_unit);
         r.wait = done_f + s;
         r.target = nblk == 1 ? 1 : di_range(0, p + 1);
         r.g0 = P.row_group[m.lidx + r0];
@@ -552,7 +551,7 @@ static void build_solve_recs(Plan& P) {
       } else {
         r.m = cols;
         r.k = br;
-        r.x0 = (int32_t)(m.lidx + r0);
+        r.x0 = (int32_t)((m.lidx + r0) / P.row_unit);
         r.y0 = m.fc + col0;
         const int par = P.sparent[s];
         if (par >= 0) r.wait = done_b + par, r.target = solve_done_count(P.meta[par].w, SB, TPT);
@@ -592,7 +591,7 @@ static void build_solve_recs(Plan& P) {
         level = P.level[t.s];
       }
       SolveRec r = make(t, fwd);
-      r.kind |= (int32_t)(i << 3);
+      r.kind |= (int32_t)((uint32_t)std::min<size_t>(i, ((size_t)1 << 29) - 1) << 3);
       if (!small(t)) {
         recs.push_back(r);
         continue;
@@ -608,7 +607,7 @@ static void build_solve_recs(Plan& P) {
   P.tiny_recs.resize(P.tiny.size());
   for (size_t i = 0; i < P.tiny.size(); ++i) {
     const SnMeta& m = P.meta[P.tiny[i]];
-    P.tiny_recs[i] = TinyRec{m.off, (int32_t)m.lidx, m.fc, m.ld, m.w, m.h, P.tiny[i]};
+    P.tiny_recs[i] = TinyRec{m.off, m.lidx, m.fc, m.ld, (int16_t)m.w, (int16_t)m.h, P.tiny[i]};
   }
   P.fwd_wait = P.fwd_pending;
   for (int32_t s : P.tiny) {

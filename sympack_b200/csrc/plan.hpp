@@ -23,6 +23,11 @@
 
 namespace spb {
 
+// Row lists are laid out so that every off-diagonal part starts on a multiple of kRowUnit
+// entries: with more than 2^31 entries the solve records count them in these units, in 32 bits
+// beyond what device memory can hold (Plan::row_unit).
+constexpr int kRowUnit = 8;
+
 // Panel descriptor (device-visible).
 struct SnMeta {
   int32_t fc;    // first column, 0-based (permuted numbering)
@@ -30,7 +35,8 @@ struct SnMeta {
   int32_t h;     // rows, including the w x w diagonal block
   int32_t ld;    // leading dimension of the panel
   int64_t off;   // element offset of the panel in the factor arena
-  int64_t lidx;  // offset of this supernode's row list in the device row array
+  int64_t lidx;  // offset of this supernode's row list in the device row array (lidx + w on a
+                 // multiple of kRowUnit)
   int32_t boff;  // first of this supernode's 64-column blocks over all supernodes
   int32_t sboff; // first of this supernode's solve super-blocks in the per-super-block solve counters
   int64_t ioff;  // element offset of its diagonal super-block inverses in the inverse arena (-1: none)
@@ -173,12 +179,13 @@ inline int32_t pack_task_i(int p, int q0) { return p | (q0 << 24); }
 struct alignas(16) SolveRec {
   int64_t a;       // element offset of the operand's first element (panel arena; DI: inverse arena)
   int64_t inv;     // one-block supernodes: element offset of the diagonal block's inverse
-  int32_t kind;    // SolveTask::kind | place in the task list << 3
+  int32_t kind;    // SolveTask::kind | place in the task list << 3 (for the trace; places beyond
+                   // 2^29 share the last one)
   int32_t s;
   int32_t ld;      // leading dimension of the operand
   int32_t m, k;    // outputs and inner length (F, G, D, B: panel columns and off-diagonal rows)
   int32_t x0, y0;  // first right-hand-side row and first output row; the gathered side of O, F, W and G
-                   // counts in the concatenated row lists
+                   // counts in the concatenated row lists, in units of Plan::row_unit entries
   int32_t wait, target;  // counter and the value to reach (wait < 0: none)
   int32_t sig;     // counter to bump (-1: none)
   int32_t g0, ng;  // O, F: relative-index groups of its rows; backward DI: first tile row and its column
@@ -215,12 +222,13 @@ SPB_HD inline int solve_done_count(int w, int sb, int tpt) {
 // A tiny leaf supernode as its kernels read it (one load before everything else).
 struct alignas(16) TinyRec {
   int64_t off;   // its panel
-  int32_t lidx;  // its row list
+  int64_t lidx;  // its row list
   int32_t fc;
   int32_t ld;
-  int32_t w, h;
+  int16_t w, h;  // at most kTinyMaxElems
   int32_t s;
 };
+static_assert(sizeof(TinyRec) == 32, "one 32-byte record per tiny leaf");
 
 // One CTA of the super-block inverse kernel: column block j of Inv_p of supernode s
 // (tiles (i, j), i = j .. nb_p - 1).
@@ -292,6 +300,7 @@ struct Plan {
   std::vector<SolveTask> fwd_tasks, bwd_tasks;
   std::vector<int32_t> fwd_pending;
   std::vector<SolveRec> fwd_recs, bwd_recs;  // the same tasks as device records
+  int32_t row_unit = 1;                      // what they count row lists in: 1 or kRowUnit entries
   std::vector<SolveRec> fwd_subs, bwd_subs;  // the records of their batches
   std::vector<int32_t> fwd_wait;             // arrivals the forward sweep waits for (without the tiny leaves')
   std::vector<int32_t> tiny;  // leaf supernodes of the forward T tasks
@@ -345,13 +354,14 @@ struct PlanParams {
   int sms = 148;                 // SMs of the device: a launch with too few tiles to fill them
                                  // splits its tiles' K range (partial products add atomically)
   bool factor_dag = true;        // build the persistent factorization's task graph
+  bool wide_rows = false;        // solve records count row lists in kRowUnit entries, however few there are
   bool dag_unless_wide = false;  // only when the tree is not too wide for it (kWideSupernodesPerStep)
   bool fp32 = false;             // FP32 factor (precision form): 128 x 128 tensor-core tiles, one CTA
                                  // per SM; FP64: 128 x 64 tiles at two CTAs per SM
   bool operator==(const PlanParams& o) const {
     return small_max_w == o.small_max_w && small_max_bytes == o.small_max_bytes && nb == o.nb &&
            outer_nb == o.outer_nb && big_tile_rows == o.big_tile_rows && solve_sb == o.solve_sb &&
-           solve_tpt == o.solve_tpt && sms == o.sms && factor_dag == o.factor_dag && dag_unless_wide == o.dag_unless_wide &&
+           solve_tpt == o.solve_tpt && sms == o.sms && factor_dag == o.factor_dag && dag_unless_wide == o.dag_unless_wide && wide_rows == o.wide_rows &&
            fp32 == o.fp32;
   }
 };

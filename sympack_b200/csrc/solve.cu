@@ -111,6 +111,12 @@ __device__ __forceinline__ unsigned long long now_ns() {
   return t;
 }
 
+// The gathered side's rows, from a record's count of kUnit entries.
+template <int kUnit>
+__device__ __forceinline__ const int32_t* row_list(const PSolveArgs& a, int32_t at) {
+  return a.rows + (int64_t)at * kUnit;
+}
+
 // Task timeline for analysis (of the first group of right-hand sides; trace may be null).
 __device__ __forceinline__ void trace_mark(unsigned long long* trace, const SolveRec& r, int slot) {
   if (trace) trace[4 * (size_t)((unsigned)r.kind >> 3) + slot] = now_ns();
@@ -503,7 +509,7 @@ __device__ __forceinline__ void correct_small(double (&d)[NG][4], const double (
     for (int e = 0; e < 4; ++e) d[n][e] += r[n][e];
 }
 
-template <class T, int NG>
+template <class T, int NG, int kUnit>
 __device__ bool warp_forward(const PSolveArgs& a, const SolveRec& r, double* zs, double* ys, double* Ls, double* X, double* Z, int32_t* sync,
                              int nc, Frag<T>& f, unsigned long long* trace) {
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3, w = r.m;
@@ -525,7 +531,7 @@ __device__ bool warp_forward(const PSolveArgs& a, const SolveRec& r, double* zs,
     tgt = gr.t;
     cnt = (hi >> 6) - (lo >> 6) + 1;
   }
-  const int32_t* rows = a.rows + r.y0;
+  const int32_t* rows = row_list<kUnit>(a, r.y0);
   bool ok = true;
   if (lane == 0) ok = poll_geq(sync + r.wait, a.expected[r.s], a.status, r.s, a.spin_limit);
   ok = __shfl_sync(0xffffffffu, ok, 0);
@@ -584,7 +590,7 @@ __device__ bool warp_forward(const PSolveArgs& a, const SolveRec& r, double* zs,
   return true;
 }
 
-template <class T, int NG>
+template <class T, int NG, int kUnit>
 __device__ bool warp_backward(const PSolveArgs& a, const SolveRec& r, double* zs, double* ys, double* Ls, double* X,
                               const double* Z, int32_t* sync, int nc, Frag<T>& f, unsigned long long* trace) {
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3, w = r.m;
@@ -599,7 +605,7 @@ __device__ bool warp_backward(const PSolveArgs& a, const SolveRec& r, double* zs
   }
   f.load(A, r.ld, 1, w, min(64, r.k));
   if constexpr (kCorrect<T>) stage_small(Ls, A - w, r.ld, w);
-  const int32_t* rows = a.rows + r.y0;
+  const int32_t* rows = row_list<kUnit>(a, r.y0);
   int idx[16];
 #pragma unroll
   for (int i = 0; i < 16; ++i) idx[i] = 4 * i + t < r.k ? rows[4 * i + t] : -1;
@@ -662,8 +668,10 @@ __device__ bool warp_backward(const PSolveArgs& a, const SolveRec& r, double* zs
 // staged right-hand sides and the product.  A ticket is one task for one group of kSolveGroup
 // right-hand sides: the groups are independent solves with counters of their own whose
 // chains run side by side, and share the operand's tiles in L2.  The next ticket is drawn
-// while the last results are on their way.
-template <class T, int NG, bool kFwd>
+// while the last results are on their way.  kUnit: Plan::row_unit (a kernel of its own, since
+// the multiplication costs the forward sweep registers: 27-point 17^3, one right-hand side, 182 ->
+// 187 us).
+template <class T, int NG, bool kFwd, int kUnit>
 __global__ void __launch_bounds__(kThreads, solve_min_blocks<T, NG>()) k_solve(PSolveArgs a) {
   extern __shared__ __align__(16) unsigned char sm_raw[];
   SolveSmem<NG>& sm = *reinterpret_cast<SolveSmem<NG>*>(sm_raw);
@@ -712,8 +720,8 @@ __global__ void __launch_bounds__(kThreads, solve_min_blocks<T, NG>()) k_solve(P
         static_assert(kXLd * NG >= kWzLd * 8 * NG && kT * kInvLd / 8 >= 16 * kWzLd, "a warp's tiles");
         unsigned long long* wtrace = grp == 0 && (tid & 31) == 0 ? a.trace : nullptr;
         if (wtrace) trace_start(wtrace, q);
-        if (kFwd) ok = warp_forward<T, NG>(a, q, zs, ys, Ls, X, Z, sync, nc, f, wtrace);
-        else ok = warp_backward<T, NG>(a, q, zs, ys, Ls, X, Z, sync, nc, f, wtrace);
+        if (kFwd) ok = warp_forward<T, NG, kUnit>(a, q, zs, ys, Ls, X, Z, sync, nc, f, wtrace);
+        else ok = warp_backward<T, NG, kUnit>(a, q, zs, ys, Ls, X, Z, sync, nc, f, wtrace);
         if (wtrace) trace_mark(wtrace, q, 2);
       }
       if (tid == 0) sh_task[turn ^ 1] = atomicAdd(a.counter, 1);
@@ -721,7 +729,7 @@ __global__ void __launch_bounds__(kThreads, solve_min_blocks<T, NG>()) k_solve(P
       continue;
     } else if (one_block) {
       stage_inverse<T>(sm.inv, sm.ldiag, a.Inv1 + r.inv, L + r.a, r.ld, r.m);
-      for (int i = tid; i < min(r.k, kRowCap); i += kThreads) sm.rows[i] = a.rows[r.y0 + i];
+      for (int i = tid; i < min(r.k, kRowCap); i += kThreads) sm.rows[i] = row_list<kUnit>(a, r.y0)[i];
       const T* A = L + r.a + r.m;  // first off-diagonal row
       if (kFwd) {
         // m-tiles of 16 off-diagonal rows dealt to the warps; a warp's 16 fragment steps hold
@@ -749,7 +757,7 @@ __global__ void __launch_bounds__(kThreads, solve_min_blocks<T, NG>()) k_solve(P
     } else if (!kFwd && kind == 3) {  // W: one 16-column tile per warp
       wm = warp;
       wk = 0;
-      for (int i = tid; i < r.k; i += kThreads) sm.rows[i] = a.rows[r.x0 + i];
+      for (int i = tid; i < r.k; i += kThreads) sm.rows[i] = row_list<kUnit>(a, r.x0)[i];
       f.load(L + r.a + (int64_t)warp * 16 * r.ld, r.ld, 1, r.m - warp * 16, r.k);
     } else if (!kFwd && kind == 5) {  // DI: this warp's tile of the inverse, transposed
       const int R = r.g0 + wk;
@@ -759,7 +767,7 @@ __global__ void __launch_bounds__(kThreads, solve_min_blocks<T, NG>()) k_solve(P
       f.load(L + r.a + (int64_t)wm * 16 * r.ld + wk * kT, r.ld, 1, r.m - wm * 16, min(kT, r.k - wk * kT));
     } else {  // DI, U, O
       if (kind == 2)
-        for (int i = tid; i < r.m; i += kThreads) sm.rows[i] = a.rows[r.y0 + i];
+        for (int i = tid; i < r.m; i += kThreads) sm.rows[i] = row_list<kUnit>(a, r.y0)[i];
       const T* A = kind == 5 ? static_cast<const T*>(a.Inv) + r.a : L + r.a;
       f.load(A + wm * 16 + (int64_t)wk * kT * r.ld, 1, r.ld, r.m - wm * 16, min(kT, r.k - wk * kT));
     }
@@ -816,7 +824,7 @@ __global__ void __launch_bounds__(kThreads, solve_min_blocks<T, NG>()) k_solve(P
                 const int row0 = rb + ((4 * q4 >> sh) * 8 + warp) * 16;
                 if (row0 < r.k) {
                   if (row0 + 16 <= kRowCap) scatter<NG>(X, a.ldx, 0, sm.rows + row0, acc, r.k - row0, nc, -1.0);
-                  else scatter<NG>(X, a.ldx, 0, a.rows + r.y0 + row0, acc, r.k - row0, nc, -1.0);
+                  else scatter<NG>(X, a.ldx, 0, row_list<kUnit>(a, r.y0) + row0, acc, r.k - row0, nc, -1.0);
                 }
                 clear<NG>(acc);
               }
@@ -834,7 +842,7 @@ __global__ void __launch_bounds__(kThreads, solve_min_blocks<T, NG>()) k_solve(P
           for (int ch = 0; ch < nch; ++ch) {
             const int rb = ch * sc, kc = min(sc, r.k - rb);
             if (ch > 0) __syncthreads();
-            stage_x(sm.x, kXLd, X, a.ldx, 0, rb + sc <= kRowCap ? sm.rows + rb : a.rows + r.y0 + rb, kc, sc, nc);
+            stage_x(sm.x, kXLd, X, a.ldx, 0, rb + sc <= kRowCap ? sm.rows + rb : row_list<kUnit>(a, r.y0) + rb, kc, sc, nc);
             if (ch > 0)
               f.load(A + (int64_t)wm * 16 * r.ld + rb + wk * rw, r.ld, 1, w - wm * 16, min(rw, kc - wk * rw));
             __syncthreads();
@@ -1276,9 +1284,9 @@ int g_solve_grid[2][2] = {};  // resident CTAs of the sweeps: [FP32][NG - 1]
 template <class T, int NG>
 void init_sweeps(int fp32, int sms) {
   int per = 0;
-  cudaFuncSetAttribute(k_solve<T, NG, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SolveSmem<NG>));
-  cudaFuncSetAttribute(k_solve<T, NG, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SolveSmem<NG>));
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_solve<T, NG, true>, kThreads, sizeof(SolveSmem<NG>));
+  for (auto f : {k_solve<T, NG, true, 1>, k_solve<T, NG, false, 1>, k_solve<T, NG, true, kRowUnit>, k_solve<T, NG, false, kRowUnit>})
+    cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SolveSmem<NG>));
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_solve<T, NG, true, 1>, kThreads, sizeof(SolveSmem<NG>));
   g_solve_grid[fp32][NG - 1] = sms * (per > 0 ? per : 1);
 }
 
@@ -1290,9 +1298,11 @@ void run_sweep(cudaStream_t st, const PSolveArgs& a, bool forward) {
   const int tiny = pairs > 148 * 16 * 128 ? 148 * 16 : (int)((pairs + 127) / 128);
   if (forward) {
     if (tiny > 0) k_solve_tiny<T, true><<<tiny, 128, 0, st>>>(a);
-    if (grid > 0) k_solve<T, NG, true><<<grid, kThreads, sizeof(SolveSmem<NG>), st>>>(a);
+    if (grid > 0)
+      (a.row_unit == 1 ? k_solve<T, NG, true, 1> : k_solve<T, NG, true, kRowUnit>)<<<grid, kThreads, sizeof(SolveSmem<NG>), st>>>(a);
   } else {
-    if (grid > 0) k_solve<T, NG, false><<<grid, kThreads, sizeof(SolveSmem<NG>), st>>>(a);
+    if (grid > 0)
+      (a.row_unit == 1 ? k_solve<T, NG, false, 1> : k_solve<T, NG, false, kRowUnit>)<<<grid, kThreads, sizeof(SolveSmem<NG>), st>>>(a);
     if (tiny > 0) k_solve_tiny<T, false><<<tiny, 128, 0, st>>>(a);
   }
 }

@@ -75,6 +75,8 @@ static void path_matrix(int n, std::vector<int64_t>& cp, std::vector<int32_t>& r
 static long long n_rel = 0;
 static int widest_small = 0;
 
+static void check_records(const Plan& P, const char* what);
+
 static void check_plan(const Symbolic& sym, const PlanParams& prm, const char* what) {
   const Plan P = build_plan(sym, prm);
   // relative indices (filled by host threads on large plans): every group's positions
@@ -106,6 +108,8 @@ static void check_plan(const Symbolic& sym, const PlanParams& prm, const char* w
     }
     CHECK(!bad, "%s: relative indices differ from a merge of the row lists", what);
   }
+  for (int s = 0; s < P.nsuper; ++s)
+    CHECK((P.meta[s].lidx + P.meta[s].w) % kRowUnit == 0, "%s: row list of supernode %d not aligned", what, s);
   // small panels: what their task keeps in shared memory holds D of the widest one, however
   // wide the caller lets them be
   for (int s = 0; s < P.nsuper; ++s) {
@@ -261,8 +265,9 @@ static void check_plan(const Symbolic& sym, const PlanParams& prm, const char* w
     CHECK(arrivals[s] == P.fwd_pending[s], "%s: supernode %d gets %lld forward arrivals, waits for %d", what, s,
           (long long)arrivals[s], P.fwd_pending[s]);
 
-  // both sweeps run one task at a time in dispatch order with the kernels' wait targets and
-  // signals (solve.cu): no task ever waits, and every supernode ends done
+  check_records(P, what);
+  // both sweeps' task lists run one task at a time in their own order, with wait targets and
+  // signals worked out here: no task ever waits, and every supernode ends done
   const int SB = P.solve_sb, TPT = P.solve_tpt;
   auto nblk_of = [&](int s) { return (P.meta[s].w + 63) / 64; };
   auto nsb_of = [&](int s) { return (nblk_of(s) + SB - 1) / SB; };
@@ -376,6 +381,141 @@ static void check_plan(const Symbolic& sym, const PlanParams& prm, const char* w
   }
 }
 
+// The records the sweeps' kernels read (solve.cu), each sweep run one ticket at a time in the
+// records' own order, batches whole: no task waits for one handed out after it (or beside it in
+// its batch), what arrives at a supernode is what its tasks wait for, every counter ends where
+// the last task expects it, and operands, right-hand-side rows and output rows are the places
+// that the plan's panels, inverses and row lists give them, each part of a panel once.
+static void check_records(const Plan& P, const char* what) {
+  const int ns = P.nsuper, SB = P.solve_sb, TPT = P.solve_tpt;
+  const int64_t nctr = (int64_t)solve_sync_ints(P);
+  CHECK((int64_t)P.fwd_wait.size() == ns, "%s: fwd_wait size", what);
+  std::vector<uint8_t> tiny(ns, 0);
+  for (size_t i = 0; i < P.tiny.size(); ++i) {
+    const SnMeta& m = P.meta[P.tiny[i]];
+    const TinyRec& t = P.tiny_recs[i];
+    tiny[P.tiny[i]] = 1;
+    CHECK(t.s == P.tiny[i] && t.off == m.off && t.lidx == m.lidx && t.fc == m.fc && t.ld == m.ld && t.w == m.w && t.h == m.h,
+          "%s: tiny record %zu", what, i);
+  }
+  std::vector<int64_t> inv_at(ns, -1);
+  for (const Inv1Item& it : P.inv1_items)
+    for (int s = std::upper_bound(P.meta.begin(), P.meta.end(), it.a, [](int64_t a, const SnMeta& m) { return a < m.off; }) -
+                 P.meta.begin() - 1;
+         s >= 0; s = -1) {
+      CHECK(P.meta[s].off == it.a && P.meta[s].w == it.w && P.meta[s].ld == it.ld && inv_at[s] < 0, "%s: inverse item of %d", what, s);
+      inv_at[s] = it.inv;
+    }
+  for (int sweep = 0; sweep < 2; ++sweep) {
+    const bool fwd = sweep == 0;
+    const std::vector<SolveRec>& recs = fwd ? P.fwd_recs : P.bwd_recs;
+    const std::vector<SolveRec>& subs = fwd ? P.fwd_subs : P.bwd_subs;
+    const std::vector<SolveTask>& tasks = fwd ? P.fwd_tasks : P.bwd_tasks;
+    std::vector<int64_t> c(nctr, 0), area(ns, 0), di(ns, 0);
+    std::set<std::pair<int64_t, int>> once;  // operand offset and kind
+    std::vector<uint8_t> placed(tasks.size(), 0);
+    size_t done = 0, nsub = 0;
+    auto need = [&](int64_t ctr, int64_t target, const SolveRec& r) {
+      CHECK(ctr >= 0 && ctr < nctr, "%s: counter %lld out of range", what, (long long)ctr);
+      if (ctr >= 0 && ctr < nctr)
+        CHECK(c[ctr] >= target, "%s: %s record of supernode %d (kind %d) waits for %lld at %lld, sees %lld", what,
+              fwd ? "forward" : "backward", r.s, r.kind & 7, (long long)target, (long long)ctr, (long long)c[ctr]);
+    };
+    auto look = [&](const SolveRec& r) {
+      const int kind = r.kind & 7, s = r.s;
+      const SnMeta& m = P.meta[s];
+      const size_t place = (uint32_t)r.kind >> 3;
+      CHECK(place < tasks.size() && !placed[place] && tasks[place].s == s && tasks[place].kind == kind, "%s: record's place", what);
+      if (place < tasks.size()) placed[place] = 1;
+      const bool one = kind == 4 || kind == 0;
+      if (fwd && (one || kind == 5)) need(2 + s, P.fwd_wait[s], r);
+      if (r.wait >= 0 && !(fwd && one)) need(r.wait, r.target, r);
+      CHECK(once.insert({r.a, kind}).second, "%s: two records on one operand", what);
+      if (one) {
+        CHECK(m.w <= 64 && r.a == m.off && r.ld == m.ld && r.m == m.w && r.x0 == m.fc && r.inv == inv_at[s] && r.inv >= 0, "%s: one-block record", what);
+        CHECK((int64_t)r.y0 * P.row_unit == m.lidx + m.w && r.k == (kind == 4 ? m.h - m.w : 0), "%s: one-block rows", what);
+        area[s] += (int64_t)r.k * r.m;
+        if (kind == 4 && fwd)
+          CHECK(r.k == 0 ? r.ng == 0 : r.g0 == P.row_group[m.lidx + m.w] && r.g0 + r.ng - 1 == P.row_group[m.lidx + m.h - 1], "%s: groups of F", what);
+      } else if (kind == 5) {
+        const SolveTask& t = tasks[place];
+        const int p = t.i & 0xffffff, q0 = t.i >> 24, rb = t.t, nblk = (m.w + 63) / 64, nb = std::min(SB, nblk - p * SB), blk = p * SB + rb;
+        const int first = fwd ? q0 : rb + q0, last = std::min(fwd ? rb + 1 : nb, first + TPT);  // tiles along the product
+        const int64_t base = m.ioff + (int64_t)p * inv_tiles(SB) * 4096;
+        CHECK(r.ld == 64 && r.m == std::min(64, m.w - blk * 64) && r.y0 == m.fc + blk * 64 && r.x0 == m.fc + (p * SB + first) * 64 &&
+                  r.k == std::min(m.w, (p * SB + last) * 64) - (p * SB + first) * 64, "%s: DI record", what);
+        if (fwd) CHECK(r.a == base + ((int64_t)rb * (rb + 1) / 2 + q0) * 4096, "%s: DI tiles", what);
+        else CHECK(r.a == base && r.g0 == first && r.ng == rb, "%s: DI tiles", what);
+        di[s] += last - first;
+        if (!fwd) once.erase({r.a, kind});  // a super-block's tasks share its base
+      } else {
+        const int64_t e = r.a - m.off, row = e % m.ld, col = e / m.ld;
+        const bool down = fwd;  // outputs are panel rows; backward: panel columns
+        const int rows = down ? r.m : r.k, cols = down ? r.k : r.m;
+        CHECK(r.ld == m.ld && e >= 0 && rows >= 1 && cols >= 1 && rows <= 64 + (kind == 1 && !fwd) * 64 * TPT && row + rows <= m.h && col + cols <= m.w,
+              "%s: operand of kind %d outside its panel", what, kind);
+        const int64_t x = fwd ? col : row, y = fwd ? row : col;
+        const bool off = kind != 1;
+        CHECK(off == (row >= m.w), "%s: kind %d on the other part of its panel", what, kind);
+        if (off && fwd) CHECK((int64_t)r.y0 * P.row_unit == m.lidx + y && r.x0 == m.fc + x, "%s: O rows", what);
+        if (off && !fwd) CHECK((int64_t)r.x0 * P.row_unit == m.lidx + x && r.y0 == m.fc + y, "%s: W rows", what);
+        if (!off) CHECK(r.x0 == m.fc + x && r.y0 == m.fc + y, "%s: U or V rows", what);
+        if (off && fwd) CHECK(r.g0 == P.row_group[m.lidx + row] && r.g0 + r.ng - 1 == P.row_group[m.lidx + row + rows - 1], "%s: groups of O", what);
+        area[s] += (int64_t)rows * cols;
+      }
+    };
+    auto signal = [&](const SolveRec& r) {
+      const int kind = r.kind & 7;
+      if (r.sig >= 0) ++c[r.sig];
+      if (fwd && (kind == 2 || kind == 4 || kind == 0))
+        for (int g = 0; g < r.ng; ++g) {
+          const RelGroup& gr = P.groups[r.g0 + g];
+          int n = 1;
+          if (kind != 2) {  // F: one arrival per 64-row tile
+            const int lo = gr.j0 - r.m, hi = (g + 1 < r.ng ? P.groups[r.g0 + g + 1].j0 - r.m : r.k) - 1;
+            n = (hi >> 6) - (lo >> 6) + 1;
+          }
+          c[2 + gr.t] += n;
+        }
+      ++done;
+    };
+    for (const SolveRec& r : recs) {
+      if ((r.kind & 7) != 7) {
+        look(r);
+        signal(r);
+        continue;
+      }
+      CHECK(r.m >= 1 && r.m <= 8 && r.x0 == (int)nsub && r.x0 + r.m <= (int)subs.size(), "%s: batch range", what);
+      for (int q = 0; q < r.m; ++q) {
+        const SolveRec& t = subs[r.x0 + q];
+        CHECK((t.kind & 7) == 4 && t.m <= kWarpMaxW && t.k <= kWarpMaxOff, "%s: batched record too large for a warp", what);
+        look(t);
+      }
+      for (int q = 0; q < r.m; ++q) signal(subs[r.x0 + q]);
+      nsub += r.m;
+    }
+    size_t batches = 0;
+    for (const SolveTask& t : tasks) batches += t.kind == 6;
+    CHECK(nsub == subs.size() && done + batches == tasks.size(), "%s: %zu records for %zu tasks", what, done, tasks.size() - batches);
+    for (int s = 0; s < ns; ++s) {
+      const SnMeta& m = P.meta[s];
+      if (tiny[s]) continue;
+      const int nblk = (m.w + 63) / 64, nsb = (nblk + SB - 1) / SB;
+      int64_t want = (int64_t)(m.h - m.w) * m.w, tiles = 0;
+      for (int p = 0; p < nsb && nblk > 1; ++p) {
+        const int64_t c0 = (int64_t)p * SB * 64, c1 = std::min<int64_t>(m.w, c0 + (int64_t)SB * 64);
+        want += (m.w - c1) * (c1 - c0);
+        tiles += inv_tiles(std::min(SB, nblk - p * SB));
+      }
+      CHECK(area[s] == want && di[s] == tiles, "%s: records of supernode %d cover %lld of %lld entries, %lld of %lld inverse tiles",
+            what, s, (long long)area[s], (long long)want, (long long)di[s], (long long)tiles);
+      const bool whole = nblk == 1 && (m.h - m.w + 63) / 64 <= kSolveFusedTiles;  // F: nobody waits for it
+      CHECK(c[(fwd ? 2 + ns : 2 + 2 * ns) + s] == (fwd && whole ? 0 : solve_done_count(m.w, SB, TPT)), "%s: supernode %d not done", what, s);
+      if (fwd) CHECK(c[2 + s] == P.fwd_wait[s], "%s: supernode %d gets %lld arrivals, waits for %d", what, s, (long long)c[2 + s], P.fwd_wait[s]);
+    }
+  }
+}
+
 int main() {
   for (int full = 0; full < 2; ++full)
     for (int k : {6, 12, 20, 28}) {
@@ -403,6 +543,13 @@ int main() {
       small.solve_tpt = 1;
       std::snprintf(what, sizeof what, "%s %d^3 FP64 small blocks", full ? "27-point" : "7-point", k);
       check_plan(sym, small, what);
+      PlanParams units;  // records as plans of more than 2^31 row-list entries have them
+      units.factor_dag = false;
+      units.wide_rows = true;
+      units.solve_sb = 2;
+      units.solve_tpt = 3;
+      std::snprintf(what, sizeof what, "%s %d^3 row units", full ? "27-point" : "7-point", k);
+      check_plan(sym, units, what);
     }
   // a plan large enough (over 2^20 relative indices) for its relative indices to be
   // filled by several host threads

@@ -4,9 +4,11 @@ tiles cut from even rows for the 16-byte bulk copies, FP32 tiles in whole 32-col
 chunks), the persistent factorization's dispatch order (run one task at a time in that
 order, no task ever waits), the tiny-leaf solve batches (first forward, last backward,
 every tiny leaf in exactly one), the forward solve's arrival counts (what the tasks
-signal equals what each supernode waits for), and both solve sweeps run one task at a time
-in dispatch order with the kernels' wait targets and signals (no task waits for one handed
-out after it, and every supernode ends done), the relative indices of the external updates
+signal equals what each supernode waits for), both solve sweeps run one task at a time in
+the order of the task lists and in the order of the records that the kernels read (their own
+waits, targets, signals and batches: no task waits for one handed out after it, and every
+supernode ends done), the records' operands and rows against the panels, inverses and row
+lists (each part once), the widths of small panels, the relative indices of the external updates
 (filled by host threads on large plans) against a merge of the row lists, and the task
 order re-built from measured durations (same tasks, waits and signals; still never
 waiting for a later task).  The matrices: 7- and 27-point grids, and a
