@@ -792,7 +792,8 @@ def run_ours(args):
     K = args.steps
     # per step: assemble, the factorization (one persistent launch), then two solves (permute in,
     # tiny leaves, forward, backward, tiny leaves, permute out), the first one after the
-    # factorization also computing the super-block and diagonal block inverses
+    # factorization also computing the super-block inverses and those of the narrow and of the
+    # wide diagonal blocks (this matrix has tiny leaves and all three)
     launches_per_step = 1 + info.factor_launches + 6 + 6 + (3 if info.inverse_bytes else 0)
     if rank == 0:
         line = {

@@ -200,11 +200,12 @@ int spb_solve_device(spb_handle* h, const double* d_rhs, double* d_x, int32_t nr
  * The first call on a device resolves the array's device address
  * (cudaGetSymbolAddress); make that first call before any stream capture.
  * Every call on a device shares the array: calls whose work overlaps on the GPU
- * (other handles or streams) race, so serialize them.  The counters are cleared
- * on every call (and for every 64 right-hand sides); nothing else is kept
- * between calls.  The first call after a factorization also computes the
- * factor's diagonal super-block inverses, in memory the handle allocated with
- * its analysis.  Like spb_solve_device, the call reads the device status word
+ * (other handles or streams) race, so serialize them.  A pass takes 16 right-hand
+ * sides for every set of counters that the room holds, at most four (so 64, or as
+ * few as 16 when the limit is nearly reached); the counters are cleared for every
+ * pass and nothing else is kept between calls.  The first call after a
+ * factorization also computes the factor's diagonal block and super-block
+ * inverses, in memory the handle allocated with its analysis.  Like spb_solve_device, the call reads the device status word
  * back before it returns, so it waits for the handle's stream. */
 int spb_solve_device_noalloc(spb_handle* h, const double* d_rhs, double* d_x, int32_t nrhs, int64_t ld);
 
@@ -273,7 +274,7 @@ int spb_set_stream(spb_handle* h, void* stream);
 #define SPB_KIND_GEMM_DMMA 5
 #define SPB_KIND_SOLVE_FORWARD 6
 #define SPB_KIND_SOLVE_BACKWARD 7
-#define SPB_KIND_SOLVE_INVERSE 8  /* diagonal super-block inverses (first solve after a factorization) */
+#define SPB_KIND_SOLVE_INVERSE 8  /* diagonal block and super-block inverses (first solve after a factorization) */
 #define SPB_KIND_COUNT 9
 typedef struct spb_profile {
   double ms[SPB_KIND_COUNT];

@@ -44,7 +44,6 @@ struct spb_handle {
   std::vector<int64_t> colptr;
   std::vector<int32_t> rowind;
   std::vector<int64_t> amap;       // arena position of each input entry (DistributeMatrix map)
-  std::vector<int32_t> level_off;  // level l covers dlevel_sn[level_off[l] .. level_off[l+1])
   // device buffers
   bool fp32 = false;        // precision form: FP32 factor + FP64 refinement
   bool ldl = false;         // LDL^T decomposition (FP64): dL unit L, dW = L D
@@ -53,7 +52,6 @@ struct spb_handle {
   double* dW = nullptr;
   spb::SnMeta* dmeta = nullptr;
   int32_t* drows = nullptr;
-  int32_t* dsupm = nullptr;
   int32_t* drowgrp = nullptr;      // relative-index group of each row-list entry
   spb::RelGroup* dgroups = nullptr;
   int32_t* drel = nullptr;
@@ -75,14 +73,12 @@ struct spb_handle {
   bool factor_trace = false;
   bool trace_fresh = false;        // the last factorization was traced in the current task order
   int32_t* dinvp0 = nullptr;
-  int32_t* dlevel_sn = nullptr;
   spb::SolveRec* dfwd = nullptr;   // records of the solve tasks
   spb::SolveRec* dbwd = nullptr;
   spb::SolveRec* dfsubs = nullptr;
   spb::SolveRec* dbsubs = nullptr;
   int32_t* dexpected = nullptr;
   spb::TinyRec* dtiny = nullptr;   // tiny leaf supernodes
-  int32_t* dsparent = nullptr;
   int32_t* dsync = nullptr;  // solve counters (spb::solve_sync_ints)
   void* dInv = nullptr;      // diagonal super-block inverses of the forward operand (L, or L D for LDL^T)
   void* dInvB = nullptr;     // LDL^T: inverses of the backward operand (unit L); else dInv
@@ -213,7 +209,6 @@ spb::dev::FactorArgs factor_args(spb_handle* h) {
   a.L = h->dL;
   a.meta = h->dmeta;
   a.rows = h->drows;
-  a.supmember = h->dsupm;
   a.status = h->dstatus;
   a.row_group = h->drowgrp;
   a.groups = h->dgroups;
@@ -467,11 +462,7 @@ void enqueue_sweeps(spb_handle* h, double* X, double* Z, int32_t* sync, int grou
     a.Inv = h->dInv;
     a.Inv1 = h->dInv1;
     a.fp32 = h->fp32;
-    a.meta = h->dmeta;
     a.rows = h->drows;
-    a.supmember = h->dsupm;
-    a.sparent = h->dsparent;
-    a.row_group = h->drowgrp;
     a.groups = h->dgroups;
     a.X = X + (int64_t)c0 * h->sym.n;
     a.Z = Z + (int64_t)c0 * h->sym.n;
@@ -902,15 +893,15 @@ int64_t predict_bytes(const spb_handle* h, bool fp32, int nrhs) {
   auto b = [](int64_t count, size_t size) { return std::max<int64_t>(count, 1) * (int64_t)size; };
   int64_t t = b(P.arena_elems, fp32 ? sizeof(float) : sizeof(double));
   if (o.decomposition == SPB_DECOMPOSITION_LDL) t += b(P.arena_elems, sizeof(double));
-  t += b(P.meta.size(), sizeof(spb::SnMeta)) + b(P.rows.size(), 4) + b(P.supmember0.size(), 4);
+  t += b(P.meta.size(), sizeof(spb::SnMeta)) + b(P.rows.size(), 4);
   t += b(P.row_group.size(), 4) + b(P.groups.size(), sizeof(spb::RelGroup)) + b(P.rel.size(), 4);
   t += b(h->amap.size(), 8) + b(h->nnz_a, 8) + b(P.small_items.size(), 4);
   t += b(P.panel_items.size(), sizeof(spb::PanelItem));
   t += b((int64_t)std::max(1, P.max_diag_slots) * (int64_t)spb::dev::kDiagSlotDoubles, 8);
-  t += b(P.tile_items.size(), sizeof(spb::TileItem)) + b(n, 4) + b(ns, 4);
+  t += b(P.tile_items.size(), sizeof(spb::TileItem)) + b(n, 4);
   t += b(P.fwd_recs.size(), sizeof(spb::SolveRec)) + b(P.bwd_recs.size(), sizeof(spb::SolveRec));
   t += b(P.fwd_subs.size(), sizeof(spb::SolveRec)) + b(P.bwd_subs.size(), sizeof(spb::SolveRec));
-  t += b(P.fwd_wait.size(), 4) + b(P.tiny_recs.size(), sizeof(spb::TinyRec)) + b(P.sparent.size(), 4) +
+  t += b(P.fwd_wait.size(), 4) + b(P.tiny_recs.size(), sizeof(spb::TinyRec)) +
        b((int64_t)spb::solve_sync_ints(P) * spb::kSolveGroups, 4);
   t += b(P.inv_elems, fp32 ? sizeof(float) : sizeof(double)) + b(P.inv_items.size(), sizeof(spb::InvItem));
   t += b(P.inv1_elems, sizeof(double)) + b(P.inv1_items.size(), sizeof(spb::Inv1Item));
@@ -966,13 +957,7 @@ int install_device(spb_handle* h) {
   const int32_t* rowind = h->rowind.data();
   const std::vector<int64_t>& amap = h->amap;
   const spb::Plan& P = h->plan;
-  std::vector<int32_t> lsn, invp0(n);
-  h->level_off.assign(P.nlevels + 1, 0);
-  for (int l = 0; l < P.nlevels; ++l) {
-    h->level_off[l] = (int32_t)lsn.size();
-    lsn.insert(lsn.end(), P.level_sn[l].begin(), P.level_sn[l].end());
-  }
-  h->level_off[P.nlevels] = (int32_t)lsn.size();
+  std::vector<int32_t> invp0(n);
   for (int i = 0; i < n; ++i) invp0[i] = h->sym.invp[i] - 1;
 
   h->fp32 = h->opt.precision == SPB_PRECISION_FP32_IR;
@@ -986,7 +971,6 @@ int install_device(spb_handle* h) {
   if (h->ldl) SPB_CK(h, dalloc(h, &h->dW, (size_t)P.arena_elems));
   SPB_CK(h, dalloc(h, &h->dmeta, P.meta.size()));
   SPB_CK(h, dalloc(h, &h->drows, P.rows.size()));
-  SPB_CK(h, dalloc(h, &h->dsupm, P.supmember0.size()));
   SPB_CK(h, dalloc(h, &h->drowgrp, P.row_group.size()));
   SPB_CK(h, dalloc(h, &h->dgroups, P.groups.size()));
   SPB_CK(h, dalloc(h, &h->drel, P.rel.size()));
@@ -997,14 +981,12 @@ int install_device(spb_handle* h) {
   SPB_CK(h, dalloc(h, &h->dwinv, (size_t)std::max(1, P.max_diag_slots) * spb::dev::kDiagSlotDoubles));
   SPB_CK(h, dalloc(h, &h->dtiles, P.tile_items.size()));
   SPB_CK(h, dalloc(h, &h->dinvp0, invp0.size()));
-  SPB_CK(h, dalloc(h, &h->dlevel_sn, lsn.size()));
   SPB_CK(h, dalloc(h, &h->dfwd, P.fwd_recs.size()));
   SPB_CK(h, dalloc(h, &h->dbwd, P.bwd_recs.size()));
   SPB_CK(h, dalloc(h, &h->dfsubs, P.fwd_subs.size()));
   SPB_CK(h, dalloc(h, &h->dbsubs, P.bwd_subs.size()));
   SPB_CK(h, dalloc(h, &h->dexpected, P.fwd_wait.size()));
   SPB_CK(h, dalloc(h, &h->dtiny, P.tiny_recs.size()));
-  SPB_CK(h, dalloc(h, &h->dsparent, P.sparent.size()));
   SPB_CK(h, dalloc(h, &h->dsync, spb::solve_sync_ints(P) * spb::kSolveGroups));
   {
     unsigned char* inv = nullptr;
@@ -1035,7 +1017,6 @@ int install_device(spb_handle* h) {
   };
   SPB_CK(h, up(h->dmeta, P.meta.data(), P.meta.size() * sizeof(spb::SnMeta)));
   SPB_CK(h, up(h->drows, P.rows.data(), P.rows.size() * 4));
-  SPB_CK(h, up(h->dsupm, P.supmember0.data(), P.supmember0.size() * 4));
   SPB_CK(h, up(h->drowgrp, P.row_group.data(), P.row_group.size() * 4));
   SPB_CK(h, up(h->dgroups, P.groups.data(), P.groups.size() * sizeof(spb::RelGroup)));
   SPB_CK(h, up(h->drel, P.rel.data(), P.rel.size() * 4));
@@ -1044,14 +1025,12 @@ int install_device(spb_handle* h) {
   SPB_CK(h, up(h->dpanel, P.panel_items.data(), P.panel_items.size() * sizeof(spb::PanelItem)));
   SPB_CK(h, up(h->dtiles, P.tile_items.data(), P.tile_items.size() * sizeof(spb::TileItem)));
   SPB_CK(h, up(h->dinvp0, invp0.data(), invp0.size() * 4));
-  SPB_CK(h, up(h->dlevel_sn, lsn.data(), lsn.size() * 4));
   SPB_CK(h, up(h->dfwd, P.fwd_recs.data(), P.fwd_recs.size() * sizeof(spb::SolveRec)));
   SPB_CK(h, up(h->dbwd, P.bwd_recs.data(), P.bwd_recs.size() * sizeof(spb::SolveRec)));
   SPB_CK(h, up(h->dfsubs, P.fwd_subs.data(), P.fwd_subs.size() * sizeof(spb::SolveRec)));
   SPB_CK(h, up(h->dbsubs, P.bwd_subs.data(), P.bwd_subs.size() * sizeof(spb::SolveRec)));
   SPB_CK(h, up(h->dexpected, P.fwd_wait.data(), P.fwd_wait.size() * 4));
   SPB_CK(h, up(h->dtiny, P.tiny_recs.data(), P.tiny_recs.size() * sizeof(spb::TinyRec)));
-  SPB_CK(h, up(h->dsparent, P.sparent.data(), P.sparent.size() * 4));
   SPB_CK(h, up(h->dinvitems, P.inv_items.data(), P.inv_items.size() * sizeof(spb::InvItem)));
   SPB_CK(h, up(h->dinv1items, P.inv1_items.data(), P.inv1_items.size() * sizeof(spb::Inv1Item)));
   SPB_CK(h, up(h->dftasks, P.ftasks.data(), P.ftasks.size() * sizeof(spb::FTask)));

@@ -21,7 +21,6 @@ struct FactorArgs {
   void* L;                   // factor arena: double, or float when fp32
   const SnMeta* meta;        // nsuper
   const int32_t* rows;       // concatenated 0-based row lists
-  const int32_t* supmember;  // 0-based supernode of each permuted column
   Status* status;
   const int32_t* row_group;  // relative-index group of each row-list entry
   const RelGroup* groups;
@@ -91,11 +90,7 @@ struct PSolveArgs {
   const void* Inv;   // diagonal super-block inverses of that operand (same type)
   const double* Inv1;  // inverses of its one-block supernodes' diagonal blocks
   bool fp32;
-  const SnMeta* meta;
   const int32_t* rows;
-  const int32_t* supmember;
-  const int32_t* sparent;
-  const int32_t* row_group;  // relative-index group of each row-list entry (arrival targets)
   const RelGroup* groups;
   double* X;
   double* Z;

@@ -131,14 +131,15 @@ struct FWait {
   int32_t target;
 };
 
-// One task of the persistent triangular solves.  A supernode of one 64-column block
-// is solved by substitution; a wider one is cut into super-blocks of sb 64-column
-// blocks (the last one shorter), and the diagonal triangle of every super-block p is
-// applied through its inverse Inv_p (computed once per factorization, in 64 x 64
-// tiles), so a super-block costs two parallel steps instead of a chain of sb block
-// solves.  Forward (permuted right-hand sides Y in, solution of L y = b in Z):
-//            kind 6  T(i, t):  t tiny leaf supernodes tiny[i .. i + t), one per thread, whole
-//                              (no arrivals to wait for; solve, scatter, signal)
+// One task of the triangular solves.  The diagonal triangle of a supernode of one 64-column
+// block is applied through its inverse (FP64: corrected by the residual); a wider supernode is
+// cut into super-blocks of sb 64-column blocks (the last one shorter), and the diagonal triangle
+// of every super-block p is applied through its inverse Inv_p, in 64 x 64 tiles, so a super-block
+// costs two parallel steps instead of a chain of sb block solves.  All inverses are computed once
+// per factorization.  Forward (permuted right-hand sides Y in, solution of L y = b in Z):
+//            kind 6  T(i, t):  t tiny leaf supernodes tiny[i .. i + t), whole, by substitution;
+//                              solved for all of them by a launch before the sweep, so that
+//                              nothing waits for them or is signalled (fwd_wait)
 //            kind 4  F:        one-block supernode with at most kSolveFusedTiles
 //                              off-diagonal tiles, whole: Z_0 <- L_00^-1 Y_0, then every
 //                              tile's Y[ancestor rows] -= L_u0 Z_0
@@ -149,9 +150,9 @@ struct FWait {
 //            kind 2  O(p, u):  Y[rows of off-diagonal tile u] -= L(u, super-block p) Z[p],
 //                              scattered into the ancestors' rows
 // Backward (Z in, solution X):
-//            kind 6  T(i, t):  the tiny leaves, one per thread, each once its parent is done
+//            kind 6  T(i, t):  the tiny leaves, by a launch after the sweep
 //            kind 4  G:        the F supernode whole: Z_0 -= L_u0^T X[ancestor rows of u] for
-//                              every tile, then X_0 <- L_00^-T Z_0
+//                              every tile, then X_0 <- L_00^-T Z_0 (once the parent is done)
 //            kind 3  W(p, u):  Z[p] -= L(u, super-block p)^T X[ancestor rows of tile u]
 //                              (final once the parent is done)
 //            kind 0  B:        one-block supernode: X_0 <- L_00^-T Z_0
@@ -325,7 +326,7 @@ struct Plan {
 // are one solve task per sweep.
 constexpr int kSolveFusedTiles = 16;
 // Tiny leaf supernodes (at most kTinyMaxW columns and kTinyMaxElems panel entries) are
-// solved forward one per thread, kTinyBatch to a task.
+// solved one per thread and right-hand side, kTinyBatch to an entry of the task list.
 // Small F / G tasks: supernodes of at most kWarpMaxW columns and kWarpMaxOff off-diagonal
 // rows, one per warp.  Right-hand sides are solved in groups of kSolveGroup columns, each
 // group with counters of its own, at most kSolveGroups groups at a time.
