@@ -50,7 +50,8 @@ extern "C" {
 #define SPB_ERR_STATE (-5)     /* call out of order (e.g. Solve before Factorize) */
 #define SPB_ERR_STRUCTURE (-6) /* inconsistent symbolic structure detected on the device */
 #define SPB_ERR_TIMEOUT (-7)   /* a bounded device wait expired */
-#define SPB_ERR_NOT_CONVERGED (-8) /* iterative refinement did not reach its tolerance */
+#define SPB_ERR_NOT_CONVERGED (-8) /* iterative refinement did not reach its tolerance, or met a
+                                      value that is not finite (backward_error is infinite then) */
 
 #define SPB_ORDERING_MMD 0
 #define SPB_ORDERING_NATURAL 1
